@@ -85,6 +85,16 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
+// One lane of a converged warp; the branch it guards is known to be taken by a single thread.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// A wait of the whole warp: every lane gets the same answer, so the warp leaves a loop together.
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(b, parity, abort_flag));
+}
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 2, %0;" :: "n"(EPI_WARPS * 32) : "memory"); }
 // consumer barrier that also ORs a flag over the consumer threads: every thread gets the same answer
 __device__ __forceinline__ bool consumer_sync_any(int flag) {
@@ -457,7 +467,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
     uint8_t* sfb1 = smem_raw + ((sizeof(SmemDf) + 15) & ~(size_t)15);    // 512 bytes of 0x38 (scale 1.0)
     uint8_t* ring = smem_raw + (((smem_u32(smem_raw) + (uint32_t)sizeof(SmemDf) + 16u + 512u + 1023u) & ~1023u) - smem_u32(smem_raw));
     uint8_t* digb = ring + (size_t)P.tc_ring * HX_RING_SLOT;              // digit columns / attention scratch (1024-aligned)
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // warp-uniform for the compiler too
     const int cta = blockIdx.x, grid = gridDim.x;
     const int pos = *P.pos;
     const uint32_t nring = (uint32_t)P.tc_ring;
@@ -548,8 +558,11 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
         }
     } else if (warp == NCW + 1) {
         // =========================== MMA issuer ===========================
-        if (lane == 0) {
-            tc_cp_sf(tmem + TM_SFB, tc_desc(smem_u32(sfb1), 16, 128));
+        // The whole warp runs the loop and one elected lane issues: with the control flow convergent, descriptors and
+        // addresses stay in uniform registers.  A single-thread branch (lane == 0) makes the compiler move every operand
+        // over for each instruction: 170 cycles per MMA (with its scale copy) against 87 at N = 16.
+        {
+            if (tc_elect()) tc_cp_sf(tmem + TM_SFB, tc_desc(smem_u32(sfb1), 16, 128));
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(TC_NDIG >> 3) << 17) | (8u << 24);
             const uint64_t a_ring = tc_desc(smem_u32(ring), 16, 1024, TC_SW128);    // 8-row groups 1024 B apart, 128-byte swizzle
             const uint64_t sf_ring = tc_desc(smem_u32(ring) + 16384, 16, 128);
@@ -563,7 +576,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                 const HxPhase& ph = P.phases[pi];
                 if (ph.type == HX_PH_LINEAR_TC) {
                     const HxCtaPlan tp = ph.plan[cta];
-                    ok = mbar_wait(&S.b_ready, tcph & 1, &S.abort_flag);        // digit columns of this phase are in place
+                    ok = warp_wait(&S.b_ready, tcph & 1, &S.abort_flag);        // digit columns of this phase are in place
                     tcph++;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     unsigned long long dbg_wait = 0; (void)dbg_wait;
@@ -574,11 +587,11 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                     for (int g = tp.b0; g < tp.b1 && ok; g++) {
                         if (fresh) {
                             const uint32_t buf = uc & 1u;
-                            if (uc >= 2) ok = mbar_wait(&S.acc_empty[buf], ((uc >> 1) - 1) & 1, &S.abort_flag);
+                            if (uc >= 2) ok = warp_wait(&S.acc_empty[buf], ((uc >> 1) - 1) & 1, &S.abort_flag);
                             if (!ok) break;
                             dcol = tmem + TM_D0 + buf * TC_NDIG;
                         }
-                        { DF_MMA_T0(); ok = mbar_wait(&S.full[slot], par, &S.abort_flag); DF_MMA_T1(); }
+                        { DF_MMA_T0(); ok = warp_wait(&S.full[slot], par, &S.abort_flag); DF_MMA_T1(); }
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         // descriptors advance in 16-byte units: a K step is 32 B of a swizzled row, a scale chunk 512 B
@@ -586,20 +599,22 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                         const uint64_t sf_slot = sf_ring + (uint64_t)(slot * (HX_RING_SLOT >> 4));
                         const uint64_t b_cell = b_base + (uint64_t)(dp * 128);
                         const uint32_t tsf = tmem + TM_SFA + slot * 16;
+                        const bool last = kc + 1 == tp.C || g + 1 == tp.b1;      // last cell of this tile's piece
+                        if (tc_elect()) {
 #pragma unroll
-                        for (int e = 0; e < 4; e++) tc_cp_sf(tsf + e * 4, sf_slot + (uint64_t)(e * 32));
+                            for (int e = 0; e < 4; e++) tc_cp_sf(tsf + e * 4, sf_slot + (uint64_t)(e * 32));
 #pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            tc_mma(dcol, a_slot + (uint64_t)(e * 2), b_cell + (uint64_t)(e * 2), idesc, tsf + e * 4, tmem + TM_SFB,
-                                   (fresh && e == 0) ? 0u : 1u);
-                        tc_commit(&S.empty[slot]);
-                        fresh = false;
+                            for (int e = 0; e < 4; e++)
+                                tc_mma(dcol, a_slot + (uint64_t)(e * 2), b_cell + (uint64_t)(e * 2), idesc, tsf + e * 4, tmem + TM_SFB,
+                                       (fresh && e == 0) ? 0u : 1u);
+                            tc_commit(&S.empty[slot]);
+                            if (last) tc_commit(&S.acc_full[uc & 1u]);
+                        }
+                        __syncwarp();
+                        fresh = last;
                         if (++slot == nring) { slot = 0; par ^= 1u; }
                         if (++dp == tp.C) dp = 0;
-                        if (++kc == tp.C || g + 1 == tp.b1) {          // last cell of this tile's piece
-                            tc_commit(&S.acc_full[uc & 1u]);
-                            uc++; kc = 0; fresh = true;
-                        }
+                        if (last) { uc++; kc = 0; } else kc++;
                     }
                     DF_MMA_OUT();
                 } else if (ph.type == HX_PH_ATTN) {

@@ -82,6 +82,17 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(s_u32(bar)) : "memory");
 }
 
+// One lane of a converged warp; the branch it guards is known to be taken by a single thread.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// A wait of the whole warp: every lane gets the same answer, so the warp leaves a loop together.
+__device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mb_wait(b, parity, abort_flag));
+}
+
 struct TcSmem {
     uint64_t full[HX_TC_STAGES], empty[HX_TC_STAGES], accum[2], acc_free[2], part_done, tk_ready, bfull[HX_TC_RES_CELLS];
     uint32_t tmem_base;
@@ -126,7 +137,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
     static_assert(sizeof(TcSmem) <= 1024, "header overlaps the unit-scale chunk");
     float* swi = reinterpret_cast<float*>(smem_raw + TC_HDR);
     uint8_t* ring = smem_raw + (((s_u32(smem_raw) + TC_HDR + TC_SWI + 1023u) & ~1023u) - s_u32(smem_raw));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // warp-uniform for the compiler too
     const int Sk = g.stage_ksteps;
     const int P = g.ksplit > 1 ? g.ksplit : 1, kcells = g.ksteps / 4;
     const bool DG = g.digit_mode != 0;      // digit mode: resident digit cells, two accumulators
@@ -200,7 +211,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
+        // The whole warp runs the loop and one elected lane issues: with the control flow convergent, descriptors and
+        // addresses stay in uniform registers.  A single-thread branch (lane == 0) makes the compiler move every operand
+        // over for each instruction: 175 .. 225 cycles per (scale copy + MMA) against 120, the pipe's own rate at N = 240.
+        {
             // instruction descriptor: E2M1 x E2M1, UE4M3 scales, K-major both, N = NB, M = 128, K = 64
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | (8u << 24);
             uint32_t git = 0;
@@ -212,69 +226,76 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const __grid_constant
                 const uint64_t dA0 = smem_desc(s_u32(ring), 16, 1024, SW128), dS0 = smem_desc(s_u32(ring) + 16384, 16, 128);
                 const uint64_t dB0 = smem_desc(s_u32(bres), 16, 1024, SW128);
                 // unit scales (E4M3 1.0) for every digit column: sixteen TMEM columns cover any N up to 256
-                for (int c = 0; c < 4; c++) tc_cp_sf(tmem + col_sfb + c * 4, smem_desc(s_u32(smem_raw + 1024), 16, 128));
+                if (tc_elect()) for (int c = 0; c < 4; c++) tc_cp_sf(tmem + col_sfb + c * 4, smem_desc(s_u32(smem_raw + 1024), 16, 128));
                 const int piece0 = ((int)blockIdx.x % PG) / G;
                 const int ncell = (piece0 + 1) * kcells / P - piece0 * kcells / P;
                 const int nu = ((int)blockIdx.x < nunits) ? (nunits - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
                 const uint32_t total = (uint32_t)(nu * ncell);
                 int ci = 0;
+                uint32_t slot = 0, par = 0;
                 for (git = 0; git < total && ok; git++) {
                     const uint32_t acc = tmem + (uint32_t)(unit_iter & 1) * HX_TC_GROUP_COLS;
                     if (ci == 0) {
                         TC_MARK(1, unit_iter, 0);
                         if (unit_iter >= 2) {      // the epilogue has read this accumulator's previous unit out
-                            if (!mb_wait(&S.acc_free[unit_iter & 1], (uint32_t)((unit_iter >> 1) - 1) & 1u, &S.abort_flag)) break;
+                            if (!warp_wait(&S.acc_free[unit_iter & 1], (uint32_t)((unit_iter >> 1) - 1) & 1u, &S.abort_flag)) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         }
                         TC_MARK(1, unit_iter, 1);
                     }
-                    const uint32_t slot = git % HX_TC_STAGES, round = git / HX_TC_STAGES;
-                    if (git < (uint32_t)ncell && !mb_wait(&S.bfull[git], 0, &S.abort_flag)) { ok = false; break; }
-                    if (!mb_wait(&S.full[slot], round & 1, &S.abort_flag)) { ok = false; break; }
+                    if (git < (uint32_t)ncell && !warp_wait(&S.bfull[git], 0, &S.abort_flag)) { ok = false; break; }
+                    if (!warp_wait(&S.full[slot], par, &S.abort_flag)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (ci == 0) TC_MARK(1, unit_iter, 2);
                     const uint64_t dA = dA0 + (uint64_t)((slot * stage_bytes) >> 4), dS = dS0 + (uint64_t)((slot * stage_bytes) >> 4);
                     const uint64_t dB = dB0 + (uint64_t)(((uint32_t)ci * b_cell_bytes) >> 4);
+                    const bool last = ci + 1 == ncell;
+                    if (tc_elect()) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) tc_cp_sf(tmem + col_sfa + k * 4, dS + (uint64_t)(k * 32));
+                        for (int k = 0; k < 4; k++) tc_cp_sf(tmem + col_sfa + k * 4, dS + (uint64_t)(k * 32));
 #pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        tc_mma(acc, dA + (uint64_t)(k * 2), dB + (uint64_t)(k * 2), idesc, tmem + col_sfa + k * 4, tmem + col_sfb, (k > 0 || ci > 0) ? 1u : 0u);
-                    tc_commit(&S.empty[slot]);          // the slot is free once these MMAs have read it
-                    if (++ci == ncell) {
-                        tc_commit(&S.accum[unit_iter & 1]);            // accumulator complete
-                        TC_MARK(1, unit_iter, 3);
-                        ci = 0; unit_iter++;
+                        for (int k = 0; k < 4; k++)
+                            tc_mma(acc, dA + (uint64_t)(k * 2), dB + (uint64_t)(k * 2), idesc, tmem + col_sfa + k * 4, tmem + col_sfb, (k > 0 || ci > 0) ? 1u : 0u);
+                        tc_commit(&S.empty[slot]);          // the slot is free once these MMAs have read it
+                        if (last) tc_commit(&S.accum[unit_iter & 1]);            // accumulator complete
                     }
+                    __syncwarp();
+                    if (++slot == HX_TC_STAGES) { slot = 0; par ^= 1u; }
+                    if (last) { TC_MARK(1, unit_iter, 3); ci = 0; unit_iter++; }
+                    else ci++;
                 }
             } else
             for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, unit_iter++) {
                 TC_UNIT(u);
                 (void)mt;
                 if (unit_iter > 0) {      // the epilogue has read the previous unit's accumulator out
-                    if (!mb_wait(&S.acc_free[0], (uint32_t)(unit_iter - 1) & 1u, &S.abort_flag)) break;
+                    if (!warp_wait(&S.acc_free[0], (uint32_t)(unit_iter - 1) & 1u, &S.abort_flag)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 for (int ks0 = ks_lo; ks0 < ks_hi; ks0 += Sk, git++) {
                     const uint32_t slot = git % HX_TC_STAGES, round = git / HX_TC_STAGES;
-                    if (!mb_wait(&S.full[slot], round & 1, &S.abort_flag)) { ok = false; break; }
+                    if (!warp_wait(&S.full[slot], round & 1, &S.abort_flag)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const int nk = min(Sk, ks_hi - ks0);
                     const uint32_t sa = s_u32(ring + (size_t)slot * stage_bytes);
                     const uint32_t sb = sa + (uint32_t)Sk * a_cell;
-                    for (int k = 0; k < nk; k++) {
-                        const uint32_t ta = tmem + col_sfa + (slot * HX_TC_MAX_SK + k) * 4;
-                        const uint32_t tb = tmem + col_sfb + (slot * HX_TC_MAX_SK + k) * 4;
-                        const uint32_t acell = sa + (uint32_t)(k >> 2) * HX_T128_CELL, bcell = sb + (uint32_t)(k >> 2) * b_cell_bytes;
-                        const uint32_t e = (uint32_t)(k & 3);
-                        tc_cp_sf(ta, smem_desc(acell + 16384 + e * 512, 16, 128));
-                        tc_cp_sf(tb, smem_desc(bcell + (uint32_t)NB * 128u + e * 512, 16, 128));
-                        tc_mma(tmem, smem_desc(acell + e * 32, 16, 1024, SW128), smem_desc(bcell + e * 32, 16, 1024, SW128), idesc,
-                               ta, tb, (ks0 > ks_lo || k > 0) ? 1u : 0u);
+                    if (tc_elect()) {
+                        for (int k = 0; k < nk; k++) {
+                            const uint32_t ta = tmem + col_sfa + (slot * HX_TC_MAX_SK + k) * 4;
+                            const uint32_t tb = tmem + col_sfb + (slot * HX_TC_MAX_SK + k) * 4;
+                            const uint32_t acell = sa + (uint32_t)(k >> 2) * HX_T128_CELL, bcell = sb + (uint32_t)(k >> 2) * b_cell_bytes;
+                            const uint32_t e = (uint32_t)(k & 3);
+                            tc_cp_sf(ta, smem_desc(acell + 16384 + e * 512, 16, 128));
+                            tc_cp_sf(tb, smem_desc(bcell + (uint32_t)NB * 128u + e * 512, 16, 128));
+                            tc_mma(tmem, smem_desc(acell + e * 32, 16, 1024, SW128), smem_desc(bcell + e * 32, 16, 1024, SW128), idesc,
+                                   ta, tb, (ks0 > ks_lo || k > 0) ? 1u : 0u);
+                        }
+                        tc_commit(&S.empty[slot]);          // the slot is free once these MMAs have read it
                     }
-                    tc_commit(&S.empty[slot]);          // the slot is free once these MMAs have read it
+                    __syncwarp();
                 }
-                if (ok) tc_commit(&S.accum[0]);         // accumulator complete
+                if (ok && tc_elect()) tc_commit(&S.accum[0]);         // accumulator complete
+                __syncwarp();
             }
         }
     } else if (warp < 2 + 4 * TC_EPI_Q) {
