@@ -95,14 +95,14 @@ struct hx_model {
     hx_config gcfg{}; int tp_rank = 0, tp_world = 1;
     float* tp_buf = nullptr; size_t tp_buf_floats = 0; float* tp_peer[8] = {nullptr}; bool tp_connected = false; unsigned tp_launches = 0;
     float* x2 = nullptr; int tp_nbar = 0;
-    // batched prefill (chunks of HX_PF_TB tokens through the tcgen05 GEMM); buffers are created on first use
-    float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_partial = nullptr; unsigned* pf_tickets = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
-    int pf_gu_ld = 0; bool pf_batched = true; size_t pf_partial_n = 0;
+    // batched prefill (chunks of up to pf_tb tokens through the tcgen05 GEMM); buffers are created on first use
+    float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
+    int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
     float* pf_part = nullptr; size_t tp_pf_off = 0, tp_pf_area = 0; unsigned tp_pf_ep = 0;      // tensor-parallel chunk exchange
     int *d_bids = nullptr, *d_bpos = nullptr, *d_bseq = nullptr, *d_bnext = nullptr; float* pf_logits = nullptr; int b_cap = 0;   // batched decode
     int* sp_next = nullptr; float* sp_margin = nullptr;                                   // speculative decode: verify rows
     cudaGraphExec_t g_bstep = nullptr; int g_bstep_n = 0;
-    int* d_pf_pos = nullptr; cudaGraphExec_t g_pf_chunk = nullptr; bool pf_graph_failed = false; int pf_chunk_launches = 0;
+    int* d_pf_pos = nullptr; int bstep_launches = 0;
     // dataflow engine (hx_decode_df.cu): vectors that cross CTAs as (value, epoch) pairs
     bool use_df = false;
     unsigned long long *xll[2] = {nullptr, nullptr}, *statll[2] = {nullptr, nullptr}, *qll = nullptr, *kvll = nullptr, *hll = nullptr;
@@ -881,7 +881,6 @@ HX_API int hx_model_free(hx_model* m) {
     if (!m) return HX_OK;
     if (m->g_decode) cudaGraphExecDestroy(m->g_decode);
     if (m->g_prefill) cudaGraphExecDestroy(m->g_prefill);
-    if (m->g_pf_chunk) cudaGraphExecDestroy(m->g_pf_chunk);
     if (m->g_bstep) cudaGraphExecDestroy(m->g_bstep);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
@@ -1261,68 +1260,48 @@ HX_API int hx_decode_step(hx_model* m, const int32_t* ids, int pos, int32_t* nex
 }
 
 // ---- batched prefill ---------------------------------------------------------------------------------
-static_assert(HX_PF_TB <= HX_TC_MAX_GROUPS * HX_TC_MAX_TOK && HX_PF_TB <= HX_TC_NTOK, "a chunk fits the token groups of the GEMM");
-// K pieces of a linear in the chunk GEMM: pieces small enough for their digit cells to stay in shared memory, and
-// with few row tiles enough of them for about one unit per SM.
-static int pf_pieces(const Fused& f) {
-    const int kcells = f.ksteps / 4;
-    int P = (kcells + HX_TC_RES_CELLS - 1) / HX_TC_RES_CELLS;
-    if (2 * f.tiles128 <= 148) {
-        int q = 148 / f.tiles128; if (q > kcells) q = kcells;
-        if (q > 148 / HX_TC_MAX_GROUPS) q = 148 / HX_TC_MAX_GROUPS;      // pieces x token groups is the least grid
-        if (q > P) P = q;
-    }
-    return P < 1 ? 1 : P;
-}
-
 static int pf_alloc(hx_model* m) {
     if (m->pf_x) return HX_OK;
-    { const int prc = hx_gemm_tc_prepare(); if (prc) return prc; }
+    { const int prc = hx_gemm_dig_prepare(); if (prc) return prc; }
     const hx_config& c = m->cfg;
+    int tb = m->kv_cap < HX_PF_MAX ? m->kv_cap : HX_PF_MAX;
+    if (tb < HX_PF_TB || m->tp_world > 1) tb = HX_PF_TB;       // (a shard's exchange areas hold HX_PF_TB tokens)
+    tb = (tb + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK * HX_TC_MAX_TOK;
     int maxK = c.d_model > m->QD ? c.d_model : m->QD; if (c.d_ff > maxK) maxK = c.d_ff;
-    const size_t cells = (size_t)((maxK + 255) / 256) * HX_TC_MAX_GROUPS * (HX_TC_GROUP_COLS * 128);
+    const size_t cells = (size_t)((maxK + 255) / 256) * (tb / HX_TC_MAX_TOK) * (HX_TC_GROUP_COLS * 128);
     m->pf_gu_ld = m->layers.empty() ? 64 : m->layers[0].gu.tiles128 * 64;      // hidden size rounded up to whole tiles
     int rc;
-    if ((rc = dalloc(m, &m->pf_x, (size_t)HX_PF_TB * c.d_model))) return rc;
-    if ((rc = dalloc(m, &m->pf_qkv, (size_t)HX_PF_TB * (m->QD + 2 * m->KVD)))) return rc;
-    if ((rc = dalloc(m, &m->pf_ctx, (size_t)HX_PF_TB * m->QD))) return rc;
-    if ((rc = dalloc(m, &m->pf_gu, (size_t)HX_PF_TB * m->pf_gu_ld))) return rc;
-    if ((rc = dalloc(m, &m->pf_scale, (size_t)HX_PF_TB))) return rc;
+    if ((rc = dalloc(m, &m->pf_x, (size_t)tb * c.d_model))) return rc;
+    if ((rc = dalloc(m, &m->pf_qkv, (size_t)tb * (m->QD + 2 * m->KVD)))) return rc;
+    if ((rc = dalloc(m, &m->pf_ctx, (size_t)tb * m->QD))) return rc;
+    if ((rc = dalloc(m, &m->pf_gu, (size_t)tb * m->pf_gu_ld))) return rc;
+    if ((rc = dalloc(m, &m->pf_scale, (size_t)tb))) return rc;
     if ((rc = dalloc(m, &m->pf_cells, cells))) return rc;
     if (m->tp_world > 1 && (rc = dalloc(m, &m->pf_part, (size_t)HX_PF_TB * c.d_model))) return rc;
     if ((rc = dalloc(m, &m->pf_err, (size_t)4))) return rc;
     if ((rc = dalloc(m, &m->d_pf_pos, (size_t)4))) return rc;
-    if ((rc = dalloc(m, &m->pf_att_part, hx_pf_attn_scratch(HX_PF_TB, c.n_heads, c.n_kv_heads, c.head_dim)))) return rc;
-    if ((rc = dalloc(m, &m->pf_att_tickets, (size_t)HX_PF_TB * c.n_kv_heads))) return rc;
-    HX_CUDA(cudaMemsetAsync(m->pf_att_tickets, 0, (size_t)HX_PF_TB * c.n_kv_heads * 4, m->st));
+    if ((rc = dalloc(m, &m->pf_att_part, hx_pf_attn_scratch(tb, c.n_heads, c.n_kv_heads, c.head_dim)))) return rc;
+    if ((rc = dalloc(m, &m->pf_att_tickets, (size_t)tb * c.n_kv_heads))) return rc;
+    HX_CUDA(cudaMemsetAsync(m->pf_att_tickets, 0, (size_t)tb * c.n_kv_heads * 4, m->st));
     HX_CUDA(cudaMemsetAsync(m->pf_err, 0, 16, m->st));
-    {   // partial sums [tile][piece][token][128] of the most demanding linear, tickets per tile
-        size_t need = 0; int maxt = m->head.tiles128;
-        auto acc = [&](const Fused& f) { const size_t v = (size_t)f.tiles128 * pf_pieces(f) * HX_PF_TB * 128; if (v > need) need = v; if (f.tiles128 > maxt) maxt = f.tiles128; };
-        for (auto& ly : m->layers) { acc(ly.qkv); acc(ly.o); acc(ly.gu); acc(ly.down); }
-        acc(m->head);
-        m->pf_partial_n = need;
-        if ((rc = dalloc(m, &m->pf_partial, need))) return rc;
-        const size_t ntk = (size_t)maxt * HX_TC_MAX_GROUPS + 8;
-        if ((rc = dalloc(m, &m->pf_tickets, ntk))) return rc;
-        HX_CUDA(cudaMemsetAsync(m->pf_tickets, 0, ntk * 4, m->st));
+    {   // sums so far of the linears whose K is done in blocks: residual ones (d_model rows) and gate/up
+        size_t w = (size_t)c.d_model;
+        for (auto& ly : m->layers) if ((size_t)ly.gu.tiles128 * 128 > w) w = (size_t)ly.gu.tiles128 * 128;
+        if ((rc = dalloc(m, &m->pf_acc, (size_t)tb * w))) return rc;
     }
+    m->pf_tb = tb;
     return HX_OK;
 }
 
 // one linear of a chunk: digits of `src` -> GEMM against f -> out (token-major)
 static int pf_linear(hx_model* m, const Fused& f, const float* src, int ld_src, int n, int swiglu, const float* g,
                      float* out, int ld_out, int rows, int resid, int pair64) {
-    hx_pf_digits(src, ld_src, n, f.K, 0, g, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st);
-    HxGemmTC q = {};
-    q.a = f.t128; q.b = m->pf_cells; q.rows = rows; q.ntiles = f.tiles128; q.ksteps = f.ksteps; q.ntok = n; q.stage_ksteps = 4;
-    q.err = m->pf_err; q.digit_mode = 1; q.col_scale = m->pf_scale; q.out = out; q.ld_out = ld_out; q.resid = resid;
+    hx_pf_digits(src, ld_src, n, f.K, g, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st);
+    HxGemmDig q = {};
+    q.a = f.t128; q.b = m->pf_cells; q.rows = rows; q.ntiles = f.tiles128; q.kcells = f.ksteps / 4; q.ntok = n;
+    q.err = m->pf_err; q.col_scale = m->pf_scale; q.out = out; q.ld_out = ld_out; q.resid = resid; q.acc = m->pf_acc;
     q.ts[0] = f.ts[0]; q.ts[1] = f.ts[1]; q.ts[2] = f.ts[2]; q.bound0 = f.bound0; q.bound1 = f.bound1; q.pair64 = pair64; q.swiglu = swiglu;
-    const int P = pf_pieces(f);
-    if (P > 148) return hx_fail(HX_ERR_ARG, "prefill: %d input columns are more than the chunk GEMM cuts into pieces", f.K);
-    q.ksplit = P; q.partial = m->pf_partial; q.tickets = m->pf_tickets; q.b_resident = 1;
-    if ((size_t)f.tiles128 * P * HX_PF_TB * 128 > m->pf_partial_n) return hx_fail(HX_ERR_ARG, "prefill: partial-sum buffer too small");
-    return hx_gemm_tc_launch(q, m->st);
+    return hx_gemm_dig_launch(q, m->st);
 }
 
 // Tensor-parallel shard: pf_part (this rank's partial rows of a row-split linear for the n tokens of the chunk) summed over
@@ -1417,35 +1396,21 @@ static int bd_enqueue_step(hx_model* m, int n_seq) {
     return HX_OK;
 }
 
-// Prompt positions [0, T) in chunks of HX_PF_TB tokens; ends like the token-by-token path: KV rows written,
-// logits of the last position in m->logits, its arg-max in d_tok / d_hist[T], *d_pos = T.
-// Full chunks replay one captured CUDA graph (the position lives in device memory); the last, shorter chunk
-// and the lm_head are launched directly.
+// Prompt positions [0, T) in equal chunks of whole token groups, as few as the buffers allow; ends like the
+// token-by-token path: KV rows written, logits of the last position in m->logits, its arg-max in d_tok / d_hist[T],
+// *d_pos = T.
 static int run_prefill_batched(hx_model* m, int T, int seq) {
     const hx_config& c = m->cfg;
     int rc = pf_alloc(m); if (rc) return rc;
     const int ps[2] = {0, seq};                      // first position of the chunk, KV slot of the sequence
     HX_CUDA(cudaMemcpyAsync(m->d_pf_pos, ps, 8, cudaMemcpyHostToDevice, m->st));
-    const int nfull = T / HX_PF_TB, rem = T - nfull * HX_PF_TB;
-    if (nfull > 1 && !m->g_pf_chunk && !m->pf_graph_failed) {
-        cudaGraph_t g = nullptr;
-        HX_CUDA(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-        const unsigned long long before = g_hx_launches;
-        rc = pf_enqueue_chunk(m, HX_PF_TB);
-        cudaError_t e = cudaStreamEndCapture(m->st, &g);
-        g_hx_launches = before;
-        if (rc) { if (g) cudaGraphDestroy(g); return rc; }
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&m->g_pf_chunk, g, 0);
-        if (g) cudaGraphDestroy(g);
-        if (e != cudaSuccess) { (void)cudaGetLastError(); m->g_pf_chunk = nullptr; m->pf_graph_failed = true; }
-        m->pf_chunk_launches = 2 + 11 * c.n_layers;
+    const int nch = (T + m->pf_tb - 1) / m->pf_tb, gr = (T + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
+    const int chunk = (gr + nch - 1) / nch * HX_TC_MAX_TOK;
+    int nlast = 0;
+    for (int t0 = 0; t0 < T; t0 += chunk) {
+        nlast = T - t0 < chunk ? T - t0 : chunk;
+        if ((rc = pf_enqueue_chunk(m, nlast))) return rc;
     }
-    for (int i = 0; i < nfull; i++) {
-        if (m->g_pf_chunk) { HX_CUDA(cudaGraphLaunch(m->g_pf_chunk, m->st)); HX_COUNT_LAUNCH(m->pf_chunk_launches); }
-        else if ((rc = pf_enqueue_chunk(m, HX_PF_TB))) return rc;
-    }
-    if (rem && (rc = pf_enqueue_chunk(m, rem))) return rc;
-    const int nlast = rem ? rem : HX_PF_TB;
     if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0))) return rc;
     hx_pf_argmax(m->logits, c.vocab, m->d_tok, m->d_hist, m->d_pos, T - 1, m->st);
     HX_CUDA(cudaGetLastError());
@@ -1763,7 +1728,7 @@ HX_API int hx_decode_batch_loop(hx_model* m, const int32_t* ids, int pos0, int n
         const unsigned long long before = g_hx_launches;
         rc = bd_enqueue_step(m, n_seq);
         cudaError_t e = cudaStreamEndCapture(m->st, &g);
-        m->pf_chunk_launches = (int)(g_hx_launches - before);
+        m->bstep_launches = (int)(g_hx_launches - before);
         g_hx_launches = before;
         if (rc) { if (g) cudaGraphDestroy(g); return rc; }
         if (e == cudaSuccess) e = cudaGraphInstantiate(&m->g_bstep, g, 0);
@@ -1773,7 +1738,7 @@ HX_API int hx_decode_batch_loop(hx_model* m, const int32_t* ids, int pos0, int n
     }
     HX_CUDA(cudaEventRecord(m->ev0, m->st));
     for (int s = 0; s < n_steps; s++) {
-        if (m->g_bstep && m->g_bstep_n == n_seq) { HX_CUDA(cudaGraphLaunch(m->g_bstep, m->st)); HX_COUNT_LAUNCH(m->pf_chunk_launches); }
+        if (m->g_bstep && m->g_bstep_n == n_seq) { HX_CUDA(cudaGraphLaunch(m->g_bstep, m->st)); HX_COUNT_LAUNCH(m->bstep_launches); }
         else if ((rc = bd_enqueue_step(m, n_seq))) return rc;
         if (out_ids) HX_CUDA(cudaMemcpyAsync(out_ids + (size_t)s * n_seq, m->d_bnext, (size_t)n_seq * 4, cudaMemcpyDeviceToHost, m->st));
     }

@@ -17,90 +17,85 @@
 
 namespace {
 
-__device__ __forceinline__ float pf_silu_mul(float g, float u) {      // same formula as the decode epilogue (silu_mul_k)
-    const float sgn = g < 0.0f ? -1.0f : 1.0f;
-    const float e = __expf(-(sgn * g));
-    const float th = sgn * ((1.0f - e) / (1.0f + e));
-    return g * (0.5f * (1.0f + th)) * u;
-}
-
 __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, HxPfWhere wh, const float* __restrict__ emb, float* __restrict__ X, int DM) {
     const float4* src = reinterpret_cast<const float4*>(emb + (size_t)ids[wh.pos_arr ? (int)blockIdx.x : *wh.posp + (int)blockIdx.x] * DM);
     float4* dst = reinterpret_cast<float4*>(X + (size_t)blockIdx.x * DM);
     for (int i = threadIdx.x; i < DM / 4; i += blockDim.x) dst[i] = src[i];
 }
 
-// grid (token, slice of K): every CTA of a token computes the token's statistics, then emits its slice of items.
-// A value becomes the integer M = round(|x| / S * 2^29) < 2^30 (S: the power of two at or below the vector's largest
-// element) and that integer ten balanced base-9 digits (-4 .. 4), least significant first: r = M mod 9, M = M div 9,
-// and a remainder above 4 becomes r - 9 with a carry.  A negative value has all its digits negated.  Digit d (d = 0:
-// weight 9^9) of token t lies in row 24 d + t % 24 of the token group t / 24 of a cell, as the E2M1 code of its value.
-__global__ void __launch_bounds__(512) k_pf_digits(const float* __restrict__ src, int ld, int K, int swiglu, const float* __restrict__ g,
-                                                    float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
+// grid (token, slice of 2048 columns), 256 threads: every CTA of a token computes the token's statistics (all its loads in
+// flight together: one round trip to L2 bounds the small launches), then a thread turns eight consecutive elements into one
+// 32-bit word per digit.
+// A value becomes the integer X = round(x / S * 2^29), |X| < 2^30 (S: the power of two at or below the vector's largest
+// element), spelled with ten balanced base-9 digits (-4 .. 4).  Adding sum_i 4 * 9^i makes it a plain base-9 number whose
+// digits are the balanced ones plus 4 -- no carries, no separate sign -- and a division by 9^5 makes two independent chains
+// of five.  Digit d (d = 0: weight 9^9) of token t lies in row 24 d + t % 24 of the token group t / 24 of a cell, as the E2M1
+// code of its value.  (Before: a chain of ten dependent 32-bit divisions per element on 128 of 512 threads; 64 tokens x 4096
+// columns 6.9 us, 64 x 12288 15.8 us.)
+#define PFD_T 256
+__global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g,
+                                                     float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = src + (size_t)t * ld;
-    __shared__ float red[32];
-    auto value = [&](int k) -> float {        // element k of the vector before the norm scale (gain applied)
-        float v;
-        if (swiglu) { const int tile = k >> 6, r = k & 63; v = pf_silu_mul(x[tile * 128 + r], x[tile * 128 + 64 + r]); }
-        else v = x[k];
-        return v;
-    };
-    // pass 1: sum of squares (of x) and largest |x * g|
+    __shared__ float red[2 * PFD_T / 32];
+    const int k0 = (blockIdx.y * PFD_T + tid) * 8;       // this thread's item, fetched with the rest
+    float v[8];
+    {
+        const bool in0 = k0 < K, in1 = k0 + 4 < K;       // K is a multiple of four
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 a = in0 ? __ldcg(reinterpret_cast<const float4*>(x + k0)) : z, b = in1 ? __ldcg(reinterpret_cast<const float4*>(x + k0 + 4)) : z;
+        const float4 ga = (g && in0) ? __ldg(reinterpret_cast<const float4*>(g + k0)) : one, gb = (g && in1) ? __ldg(reinterpret_cast<const float4*>(g + k0 + 4)) : one;
+        v[0] = a.x * ga.x; v[1] = a.y * ga.y; v[2] = a.z * ga.z; v[3] = a.w * ga.w;
+        v[4] = b.x * gb.x; v[5] = b.y * gb.y; v[6] = b.z * gb.z; v[7] = b.w * gb.w;
+    }
+    // sum of squares (of x) and largest |x * g| of the whole vector
     float ss = 0.0f, mx = 0.0f;
-    for (int k = tid; k < K; k += 512) {
-        const float v = value(k);
-        ss = fmaf(v, v, ss);
-        mx = fmaxf(mx, fabsf(g ? v * g[k] : v));
+    #pragma unroll 4
+    for (int k = tid * 4; k < K; k += PFD_T * 4) {
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k));
+        const float4 ga = g ? __ldg(reinterpret_cast<const float4*>(g + k)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        ss = fmaf(a.x, a.x, ss); ss = fmaf(a.y, a.y, ss); ss = fmaf(a.z, a.z, ss); ss = fmaf(a.w, a.w, ss);
+        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(a.x * ga.x), fabsf(a.y * ga.y)), fmaxf(fabsf(a.z * ga.z), fabsf(a.w * ga.w))));
     }
     ss = hx_warp_sum(ss); mx = hx_warp_max(mx);
-    if (lane == 0) { red[warp] = ss; red[16 + warp] = mx; }
+    if (lane == 0) { red[warp] = ss; red[PFD_T / 32 + warp] = mx; }
     __syncthreads();
     float tss = 0.0f, tmx = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 16; i++) { tss += red[i]; tmx = fmaxf(tmx, red[16 + i]); }
+    for (int i = 0; i < PFD_T / 32; i++) { tss += red[i]; tmx = fmaxf(tmx, red[PFD_T / 32 + i]); }
     const float inv = g ? rsqrtf(tss / (float)K + eps) : 1.0f;
     float Sg = 1.0f;
     const float vmax = tmx * inv * 1.0000005f;
     if (vmax > 0.0f && vmax < INFINITY) Sg = __uint_as_float(__float_as_uint(vmax) & 0x7F800000u);
     if (tid == 0 && blockIdx.y == 0) scale[t] = Sg * (1.0f / HX_TC_DIGIT_UNIT);
     const float mul = (inv / Sg) * HX_TC_DIGIT_UNIT;
-    // pass 2: items of 8 consecutive elements -> one word per digit
-    const int Kc = ((K + 255) / 256) * 256;
-    const size_t cell_bytes = (size_t)groups * (HX_TC_GROUP_COLS * 128);
-    const int tg = t / HX_TC_MAX_TOK, tl = t - tg * HX_TC_MAX_TOK;
-    const int nit = Kc / 8, per = (nit + gridDim.y - 1) / gridDim.y;
-    const int it_hi = min(nit, (int)(blockIdx.y + 1) * per);
-    for (int it = blockIdx.y * per + tid; it < it_hi; it += 512) {
-        const int k = it * 8;
-        uint32_t word[HX_TC_DIGITS];
+    if (k0 >= ((K + 255) & ~255)) return;
+    uint32_t word[HX_TC_DIGITS];
 #pragma unroll
-        for (int n = 0; n < HX_TC_DIGITS; n++) word[n] = 0u;
+    for (int n = 0; n < HX_TC_DIGITS; n++) word[n] = 0u;
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            float v = 0.0f;
-            if (k + e < K) { v = value(k + e); if (g) v *= g[k + e]; }
-            uint32_t m = __float2uint_rn(fabsf(v) * mul);
-            const uint32_t neg = v < 0.0f ? 8u : 0u;
+    for (int e = 0; e < 8; e++) {
+        const uint32_t u = 1743392200u + (uint32_t)__float2int_rn(v[e] * mul);      // (9^10 - 1) / 2 + X
+        const uint32_t hi = u / 59049u;
+        uint32_t part[2] = {hi, u - hi * 59049u};                                    // both below 2^16
 #pragma unroll
-            for (int n = HX_TC_DIGITS - 1; n >= 0; n--) {
-                const uint32_t q = __umulhi(m, 0x38E38E39u) >> 1;      // m / 9
-                uint32_t r = m - 9u * q;                                // 0 .. 8
-                const bool up = r > 4u;                                 // balanced: 5 .. 8 are -4 .. -1 of the next power
-                m = q + (up ? 1u : 0u);
-                const uint32_t mag = up ? 9u - r : r;                   // 0 .. 4
-                const uint32_t code = (0x65420u >> (4u * mag)) & 0xFu;  // E2M1 codes of 0, 1, 2, 3, 4
-                const uint32_t sgn = (mag != 0u && (up != (neg != 0u))) ? 8u : 0u;
-                word[n] |= (code | sgn) << (4 * e);
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int n = 4; n >= 0; n--) {
+                const uint32_t qn = (part[h] * 58255u) >> 19;                        // / 9, exact below 2^16
+                const uint32_t r = part[h] - 9u * qn;                                // digit + 4
+                part[h] = qn;
+                // E2M1 codes of -4, -3, -2, -1, 0, 1, 2, 3, 4: E D C A 0 2 4 5 6
+                word[h * 5 + n] |= (__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * r) & 0xFu) << (4 * e);
             }
-        }
-        const int j = (it >> 2) & 7, w = it & 3;
-        uint8_t* dst = cells + (size_t)(it >> 5) * cell_bytes + (size_t)tg * (HX_TC_GROUP_COLS * 128) + w * 4;
+    }
+    const int it = k0 >> 3, j = (it >> 2) & 7, w = it & 3;
+    const int tg = t / HX_TC_MAX_TOK, tl = t - tg * HX_TC_MAX_TOK;
+    uint8_t* dst = cells + ((size_t)(it >> 5) * groups + tg) * (HX_TC_GROUP_COLS * 128) + w * 4;
 #pragma unroll
-        for (int n = 0; n < HX_TC_DIGITS; n++) {
-            const int row = n * HX_TC_MAX_TOK + tl;
-            *reinterpret_cast<uint32_t*>(dst + (size_t)row * 128 + ((j ^ (row & 7)) << 4)) = word[n];
-        }
+    for (int n = 0; n < HX_TC_DIGITS; n++) {
+        const int row = n * HX_TC_MAX_TOK + tl;
+        *reinterpret_cast<uint32_t*>(dst + (size_t)row * 128 + ((j ^ (row & 7)) << 4)) = word[n];
     }
 }
 
@@ -611,11 +606,9 @@ void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, float* X, int n
     HX_COUNT_LAUNCH(1);
 }
 
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, int swiglu, const float* g, float eps,
-                  uint8_t* cells, float* scale, cudaStream_t st) {
-    const int slices = K >= 8192 ? 8 : 4;
+void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
     const int groups = (n_tok + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
-    k_pf_digits<<<dim3(n_tok, slices), 512, 0, st>>>(src, ld, K, swiglu, g, eps, cells, groups, scale);
+    k_pf_digits<<<dim3(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8)), PFD_T, 0, st>>>(src, ld, K, g, eps, cells, groups, scale);
     HX_COUNT_LAUNCH(1);
 }
 
@@ -626,8 +619,21 @@ void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, 
     HX_COUNT_LAUNCH(1);
 }
 
+// Runs of key tiles per (token group, kv head): about two CTAs per SM, no more than the cache has tiles.
+static int pf_attn_runs(int groups, int NKV, int DH, int cap) {
+    const int KT = 128 < PF_TILE_BYTES / (DH * 4) ? 128 : PF_TILE_BYTES / (DH * 4);
+    int ns = (2 * 148 + NKV * groups - 1) / (NKV * groups);
+    const int cap_tiles = (cap + KT - 1) / KT;
+    if (ns > cap_tiles) ns = cap_tiles;
+    if (ns > PF_NS_MAX) ns = PF_NS_MAX;
+    return ns < 1 ? 1 : ns;
+}
+// Floats of scratch for chunks of up to n_tok tokens.  Only launches with several runs use it, and those have fewer than
+// 2 * 148 (token group, kv head) pairs, so runs x pairs stays below 4 * 148 and a pair has at most four tokens.
 size_t hx_pf_attn_scratch(int n_tok, int NH, int NKV, int DH) {
-    return (size_t)n_tok * NKV * PF_NS_MAX * (NH / NKV) * (DH + 2);
+    size_t rows = (size_t)n_tok * NKV * PF_NS_MAX;
+    if (rows > 4 * 4 * 148) rows = 4 * 4 * 148;
+    return rows * (NH / NKV) * (DH + 2);
 }
 
 template <int GRP, int TG>
@@ -652,13 +658,7 @@ int hx_pf_attn(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NK
     const int groups = (n_tok + TG - 1) / TG;
     const size_t smem = smem_of(TG);
     if (smem > smem_max) return hx_fail(HX_ERR_ARG, "batched prefill attention: %zu bytes of shared memory", smem);
-    // runs of key tiles per (token group, kv head): about two CTAs per SM, no more than the cache has tiles
-    const int KT = 128 < PF_TILE_BYTES / (DH * 4) ? 128 : PF_TILE_BYTES / (DH * 4);
-    int ns = (2 * 148 + NKV * groups - 1) / (NKV * groups);
-    const int cap_tiles = (cap + KT - 1) / KT;
-    if (ns > cap_tiles) ns = cap_tiles;
-    if (ns > PF_NS_MAX) ns = PF_NS_MAX;
-    if (ns < 1) ns = 1;
+    const int ns = pf_attn_runs(groups, NKV, DH, cap);
     dim3 grid(NKV, groups, ns);
     int rc;
 #define HX_PF_ATTN(G) case G: rc = TG == 1 ? pf_attn_launch<G, 1>(grid, smem, st, qkv, ld, wh, n_tok, NH, DH, kc, vc, cap, scale, ctx, ld_ctx, part, tickets, err) \

@@ -1,30 +1,30 @@
-// hx_prefill.cuh -- kernels of the batched prefill (hx_prefill.cu): a chunk of up to 16 prompt tokens goes through
-// every linear as ONE tcgen05 block-scaled GEMM (hx_gemm_tc.cu, digit mode).
+// hx_prefill.cuh -- kernels of the batched prefill (hx_prefill.cu): a chunk of tokens goes through every linear as ONE
+// tcgen05 block-scaled GEMM (hx_gemm_dig.cu).
 #pragma once
 #include "hx_common.cuh"
 
-#define HX_PF_TB 64                // tokens per chunk: three groups of up to 24 tokens x 10 digit columns = the 240 columns of one MMA
+#define HX_PF_TB 64                // tokens per chunk of the batched decode (its logits take vocab floats each), of a verify window and inside a tensor-parallel group
+#define HX_PF_MAX 1008             // tokens per chunk of a prompt: 42 groups of 24.  A launch's ramp and drain (about 6 us) are a
+                                   // twentieth of its work there; the activations of a chunk stay within about 200 MB
 
 // Where the tokens of a chunk sit.  Prefill: consecutive positions of one sequence starting at *posp (device memory, so
-// that the launches of a chunk can be replayed as one CUDA graph).  Batched decode: token t is at position pos_arr[t] of
+// that captured launches can be replayed).  Batched decode: token t is at position pos_arr[t] of
 // sequence seq_arr[t], whose KV cache starts seq_stride floats after the previous sequence's.
 // With pos_arr == null and seqp != null the whole chunk belongs to sequence *seqp (prefill into one KV slot of a batch).
 struct HxPfWhere { const int* posp; const int* pos_arr; const int* seq_arr; size_t seq_stride; const int* seqp; };
 
 // Positions are read from device memory (*posp = position of the chunk's first token) so that the launches of a
-// chunk can be replayed as one CUDA graph.
+// chunk can be captured once and replayed.
 // X[t][:] = emb[ids[*posp + t]][:]
 void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, float* X, int n_tok, int DM, cudaStream_t st);
 
 // Digit columns of a chunk of activation vectors, in the B-cell layout of the digit-mode GEMM.
-//   src [n_tok][ld] f32; swiglu != 0: the vector is silu(gate)*up read from gate/up tiles of 128 rows
-//   (64 gate rows then the 64 matching up rows), K = hidden size;
+//   src [n_tok][ld] f32, K a multiple of four;
 //   g != null: RMSNorm with gain g and eps first;
 //   cells: K rounded up to 256 columns; per 256-column cell and group of 24 tokens 240 rows of 128 bytes, row 24 d + t % 24 =
 //   digit d of token t (ten balanced base-9 digits, most significant first, as E2M1 codes);
 //   scale[t]: x_n = scale[t] * sum_d digit_d 9^(9-d)  (a power of two).
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, int swiglu, const float* g, float eps,
-                  uint8_t* cells, float* scale, cudaStream_t st);
+void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, float eps, uint8_t* cells, float* scale, cudaStream_t st);
 
 // Per token and head of a chunk: RMSNorm (gains qn_g / kn_g, may be null) + rotate_half RoPE at position *posp + t on
 // q (in place) and k; k and v are written to the cache rows of their positions.
