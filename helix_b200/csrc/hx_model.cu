@@ -98,6 +98,7 @@ struct hx_model {
     // batched prefill (chunks of up to pf_tb tokens through the tcgen05 GEMM); buffers are created on first use
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
     int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
+    uint8_t* pf_pieces = nullptr; size_t pf_pieces_bytes = 0; int pf_ctx_hint = 0;      // bf16 terms of K and V of a layer for the tensor-core attention, grown to the longest context seen
     float* pf_part = nullptr; size_t tp_pf_off = 0, tp_pf_area = 0; unsigned tp_pf_ep = 0;      // tensor-parallel chunk exchange
     int *d_bids = nullptr, *d_bpos = nullptr, *d_bseq = nullptr, *d_bnext = nullptr; float* pf_logits = nullptr; int b_cap = 0;   // batched decode
     int* sp_next = nullptr; float* sp_margin = nullptr;                                   // speculative decode: verify rows
@@ -887,6 +888,7 @@ HX_API int hx_model_free(hx_model* m) {
     for (int w = 0; w < 8; w++)                      // mappings of the peers' exchange buffers
         if (m->tp_peer[w] && w != m->tp_rank) cudaIpcCloseMemHandle(m->tp_peer[w]);
     for (void* p : m->allocs) cudaFree(p);
+    if (m->pf_pieces) cudaFree(m->pf_pieces);
     if (m->h_flags) cudaFreeHost(m->h_flags);
     for (cudaEvent_t e : m->prof_ev) cudaEventDestroy(e);
     if (m->st) cudaStreamDestroy(m->st);
@@ -1318,20 +1320,36 @@ static int pf_tp_reduce(hx_model* m, int n) {
     return HX_OK;
 }
 
-// The launches of the layers for one chunk of n tokens (ids[t] / wh say which token, position and sequence each is).
-static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh) {
+// The launches of the layers for one chunk of n tokens (ids[t] / wh say which token, position and sequence each is).  A chunk
+// of one sequence ends at position ctx_end (0: batched decode, every token has a sequence of its own).
+static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, int ctx_end) {
     const hx_config& c = m->cfg;
     const int DH = c.head_dim, DM = c.d_model, QD = m->QD, KVD = m->KVD, cap = m->kv_cap;
     const int ldq = QD + 2 * KVD;
     const float att_scale = 1.0f / sqrtf((float)DH);
     int rc;
+    bool tc = ctx_end > 0 && hx_pf_attn_tc_wanted(n, ctx_end, c.n_heads, c.n_kv_heads, DH);
+    if (tc) {
+        size_t need = hx_pf_attn_tc_bytes(ctx_end, c.n_kv_heads);
+        if (need > m->pf_pieces_bytes) {
+            if (m->pf_ctx_hint > ctx_end) need = hx_pf_attn_tc_bytes(m->pf_ctx_hint, c.n_kv_heads);      // the prompt's later chunks
+            HX_CUDA(cudaStreamSynchronize(m->st));
+            if (m->pf_pieces) cudaFree(m->pf_pieces);
+            m->pf_pieces_bytes = 0;
+            const cudaError_t e = cudaMalloc(&m->pf_pieces, need);
+            if (e != cudaSuccess) { m->pf_pieces = nullptr; (void)cudaGetLastError(); tc = false; }      // no room: the vector kernel needs none
+            else m->pf_pieces_bytes = need;
+        }
+    }
     hx_pf_embed(ids, wh, m->emb, m->pf_x, n, DM, m->st);
     for (int L = 0; L < c.n_layers; L++) {
         Layer& ly = m->layers[L];
         float* kc = m->kc + (size_t)L * c.n_kv_heads * cap * DH; float* vc = m->vc + (size_t)L * c.n_kv_heads * cap * DH;
         if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0))) return rc;
         hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, m->cosT, m->sinT, kc, vc, cap, m->st);
-        if ((rc = hx_pf_attn(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_att_part, m->pf_att_tickets, m->pf_err, m->st))) return rc;
+        if (tc) {
+            if ((rc = hx_pf_attn_tc(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_pieces, ctx_end, m->pf_err, m->st))) return rc;
+        } else if ((rc = hx_pf_attn(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_att_part, m->pf_att_tickets, m->pf_err, m->st))) return rc;
         if (m->tp_world > 1) {
             if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_part, DM, ly.o.N, 0, 0))) return rc;
             if ((rc = pf_tp_reduce(m, n))) return rc;
@@ -1345,11 +1363,11 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh) {
     return HX_OK;
 }
 
-// One prefill chunk of n tokens whose first position is *d_pf_pos; ends by advancing that position.
-static int pf_enqueue_chunk(hx_model* m, int n) {
+// One prefill chunk of n tokens whose first position is *d_pf_pos = t0; ends by advancing that position.
+static int pf_enqueue_chunk(hx_model* m, int t0, int n) {
     const hx_config& c = m->cfg;
     HxPfWhere wh = {m->d_pf_pos, nullptr, nullptr, (size_t)c.n_layers * c.n_kv_heads * m->kv_cap * c.head_dim, m->d_pf_pos + 1};
-    int rc = pf_enqueue_layers(m, n, m->d_prompt, wh); if (rc) return rc;
+    int rc = pf_enqueue_layers(m, n, m->d_prompt, wh, t0 + n); if (rc) return rc;
     hx_pf_advance(m->d_pf_pos, n, m->st);
     return HX_OK;
 }
@@ -1379,7 +1397,7 @@ static int bd_enqueue_step(hx_model* m, int n_seq) {
     for (int c0 = 0; c0 < n_seq; c0 += HX_PF_TB) {
         const int n = n_seq - c0 < HX_PF_TB ? n_seq - c0 : HX_PF_TB;
         HxPfWhere wh = {nullptr, m->d_bpos + c0, m->d_bseq + c0, seq_stride, nullptr};
-        if ((rc = pf_enqueue_layers(m, n, m->d_bids + c0, wh))) return rc;
+        if ((rc = pf_enqueue_layers(m, n, m->d_bids + c0, wh, 0))) return rc;
         if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
         if (m->tp_world > 1) {
             // every rank holds a slice of the vocabulary: local first maximum, then the best over the ranks
@@ -1409,7 +1427,7 @@ static int run_prefill_batched(hx_model* m, int T, int seq) {
     int nlast = 0;
     for (int t0 = 0; t0 < T; t0 += chunk) {
         nlast = T - t0 < chunk ? T - t0 : chunk;
-        if ((rc = pf_enqueue_chunk(m, nlast))) return rc;
+        if ((rc = pf_enqueue_chunk(m, t0, nlast))) return rc;
     }
     if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0))) return rc;
     hx_pf_argmax(m->logits, c.vocab, m->d_tok, m->d_hist, m->d_pos, T - 1, m->st);
@@ -1419,6 +1437,7 @@ static int run_prefill_batched(hx_model* m, int T, int seq) {
 
 static int run_prefill(hx_model* m, const int32_t* ids, int T, int seq = 0) {
     // positions 0..T-2 without the head, position T-1 with it
+    m->pf_ctx_hint = T;
     HX_CUDA(cudaMemcpyAsync(m->d_prompt, ids, (size_t)T * 4, cudaMemcpyHostToDevice, m->st));
     if (m->tp_world > 1 && m->use_tc && m->pf_batched && m->head.t128 && m->use_df) {
         // a shard: positions [0, T-1) in chunks (the exchanges are epoch-numbered kernel arguments, so no graph replay),
@@ -1432,7 +1451,7 @@ static int run_prefill(hx_model* m, const int32_t* ids, int T, int seq = 0) {
         int nlast = 0;
         for (int t0 = 0; t0 < Tc; t0 += HX_PF_TB) {
             nlast = Tc - t0 < HX_PF_TB ? Tc - t0 : HX_PF_TB;
-            if ((rc = pf_enqueue_chunk(m, nlast))) return rc;
+            if ((rc = pf_enqueue_chunk(m, t0, nlast))) return rc;
         }
         if (slot) {
             // the head on the last position, then the first maximum over the ranks' vocabulary slices
@@ -1589,7 +1608,7 @@ static int spec_verify(hx_model* m, const int32_t* win, int n, int pos, int32_t*
     HX_CUDA(cudaMemcpyAsync(m->d_prompt + pos, win, (size_t)n * 4, cudaMemcpyHostToDevice, m->st));
     HX_CUDA(cudaMemcpyAsync(m->d_pf_pos, ps, 8, cudaMemcpyHostToDevice, m->st));
     HxPfWhere wh = {m->d_pf_pos, nullptr, nullptr, (size_t)c.n_layers * c.n_kv_heads * m->kv_cap * c.head_dim, m->d_pf_pos + 1};
-    int rc = pf_enqueue_layers(m, n, m->d_prompt, wh); if (rc) return rc;
+    int rc = pf_enqueue_layers(m, n, m->d_prompt, wh, pos + n); if (rc) return rc;
     if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
     hx_pf_top2_rows(m->pf_logits, c.vocab, c.vocab, n, m->sp_next, m->sp_margin, m->st);
     HX_CUDA(cudaMemcpyAsync(a, m->sp_next, (size_t)n * 4, cudaMemcpyDeviceToHost, m->st));
