@@ -15,6 +15,7 @@
 #include "hx_persist.cuh"
 #include "hx_gemm_tc.cuh"
 #include "hx_prefill.cuh"
+#include "hx_stage.cuh"
 #include <fcntl.h>
 #include <sys/mman.h>
 #include <sys/stat.h>
@@ -118,6 +119,7 @@ template <typename T>
 int dalloc(hx_model* m, T** p, size_t n) {
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, n * sizeof(T) ? n * sizeof(T) : 16);
+    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(&q, n * sizeof(T) ? n * sizeof(T) : 16); }
     if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
     m->allocs.push_back(q);
     *p = (T*)q;
@@ -1812,23 +1814,23 @@ HX_API int hx_model_kv_write(hx_model* m, int seq, int layer, int kv_head, int p
 HX_API int hx_roundtrip_host(const float* w, int rows, int K, const float* x, float* y, int* kpad_out) {
     HX_CHECK_ARG(w && x && y && rows > 0 && K > 0 && K % 4 == 0);
     const int Kpad = hx_kpad(K), Kd = hx_kd(K);
-    float *dw = nullptr, *dx = nullptr, *dy = nullptr, *dts = nullptr; int32_t* dq = nullptr; uint8_t *dm = nullptr, *dc = nullptr, *ds = nullptr;
-    int rc = HX_OK;
-    auto fr = [&]() { cudaFree(dw); cudaFree(dx); cudaFree(dy); cudaFree(dts); cudaFree(dq); cudaFree(dm); cudaFree(dc); cudaFree(ds); };
-#define RT(call) do { cudaError_t _e = (call); if (_e != cudaSuccess) { fr(); return hx_fail(HX_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e)); } } while (0)
-    RT(cudaMalloc(&dw, (size_t)rows * K * 4)); RT(cudaMalloc(&dx, (size_t)Kd * 4)); RT(cudaMalloc(&dy, (size_t)rows * 4));
-    RT(cudaMalloc(&dts, 4)); RT(cudaMalloc(&dq, (size_t)rows * (Kpad / 7) * 4)); RT(cudaMalloc(&dm, (size_t)rows * (Kpad / 16)));
-    RT(cudaMalloc(&dc, (size_t)rows * (Kd / 2))); RT(cudaMalloc(&ds, (size_t)rows * (Kd / 16)));
-    RT(cudaMemcpy(dw, w, (size_t)rows * K * 4, cudaMemcpyHostToDevice));
-    RT(cudaMemset(dx, 0, (size_t)Kd * 4));
-    RT(cudaMemcpy(dx, x, (size_t)K * 4, cudaMemcpyHostToDevice));
-    rc = hx_quantize_nvfp4(dw, rows, K, dq, dm, nullptr, dts, nullptr);
-    if (!rc) rc = hx_repack_d16(dq, dm, rows, K, Kpad, dc, ds, nullptr);
-    if (!rc) rc = hx_gemv_d16(dx, dc, ds, dts, dy, rows, Kd, nullptr);
-    if (rc) { fr(); return rc; }
-    RT(cudaMemcpy(y, dy, (size_t)rows * 4, cudaMemcpyDeviceToHost));
-#undef RT
-    fr();
+    const size_t sz[8] = {(size_t)rows * K * 4, (size_t)Kd * 4, (size_t)rows * 4, 4, (size_t)rows * (Kpad / 7) * 4, (size_t)rows * (Kpad / 16), (size_t)rows * (Kd / 2), (size_t)rows * (Kd / 16)};
+    uint8_t* p[8]; size_t total = 0;
+    for (size_t b : sz) total += (b + 255) & ~(size_t)255;
+    HxStage s;
+    if (s.status()) return s.status();
+    uint8_t* base = nullptr;
+    int rc = s.workspace((void**)&base, total); if (rc) return rc;
+    for (int i = 0; i < 8; i++) { p[i] = base; base += (sz[i] + 255) & ~(size_t)255; }
+    float *dw = (float*)p[0], *dx = (float*)p[1], *dy = (float*)p[2], *dts = (float*)p[3];
+    HX_CUDA(cudaMemsetAsync(dx, 0, (size_t)Kd * 4, s.stream()));
+    const HxCopy in[2] = {{dw, const_cast<float*>(w), sz[0]}, {dx, const_cast<float*>(x), (size_t)K * 4}};
+    if ((rc = s.upload(in, 2))) return rc;
+    if ((rc = hx_quantize_nvfp4(dw, rows, K, (int32_t*)p[4], p[5], nullptr, dts, s.stream()))) return rc;
+    if ((rc = hx_repack_d16((int32_t*)p[4], p[5], rows, K, Kpad, p[6], p[7], s.stream()))) return rc;
+    if ((rc = hx_gemv_d16(dx, p[6], p[7], dts, dy, rows, Kd, s.stream()))) return rc;
+    const HxCopy out = {dy, y, sz[2]};
+    if ((rc = s.download(&out, 1))) return rc;
     if (kpad_out) *kpad_out = Kpad;
     return HX_OK;
 }
