@@ -94,49 +94,74 @@ __device__ __forceinline__ void q_load(const float* __restrict__ wr, int c, int 
     }
 }
 
-// one unit of row r per half-warp; `on`: this half-warp has one
-__device__ __forceinline__ void q_unit(const float (&v)[8], bool on, size_t r, int u, int units, float ts, float ts6, const QOut& o) {
+// what the whole tensor shares
+struct QScale { float ts, ts6, rts6; bool fast; };
+__device__ __forceinline__ QScale q_scale(float amax) {
+    QScale q;
+    q.ts = __fdiv_rn(amax, 2688.0f);                      // 6.0f*448.0f folds to 2688.0f in the reference build
+    if (!(q.ts > 0.0f)) q.ts = 1.0f;                      // `if (ts <= 0) ts = 1`; amax is never NaN
+    q.ts6 = __fmul_rn(q.ts, 6.0f);
+    q.rts6 = __frcp_rn(q.ts6);
+    q.fast = q.ts >= 8.6736174e-19f && q.ts <= 1.1529215e18f;      // 2^-60 .. 2^60: nothing in the fast path over- or underflows
+    return q;
+}
+
+// one unit of row r per half-warp; `on`: this half-warp has one; `out`: its index among all units
+__device__ __forceinline__ void q_unit(const float (&v)[8], bool on, size_t out, const QScale& q, const QOut& o) {
     const int lane = threadIdx.x & 31, l = lane & 15;
     float bm = 0.0f;                                      // the reference's compare: NaN never replaces the running maximum
 #pragma unroll
     for (int e = 0; e < 8; e++) bm = fmaxf(bm, fabsf(v[e]));
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
-    const int mc = hx_e4m3_enc(__fdiv_rn(bm, ts6));
-    const float eff = __fmul_rn(hx_e4m3_dec(mc), ts);
-    uint32_t c8 = 0;
-    if (eff >= 8.6736174e-19f && eff <= 1.1529215e18f) {  // 2^-60 .. 2^60: nothing below over- or underflows
-        const float inv = __frcp_rn(eff), ih = inv * 1.00000095f, il = inv * 0.99999905f;
+    uint32_t c8 = 0, mc;
+    float eff;
+    if (q.fast) {
+        // the scale code the same way: both ends of a window around bm / ts6 through the hardware's E4M3 conversion
+        const float ra = bm * q.rts6;
+        uint16_t two;
+        asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(two) : "f"(ra * 1.00000095f), "f"(ra * 0.99999905f));
+        mc = two & 0xFFu;
+        if ((two >> 8) != mc) mc = (uint32_t)hx_e4m3_enc(__fdiv_rn(bm, q.ts6));
+        eff = __fmul_rn(__uint_as_float(mc << 20) * 1.329227995784916e36f, q.ts);      // decode: bit pattern times 2^120 (never the NaN code here)
+        float inv;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(eff));
+        const float ih = inv * 1.00000095f, il = inv * 0.99999905f;
         float h[8], d[8];
 #pragma unroll
         for (int e = 0; e < 8; e++) { h[e] = v[e] * ih; d[e] = v[e] * il; }
         c8 = q_cvt8(h);
-        uint32_t diff = c8 ^ q_cvt8(d);
+        const uint32_t diff = mc ? c8 ^ q_cvt8(d) : 0u;
         const uint32_t mag = (c8 | (c8 >> 1) | (c8 >> 2)) & 0x11111111u;      // a zero code carries no sign
         c8 &= 0x77777777u | (mag << 3);
+        if (!mc) c8 = 0;                                  // eff == 0: every code of the block is zero
         if (diff) {
+#pragma unroll 1
+            for (int e = 0; e < 8; e++) {
+                if (!((diff >> (4 * e)) & 0xFu)) continue;
+                float x = v[0];
 #pragma unroll
-            for (int e = 0; e < 8; e++)
-                if ((diff >> (4 * e)) & 0xFu) c8 = (c8 & ~(0xFu << (4 * e))) | ((uint32_t)hx_e2m1_enc(__fdiv_rn(v[e], eff)) << (4 * e));
+                for (int k = 1; k < 8; k++) x = e == k ? v[k] : x;
+                c8 = (c8 & ~(0xFu << (4 * e))) | ((uint32_t)hx_e2m1_enc(__fdiv_rn(x, eff)) << (4 * e));
+            }
         }
-    } else if (eff > 0.0f) {
+    } else {
+        mc = (uint32_t)hx_e4m3_enc(__fdiv_rn(bm, q.ts6));
+        eff = __fmul_rn(hx_e4m3_dec((int)mc), q.ts);
+        if (eff > 0.0f) {
 #pragma unroll
-        for (int e = 0; e < 8; e++) c8 |= (uint32_t)hx_e2m1_enc(__fdiv_rn(v[e], eff)) << (4 * e);
+            for (int e = 0; e < 8; e++) c8 |= (uint32_t)hx_e2m1_enc(__fdiv_rn(v[e], eff)) << (4 * e);
+        }
     }
     if (l >= 14) c8 = 0;
     const int w0 = (lane & 16) + ((7 * l) >> 3);          // 28 l bits into the stream
     const uint32_t lo = __shfl_sync(0xffffffffu, c8, w0), hi = __shfl_sync(0xffffffffu, c8, w0 + 1);
     if (!on) return;
-    o.words[r * (size_t)units * 16 + (size_t)u * 16 + l] = (int32_t)(__funnelshift_r(lo, hi, (28 * l) & 31) & 0x0FFFFFFFu);
+    o.words[out * 16 + l] = (int32_t)(__funnelshift_r(lo, hi, (28 * l) & 31) & 0x0FFFFFFFu);
     if (l < 14 && (l & 1) == 0) {
-        const size_t bi = r * (size_t)units * 7 + (size_t)u * 7 + (l >> 1);
+        const size_t bi = out * 7 + (l >> 1);
         if (o.micro) o.micro[bi] = (uint8_t)mc;
         if (o.sc) o.sc[bi] = eff;
     }
-}
-
-__device__ __forceinline__ float q_ts(float amax) {
-    const float ts = __fdiv_rn(amax, 2688.0f);            // 6.0f*448.0f folds to 2688.0f in the reference build
-    return ts > 0.0f ? ts : 1.0f;                         // `if (ts <= 0) ts = 1`; amax is never NaN
 }
 
 #define Q_THREADS 256
@@ -146,23 +171,32 @@ __global__ void __launch_bounds__(Q_THREADS, 4) k_quantize(const float* __restri
     hx_grid_dep_wait();
     float m = 0.0f;
     for (int i = threadIdx.x; i < nparts; i += Q_THREADS) m = fmaxf(m, __ldcg(part + i));
-    const float ts = q_ts(q_block_max<Q_THREADS>(m, sm)), ts6 = __fmul_rn(ts, 6.0f);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && ts_out) *ts_out = ts;
+    const QScale qs = q_scale(q_block_max<Q_THREADS>(m, sm));
+    if (blockIdx.x == 0 && threadIdx.x == 0 && ts_out) *ts_out = qs.ts;
     const bool vec = ((K & 3) == 0) && ((((uintptr_t)w) & 15) == 0);
     const int lane = threadIdx.x & 31, h = lane >> 4, l = lane & 15;
+    // pairs of units, the last ones first; a warp's next pair is nw pairs before: (row, pair) move by a fixed step
     const unsigned np = (unsigned)(units + 1) / 2, total = (unsigned)rows * np, nw = gridDim.x * (Q_THREADS / 32);
-    for (unsigned i = blockIdx.x * (Q_THREADS / 32) + (threadIdx.x >> 5); i < total; i += 2 * nw) {
+    const unsigned dr = nw / np, dp = nw - dr * np;
+    unsigned i = blockIdx.x * (Q_THREADS / 32) + (threadIdx.x >> 5);
+    if (i >= total) return;
+    unsigned r = (total - 1 - i) / np, p = (total - 1 - i) - r * np;
+    for (; i < total; i += 2 * nw) {
         float v[2][8];
-        unsigned r[2]; int u[2]; bool on[2];
+        size_t out[2]; bool on[2];
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const unsigned it = total - 1 - min(i + (unsigned)j * nw, total - 1);
-            r[j] = it / np; u[j] = (int)(it - r[j] * np) * 2 + h;
-            on[j] = u[j] < units && i + (unsigned)j * nw < total;
-            q_load(w + (size_t)r[j] * K, (on[j] && l < 14) ? u[j] * 112 + l * 8 : K, K, vec, v[j]);
+            const int u = (int)p * 2 + h;
+            on[j] = u < units && i + (unsigned)j * nw < total;
+            out[j] = (size_t)r * units + u;
+            q_load(w + (size_t)r * K, (on[j] && l < 14) ? u * 112 + l * 8 : K, K, vec, v[j]);
+            const bool borrow = p < dp;
+            p = borrow ? p + np - dp : p - dp;
+            r -= dr + (borrow ? 1u : 0u);
+            if (i + (unsigned)(j + 1) * nw >= total) r = 0;      // nothing follows: keep the row in range
         }
 #pragma unroll
-        for (int j = 0; j < 2; j++) q_unit(v[j], on[j], r[j], u[j], units, ts, ts6, o);
+        for (int j = 0; j < 2; j++) q_unit(v[j], on[j], out[j], qs, o);
     }
 }
 
@@ -170,7 +204,7 @@ __global__ void __launch_bounds__(Q_THREADS, 4) k_quantize(const float* __restri
 // memory.  Launches are what a small call costs (a fill and two kernels before: 12.5 us for 48 x 1000); up to Q_SMALL
 // elements eight SMs are not slower than two launches over all of them.
 #define Q_SMALL 131072
-#define QS_THREADS 512
+#define QS_THREADS 1024
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(QS_THREADS) k_quantize_small(const float* __restrict__ w, int rows, int K, int units, QOut o, float* __restrict__ ts_out) {
     __shared__ float sm[32];
     __shared__ float cmax[8];
@@ -179,14 +213,18 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(QS_THREADS) k_quanti
     const unsigned np = (unsigned)(units + 1) / 2, total = (unsigned)rows * np, nw = 8 * (QS_THREADS / 32);
     const unsigned i0 = blockIdx.x * (QS_THREADS / 32) + (threadIdx.x >> 5);
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // waited for before the first remote store
-    float m = 0.0f;
-    for (unsigned i = i0; i < total; i += nw) {
+    float m = 0.0f, v0[8];                                // the warp's first pair of units stays in registers
+    auto fetch = [&](unsigned i, float (&v)[8]) {
         const unsigned r = i / np; const int u = (int)(i - r * np) * 2 + h;
-        float v[8];
-        q_load(w + (size_t)r * K, (u < units && l < 14) ? u * 112 + l * 8 : K, K, vec, v);
+        q_load(w + (size_t)r * K, (i < total && u < units && l < 14) ? u * 112 + l * 8 : K, K, vec, v);
+    };
+    auto largest = [&](const float (&v)[8]) {
 #pragma unroll
         for (int e = 0; e < 8; e++) m = fmaxf(m, fabsf(v[e]));
-    }
+    };
+    fetch(i0 < total ? i0 : total, v0);
+    largest(v0);
+    for (unsigned i = i0 + nw; i < total; i += nw) { float v[8]; fetch(i, v); largest(v); }
     m = q_block_max<QS_THREADS>(m, sm);
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every CTA of the cluster has started
     if (threadIdx.x < 8) {                                // this CTA's maximum to every CTA of the cluster
@@ -198,13 +236,16 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(QS_THREADS) k_quanti
     m = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; i++) m = fmaxf(m, cmax[i]);
-    const float ts = q_ts(m), ts6 = __fmul_rn(ts, 6.0f);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && ts_out) *ts_out = ts;
+    const QScale qs = q_scale(m);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && ts_out) *ts_out = qs.ts;
     for (unsigned i = i0; i < total; i += nw) {
         const unsigned r = i / np; const int u = (int)(i - r * np) * 2 + h;
         float v[8];
-        q_load(w + (size_t)r * K, (u < units && l < 14) ? u * 112 + l * 8 : K, K, vec, v);
-        q_unit(v, u < units, r, u, units, ts, ts6, o);
+        if (i == i0) {
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = v0[e];
+        } else fetch(i, v);
+        q_unit(v, u < units, (size_t)r * units + u, qs, o);
     }
 }
 
