@@ -141,4 +141,18 @@ __device__ __forceinline__ float hx_warp_max(float v) {
 // Programmatic dependent launch: wait for the kernels this one depends on / let dependents start.
 __device__ __forceinline__ void hx_grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void hx_grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launch with programmatic stream serialization: the kernel may start while the one before it in the stream drains, and
+// calls hx_grid_dep_wait() before it touches anything that an earlier kernel writes or reads.  Every kernel launched this
+// way waits in at least one CTA before it ends -- otherwise it could complete ahead of its predecessor, and the wait of its
+// successor would not cover that one.
+template <class... KArgs, class... Args>
+static inline cudaError_t hx_launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
+}
 #endif

@@ -93,6 +93,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
     const int units = g.ntiles * g.groups;
     const int u0 = (int)((long long)units * cl / ncl), u1 = (int)((long long)units * (cl + 1) / ncl);
 
+    // The next kernel may start; this one has its barriers, tensor memory and first weight cells (which no kernel writes) ready
+    // before it waits for the one before: the digit loader and the finishing warps do.
+    hx_grid_dep_launch();
     if (tid < 128) reinterpret_cast<uint32_t*>(ones)[tid] = 0x38383838u;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (tid == 0) {
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         }
     } else if (warp == 2) {
         // ------------------------------ digit-cell loader ------------------------------
+        hx_grid_dep_wait();
         if (lane == 0) {
             uint32_t uses[HX_TC_RES_CELLS] = {0, 0, 0, 0};
             bool ok = true;
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         // and the up row.  K in blocks: the sums so far wait in `part` (the output itself when nothing else lies there); the
         // thread that wrote them reads them back.
         const int ft = tid - DG_W_FIN * 32;
+        hx_grid_dep_wait();
         uint32_t free_bar[2] = {0u, 0u};
         if (lane < C) { free_bar[0] = cl_map(s_u32(&S.rx_free[0]), (uint32_t)lane); free_bar[1] = cl_map(s_u32(&S.rx_free[1]), (uint32_t)lane); }
         DgStep it = {u0, u1, 0, 0, 0, 0, 0};
@@ -286,7 +291,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                 if (cur.grp != cs_grp) {
                     cs_grp = cur.grp;
 #pragma unroll
-                    for (int j = 0; j < TB; j++) { const int tk = cur.grp * DG_TOK + q * tpc + j0 + j; cs[j] = tk < g.ntok ? __ldg(g.col_scale + tk) : 0.0f; }
+                    for (int j = 0; j < TB; j++) { const int tk = cur.grp * DG_TOK + q * tpc + j0 + j; cs[j] = tk < g.ntok ? __ldcg(g.col_scale + tk) : 0.0f; }
                 }
                 if (!__all_sync(0xffffffffu, mb_wait_cl(&S.rx_full[buf], (uint32_t)(ou >> 1) & 1u, ab_flag))) break;
                 const float* src = rx + ((size_t)buf * C * tpc + j0) * 128 + r;
@@ -337,7 +342,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                 if (cur.grp != cs_grp) {
                     cs_grp = cur.grp;
 #pragma unroll
-                    for (int j = 0; j < TB; j++) cs[j] = j < nt ? __ldg(g.col_scale + tok0 + j) : 0.0f;
+                    for (int j = 0; j < TB; j++) cs[j] = j < nt ? __ldcg(g.col_scale + tok0 + j) : 0.0f;
                 }
                 if (!__all_sync(0xffffffffu, mb_wait_cl(&S.rx_full[buf], (uint32_t)(ou >> 1) & 1u, ab_flag))) break;
                 const float* src = rx + ((size_t)buf * C * tpc + j0) * 128 + rr;
@@ -446,8 +451,10 @@ int hx_gemm_dig_launch(HxGemmDig g, cudaStream_t st) {
     }
     g.nblk = nblk;
     HX_CHECK_ARG((!g.resid && !g.swiglu) || g.nblk == 1 || g.acc);
-    cudaLaunchConfig_t cfg; cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg; cudaLaunchAttribute at[2];
     dg_config(cfg, at, ncl, C, st);
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     HX_CUDA(cudaLaunchKernelEx(&cfg, dg_kernel(C), g));
     HX_COUNT_LAUNCH(1);
     return HX_OK;

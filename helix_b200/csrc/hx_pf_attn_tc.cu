@@ -57,8 +57,10 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4& h, uint4& m, 
 // Bound by HBM / L2: 8 bytes read and 12 written per (key, dim).
 __global__ void __launch_bounds__(256) k_pf_kv_split(const float* __restrict__ kc, const float* __restrict__ vc, HxPfWhere wh, int n_tok, int cap, uint8_t* __restrict__ dst) {
     const int tile = blockIdx.x, kvh = blockIdx.y, part = blockIdx.z, isv = part >> 1;
-    const int ctx = *wh.posp + n_tok, k0 = tile * AT_KT;
-    const size_t seq_off = wh.seqp ? (size_t)(*wh.seqp) * wh.seq_stride : 0;
+    hx_grid_dep_launch();
+    hx_grid_dep_wait();
+    const int ctx = __ldcg(wh.posp) + n_tok, k0 = tile * AT_KT;
+    const size_t seq_off = wh.seqp ? (size_t)__ldcg(wh.seqp) * wh.seq_stride : 0;
     const float* src = (isv ? vc : kc) + seq_off + ((size_t)kvh * cap) * AT_DH;
     uint8_t* out = dst + (((size_t)kvh * gridDim.x + tile) * 2 + isv) * 6 * AT_PIECE;
 #pragma unroll
@@ -110,9 +112,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_pf_attn_tc(const float* __res
     AtSmem& S = *reinterpret_cast<AtSmem*>(base);
     uint8_t* sq = base + AT_HDR;                              // Q terms: [hi, mid, lo][half]
     uint8_t* ring = sq + 6 * AT_PIECE;
+    hx_grid_dep_launch();
+    hx_grid_dep_wait();
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int kvh = blockIdx.x, TPT = 128 / GRP, t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * TPT;
-    const int pos0 = *wh.posp, tlast = min(n_tok, t0 + TPT) - 1;
+    const int pos0 = __ldcg(wh.posp), tlast = min(n_tok, t0 + TPT) - 1;
     const int ntile = (pos0 + tlast + AT_KT) / AT_KT;         // key tiles that the last token sees
     volatile int* ab = &S.abort_flag;
 
@@ -318,8 +322,8 @@ int hx_pf_attn_tc(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int
     const size_t smem = 1024 + AT_HDR + (size_t)(6 + AT_RING) * AT_PIECE;
     static std::atomic<unsigned long long> attr_seen{0};
     if (hx_first_on_device(attr_seen)) HX_CUDA(cudaFuncSetAttribute(k_pf_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    k_pf_kv_split<<<dim3(kt, NKV, 4), 256, 0, st>>>(kc, vc, wh, n_tok, cap, pieces);
-    k_pf_attn_tc<<<dim3(NKV, (n_tok + tpt - 1) / tpt), AT_THREADS, smem, st>>>(qkv, ld, wh, n_tok, GRP, pieces, kt, scale, ctx, ld_ctx, err);
+    HX_CUDA(hx_launch_pdl(k_pf_kv_split, dim3(kt, NKV, 4), dim3(256), 0, st, kc, vc, wh, n_tok, cap, pieces));
+    HX_CUDA(hx_launch_pdl(k_pf_attn_tc, dim3(NKV, (n_tok + tpt - 1) / tpt), dim3(AT_THREADS), smem, st, qkv, ld, wh, n_tok, GRP, pieces, kt, scale, ctx, ld_ctx, err));
     HX_COUNT_LAUNCH(2);
     HX_CUDA(cudaGetLastError());
     return HX_OK;

@@ -18,7 +18,8 @@
 namespace {
 
 __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, HxPfWhere wh, const float* __restrict__ emb, float* __restrict__ X, int DM) {
-    const float4* src = reinterpret_cast<const float4*>(emb + (size_t)ids[wh.pos_arr ? (int)blockIdx.x : *wh.posp + (int)blockIdx.x] * DM);
+    hx_grid_dep_launch();
+    const float4* src = reinterpret_cast<const float4*>(emb + (size_t)ids[wh.pos_arr ? (int)blockIdx.x : __ldcg(wh.posp) + (int)blockIdx.x] * DM);
     float4* dst = reinterpret_cast<float4*>(X + (size_t)blockIdx.x * DM);
     for (int i = threadIdx.x; i < DM / 4; i += blockDim.x) dst[i] = src[i];
 }
@@ -36,6 +37,8 @@ __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, H
 __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g,
                                                      float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    hx_grid_dep_launch();
+    hx_grid_dep_wait();
     const float* x = src + (size_t)t * ld;
     __shared__ float red[2 * PFD_T / 32];
     const int k0 = (blockIdx.y * PFD_T + tid) * 8;       // this thread's item, fetched with the rest
@@ -104,12 +107,14 @@ __global__ void __launch_bounds__(256) k_pf_qkpost(float* __restrict__ qkv, int 
                                                     const float* __restrict__ qn_g, const float* __restrict__ kn_g, float eps,
                                                     const float* __restrict__ cosT, const float* __restrict__ sinT,
                                                     float* __restrict__ kc, float* __restrict__ vc, int cap) {
-    const int hs = blockIdx.x, t = blockIdx.y, e = threadIdx.x, half = DH >> 1, pos = wh.pos_arr ? wh.pos_arr[t] : *wh.posp + t;
-    const size_t seq_off = wh.seq_arr ? (size_t)wh.seq_arr[t] * wh.seq_stride : (wh.seqp ? (size_t)(*wh.seqp) * wh.seq_stride : 0);
+    hx_grid_dep_launch();
+    hx_grid_dep_wait();
+    const int hs = blockIdx.x, t = blockIdx.y, e = threadIdx.x, half = DH >> 1, pos = wh.pos_arr ? __ldcg(wh.pos_arr + t) : __ldcg(wh.posp) + t;
+    const size_t seq_off = wh.seq_arr ? (size_t)__ldcg(wh.seq_arr + t) * wh.seq_stride : (wh.seqp ? (size_t)__ldcg(wh.seqp) * wh.seq_stride : 0);
     const int sec = hs < NH ? 0 : (hs < NH + NKV ? 1 : 2);
     float* row = qkv + (size_t)t * ld + (size_t)hs * DH;
     __shared__ float sm[256]; __shared__ float red[8];
-    float v = e < DH ? row[e] : 0.0f;
+    float v = e < DH ? __ldcg(row + e) : 0.0f;
     const float* gg = sec == 0 ? qn_g : (sec == 1 ? kn_g : nullptr);
     float ssq = hx_warp_sum(v * v);
     if ((e & 31) == 0) red[e >> 5] = ssq;
@@ -166,6 +171,8 @@ __global__ void __launch_bounds__(PF_AT) k_pf_attn(const float* __restrict__ qkv
                                                     const float* __restrict__ kc, const float* __restrict__ vc, int cap, float scale,
                                                     float* __restrict__ ctx, int ld_ctx, float* __restrict__ part, unsigned* __restrict__ tickets, int* err) {
     extern __shared__ __align__(128) float smf[];
+    hx_grid_dep_launch();
+    hx_grid_dep_wait();
     const int kvh = blockIdx.x, t0 = blockIdx.y * TG, s = blockIdx.z, NS = gridDim.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = PF_AT / 32;
     constexpr int GP = GRP <= 1 ? 1 : (GRP <= 2 ? 2 : (GRP <= 4 ? 4 : 8));      // GRP rounded up to a power of two
@@ -173,13 +180,13 @@ __global__ void __launch_bounds__(PF_AT) k_pf_attn(const float* __restrict__ qkv
     constexpr int LG = NP == 4 ? 2 : (NP == 8 ? 3 : (NP == 16 ? 4 : 5));
     const int KT = min(128, PF_TILE_BYTES / (DH * 4));                           // keys per tile (32 .. 128, a multiple of 32)
     const int ntk = min(TG, n_tok - t0);                                         // tokens of this group
-    const int pos0 = wh.pos_arr ? wh.pos_arr[t0] : *wh.posp + t0;                // TG > 1 only with consecutive positions
+    const int pos0 = wh.pos_arr ? __ldcg(wh.pos_arr + t0) : __ldcg(wh.posp) + t0;                // TG > 1 only with consecutive positions
     const int Tmax = pos0 + ntk;                                                 // context of the group's last token
     const int tiles = (Tmax + KT - 1) / KT, per = ((tiles + NS - 1) / NS) * KT;  // keys per run: whole tiles
     const int n_act = (Tmax + per - 1) / per;
     if (s >= n_act) return;
     const int j_lo = s * per, j_hi = min(Tmax, j_lo + per);
-    const size_t seq_off = wh.seq_arr ? (size_t)wh.seq_arr[t0] * wh.seq_stride : (wh.seqp ? (size_t)(*wh.seqp) * wh.seq_stride : 0);
+    const size_t seq_off = wh.seq_arr ? (size_t)__ldcg(wh.seq_arr + t0) * wh.seq_stride : (wh.seqp ? (size_t)__ldcg(wh.seqp) * wh.seq_stride : 0);
     // shared memory: ring [PF_ST][K tile | V tile], then q, p and the P*V partial outputs
     float* ringf = smf;
     const int stage_f = 2 * (PF_TILE_BYTES / 4);
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(PF_AT) k_pf_attn(const float* __restrict__ qkv
     __shared__ __align__(8) uint64_t full[PF_ST];
     for (int i = tid; i < ntk * GRP * DH; i += PF_AT) {
         const int tk = i / (GRP * DH), r = i - tk * GRP * DH;
-        sq[i] = qkv[(size_t)(t0 + tk) * ld + (size_t)kvh * GRP * DH + r];
+        sq[i] = __ldcg(qkv + (size_t)(t0 + tk) * ld + (size_t)kvh * GRP * DH + r);
     }
     if (tid < TG * GRP) { sm_m[tid / GRP][tid % GRP] = -100000000.0f; sm_l[tid / GRP][tid % GRP] = 0.0f; }
     if (tid == 0) {
@@ -536,7 +543,7 @@ __global__ void __launch_bounds__(1024) k_pf_tp_argmax_rows(const float* __restr
     }
 }
 
-__global__ void k_pf_advance(int* posp, int n) { if (threadIdx.x == 0) *posp += n; }
+__global__ void k_pf_advance(int* posp, int n) { hx_grid_dep_launch(); hx_grid_dep_wait(); if (threadIdx.x == 0) *posp += n; }
 // one CTA per token row: first maximum of logits[row][0..n) -> next[row]; the row's position advances by one
 __global__ void __launch_bounds__(1024) k_pf_argmax_rows(const float* __restrict__ logits, int n, int ld, int* __restrict__ next, int* __restrict__ pos_arr) {
     const float* lg = logits + (size_t)blockIdx.x * ld;
@@ -608,31 +615,37 @@ void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, float* X, int n
 
 void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
     const int groups = (n_tok + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
-    k_pf_digits<<<dim3(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8)), PFD_T, 0, st>>>(src, ld, K, g, eps, cells, groups, scale);
+    const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
+    // Started early, this kernel's CTAs wait beside the GEMM's and the step got slower up to some hundred tokens (64 sequences
+    // 3.72 -> 3.85 ms for twelve layers, five sequences 0.97 -> 1.03); at 512 tokens it gains 3 %.
+    if (n_tok >= 256) hx_launch_pdl(k_pf_digits, grid, dim3(PFD_T), 0, st, src, ld, K, g, eps, cells, groups, scale);
+    else k_pf_digits<<<grid, PFD_T, 0, st>>>(src, ld, K, g, eps, cells, groups, scale);
     HX_COUNT_LAUNCH(1);
 }
 
 void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
                   float eps, const float* cosT, const float* sinT, float* kc, float* vc, int cap, cudaStream_t st) {
     const int threads = ((DH + 31) / 32) * 32;
-    k_pf_qkpost<<<dim3(NH + 2 * NKV, n_tok), threads, 0, st>>>(qkv, ld, wh, NH, NKV, DH, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap);
+    hx_launch_pdl(k_pf_qkpost, dim3(NH + 2 * NKV, n_tok), dim3(threads), 0, st, qkv, ld, wh, NH, NKV, DH, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap);
     HX_COUNT_LAUNCH(1);
 }
 
-// Runs of key tiles per (token group, kv head): about two CTAs per SM, no more than the cache has tiles.
+// Runs of key tiles per (token group, kv head): as many as one wave of CTAs holds (a CTA fills an SM's shared memory; with
+// two CTAs per SM asked for, five sequences took 2.2 waves of short runs: 24.5 us per layer at 900 positions against 13),
+// no more than the cache has tiles.
 static int pf_attn_runs(int groups, int NKV, int DH, int cap) {
     const int KT = 128 < PF_TILE_BYTES / (DH * 4) ? 128 : PF_TILE_BYTES / (DH * 4);
-    int ns = (2 * 148 + NKV * groups - 1) / (NKV * groups);
+    int ns = 148 / (NKV * groups);
     const int cap_tiles = (cap + KT - 1) / KT;
     if (ns > cap_tiles) ns = cap_tiles;
     if (ns > PF_NS_MAX) ns = PF_NS_MAX;
     return ns < 1 ? 1 : ns;
 }
-// Floats of scratch for chunks of up to n_tok tokens.  Only launches with several runs use it, and those have fewer than
-// 2 * 148 (token group, kv head) pairs, so runs x pairs stays below 4 * 148 and a pair has at most four tokens.
+// Floats of scratch for chunks of up to n_tok tokens: runs x (token group, kv head) pairs stays within 148 where there are
+// several runs, and a pair has at most four tokens.
 size_t hx_pf_attn_scratch(int n_tok, int NH, int NKV, int DH) {
     size_t rows = (size_t)n_tok * NKV * PF_NS_MAX;
-    if (rows > 4 * 4 * 148) rows = 4 * 4 * 148;
+    if (rows > 4 * 148) rows = 4 * 148;
     return rows * (NH / NKV) * (DH + 2);
 }
 
@@ -641,7 +654,7 @@ static int pf_attn_launch(dim3 grid, size_t smem, cudaStream_t st, const float* 
                           const float* vc, int cap, float scale, float* ctx, int ld_ctx, float* part, unsigned* tickets, int* err) {
     static std::atomic<unsigned long long> attr_seen{0};
     if (hx_first_on_device(attr_seen)) HX_CUDA(cudaFuncSetAttribute(k_pf_attn<GRP, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));      // the kernel has some static shared memory too
-    k_pf_attn<GRP, TG><<<grid, PF_AT, smem, st>>>(qkv, ld, wh, n_tok, NH, DH, kc, vc, cap, scale, ctx, ld_ctx, part, tickets, err);
+    HX_CUDA(hx_launch_pdl(k_pf_attn<GRP, TG>, grid, dim3(PF_AT), smem, st, qkv, ld, wh, n_tok, NH, DH, kc, vc, cap, scale, ctx, ld_ctx, part, tickets, err));
     return HX_OK;
 }
 
@@ -691,7 +704,7 @@ void hx_pf_tp_argmax_rows(const float* logits, int n, int ld, int rows, int voca
 }
 
 void hx_pf_advance(int* posp, int n, cudaStream_t st) {
-    k_pf_advance<<<1, 32, 0, st>>>(posp, n);
+    hx_launch_pdl(k_pf_advance, dim3(1), dim3(32), 0, st, posp, n);
     HX_COUNT_LAUNCH(1);
 }
 

@@ -286,12 +286,7 @@ static int quantize_launch(const float* w, int rows, int K, int32_t* words, uint
     k_amax<<<g1, AMAX_THREADS, 0, st>>>(w, n, part);
     // pass 2 is launched while pass 1 drains; it waits for its results before the first read
     const size_t ctas = (items + Q_THREADS / 32 - 1) / (Q_THREADS / 32);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8)); cfg.blockDim = dim3(Q_THREADS); cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    HX_CUDA(cudaLaunchKernelEx(&cfg, k_quantize, w, rows, K, units, (const float*)part, g1, o, ts));
+    HX_CUDA(hx_launch_pdl(k_quantize, dim3((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8)), dim3(Q_THREADS), 0, st, w, rows, K, units, (const float*)part, g1, o, ts));
     HX_COUNT_LAUNCH(2);
     HX_CUDA(cudaGetLastError());
     return HX_OK;
