@@ -75,6 +75,14 @@ struct DgStep {
     }
 };
 
+__device__ __forceinline__ float dg_gelu(float x) {      // gpu_gelu_stable_kernel.hx:15-28
+    const float inner = 0.7978846f * (x + (0.044715f * (x * x * x))), two = 2.0f * inner;
+    const float sgn = inner < 0.0f ? -1.0f : 1.0f;
+    const float e = __expf(-(sgn * two));
+    const float th = sgn * ((1.0f - e) / (1.0f + e));
+    return 0.5f * x * (1.0f + th);
+}
+
 template <int C>
 __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constant__ HxGemmDig g) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -304,12 +312,14 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                     for (int j = 0; j < TB; j++) v[j] += (j0 + j < tpc) ? src[(p * tpc + j) * 128] : 0.0f;
                 __syncwarp();
                 if (lane < C) cl_arrive_relaxed(free_bar[buf]);
+                const float bias = (g.bias && lastb && row < g.rows) ? __ldg(g.bias + row) : 0.0f;
                 const float tsr = g.pair64 ? (r < 64 ? g.ts[0] : g.ts[1]) : (row < g.bound0 ? g.ts[0] : (row < g.bound1 ? g.ts[1] : g.ts[2]));
                 float* dst = (lastb ? g.out : part) + offset(cur);
 #pragma unroll
                 for (int j = 0; j < TB; j++) {
                     float y = v[j] * cs[j] * tsr;
                     if (!firstb) y += sofar[j];
+                    if (lastb) { y += bias; if (g.gelu) y = dg_gelu(y); }
                     v[j] = (g.resid && lastb) ? prev[j] + y : y;
                 }
                 more = it.next(g);

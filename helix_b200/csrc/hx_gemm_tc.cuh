@@ -23,7 +23,7 @@ int hx_gemm_tc_launch(const HxGemmTC& g, cudaStream_t st);
 size_t hx_gemm_tc_smem(int ncols, int stage_ksteps);
 
 // A linear of a chunk: out[t * ld_out + row] = resid ? out + y : y with
-//   y = col_scale[t] * ts(row) * sum_d 9^(9-d) D[row][group of t][24 d + t % 24]
+//   y = act(col_scale[t] * ts(row) * sum_d 9^(9-d) D[row][group of t][24 d + t % 24] + bias[row])
 struct HxGemmDig {
     const uint8_t* a;              // T128 weight cells [tile][cell of 256 columns]
     const uint8_t* b;              // digit cells [cell of 256 columns][token group]: 240 rows of 128 swizzled bytes
@@ -35,6 +35,8 @@ struct HxGemmDig {
     float ts[3]; int bound0, bound1;   // per-row tensor scale: rows < bound0 ts[0], < bound1 ts[1], else ts[2]
     int pair64;                    // 1: ts[0] for rows with (row % 128) < 64, ts[1] for the others (gate/up tiles)
     int swiglu;                    // 1: tiles hold 64 gate + 64 up rows; out[t][tile * 64 + r] = silu(gate_r) * up_r, rows = hidden size
+    const float* bias;             // [rows] or null; gelu: gelu_new after it (plain linears)
+    int gelu;
     int* err;                      // set when a bounded wait ran out
     int groups, nblk;              // filled in by the launch: token groups, blocks of K
 };

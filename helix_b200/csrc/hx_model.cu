@@ -958,7 +958,10 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
     hx_model* m = new hx_model();
     m->cfg = c; m->gcfg = c; m->cfg.qk_norm = 0; m->QD = c.d_model; m->KVD = c.d_model;
     m->kv_cap = kv_cap; m->batch = 1; m->flags = 0;
-    m->persist = false; m->use_tc = false; m->want_t128 = false; m->pf_batched = false;     // per-op kernels in one CUDA graph
+    // tokens one at a time through per-op kernels in one CUDA graph, prompts through the chunk GEMM (its weight cells beside
+    // the dense layout: 0.56 bytes per weight once more)
+    m->persist = false; m->use_tc = false; m->want_t128 = true;
+    { const char* pf = getenv("HX_PREFILL"); m->pf_batched = !(pf && strcmp(pf, "token") == 0); }
     int rc = HX_OK;
     float* stage = nullptr; int32_t* wtmp = nullptr; uint8_t* mtmp = nullptr; float* tstmp = nullptr;
     do {
@@ -1273,7 +1276,7 @@ static int pf_alloc(hx_model* m) {
     tb = (tb + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK * HX_TC_MAX_TOK;
     int maxK = c.d_model > m->QD ? c.d_model : m->QD; if (c.d_ff > maxK) maxK = c.d_ff;
     const size_t cells = (size_t)((maxK + 255) / 256) * (tb / HX_TC_MAX_TOK) * (HX_TC_GROUP_COLS * 128);
-    m->pf_gu_ld = m->layers.empty() ? 64 : m->layers[0].gu.tiles128 * 64;      // hidden size rounded up to whole tiles
+    m->pf_gu_ld = m->layers.empty() ? 64 : m->layers[0].gu.tiles128 * (c.arch == 0 ? 128 : 64);      // hidden size rounded up to whole tiles
     int rc;
     if ((rc = dalloc(m, &m->pf_x, (size_t)tb * c.d_model))) return rc;
     if ((rc = dalloc(m, &m->pf_qkv, (size_t)tb * (m->QD + 2 * m->KVD)))) return rc;
@@ -1299,12 +1302,12 @@ static int pf_alloc(hx_model* m) {
 
 // one linear of a chunk: digits of `src` -> GEMM against f -> out (token-major)
 static int pf_linear(hx_model* m, const Fused& f, const float* src, int ld_src, int n, int swiglu, const float* g,
-                     float* out, int ld_out, int rows, int resid, int pair64) {
-    hx_pf_digits(src, ld_src, n, f.K, g, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st);
+                     float* out, int ld_out, int rows, int resid, int pair64, const float* nb = nullptr, const float* bias = nullptr, int gelu = 0) {
+    hx_pf_digits(src, ld_src, n, f.K, g, nb, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st);
     HxGemmDig q = {};
     q.a = f.t128; q.b = m->pf_cells; q.rows = rows; q.ntiles = f.tiles128; q.kcells = f.ksteps / 4; q.ntok = n;
     q.err = m->pf_err; q.col_scale = m->pf_scale; q.out = out; q.ld_out = ld_out; q.resid = resid; q.acc = m->pf_acc;
-    q.ts[0] = f.ts[0]; q.ts[1] = f.ts[1]; q.ts[2] = f.ts[2]; q.bound0 = f.bound0; q.bound1 = f.bound1; q.pair64 = pair64; q.swiglu = swiglu;
+    q.ts[0] = f.ts[0]; q.ts[1] = f.ts[1]; q.ts[2] = f.ts[2]; q.bound0 = f.bound0; q.bound1 = f.bound1; q.pair64 = pair64; q.swiglu = swiglu; q.bias = bias; q.gelu = gelu;
     return hx_gemm_dig_launch(q, m->st);
 }
 
@@ -1343,19 +1346,25 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, i
             else m->pf_pieces_bytes = need;
         }
     }
-    hx_pf_embed(ids, wh, m->emb, m->pf_x, n, DM, m->st);
+    hx_pf_embed(ids, wh, m->emb, c.arch == 0 ? m->wpe : nullptr, m->pf_x, n, DM, m->st);
     for (int L = 0; L < c.n_layers; L++) {
         Layer& ly = m->layers[L];
         float* kc = m->kc + (size_t)L * c.n_kv_heads * cap * DH; float* vc = m->vc + (size_t)L * c.n_kv_heads * cap * DH;
-        if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0))) return rc;
-        hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, m->cosT, m->sinT, kc, vc, cap, m->st);
+        const bool g2 = c.arch == 0;         // GPT-2: LayerNorm, biases, gelu_new, no rotation, no q/k norm
+        if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0, ly.ln1_b, ly.b_qkv))) return rc;
+        hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, g2 ? nullptr : m->cosT, g2 ? nullptr : m->sinT, kc, vc, cap, m->st);
         if (tc) {
             if ((rc = hx_pf_attn_tc(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_pieces, ctx_end, m->pf_err, m->st))) return rc;
         } else if ((rc = hx_pf_attn(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_att_part, m->pf_att_tickets, m->pf_err, m->st))) return rc;
         if (m->tp_world > 1) {
             if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_part, DM, ly.o.N, 0, 0))) return rc;
             if ((rc = pf_tp_reduce(m, n))) return rc;
-        } else if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_x, DM, ly.o.N, 1, 0))) return rc;
+        } else if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_x, DM, ly.o.N, 1, 0, nullptr, ly.b_o))) return rc;
+        if (g2) {
+            if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, 0, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 0, ly.ln2_b, ly.b_fc, 1))) return rc;
+            if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, 0, nullptr, m->pf_x, DM, ly.down.N, 1, 0, nullptr, ly.b_down))) return rc;
+            continue;
+        }
         if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, 1, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 1))) return rc;       // SwiGLU in the epilogue
         if (m->tp_world > 1) {
             if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, 0, nullptr, m->pf_part, DM, ly.down.N, 0, 0))) return rc;
@@ -1431,7 +1440,7 @@ static int run_prefill_batched(hx_model* m, int T, int seq) {
         nlast = T - t0 < chunk ? T - t0 : chunk;
         if ((rc = pf_enqueue_chunk(m, t0, nlast))) return rc;
     }
-    if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0))) return rc;
+    if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0, m->final_b))) return rc;
     hx_pf_argmax(m->logits, c.vocab, m->d_tok, m->d_hist, m->d_pos, T - 1, m->st);
     HX_CUDA(cudaGetLastError());
     return HX_OK;
@@ -1471,7 +1480,7 @@ static int run_prefill(hx_model* m, const int32_t* ids, int T, int seq = 0) {
         HX_CUDA(cudaMemcpyAsync(m->d_tok, m->d_prompt + (T - 1), 4, cudaMemcpyDeviceToDevice, m->st));
         return step_decode(m);
     }
-    if (m->use_tc && m->pf_batched && m->head.t128) return run_prefill_batched(m, T, seq);
+    if ((m->use_tc || m->cfg.arch == 0) && m->pf_batched && m->head.t128) return run_prefill_batched(m, T, seq);
     if (seq != 0) return hx_fail(HX_ERR_STATE, "prefill into KV slot %d needs the batched prefill path", seq);
     int rc = set_pos_tok(m, 0, nullptr); if (rc) return rc;
     for (int s = 0; s < T - 1; s++) if ((rc = step_prefill(m))) return rc;

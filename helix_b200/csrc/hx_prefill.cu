@@ -17,11 +17,17 @@
 
 namespace {
 
-__global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, HxPfWhere wh, const float* __restrict__ emb, float* __restrict__ X, int DM) {
+__global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, HxPfWhere wh, const float* __restrict__ emb, const float* __restrict__ wpe, float* __restrict__ X, int DM) {
     hx_grid_dep_launch();
-    const float4* src = reinterpret_cast<const float4*>(emb + (size_t)ids[wh.pos_arr ? (int)blockIdx.x : __ldcg(wh.posp) + (int)blockIdx.x] * DM);
-    float4* dst = reinterpret_cast<float4*>(X + (size_t)blockIdx.x * DM);
-    for (int i = threadIdx.x; i < DM / 4; i += blockDim.x) dst[i] = src[i];
+    const int t = blockIdx.x, pos = wh.pos_arr ? __ldcg(wh.pos_arr + t) : __ldcg(wh.posp) + t;
+    const float4* src = reinterpret_cast<const float4*>(emb + (size_t)ids[wh.pos_arr ? t : pos] * DM);
+    const float4* add = wpe ? reinterpret_cast<const float4*>(wpe + (size_t)pos * DM) : nullptr;
+    float4* dst = reinterpret_cast<float4*>(X + (size_t)t * DM);
+    for (int i = threadIdx.x; i < DM / 4; i += blockDim.x) {
+        float4 v = src[i];
+        if (add) { const float4 p = add[i]; v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w; }
+        dst[i] = v;
+    }
 }
 
 // grid (token, slice of 2048 columns), 256 threads: every CTA of a token computes the token's statistics (all its loads in
@@ -34,7 +40,7 @@ __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, H
 // code of its value.  (Before: a chain of ten dependent 32-bit divisions per element on 128 of 512 threads; 64 tokens x 4096
 // columns 6.9 us, 64 x 12288 15.8 us.)
 #define PFD_T 256
-__global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g,
+__global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g, const float* __restrict__ lb,
                                                      float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     hx_grid_dep_launch();
@@ -51,8 +57,41 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
         v[0] = a.x * ga.x; v[1] = a.y * ga.y; v[2] = a.z * ga.z; v[3] = a.w * ga.w;
         v[4] = b.x * gb.x; v[5] = b.y * gb.y; v[6] = b.z * gb.z; v[7] = b.w * gb.w;
     }
+    float inv = 1.0f, mx = 0.0f;
+    if (lb) {
+        // LayerNorm (GPT-2): mean, then variance about it, then the largest result
+        float mean = 0.0f;
+        for (int ps = 0; ps < 2; ps++) {
+            float s = 0.0f;
+            for (int k = tid * 4; k < K; k += PFD_T * 4) {
+                const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k));
+                if (ps == 0) s += (a.x + a.y) + (a.z + a.w);
+                else s += ((a.x - mean) * (a.x - mean) + (a.y - mean) * (a.y - mean)) + ((a.z - mean) * (a.z - mean) + (a.w - mean) * (a.w - mean));
+            }
+            s = hx_warp_sum(s);
+            __syncthreads();
+            if (lane == 0) red[warp] = s;
+            __syncthreads();
+            s = 0.0f;
+#pragma unroll
+            for (int i = 0; i < PFD_T / 32; i++) s += red[i];
+            if (ps == 0) mean = s / (float)K; else inv = rsqrtf(s / (float)K + eps);
+        }
+        for (int k = tid * 4; k < K; k += PFD_T * 4) {
+            const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k)), ga = __ldg(reinterpret_cast<const float4*>(g + k)), ba = __ldg(reinterpret_cast<const float4*>(lb + k));
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(ga.x * ((a.x - mean) * inv) + ba.x), fabsf(ga.y * ((a.y - mean) * inv) + ba.y)),
+                                 fmaxf(fabsf(ga.z * ((a.z - mean) * inv) + ba.z), fabsf(ga.w * ((a.w - mean) * inv) + ba.w))));
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[e] = k0 + e < K ? __ldg(g + k0 + e) * ((__ldcg(x + k0 + e) - mean) * inv) + __ldg(lb + k0 + e) : 0.0f;
+        inv = 1.0f;
+        mx = hx_warp_max(mx);
+        __syncthreads();
+        if (lane == 0) red[PFD_T / 32 + warp] = mx;
+        __syncthreads();
+    } else {
     // sum of squares (of x) and largest |x * g| of the whole vector
-    float ss = 0.0f, mx = 0.0f;
+    float ss = 0.0f;
     #pragma unroll 4
     for (int k = tid * 4; k < K; k += PFD_T * 4) {
         const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k));
@@ -63,10 +102,14 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
     ss = hx_warp_sum(ss); mx = hx_warp_max(mx);
     if (lane == 0) { red[warp] = ss; red[PFD_T / 32 + warp] = mx; }
     __syncthreads();
-    float tss = 0.0f, tmx = 0.0f;
+    float tss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < PFD_T / 32; i++) { tss += red[i]; tmx = fmaxf(tmx, red[PFD_T / 32 + i]); }
-    const float inv = g ? rsqrtf(tss / (float)K + eps) : 1.0f;
+    for (int i = 0; i < PFD_T / 32; i++) tss += red[i];
+    if (g) inv = rsqrtf(tss / (float)K + eps);
+    }
+    float tmx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PFD_T / 32; i++) tmx = fmaxf(tmx, red[PFD_T / 32 + i]);
     float Sg = 1.0f;
     const float vmax = tmx * inv * 1.0000005f;
     if (vmax > 0.0f && vmax < INFINITY) Sg = __uint_as_float(__float_as_uint(vmax) & 0x7F800000u);
@@ -608,18 +651,18 @@ __global__ void __launch_bounds__(1024) k_pf_argmax(const float* __restrict__ lo
 
 }  // namespace
 
-void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, float* X, int n_tok, int DM, cudaStream_t st) {
-    k_pf_embed<<<n_tok, 256, 0, st>>>(ids, wh, emb, X, DM);
+void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st) {
+    k_pf_embed<<<n_tok, 256, 0, st>>>(ids, wh, emb, wpe, X, DM);
     HX_COUNT_LAUNCH(1);
 }
 
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
+void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
     const int groups = (n_tok + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
     const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
     // Started early, this kernel's CTAs wait beside the GEMM's and the step got slower up to some hundred tokens (64 sequences
     // 3.72 -> 3.85 ms for twelve layers, five sequences 0.97 -> 1.03); at 512 tokens it gains 3 %.
-    if (n_tok >= 256) hx_launch_pdl(k_pf_digits, grid, dim3(PFD_T), 0, st, src, ld, K, g, eps, cells, groups, scale);
-    else k_pf_digits<<<grid, PFD_T, 0, st>>>(src, ld, K, g, eps, cells, groups, scale);
+    if (n_tok >= 256) hx_launch_pdl(k_pf_digits, grid, dim3(PFD_T), 0, st, src, ld, K, g, b, eps, cells, groups, scale);
+    else k_pf_digits<<<grid, PFD_T, 0, st>>>(src, ld, K, g, b, eps, cells, groups, scale);
     HX_COUNT_LAUNCH(1);
 }
 

@@ -15,16 +15,16 @@ struct HxPfWhere { const int* posp; const int* pos_arr; const int* seq_arr; size
 
 // Positions are read from device memory (*posp = position of the chunk's first token) so that the launches of a
 // chunk can be captured once and replayed.
-// X[t][:] = emb[ids[*posp + t]][:]
-void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, float* X, int n_tok, int DM, cudaStream_t st);
+// X[t][:] = emb[ids[*posp + t]][:] (+ wpe[*posp + t][:])
+void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st);
 
 // Digit columns of a chunk of activation vectors, in the B-cell layout of the digit-mode GEMM.
 //   src [n_tok][ld] f32, K a multiple of four;
-//   g != null: RMSNorm with gain g and eps first;
+//   g != null: RMSNorm with gain g and eps first, or with b != null LayerNorm with gain g and bias b;
 //   cells: K rounded up to 256 columns; per 256-column cell and group of 24 tokens 240 rows of 128 bytes, row 24 d + t % 24 =
 //   digit d of token t (ten balanced base-9 digits, most significant first, as E2M1 codes);
 //   scale[t]: x_n = scale[t] * sum_d digit_d 9^(9-d)  (a power of two).
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, float eps, uint8_t* cells, float* scale, cudaStream_t st);
+void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st);
 
 // Per token and head of a chunk: RMSNorm (gains qn_g / kn_g, may be null) + rotate_half RoPE at position *posp + t on
 // q (in place) and k; k and v are written to the cache rows of their positions.
