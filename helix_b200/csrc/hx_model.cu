@@ -16,6 +16,7 @@
 #include "hx_gemm_tc.cuh"
 #include "hx_prefill.cuh"
 #include "hx_stage.cuh"
+#include "hx_gpt2_step.cuh"
 #include <fcntl.h>
 #include <sys/mman.h>
 #include <sys/stat.h>
@@ -89,13 +90,14 @@ struct hx_model {
     bool profile = false;
     std::vector<cudaEvent_t> prof_ev; std::vector<int> prof_cat; size_t prof_n = 0;
     hx_step_stats stats{};
-    std::vector<void*> allocs;
+    std::vector<void*> allocs; uint8_t* slab = nullptr; size_t slab_left = 0;
     uint64_t decode_bytes = 0, committed_bytes = 0;
     int kv_len = 0;
     // tensor parallel: cfg holds THIS RANK's shard dimensions (heads, kv heads, hidden, vocabulary slice); gcfg the model's
     hx_config gcfg{}; int tp_rank = 0, tp_world = 1;
     float* tp_buf = nullptr; size_t tp_buf_floats = 0; float* tp_peer[8] = {nullptr}; bool tp_connected = false; unsigned tp_launches = 0;
     float* x2 = nullptr; int tp_nbar = 0;
+    HxGpt2LayerDev* g2_layers = nullptr;           // GPT-2: layer table of the one-launch layers (null: per-op launches)
     // batched prefill (chunks of up to pf_tb tokens through the tcgen05 GEMM); buffers are created on first use
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
     int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
@@ -115,13 +117,25 @@ struct hx_model {
 
 namespace {
 
+// Device memory of a model.  Small buffers (gains, biases, scratch words: several hundred of them) are cut from slabs, since
+// an allocation of the driver's costs tens of microseconds whatever its size; `own`: an allocation of its own all the same.
 template <typename T>
-int dalloc(hx_model* m, T** p, size_t n) {
+int dalloc(hx_model* m, T** p, size_t n, bool own = false) {
+    constexpr size_t SMALL = 256 << 10, SLAB = 4 << 20;
+    const size_t bytes = n * sizeof(T) ? (n * sizeof(T) + 255) & ~(size_t)255 : 256;
+    const bool small = bytes <= SMALL && !own;
+    if (small && m->slab_left >= bytes) {
+        *p = (T*)m->slab;
+        m->slab += bytes; m->slab_left -= bytes;
+        return HX_OK;
+    }
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, n * sizeof(T) ? n * sizeof(T) : 16);
-    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(&q, n * sizeof(T) ? n * sizeof(T) : 16); }
-    if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
+    const size_t want = small ? SLAB : bytes;
+    cudaError_t e = cudaMalloc(&q, want);
+    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(&q, want); }
+    if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want, cudaGetErrorString(e));
     m->allocs.push_back(q);
+    if (small) { m->slab = (uint8_t*)q + bytes; m->slab_left = SLAB - bytes; }
     *p = (T*)q;
     return HX_OK;
 }
@@ -393,6 +407,16 @@ struct ProfScope {
     ~ProfScope() { if (on) { cudaEventRecord(m->prof_ev[m->prof_n + 1], m->st); m->prof_n += 2; } }
 };
 
+// ln_f and the tied lm_head of a GPT-2 token
+int enqueue_head_gpt2(hx_model* m, bool pdl, bool prof) {
+    HxLinear hd = lin(m->head, m->x, m->logits, HX_EPI_ARGMAX);
+    hd.norm = HX_NORM_LAYER; hd.norm_g = m->final_g; hd.norm_b = m->final_b; hd.eps = m->cfg.norm_eps;
+    hd.part_val = m->am_val; hd.part_idx = m->am_idx; hd.counter = m->am_cnt; hd.next_tok = m->d_tok; hd.pos_inc = m->d_pos;
+    hd.hist = m->d_hist;
+    ProfScope ps(m, CAT_GEMV, prof);
+    return hx_launch_linear(hd, m->st, pdl);
+}
+
 // Enqueue one token step on m->st.  from_prompt: the input token is d_prompt[*pos] and no logits are
 // computed (prefill); otherwise the input token is *d_tok and the head + arg-max run.
 // GPT-2 block sequencing (forward_layer_gpt2, helixc/runtime/gpt2_infer.c:1131-1193, with a KV cache): LayerNorm ->
@@ -426,17 +450,10 @@ int enqueue_step_gpt2(hx_model* m, bool from_prompt, bool with_head, bool prof) 
         HxLinear dn = lin(ly.down, m->h, m->x, HX_EPI_RESID); dn.resid = m->x; dn.bias = ly.b_down;
         { ProfScope ps(m, CAT_GEMV, prof); if ((rc = hx_launch_linear(dn, m->st, pdl))) return rc; }
     }
-    if (with_head) {
-        HxLinear hd = lin(m->head, m->x, m->logits, HX_EPI_ARGMAX);
-        hd.norm = HX_NORM_LAYER; hd.norm_g = m->final_g; hd.norm_b = m->final_b; hd.eps = c.norm_eps;
-        hd.part_val = m->am_val; hd.part_idx = m->am_idx; hd.counter = m->am_cnt; hd.next_tok = m->d_tok; hd.pos_inc = m->d_pos;
-        hd.hist = m->d_hist;
-        { ProfScope ps(m, CAT_GEMV, prof); if ((rc = hx_launch_linear(hd, m->st, pdl))) return rc; }
-    } else {
-        k_advance<<<1, 32, 0, m->st>>>(m->d_pos);
-        HX_COUNT_LAUNCH(1);
-        HX_CUDA(cudaGetLastError());
-    }
+    if (with_head) return enqueue_head_gpt2(m, pdl, prof);
+    k_advance<<<1, 32, 0, m->st>>>(m->d_pos);
+    HX_COUNT_LAUNCH(1);
+    HX_CUDA(cudaGetLastError());
     return HX_OK;
 }
 
@@ -445,6 +462,13 @@ int enqueue_step(hx_model* m, bool from_prompt, bool with_head, bool prof = fals
     const int DM = c.d_model, DH = c.head_dim, cap = m->kv_cap;
     const bool pdl = m->pdl && !prof;
     int rc;
+    if (m->g2_layers && !from_prompt && with_head && !prof) {      // GPT-2: all layers in one launch, then the head
+        HxGpt2Step s = {};
+        s.layers = m->g2_layers; s.n_layers = c.n_layers; s.emb = m->emb; s.wpe = m->wpe; s.tok = m->d_tok; s.pos = m->d_pos;
+        s.kc = m->kc; s.vc = m->vc; s.cap = cap; s.x_out = m->x; s.eps = c.norm_eps; s.scale = 1.0f / sqrtf((float)DH); s.err = m->d_err;
+        if ((rc = hx_gpt2_step_launch(s, DM, m->st, pdl))) return rc;
+        return enqueue_head_gpt2(m, pdl, false);
+    }
     {
         // the first kernel of a step follows the last kernel of the previous step
         const int* tok = from_prompt ? m->d_prompt : m->d_tok;
@@ -504,7 +528,7 @@ int capture(hx_model* m, bool from_prompt, bool with_head, cudaGraphExec_t* out)
     return HX_OK;
 }
 
-int kernels_per_step(const hx_model* m, bool with_head) { (void)with_head; return 1 + 6 * m->cfg.n_layers + 1; }
+int kernels_per_step(const hx_model* m, bool with_head) { return m->g2_layers && with_head ? 2 : 1 + 6 * m->cfg.n_layers + 1; }
 
 // Phase table of one token for the persistent kernel: per layer qkv, attention, o_proj, gate+up, down;
 // then (with_head) the lm_head.  from_prompt: layer 0 reads the token from the prompt array.
@@ -726,7 +750,7 @@ int init_persist(hx_model* m) {
         m->tp_pf_off = m->tp_buf_floats / 2;                                       // in pairs
         m->tp_pf_area = (size_t)HX_PF_TB * m->cfg.d_model;                         // pairs per slot
         m->tp_buf_floats += (size_t)2 * 2 * m->tp_world * m->tp_pf_area;
-        if ((rc = dalloc(m, &m->tp_buf, m->tp_buf_floats))) return rc;
+        if ((rc = dalloc(m, &m->tp_buf, m->tp_buf_floats, true))) return rc;      // (its handle is opened by the peers)
         HX_CUDA(cudaMemset(m->tp_buf, 0, m->tp_buf_floats * 4));
         m->tp_peer[m->tp_rank] = m->tp_buf;
     }
@@ -799,7 +823,7 @@ static void flags_enqueue(hx_model* m) {
     if (!m->h_flags && cudaMallocHost((void**)&m->h_flags, 16) != cudaSuccess) { (void)cudaGetLastError(); m->h_flags = nullptr; return; }
     m->h_flags[0] = m->h_flags[1] = 0;
     if (m->pf_err) cudaMemcpyAsync(&m->h_flags[0], m->pf_err, 4, cudaMemcpyDeviceToHost, m->st);
-    if (m->persist) cudaMemcpyAsync(&m->h_flags[1], m->d_err, 4, cudaMemcpyDeviceToHost, m->st);
+    if (m->d_err) cudaMemcpyAsync(&m->h_flags[1], m->d_err, 4, cudaMemcpyDeviceToHost, m->st);
     m->h_flags[2] = 1;       // fetched: valid after the next synchronize of the stream
 }
 
@@ -813,9 +837,10 @@ int persist_check(hx_model* m) {
         HX_CUDA(cudaMemcpy(&pe, m->pf_err, 4, cudaMemcpyDeviceToHost));
         if (pe) { cudaMemset(m->pf_err, 0, 4); return hx_fail(HX_ERR_TIMEOUT, "a bounded wait in the prefill GEMM ran out"); }
     }
-    if (!m->persist) return HX_OK;
+    if (!m->d_err) return HX_OK;
     int e = 0;
     HX_CUDA(cudaMemcpy(&e, m->d_err, 4, cudaMemcpyDeviceToHost));
+    if (e && !m->persist) { cudaMemset(m->d_err, 0, 16); return hx_fail(HX_ERR_TIMEOUT, "a bounded wait in the GPT-2 layer kernel ran out"); }
     if (e) {
         // every counter a launch leaves behind goes back to its idle value, so the next step starts clean (the pair
         // buffers need nothing: epochs only grow)
@@ -837,6 +862,21 @@ int finish_init(hx_model* m) {
         if (rc) return rc;
     }
     if (m->persist) return HX_OK;               // the per-op launch graphs belong to the graph engine alone
+    if (m->cfg.arch == 0 && hx_gpt2_step_fits(m->cfg, m->kv_cap)) {
+        std::vector<HxGpt2LayerDev> tab;
+        for (auto& ly : m->layers) {
+            HxGpt2LayerDev d = {};
+            const Fused* f[4] = {&ly.qkv, &ly.o, &ly.gu, &ly.down};
+            const float* b[4] = {ly.b_qkv, ly.b_o, ly.b_fc, ly.b_down};
+            for (int i = 0; i < 4; i++) { d.codes[i] = f[i]->codes; d.scales[i] = f[i]->scales; d.bias[i] = b[i]; d.ts[i] = f[i]->ts[0]; }
+            d.ln1g = ly.in_g; d.ln1b = ly.ln1_b; d.ln2g = ly.post_g; d.ln2b = ly.ln2_b;
+            tab.push_back(d);
+        }
+        if ((rc = dalloc(m, &m->d_err, (size_t)4))) return rc;
+        HX_CUDA(cudaMemset(m->d_err, 0, 16));
+        if ((rc = dalloc(m, &m->g2_layers, tab.size()))) return rc;
+        HX_CUDA(cudaMemcpy(m->g2_layers, tab.data(), tab.size() * sizeof(HxGpt2LayerDev), cudaMemcpyHostToDevice));
+    }
     rc = capture(m, false, true, &m->g_decode);
     if (rc && m->pdl) {     // programmatic edges not capturable on this driver: plain stream order
         m->pdl = false;

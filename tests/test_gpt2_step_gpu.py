@@ -1,0 +1,28 @@
+"""GPT-2 prompts through the chunk GEMM and tokens through the one-launch layer kernel (d_model 256, 512 and 768), against the
+fp32 CPU restatement: contexts around the kernel's passes of 128 keys, the first position, and the last of the cache."""
+import numpy as np
+import pytest
+
+import helix_b200 as hb
+from test_gpt2_gpu import OracleGpt2, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d_model,n_layers,T,cap", [(256, 3, 1, 40), (256, 2, 126, 136), (512, 2, 25, 40), (768, 2, 255, 262)])
+def test_prompt_then_tokens_match_checker(d_model, n_layers, T, cap):
+    shape = dict(n_layers=n_layers, d_model=d_model, n_heads=d_model // 64, d_ff=4 * d_model, vocab=517, max_ctx=cap)
+    wt = synth(shape, d_model + T)
+    om = OracleGpt2(shape, wt, cap)
+    gm = hb.Model.gpt2(shape, wt, kv_cap=cap)
+    ids = np.random.default_rng(T).integers(0, shape["vocab"], T).astype(np.int32)
+    for p in range(T):
+        want = om.decode(ids[p], p)
+    tok, lg = gm.prefill(ids, want_logits=True)
+    assert np.max(np.abs(lg - want)) < 2e-4 and tok == int(np.argmax(want))
+    for p in range(T, min(cap, T + 6)):
+        want = om.decode(tok, p)
+        tok, lg = gm.decode_step(tok, p, want_logits=True)
+        assert np.max(np.abs(lg - want)) < 2e-4, p
+        assert tok == int(np.argmax(want))
+    gm.close()
