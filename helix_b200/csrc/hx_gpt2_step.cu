@@ -227,17 +227,22 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 const float* kb = kc + (size_t)cta * P.cap * 64;
                 const float* vb = vc + (size_t)cta * P.cap * 64;
                 const int kp = tid & 3, c4 = tid & 15, kg = tid >> 4;
-                float4 kr[4], vr[4];
-                auto load_k = [&](int key) {
+                // Passes of 256 keys: a thread holds a quarter of two K rows, later a chunk of eight V rows.  The first pass of K
+                // travels while q is on its way, the first of V during the softmax.
+                float4 kr[8];
+                auto load_k = [&](int k0) {
 #pragma unroll
-                    for (int c = 0; c < 4; c++) kr[c] = key < pos ? __ldcg(reinterpret_cast<const float4*>(kb + (size_t)key * 64 + (kp + 4 * c) * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                };
-                auto load_v = [&](int key0) {
+                    for (int p = 0; p < 2; p++) {
+                        const int key = k0 + (tid >> 2) + 128 * p;
 #pragma unroll
-                    for (int i = 0; i < 4; i++) { const int key = key0 + 32 * i; vr[i] = key < pos ? __ldcg(reinterpret_cast<const float4*>(vb + (size_t)key * 64 + c4 * 4)) : make_float4(0.f, 0.f, 0.f, 0.f); }
+                        for (int c = 0; c < 4; c++) kr[4 * p + c] = key < pos ? __ldcg(reinterpret_cast<const float4*>(kb + (size_t)key * 64 + (kp + 4 * c) * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
                 };
-                load_k(tid >> 2);                                  // rows of the cache travel while q is on its way
-                load_v(kg);
+                auto load_v = [&](int k0) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) { const int key = k0 + kg + 32 * i; kr[i] = key < pos ? __ldcg(reinterpret_cast<const float4*>(vb + (size_t)key * 64 + c4 * 4)) : make_float4(0.f, 0.f, 0.f, 0.f); }
+                };
+                load_k(0);
                 if (tid < 192) {
                     const float x = g2_wait(&S.qkv[tid], ep, ab);
                     (tid < 64 ? S.q : (tid < 128 ? S.k : S.v))[tid & 63] = x;
@@ -250,20 +255,23 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 float* sc = S.xs;
                 float* pv = S.xs + G2_CAP;
                 float mx = -INFINITY;
-                for (int k0 = 0; k0 <= pos; k0 += 128) {
-                    const int key = k0 + (tid >> 2);
-                    if (k0 > 0) load_k(key);
-                    if (key == pos) {
+                for (int k0 = 0; k0 <= pos; k0 += 256) {
+                    if (k0 > 0) load_k(k0);
 #pragma unroll
-                        for (int c = 0; c < 4; c++) kr[c] = *reinterpret_cast<const float4*>(S.k + (kp + 4 * c) * 4);
+                    for (int p = 0; p < 2; p++) {
+                        const int key = k0 + (tid >> 2) + 128 * p;
+                        float d = 0.0f;
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const float4 k4 = key == pos ? *reinterpret_cast<const float4*>(S.k + (kp + 4 * c) * 4) : kr[4 * p + c];
+                            d = fmaf(q4[c].x, k4.x, d); d = fmaf(q4[c].y, k4.y, d); d = fmaf(q4[c].z, k4.z, d); d = fmaf(q4[c].w, k4.w, d);
+                        }
+                        d += __shfl_xor_sync(0xffffffffu, d, 1); d += __shfl_xor_sync(0xffffffffu, d, 2);
+                        d *= P.scale;
+                        if (key <= pos) { mx = fmaxf(mx, d); if (kp == 0) sc[key] = d; }
                     }
-                    float d = 0.0f;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) { d = fmaf(q4[c].x, kr[c].x, d); d = fmaf(q4[c].y, kr[c].y, d); d = fmaf(q4[c].z, kr[c].z, d); d = fmaf(q4[c].w, kr[c].w, d); }
-                    d += __shfl_xor_sync(0xffffffffu, d, 1); d += __shfl_xor_sync(0xffffffffu, d, 2);
-                    d *= P.scale;
-                    if (key <= pos) { mx = fmaxf(mx, d); if (kp == 0) sc[key] = d; }
                 }
+                load_v(0);
                 mx = hx_warp_max(mx);
                 if (lane == 0) S.red[2][warp] = mx;
                 g2_sync();
@@ -276,14 +284,14 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 if (lane == 0) S.red[3][warp] = ls;
                 g2_sync();
                 float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k0 = kg; k0 <= pos; k0 += 128) {
-                    if (k0 != kg) load_v(k0);
+                for (int k0 = 0; k0 <= pos; k0 += 256) {
+                    if (k0 > 0) load_v(k0);
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int key = k0 + 32 * i;
+                    for (int i = 0; i < 8; i++) {
+                        const int key = k0 + kg + 32 * i;
                         if (key > pos) break;
                         const float p = sc[key];
-                        const float4 v4 = key == pos ? *reinterpret_cast<const float4*>(S.v + c4 * 4) : vr[i];
+                        const float4 v4 = key == pos ? *reinterpret_cast<const float4*>(S.v + c4 * 4) : kr[i];
                         acc.x = fmaf(p, v4.x, acc.x); acc.y = fmaf(p, v4.y, acc.y); acc.z = fmaf(p, v4.z, acc.z); acc.w = fmaf(p, v4.w, acc.w);
                     }
                 }
