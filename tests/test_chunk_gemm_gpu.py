@@ -1,0 +1,36 @@
+"""The chunk GEMM's kinds (pairs of CTAs, clusters over K, K in several blocks, an odd number of row tiles) and the prompt
+attention at token counts around their groups of 24 and row tiles, through a prompt's logits and cached rows
+against the CPU restatement."""
+import numpy as np
+import pytest
+
+import helix_b200 as hb
+import oracle_lib as ol
+
+pytestmark = pytest.mark.gpu
+
+# K of 9 and 17 cells of 256 columns, 30 and 68 row tiles, a vocabulary of three tiles
+CFG = dict(NL=1, DM=2304, NH=18, NKV=6, DH=128, DFF=4352, NV=300)
+
+
+@pytest.fixture(scope="module")
+def model(tmp_path_factory):
+    path = str(tmp_path_factory.mktemp("chunk") / "m.weights")
+    ol.write_v3(path, CFG, ol.synth_tensors(CFG, seed=41))
+    return path
+
+
+@pytest.mark.parametrize("T", [1, 24, 25, 130])
+def test_prompt_logits_and_cache_rows(model, T):
+    om, gm = ol.OracleModel(model, kv_cap=T + 8), hb.Model.load(model, kv_cap=T + 8)
+    ids = np.random.default_rng(T).integers(0, CFG["NV"], T).astype(np.int32)
+    lo = om.prefill(ids)
+    nx, lg = gm.prefill(ids, want_logits=True)
+    assert np.max(np.abs(lo - lg)) < 2e-4 and nx == int(np.argmax(lo))
+    one = hb.Model.load(model, kv_cap=T + 8)                       # the same rows written token by token
+    for p in range(T):
+        one.decode_step(int(ids[p]), p)
+    for layer, head in ((0, 1), (0, 5)):
+        for a, b in zip(gm.kv_read(layer, head, 0, T), one.kv_read(layer, head, 0, T)):
+            assert np.max(np.abs(a - b)) < 1e-4 * max(1.0, float(np.max(np.abs(b))))
+    om.close(); gm.close(); one.close()
