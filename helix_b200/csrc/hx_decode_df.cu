@@ -46,6 +46,7 @@
 #define TM_D0 0                     // two accumulators of TC_NDIG columns
 #define TM_SFB 32                   // constant unit scales for the digit columns
 #define TM_SFA 64                   // + slot * 16 + K step * 4
+#define ATT_ROWS 160                // rows of an attention tile at most, and the stride of a head's probabilities
 #define EPI_WARPS 4                 // warps 0..3 own TMEM lanes 0..127 = the rows of a tile
 #define DRAIN_LIMIT (1u << 22)
 
@@ -110,12 +111,12 @@ struct SmemDf {
     uint64_t acc_full[2], acc_empty[2], b_ready;
     float red[NCW * 2];
     float att_m[8], att_l[8], att_r[8];
-    float wgt[2304];                // merge weights of the attention splits, [head][split] (o_proj prologue)
     float bv[NCW]; int bi[NCW];
     float swi[128];
     HxPhase ph[2];
     AttPlan ap; int att_ns, ap_tile_rows, ap_ntiles;      // attention work split of this launch (depends on the position only)
-    int tile_off[8], tile_slot[8];                        // ring slots of the attention tile in flight (K: 0.., V: 4..)
+    int tile_slot[8];                                     // ring slots of the attention tile in flight (K, then V)
+    int rowk[ATT_ROWS], rowv[ATT_ROWS];                   // where its rows lie
     unsigned ticket;
     uint32_t tmem_base;
     volatile int abort_flag; unsigned wait_limit;      // adjacent: bounded waits read the limit at (&abort_flag)[1]
@@ -234,74 +235,84 @@ __device__ __noinline__ AttPlan att_plan_df(const HxPersist& P, int cta, int pos
 // ------------------------------------------------------------------------------------------------
 // Attention phase of one CTA: (kv head, split of the cached positions); the split of the work depends on the
 // position only and is worked out once per launch (SmemDf::ap).  q (normed, rotated) and this position's k and v
-// arrive as pairs from the qkv epilogue; older rows stream through the ring from the cache.
-//  * scores: eight threads per (row, head), each holding its DH/8 query dimensions in registers, one shuffle
-//    tree per row;
+// arrive as pairs from the qkv epilogue; older rows stream through the ring from the cache in tiles of up to four slots.
+//  * scores: a warp takes four rows at a time against all heads of the group, eight lanes per row; the heads' sums are
+//    reduced across the eight lanes together (each exchange halves the values a lane carries);
 //  * soft-max statistics (online, m seeded -1e8 like the reference, fused_decode_attn_kernel.hx:74-102): one warp
 //    per head;
-//  * P*V: a thread owns four output dimensions of ALL heads of the group over a subset of the rows (a V row is read
-//    once, not once per head); the subsets are folded through shared memory.
-// The split's partial output and (max, sum) leave as pairs; the o_proj prologue merges the splits.
-// The phase runs once per layer from a cold instruction cache: loops stay rolled and waits have one site each.
+//  * P*V: a thread owns four output dimensions of ALL heads of the group over a contiguous run of the tile's rows, four
+//    rows per step (a V row and a vector of four probabilities are read once); the runs are folded through shared memory.
+// The split's partial output and (max, sum) leave as pairs; one CTA per head merges the splits.
+// What bounds it: the arithmetic of the two products for groups of eight heads at long contexts (228 rows x 8 heads: about
+// 4 us), latency below.  (A thread per (row, head, eighth), with the row looked up in every step, took 44 ns per row for
+// eight heads: 25 us of a 30 us phase at 4096 positions.)
 // ------------------------------------------------------------------------------------------------
-#define ATT_GP 8                       // stride of a row's probabilities (one float per head of the group, GRP <= 8)
 __device__ __forceinline__ void ring_adv(uint32_t& slot, uint32_t& par, uint32_t n, uint32_t nring) {
     slot += n;
     while (slot >= nring) { slot -= nring; par ^= 1u; }
 }
+// two pairs to a 16-byte aligned address (each of them is single-copy atomic)
+__device__ __forceinline__ void ll_st2(u64* p, float a, float b, unsigned ep) {
+    const u64 x = ((u64)ep << 32) | (u64)__float_as_uint(a), y = ((u64)ep << 32) | (u64)__float_as_uint(b);
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" :: "l"(p), "l"(x), "l"(y) : "memory");
+}
 // The splits of a head merged into the attention output, by one CTA per head: the CTA of (kv head, split s) takes
-// the heads s, s + ns, ... of its group once its own partial is out.  out[d] = sum_s w_s acc_s[d] with
-// w_s = exp(m_s - M) / sum_s l_s exp(m_s - M); splits are added in split order, so the result does not depend on
-// timing.  The o_proj phase then reads a plain vector.
-__device__ __noinline__ void attention_merge_df(const HxPersist& P, const HxPhase& ph, SmemDf& S, int kv, int split, int ns, int grp, unsigned ep) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int DH = ph.DH;
-    float* wm = S.wgt; float* wl = S.wgt + 1152;                  // ns <= 1152 (the host checks heads * splits <= 2304)
+// the heads s, s + ns, ... of its group once its own partial is out.  out[d] = sum_s w_s acc_s[d] / sum_s w_s l_s with
+// w_s = exp(m_s - M).  The threads form groups of DH / 2; group g polls the splits g, g + NG, ... -- their statistics and
+// its two dimensions in the same breath, so a merge costs one round trip -- and the groups are combined in order, so the
+// result does not depend on timing.  The o_proj phase then reads a plain vector.
+__device__ __noinline__ void attention_merge_df(const HxPersist& P, const HxPhase& ph, SmemDf& S, float4* sm, int kv, int split, int ns, int grp, unsigned ep) {
+    constexpr int SB = 5;
+    const int DH = ph.DH, H2 = DH >> 1, NG = NCT / H2;
+    const int tid = threadIdx.x, g = tid / H2, d2 = tid - g * H2;
     #pragma unroll 1
     for (int i = split; i < grp; i += ns) {
         const int h = kv * grp + i;
-        if (warp == 0) {
-            const u64* pml = ph.pml_ll + 2 * (size_t)h * ns;
-            float M = -INFINITY;
-            #pragma unroll 1
-            for (int s = lane; s < ns; s += 32) { float m, l; df_wait2(pml + 2 * s, ep, m, l, S, P); wm[s] = m; wl[s] = l; M = fmaxf(M, m); }
-            M = hx_warp_max(M);
-            float L = 0.0f;
-            #pragma unroll 1
-            for (int s = lane; s < ns; s += 32) { const float w = __expf(wm[s] - M); wm[s] = w; L = fmaf(wl[s], w, L); }
-            L = hx_warp_sum(L);
-            #pragma unroll 1
-            for (int s = lane; s < ns; s += 32) wm[s] = wm[s] / L;
-        }
-        consumer_sync();
-        constexpr int SB = 12;
+        const u64* pml = ph.pml_ll + 2 * (size_t)h * ns;
+        const u64* pa = ph.pacc_ll + (size_t)h * ns * DH + 2 * d2;
+        float M = -INFINITY, Ls = 0.0f, o0 = 0.0f, o1 = 0.0f;
         #pragma unroll 1
-        for (int d2 = tid; d2 < (DH >> 1); d2 += NCT) {
-            const u64* pa = ph.pacc_ll + (size_t)h * ns * DH + 2 * d2;
-            float o0 = 0.0f, o1 = 0.0f;
+        for (int s0 = g; s0 < ns; s0 += SB * NG) {
+            u64 w[SB][2], q[SB][2];
+            const unsigned lim = S.abort_flag ? 1u : S.wait_limit;
+            bool ok = false;
             #pragma unroll 1
-            for (int s0 = 0; s0 < ns; s0 += SB) {
-                const int n = min(SB, ns - s0);
-                u64 w[SB][2];
-                const unsigned lim = S.abort_flag ? 1u : S.wait_limit;
-                bool ok = false;
-                #pragma unroll 1
-                for (unsigned t = 0; t < lim && !ok; t++) {
+            for (unsigned t = 0; t < lim && !ok; t++) {
+                ok = true;
 #pragma unroll
-                    for (int c = 0; c < SB; c++) { w[c][0] = w[c][1] = 0; if (c < n) ll_ld2(pa + (size_t)(s0 + c) * DH, w[c][0], w[c][1]); }
-                    ok = true;
+                for (int c = 0; c < SB; c++) if (s0 + c * NG < ns) { ll_ld2(pml + 2 * (s0 + c * NG), q[c][0], q[c][1]); ll_ld2(pa + (size_t)(s0 + c * NG) * DH, w[c][0], w[c][1]); }
 #pragma unroll
-                    for (int c = 0; c < SB; c++) if (c < n) ok = ok && ll_ok(w[c][0], ep) && ll_ok(w[c][1], ep);
-                    if (!ok && (t & 63u) == 63u && df_gave_up(S, P)) break;
-                }
-                if (!ok) df_fail(S, P);
-#pragma unroll
-                for (int c = 0; c < SB; c++) if (c < n) { const float wg = wm[s0 + c]; o0 = fmaf(ll_val(w[c][0]), wg, o0); o1 = fmaf(ll_val(w[c][1]), wg, o1); }
+                for (int c = 0; c < SB; c++) if (s0 + c * NG < ns) ok = ok && ll_ok(q[c][0], ep) && ll_ok(q[c][1], ep) && ll_ok(w[c][0], ep) && ll_ok(w[c][1], ep);
+                if (!ok && (t & 63u) == 63u && df_gave_up(S, P)) break;
             }
-            ll_st(ph.out_ll + (size_t)h * DH + 2 * d2, o0, ep);
-            ll_st(ph.out_ll + (size_t)h * DH + 2 * d2 + 1, o1, ep);
+            if (!ok) df_fail(S, P);
+            float mx = M;
+#pragma unroll
+            for (int c = 0; c < SB; c++) if (s0 + c * NG < ns) mx = fmaxf(mx, ll_val(q[c][0]));
+            const float r = __expf(M - mx);
+            M = mx; Ls *= r; o0 *= r; o1 *= r;
+#pragma unroll
+            for (int c = 0; c < SB; c++) if (s0 + c * NG < ns) {
+                const float e = __expf(ll_val(q[c][0]) - M);
+                Ls = fmaf(e, ll_val(q[c][1]), Ls); o0 = fmaf(e, ll_val(w[c][0]), o0); o1 = fmaf(e, ll_val(w[c][1]), o1);
+            }
         }
-        consumer_sync();                                            // the weights are reused by the next head
+        sm[tid] = make_float4(M, Ls, o0, o1);
+        consumer_sync();
+        if (g == 0) {
+            float mx = -INFINITY;
+            #pragma unroll 1
+            for (int k = 0; k < NG; k++) mx = fmaxf(mx, sm[k * H2 + d2].x);
+            float L = 0.0f, a = 0.0f, b = 0.0f;
+            #pragma unroll 1
+            for (int k = 0; k < NG; k++) {
+                const float4 v = sm[k * H2 + d2];
+                const float e = __expf(v.x - mx);
+                L = fmaf(e, v.y, L); a = fmaf(e, v.z, a); b = fmaf(e, v.w, b);
+            }
+            ll_st2(ph.out_ll + (size_t)h * DH + 2 * d2, a / L, b / L, ep);
+        }
+        if (i + ns < grp) consumer_sync();                         // the scratch is reused by the next head
     }
 }
 
@@ -309,26 +320,21 @@ template <int GRP>
 __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph, SmemDf& S, uint8_t* ring, uint8_t* digb,
                                           uint32_t& cslot, uint32_t& cpar, int pi, int pos) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, cta = blockIdx.x;
-    (void)cta;
+    (void)cta; (void)pos;
     const int ns = S.att_ns;
     const AttPlan ap = S.ap;
     const int tr_rows = S.ap_tile_rows, ntiles = S.ap_ntiles;
     const unsigned ep = P.ep_base + (unsigned)pi + 1u, in_ep = P.ep_base + (unsigned)ph.in_dep + 1u;
-    const int DH = ph.DH, rps = ap.rows_per_slot, KVD = ph.NKV * DH;
+    const int DH = ph.DH, HD = GRP * DH, CPT = DH >> 5, CH4 = DH >> 2, NSUB = NCT / CH4;
+    constexpr int GP = GRP <= 1 ? 1 : (GRP <= 2 ? 2 : (GRP <= 4 ? 4 : 8)), LG = GP == 1 ? 0 : (GP == 2 ? 1 : (GP == 4 ? 2 : 3));
+    const int rps = ap.rows_per_slot, KVD = ph.NKV * DH;
     const uint32_t nring = RING_SLOTS;
-    float* sq = reinterpret_cast<float*>(digb);                 // [GRP][DH] queries
-    float* knew = sq + 8 * 256;                                  // [DH] current k
-    float* vnew = knew + 256;                                    // [DH] current v
-    float* sp = vnew + 256;                                      // [160 rows][ATT_GP] scores / probabilities
-    float* accx = sp + 160 * ATT_GP;                             // [row subset][GRP][DH] partial outputs
+    float* sq = reinterpret_cast<float*>(digb);                 // [GRP][128] queries, zero from DH on
+    float* knew = sq + 8 * 128;                                  // [DH] current k
+    float* vnew = knew + 128;                                    // [DH] current v
+    float* sp = vnew + 128;                                      // [GRP][ATT_ROWS] scores / probabilities; merge scratch
+    float* accx = sp + 8 * ATT_ROWS;                             // [row run][GRP][DH] partial outputs
     const float* ringf = reinterpret_cast<const float*>(ring);
-    const int HD = GRP * DH;
-    // score pass: thread = (row group, head, part of 8)
-    constexpr int TPR = GRP * 8, NRG = NCT / TPR;
-    const int a_rg = tid / TPR, a_i = (tid >> 3) % GRP, a_p = tid & 7;
-    const int CPT = DH >> 5;                                     // float4 chunks of a row per score thread
-    // P*V pass: thread = (row subset, float4 chunk of the head dimension), all heads of the group
-    const int CH4 = DH >> 2, NSUB = NCT / CH4;
     const int c_sub = tid / CH4, c_c = tid - c_sub * CH4;
     if (!ap.active) return;
     if (ap.t1 <= ap.t0) {
@@ -341,7 +347,7 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
             const int hs = (ap.kv * GRP + i / DH) * ns + ap.split;
             ll_st(ph.pacc_ll + (size_t)hs * DH + i % DH, 0.0f, ep);
         }
-        attention_merge_df(P, ph, S, ap.kv, ap.split, ns, GRP, ep);
+        attention_merge_df(P, ph, S, reinterpret_cast<float4*>(sp), ap.kv, ap.split, ns, GRP, ep);
         return;
     }
     float4 acc[GRP];
@@ -353,18 +359,17 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         #pragma unroll 1
         for (int i = tid; i < nq + 2 * nkv; i += NCT) {
             const u64* src; float* dst;
-            if (i < nq) { src = ph.in_ll + (size_t)ap.kv * HD + 2 * i; dst = sq + 2 * i; }
+            if (i < nq) { const int h = 2 * i / DH; src = ph.in_ll + (size_t)ap.kv * HD + 2 * i; dst = sq + h * 128 + 2 * i - h * DH; }
             else if (i < nq + nkv) { src = ph.kv_ll + (size_t)ap.kv * DH + 2 * (i - nq); dst = knew + 2 * (i - nq); }
             else { src = ph.kv_ll + (size_t)KVD + (size_t)ap.kv * DH + 2 * (i - nq - nkv); dst = vnew + 2 * (i - nq - nkv); }
             df_wait2(src, in_ep, dst[0], dst[1], S, P);
         }
     }
+    #pragma unroll 1
+    for (int i = tid; i < GRP * (128 - DH); i += NCT) sq[(i / (128 - DH)) * 128 + DH + i % (128 - DH)] = 0.0f;
     if (tid < 8) { S.att_m[tid] = -100000000.0f; S.att_l[tid] = 0.0f; }
     consumer_sync();
     DF_STAMP(7); DF_MARK(1);
-    float4 qf[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) qf[c] = (c < CPT && a_rg < NRG) ? *reinterpret_cast<const float4*>(sq + a_i * DH + (a_p + 8 * c) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int ntile = ntiles + ((ap.has_new && ap.n_old % tr_rows == 0) ? 1 : 0);
     #pragma unroll 1
     for (int s = 0; s < ntile; s++) {
@@ -373,34 +378,65 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         const int nsl = (nr + rps - 1) / rps;                       // ring slots of this tile (K, then as many of V)
         const bool add_new = ap.has_new && (s == ntile - 1);       // the current position rides on the last tile
         const int ntot = nr + (add_new ? 1 : 0);
-        // one thread per ring slot waits for the rows and publishes where they are: K slots 0.., V slots 4..
+        // where the rows lie (floats from the ring's base); one thread per ring slot waits for its rows
+        for (int r = tid; r < ntot; r += NCT) {
+            const int j = (r >= rps) + (r >= 2 * rps) + (r >= 3 * rps);
+            uint32_t ks = cslot + (uint32_t)j, vs = ks + (uint32_t)nsl;
+            while (ks >= nring) ks -= nring;
+            while (vs >= nring) vs -= nring;
+            S.rowk[r] = r < nr ? (int)(ks * (HX_RING_SLOT / 4)) + (r - j * rps) * DH : (int)(knew - ringf);
+            S.rowv[r] = r < nr ? (int)(vs * (HX_RING_SLOT / 4)) + (r - j * rps) * DH : (int)(vnew - ringf);
+        }
         if (tid < 2 * nsl) {
             uint32_t sl = cslot, pr = cpar;
             ring_adv(sl, pr, (uint32_t)tid, nring);
             mbar_wait(&S.full[sl], pr, &S.abort_flag);
-            S.tile_off[tid < nsl ? tid : 4 + tid - nsl] = (int)(sl * (HX_RING_SLOT / 4));
             S.tile_slot[tid] = (int)sl;
         }
         ring_adv(cslot, cpar, (uint32_t)(2 * nsl), nring);
         consumer_sync();
         if (s == 0) { DF_STAMP(8); DF_MARK(2); }
         // scores
-        const int nk = (ntot + NRG - 1) / NRG;
-        #pragma unroll 3
-        for (int k = 0; k < nk; k++) {
-            const int r = a_rg + k * NRG;
-            const bool valid = a_rg < NRG && r < ntot;
-            const int j = (r >= rps) + (r >= 2 * rps) + (r >= 3 * rps);
-            const float* kr = (valid && r < nr) ? ringf + S.tile_off[j] + (r - j * rps) * DH : knew;
-            float d0 = 0.0f, d1 = 0.0f;
+        {
+            const int p = lane & 7;
+            #pragma unroll 1
+            for (int r0 = warp * 4; r0 < ntot; r0 += NCW * 4) {
+                const int r = r0 + (lane >> 3);
+                const float* kr = ringf + S.rowk[min(r, ntot - 1)];
+                float4 k4[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) if (c < CPT) {
-                const float4 k4 = *reinterpret_cast<const float4*>(kr + (a_p + 8 * c) * 4);
-                d0 = fmaf(qf[c].x, k4.x, d0); d1 = fmaf(qf[c].y, k4.y, d1); d0 = fmaf(qf[c].z, k4.z, d0); d1 = fmaf(qf[c].w, k4.w, d1);
+                for (int c = 0; c < 4; c++) k4[c] = *reinterpret_cast<const float4*>((c < CPT ? kr : sq) + (p + 8 * c) * 4);     // narrow heads: zeros
+                float v[GP];
+#pragma unroll
+                for (int i = 0; i < GP; i++) {
+                    v[i] = 0.0f;
+                    if (i < GRP) {
+                        float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            const float4 q4 = *reinterpret_cast<const float4*>(sq + i * 128 + (p + 8 * c) * 4);
+                            d0 = fmaf(q4.x, k4[c].x, d0); d1 = fmaf(q4.y, k4[c].y, d1); d0 = fmaf(q4.z, k4[c].z, d0); d1 = fmaf(q4.w, k4[c].w, d1);
+                        }
+                        v[i] = d0 + d1;
+                    }
+                    if (i & 1) asm volatile("" ::: "memory");          // two heads' queries in registers at a time
+                }
+#pragma unroll
+                for (int st = 0; st < 3; st++) {
+                    const int o = 4 >> st;
+                    if (st < LG) {
+                        const int hh = GP >> (st + 1);
+                        const bool up = (lane & o) != 0;
+#pragma unroll
+                        for (int k = 0; k < hh; k++) {
+                            const float send = up ? v[k] : v[k + hh], keep = up ? v[k + hh] : v[k];
+                            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                        }
+                    } else v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                }
+                const int i = p >> (3 - LG);
+                if ((p & ((1 << (3 - LG)) - 1)) == 0 && i < GRP && r < ntot) sp[i * ATT_ROWS + r] = v[0] * ph.scale;
             }
-            float d = d0 + d1;
-            d += __shfl_xor_sync(0xffffffffu, d, 1); d += __shfl_xor_sync(0xffffffffu, d, 2); d += __shfl_xor_sync(0xffffffffu, d, 4);
-            if (valid && a_p == 0) sp[r * ATT_GP + a_i] = d * ph.scale;
         }
         consumer_sync();
         if (s == 0) DF_STAMP(9);
@@ -408,12 +444,15 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         // online softmax state per head
         if (warp < GRP) {
             const int i = warp;
-            float tm = -INFINITY;
-            for (int r = lane; r < ntot; r += 32) tm = fmaxf(tm, sp[r * ATT_GP + i]);
+            float* row = sp + i * ATT_ROWS;
+            float x[ATT_ROWS / 32], tm = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < ATT_ROWS / 32; k++) { x[k] = lane + 32 * k < ntot ? row[lane + 32 * k] : -INFINITY; tm = fmaxf(tm, x[k]); }
             tm = hx_warp_max(tm);
             const float mo = S.att_m[i], mn = fmaxf(mo, tm);
             float ls = 0.0f;
-            for (int r = lane; r < ntot; r += 32) { const float pr = __expf(sp[r * ATT_GP + i] - mn); sp[r * ATT_GP + i] = pr; ls += pr; }
+#pragma unroll
+            for (int k = 0; k < ATT_ROWS / 32; k++) if (lane + 32 * k < ntot) { const float pr = __expf(x[k] - mn); row[lane + 32 * k] = pr; ls += pr; }
             ls = hx_warp_sum(ls);
             if (lane == 0) { const float rr = __expf(mo - mn); S.att_r[i] = rr; S.att_l[i] = S.att_l[i] * rr + ls; S.att_m[i] = mn; }
         }
@@ -421,43 +460,55 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         if (s == 0) DF_STAMP(10);
         // P*V
         {
+            if (s > 0) {
 #pragma unroll
-            for (int i = 0; i < GRP; i++) { const float rr = S.att_r[i]; acc[i].x *= rr; acc[i].y *= rr; acc[i].z *= rr; acc[i].w *= rr; }
-            #pragma unroll 2
-            for (int r = c_sub; r < ntot; r += NSUB) {
-                const int j = (r >= rps) + (r >= 2 * rps) + (r >= 3 * rps);
-                const float* vr = (r < nr) ? ringf + S.tile_off[4 + j] + (r - j * rps) * DH : vnew;
-                const float4 v4 = *reinterpret_cast<const float4*>(vr + c_c * 4);
-                const float4 pa = *reinterpret_cast<const float4*>(sp + r * ATT_GP);
-                const float4 pb = GRP > 4 ? *reinterpret_cast<const float4*>(sp + r * ATT_GP + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float pw[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+                for (int i = 0; i < GRP; i++) { const float rr = S.att_r[i]; acc[i].x *= rr; acc[i].y *= rr; acc[i].z *= rr; acc[i].w *= rr; }
+            }
+            const int run = ((ntot + NSUB - 1) / NSUB + 3) & ~3, ra = c_sub * run, rb = min(ntot, ra + run);
+            #pragma unroll 1
+            for (int r = ra; r < rb; r += 4) {
+                float4 v4[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) v4[u] = r + u < rb ? *reinterpret_cast<const float4*>(ringf + S.rowv[r + u] + c_c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < GRP; i++) {
-                    acc[i].x = fmaf(pw[i], v4.x, acc[i].x); acc[i].y = fmaf(pw[i], v4.y, acc[i].y);
-                    acc[i].z = fmaf(pw[i], v4.z, acc[i].z); acc[i].w = fmaf(pw[i], v4.w, acc[i].w);
+                    const float4 p4 = *reinterpret_cast<const float4*>(sp + i * ATT_ROWS + r);
+                    const float pw[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) if (r + u < rb) {
+                        acc[i].x = fmaf(pw[u], v4[u].x, acc[i].x); acc[i].y = fmaf(pw[u], v4[u].y, acc[i].y);
+                        acc[i].z = fmaf(pw[u], v4[u].z, acc[i].z); acc[i].w = fmaf(pw[u], v4[u].w, acc[i].w);
+                    }
                 }
             }
+        }
+        if (s + 1 == ntile) {
+#pragma unroll
+            for (int i = 0; i < GRP; i++) *reinterpret_cast<float4*>(accx + (c_sub * GRP + i) * DH + c_c * 4) = acc[i];
         }
         consumer_sync();
         if (tid < nsl) mbar_arrive(&S.empty[S.tile_slot[nsl + tid]]);
     }
     DF_STAMP(11); DF_MARK(3);
-    // fold the row subsets and hand the split's partial over
-#pragma unroll
-    for (int i = 0; i < GRP; i++) *reinterpret_cast<float4*>(accx + (c_sub * GRP + i) * DH + c_c * 4) = acc[i];
-    consumer_sync();
+    // fold the row runs and hand the split's partial over
     #pragma unroll 1
-    for (int hd = tid; hd < HD; hd += NCT) {
-        const int i = hd / DH, d = hd - i * DH;
-        float O = 0.0f;
-        for (int u = 0; u < NSUB; u++) O += accx[(u * GRP + i) * DH + d];
+    for (int o = tid; o < GRP * CH4; o += NCT) {
+        const int i = o / CH4, c = o - i * CH4;
+        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+        #pragma unroll 1
+        for (int u = 0; u < NSUB; u++) {
+            const float4 a = *reinterpret_cast<const float4*>(accx + (u * GRP + i) * DH + c * 4);
+            O.x += a.x; O.y += a.y; O.z += a.z; O.w += a.w;
+        }
         const int hs = (ap.kv * GRP + i) * ns + ap.split;
-        ll_st(ph.pacc_ll + (size_t)hs * DH + d, O, ep);
-        if (d == 0) { ll_st(ph.pml_ll + 2 * hs, S.att_m[i], ep); ll_st(ph.pml_ll + 2 * hs + 1, S.att_l[i], ep); }
+        u64* dst = ph.pacc_ll + (size_t)hs * DH + c * 4;
+        ll_st2(dst, O.x, O.y, ep); ll_st2(dst + 2, O.z, O.w, ep);
+        if (c == 0) ll_st2(ph.pml_ll + 2 * hs, S.att_m[i], S.att_l[i], ep);
     }
     DF_MARK(4);
-    attention_merge_df(P, ph, S, ap.kv, ap.split, ns, GRP, ep);
+    attention_merge_df(P, ph, S, reinterpret_cast<float4*>(sp), ap.kv, ap.split, ns, GRP, ep);
 }
+
 
 template <bool TP>
 __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxPersist P) {
@@ -978,7 +1029,7 @@ size_t df_smem_fixed(int bdig_bytes) {
 
 // Shared-memory scratch of the attention phase for a group of `grp` query heads per kv head (queries, the position's k
 // and v, probabilities, partial outputs of the row subsets); the digit columns share the space.
-int hx_decode_df_att_bytes(int grp) { return (8 * 256 + 256 + 256 + 160 * ATT_GP + NCT * 4 * grp) * 4; }
+int hx_decode_df_att_bytes(int grp) { return (8 * 128 + 128 + 128 + 8 * ATT_ROWS + NCT * 4 * grp) * 4; }
 
 // Ring depth that fits beside the digit columns (0 = does not fit).
 int hx_decode_df_ring(int bdig_bytes) {

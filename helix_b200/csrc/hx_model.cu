@@ -701,12 +701,12 @@ int init_persist(hx_model* m) {
     if (const char* e = getenv("HX_ATT_SPLIT")) { const int v = atoi(e); if (v >= 1 && v <= m->nsplit_persist) m->nsplit_persist = v; }
     if (256 % m->cfg.head_dim) return hx_fail(HX_ERR_ARG, "persistent decode needs head_dim dividing 256");
     int rc;
-    {   // the dataflow engine needs the fused qkv epilogue (whole heads per tile) and room for the split weights
+    {   // the dataflow engine needs the fused qkv epilogue (whole heads per tile)
         const hx_config& c = m->cfg;
         const char* sy = getenv("HX_SYNC");
         const bool fuse_qk = c.head_dim == 32 || c.head_dim == 64 || c.head_dim == 128;
         // (the prologue polls at most 64 per-tile sums of squares: d_model up to 8192)
-        m->use_df = m->use_tc && fuse_qk && (size_t)c.n_heads * m->nsplit_persist <= 2304 && c.d_model <= 8192 && !(sy && strcmp(sy, "barrier") == 0);
+        m->use_df = m->use_tc && fuse_qk && c.d_model <= 8192 && !(sy && strcmp(sy, "barrier") == 0);
     }
     if (m->tp_world > 1 && !m->use_df) m->pf_batched = false;       // the chunk exchange of a shard belongs to the pair engine
     if (m->use_df) {
