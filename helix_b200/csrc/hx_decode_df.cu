@@ -115,8 +115,7 @@ struct SmemDf {
     float swi[128];
     HxPhase ph[2];
     AttPlan ap; int att_ns, ap_tile_rows, ap_ntiles;      // attention work split of this launch (depends on the position only)
-    int tile_slot[8];                                     // ring slots of the attention tile in flight (K, then V)
-    int rowk[ATT_ROWS], rowv[ATT_ROWS];                   // where its rows lie
+    int rowk[ATT_ROWS], rowv[ATT_ROWS];                   // where the rows of the attention tile in flight lie
     unsigned ticket;
     uint32_t tmem_base;
     volatile int abort_flag; unsigned wait_limit;      // adjacent: bounded waits read the limit at (&abort_flag)[1]
@@ -190,26 +189,6 @@ __device__ __forceinline__ void df_wait2(const u64* p, unsigned ep, float& a, fl
     df_fail(S, P);
     a = ll_val(x); b = ll_val(y);
 }
-// Eight consecutive pairs at a 16-byte aligned address (one item of the digit prologue).
-__device__ __forceinline__ void df_wait8(const u64* p, unsigned ep, float (&v)[8], SmemDf& S, const HxPersist& P) {
-    const unsigned lim = S.abort_flag ? 1u : S.wait_limit;
-    u64 w[8];
-#pragma unroll
-    for (int e = 0; e < 8; e++) w[e] = 0;
-    bool ok = false;
-    for (unsigned i = 0; i < lim && !ok; i++) {
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) ll_ld2(p + e, w[e], w[e + 1]);
-        ok = true;
-#pragma unroll
-        for (int e = 0; e < 8; e++) ok = ok && ll_ok(w[e], ep);
-        if (!ok && (i & 63u) == 63u && df_gave_up(S, P)) break;
-    }
-    if (!ok) df_fail(S, P);
-#pragma unroll
-    for (int e = 0; e < 8; e++) v[e] = ll_val(w[e]);
-}
-
 // ---- attention work split: the number of splits follows the context length (about 64 positions each) ----
 __device__ __noinline__ AttPlan att_plan_df(const HxPersist& P, int cta, int pos, int nring, int* ns_out, int* tile_rows, int* ntiles) {
 #ifndef DF_SPLIT_ROWS_LOG2
@@ -378,6 +357,7 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         const int nsl = (nr + rps - 1) / rps;                       // ring slots of this tile (K, then as many of V)
         const bool add_new = ap.has_new && (s == ntile - 1);       // the current position rides on the last tile
         const int ntot = nr + (add_new ? 1 : 0);
+        uint32_t myslot = 0;
         // where the rows lie (floats from the ring's base); one thread per ring slot waits for its rows
         for (int r = tid; r < ntot; r += NCT) {
             const int j = (r >= rps) + (r >= 2 * rps) + (r >= 3 * rps);
@@ -391,7 +371,7 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
             uint32_t sl = cslot, pr = cpar;
             ring_adv(sl, pr, (uint32_t)tid, nring);
             mbar_wait(&S.full[sl], pr, &S.abort_flag);
-            S.tile_slot[tid] = (int)sl;
+            myslot = sl;
         }
         ring_adv(cslot, cpar, (uint32_t)(2 * nsl), nring);
         consumer_sync();
@@ -440,7 +420,7 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         }
         consumer_sync();
         if (s == 0) DF_STAMP(9);
-        if (tid < nsl) mbar_arrive(&S.empty[S.tile_slot[tid]]);
+        if (tid < nsl) mbar_arrive(&S.empty[myslot]);
         // online softmax state per head
         if (warp < GRP) {
             const int i = warp;
@@ -487,7 +467,7 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
             for (int i = 0; i < GRP; i++) *reinterpret_cast<float4*>(accx + (c_sub * GRP + i) * DH + c_c * 4) = acc[i];
         }
         consumer_sync();
-        if (tid < nsl) mbar_arrive(&S.empty[S.tile_slot[nsl + tid]]);
+        if (tid >= nsl && tid < 2 * nsl) mbar_arrive(&S.empty[myslot]);
     }
     DF_STAMP(11); DF_MARK(3);
     // fold the row runs and hand the split's partial over
@@ -718,7 +698,9 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                     }
                     // A unit is two consecutive elements (one 16-byte load), so a warp's load is 512 contiguous bytes.  UI
                     // units per thread and round are in flight together, with the norm gains fetched before the wait and,
-                    // in the first round of warp 0, the per-tile sums of squares polled in the same breath.
+                    // in the first round of warp 0, the per-tile sums of squares polled in the same breath.  A poll asks only
+                    // for what has not come yet: the tiles arrive over a microsecond or two, and 148 CTAs asking for the whole
+                    // vector again and again (4.8 MB a round at K = 4096) would keep L2 busy for longer than a round trip.
                     constexpr int UI = 8;
                     const int nunits = nitems * 4;
                     #pragma unroll 1
@@ -742,9 +724,10 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                             #pragma unroll 1
                             for (unsigned t = 0; t < lim && !ok; t++) {
 #pragma unroll
-                                for (int j = 0; j < UI; j++) if (kk[j] >= 0) ll_ld2(ph.in_ll + kk[j], w[j][0], w[j][1]);
-                                if (st_a) sa = ll_ld(ph.in_stat + lane);
-                                if (st_b) sb = ll_ld(ph.in_stat + lane + 32);
+                                for (int j = 0; j < UI; j++)
+                                    if (kk[j] >= 0 && !(ll_ok(w[j][0], in_ep) && ll_ok(w[j][1], in_ep))) ll_ld2(ph.in_ll + kk[j], w[j][0], w[j][1]);
+                                if (st_a && !ll_ok(sa, in_ep)) sa = ll_ld(ph.in_stat + lane);
+                                if (st_b && !ll_ok(sb, in_ep)) sb = ll_ld(ph.in_stat + lane + 32);
                                 ok = (!st_a || ll_ok(sa, in_ep)) && (!st_b || ll_ok(sb, in_ep));
 #pragma unroll
                                 for (int j = 0; j < UI; j++) if (kk[j] >= 0) ok = ok && ll_ok(w[j][0], in_ep) && ll_ok(w[j][1], in_ep);
