@@ -34,7 +34,8 @@
 #define NCW 8
 #endif
 #define NCT (NCW * 32)
-#define PT (NCT + 64)               // + producer warp (16) + MMA warp (17)
+#define NMW 2                       // MMA warps
+#define PT (NCT + 32 + NMW * 32)    // + producer warp + MMA warps
 // mbar_wait (hx_persist_common.cuh) reads its limit from the word after the abort flag it is given
 #define WAIT_LIMIT (reinterpret_cast<volatile unsigned*>(abort_flag)[1])
 #include "hx_persist.cuh"
@@ -43,9 +44,9 @@
 
 #define TC_NDIG 16
 #define TM_COLS 256
-#define TM_D0 0                     // two accumulators of TC_NDIG columns
-#define TM_SFB 32                   // constant unit scales for the digit columns
-#define TM_SFA 64                   // + slot * 16 + K step * 4
+#define TM_D0 0                     // accumulators of TC_NDIG columns: two pieces in flight, one per MMA warp
+#define TM_SFB 64                   // constant unit scales for the digit columns, + MMA warp * 4
+#define TM_SFA 96                   // + slot * 16 + K step * 4
 #define ATT_ROWS 160                // rows of an attention tile at most, and the stride of a head's probabilities
 #define EPI_WARPS 4                 // warps 0..3 own TMEM lanes 0..127 = the rows of a tile
 #define DRAIN_LIMIT (1u << 22)
@@ -59,7 +60,7 @@ typedef unsigned long long u64;
 #define DF_GT(v) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v))
 #define DF_MMA_T0() unsigned long long _w0; DF_GT(_w0)
 #define DF_MMA_T1() do { unsigned long long _w1; DF_GT(_w1); dbg_wait += _w1 - _w0; } while (0)
-#define DF_MMA_OUT() do { if (P.dbg_all) { unsigned long long _t; DF_GT(_t); P.dbg_all[((size_t)pi * gridDim.x + blockIdx.x) * 8 + 7] = _t; P.dbg_all[((size_t)pi * gridDim.x + blockIdx.x) * 8 + 6] = dbg_wait; } } while (0)
+#define DF_MMA_OUT() do { if (P.dbg_all && mw == 0) { unsigned long long _t; DF_GT(_t); P.dbg_all[((size_t)pi * gridDim.x + blockIdx.x) * 8 + 7] = _t; P.dbg_all[((size_t)pi * gridDim.x + blockIdx.x) * 8 + 6] = dbg_wait; } } while (0)
 #else
 #define DF_STAMP(i) do { } while (0)
 #define DF_MARK(ev) do { } while (0)
@@ -94,6 +95,7 @@ __device__ __forceinline__ bool tc_elect() {
 }
 // A wait of the whole warp: every lane gets the same answer, so the warp leaves a loop together.
 __device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, mbar_try(b, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait(b, parity, abort_flag));
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 2, %0;" :: "n"(EPI_WARPS * 32) : "memory"); }
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
 
     if (tid == 0) {
         for (int i = 0; i < HX_TC_MAX_RING; i++) { mbar_init(&S.full[i], 1); mbar_init(&S.empty[i], 1); }
-        mbar_init(&S.acc_full[0], 1); mbar_init(&S.acc_full[1], 1);
+        mbar_init(&S.acc_full[0], NMW); mbar_init(&S.acc_full[1], NMW);
         mbar_init(&S.acc_empty[0], EPI_WARPS); mbar_init(&S.acc_empty[1], EPI_WARPS);
         mbar_init(&S.b_ready, 1);
         S.abort_flag = 0; S.wait_limit = P.wait_limit;
@@ -587,13 +589,18 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                 for (uint32_t i = 0; i < DRAIN_LIMIT; i++) if (mbar_try(&S.full[s], pr)) break;
             }
         }
-    } else if (warp == NCW + 1) {
-        // =========================== MMA issuer ===========================
+    } else if (warp > NCW) {
+        // =========================== MMA issuers ===========================
+        // Two warps: what one cell costs its issuer -- wait for the ring slot, copies, MMAs, commit -- is about 700 cycles of
+        // latencies one after the other, against 350 on the tensor pipe, so with a single warp the cells that lay in the
+        // ring already went by at 0.37 us each.  A warp takes the cells of the ring slots of its parity (so it sees every use
+        // of a slot that it waits for) into its own accumulator; the read-out adds the two.
         // The whole warp runs the loop and one elected lane issues: with the control flow convergent, descriptors and
         // addresses stay in uniform registers.  A single-thread branch (lane == 0) makes the compiler move every operand
         // over for each instruction: 170 cycles per MMA (with its scale copy) against 87 at N = 16.
         {
-            if (tc_elect()) tc_cp_sf(tmem + TM_SFB, tc_desc(smem_u32(sfb1), 16, 128));
+            const uint32_t mw = (uint32_t)(warp - NCW - 1), sfb = tmem + TM_SFB + mw * 4;
+            if (tc_elect()) tc_cp_sf(sfb, tc_desc(smem_u32(sfb1), 16, 128));
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(TC_NDIG >> 3) << 17) | (8u << 24);
             const uint64_t a_ring = tc_desc(smem_u32(ring), 16, 1024, TC_SW128);    // 8-row groups 1024 B apart, 128-byte swizzle
             const uint64_t sf_ring = tc_desc(smem_u32(ring) + 16384, 16, 128);
@@ -612,7 +619,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     unsigned long long dbg_wait = 0; (void)dbg_wait;
                     int kc = tp.k0, dp = 0;              // K cell of the tile, its position among the digit cells
-                    bool fresh = true;
+                    bool fresh = true, first = true;     // at the start of a piece; before this warp's first cell of it
                     uint32_t dcol = 0;
 #pragma unroll 1
                     for (int g = tp.b0; g < tp.b1 && ok; g++) {
@@ -620,28 +627,35 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                             const uint32_t buf = uc & 1u;
                             if (uc >= 2) ok = warp_wait(&S.acc_empty[buf], ((uc >> 1) - 1) & 1, &S.abort_flag);
                             if (!ok) break;
-                            dcol = tmem + TM_D0 + buf * TC_NDIG;
+                            dcol = tmem + TM_D0 + (buf * NMW + mw) * TC_NDIG;
+                            first = true;
                         }
-                        { DF_MMA_T0(); ok = warp_wait(&S.full[slot], par, &S.abort_flag); DF_MMA_T1(); }
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        // descriptors advance in 16-byte units: a K step is 32 B of a swizzled row, a scale chunk 512 B
-                        const uint64_t a_slot = a_ring + (uint64_t)(slot * (HX_RING_SLOT >> 4));
-                        const uint64_t sf_slot = sf_ring + (uint64_t)(slot * (HX_RING_SLOT >> 4));
-                        const uint64_t b_cell = b_base + (uint64_t)(dp * 128);
-                        const uint32_t tsf = tmem + TM_SFA + slot * 16;
                         const bool last = kc + 1 == tp.C || g + 1 == tp.b1;      // last cell of this tile's piece
-                        if (tc_elect()) {
+                        if ((slot & 1u) == mw) {
+                            { DF_MMA_T0(); ok = warp_wait(&S.full[slot], par, &S.abort_flag); DF_MMA_T1(); }
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            // descriptors advance in 16-byte units: a K step is 32 B of a swizzled row, a scale chunk 512 B
+                            const uint64_t a_slot = a_ring + (uint64_t)(slot * (HX_RING_SLOT >> 4));
+                            const uint64_t sf_slot = sf_ring + (uint64_t)(slot * (HX_RING_SLOT >> 4));
+                            const uint64_t b_cell = b_base + (uint64_t)(dp * 128);
+                            const uint32_t tsf = tmem + TM_SFA + slot * 16;
+                            if (tc_elect()) {
 #pragma unroll
-                            for (int e = 0; e < 4; e++) tc_cp_sf(tsf + e * 4, sf_slot + (uint64_t)(e * 32));
+                                for (int e = 0; e < 4; e++) tc_cp_sf(tsf + e * 4, sf_slot + (uint64_t)(e * 32));
 #pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                tc_mma(dcol, a_slot + (uint64_t)(e * 2), b_cell + (uint64_t)(e * 2), idesc, tsf + e * 4, tmem + TM_SFB,
-                                       (fresh && e == 0) ? 0u : 1u);
-                            tc_commit(&S.empty[slot]);
-                            if (last) tc_commit(&S.acc_full[uc & 1u]);
+                                for (int e = 0; e < 4; e++)
+                                    tc_mma(dcol, a_slot + (uint64_t)(e * 2), b_cell + (uint64_t)(e * 2), idesc, tsf + e * 4, sfb,
+                                           (first && e == 0) ? 0u : 1u);
+                                tc_commit(&S.empty[slot]);
+                            }
+                            __syncwarp();
+                            first = false;
                         }
-                        __syncwarp();
+                        if (last) {
+                            if (tc_elect()) tc_commit(&S.acc_full[uc & 1u]);     // arrives at once where this warp had no cell
+                            __syncwarp();
+                        }
                         fresh = last;
                         if (++slot == nring) { slot = 0; par ^= 1u; }
                         if (++dp == tp.C) dp = 0;
@@ -793,6 +807,8 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                 DF_STAMP(1); DF_MARK(2);
 
                 // ---------- pieces of tiles: accumulator -> digits recombined -> merge -> epilogue ----------
+                uint32_t pslot = cslot;                    // ring slot of the first cell of a piece
+                int pleft = tp.b1 - tp.b0, pk = tp.k0;     // cells left, first K cell of the piece
                 ring_adv(cslot, cpar, (uint32_t)(tp.b1 - tp.b0), nring);
                 const int t_first = tp.t_first, t_last = tp.t_last;
                 if (warp < EPI_WARPS) {
@@ -802,6 +818,12 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
 #pragma unroll 1
                     for (int tile = t_first; tile <= t_last; tile++) {
                         const uint32_t buf = uc & 1u;
+                        // the MMA warps that had a cell of this piece (both from three cells on: two neighbours are of one
+                        // parity only where an odd ring wraps)
+                        const int pn = min(tp.C - pk, pleft);
+                        const uint32_t pnext = pslot + 1 == nring ? 0u : pslot + 1;
+                        const bool had0 = pn > 2 || !(pslot & 1u) || (pn == 2 && !(pnext & 1u)), had1 = pn > 2 || (pslot & 1u) || (pn == 2 && (pnext & 1u));
+                        pslot = (pslot + (uint32_t)pn) % nring; pleft -= pn; pk = 0;
                         // the CTA holding a tile's first cell merges it (see HxCtaPlan)
                         const bool merger = tile > t_first || tp.first_merger;
                         const int others = tile == t_last ? tp.last_others : 0;
@@ -821,19 +843,25 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                         uc++;
                         if (tile == t_last) DF_MARK(3);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        uint32_t r[16];
-                        const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + TM_D0 + buf * TC_NDIG;
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                                       "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                                     : "r"(ta));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        float v = 0.0f;
+#pragma unroll
+                        for (int h = 0; h < NMW; h++) {
+                            if (h == 0 ? !had0 : !had1) continue;
+                            uint32_t r[16];
+                            const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + TM_D0 + (buf * NMW + h) * TC_NDIG;
+                            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                                           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                                         : "r"(ta));
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            float a = 0.0f;
+#pragma unroll
+                            for (int j = TC_NDIG - 1; j >= 0; j--) a = fmaf(a, 0.25f, __uint_as_float(r[j]));
+                            v += a;
+                        }
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&S.acc_empty[buf]);
-                        float v = 0.0f;
-#pragma unroll
-                        for (int j = TC_NDIG - 1; j >= 0; j--) v = fmaf(v, 0.25f, __uint_as_float(r[j]));
                         v *= out_scale;
                         if (!merger) {            // pieces 1.. hand their rows to the merger
                             ll_st(ph.part_ll + ((size_t)tile * ph.pieces + (size_t)tp.first_piece) * 128 + rl, v, ep);
