@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
 #pragma unroll
                     for (int e = 0; e < 8; e++) {
                         M[e] = __float2uint_rn(fabsf(v[e]) * mul);
-                        sg |= (v[e] < 0.0f ? 8u : 0u) << (4 * e);
+                        sg |= (__float_as_uint(v[e]) >> (28 - 4 * e)) & (8u << (4 * e));
                     }
                     // digit n of element e is bits 31-2n, 30-2n of M[e]; it lands on bits 4e+1, 4e of the word of row n
                     const int j = (it >> 2) & 7, w = it & 3;               // 16-byte chunk and word of this item in its cell
