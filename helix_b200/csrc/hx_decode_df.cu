@@ -28,7 +28,7 @@
 // the arithmetic runs on whatever is there) and the phase boundary decides with a barrier-wide OR, so all
 // threads leave together through the common exit, which waits for the CTA's own bulk copies in flight
 // and frees its tensor memory.  The host reports HX_ERR_TIMEOUT.
-#define HX_TC_MAX_RING 10
+#define HX_TC_MAX_RING 12
 #define RING_SLOTS ((uint32_t)P.tc_ring)
 #ifndef NCW
 #define NCW 8
@@ -43,7 +43,7 @@
 #include "hx_gemm_tc.cuh"
 
 #define TC_NDIG 16
-#define TM_COLS 256
+#define TM_COLS 512
 #define TM_D0 0                     // accumulators of TC_NDIG columns: two pieces in flight, one per MMA warp
 #define TM_SFB 64                   // constant unit scales for the digit columns, + MMA warp * 4
 #define TM_SFA 96                   // + slot * 16 + K step * 4
@@ -688,8 +688,8 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                              "l"(reinterpret_cast<const uint4*>(P.phases + pi + 1) + tid) : "memory");
             if (ph.type == HX_PH_LINEAR_TC) {
                 // ---------- prologue: x -> (norm) -> sixteen base-4 digit columns in operand layout ----------
-                // Pass 1 stages the CTA's K slice of the input (times the norm gain) in shared memory behind the digit
-                // cells and finds its largest magnitude; pass 2 turns the staged values into digit words.  The code runs
+                // Pass 1 stages the CTA's K slice of the input (times the norm gain) in the first half of each digit
+                // cell and finds its largest magnitude; pass 2 turns the staged values into digit words.  The code runs
                 // once per phase from a cold instruction cache, so it is kept small: one polling site, one digit site.
                 const int K = ph.K;
                 const HxCtaPlan tp = ph.plan[cta];
@@ -698,7 +698,6 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                 // layer 0: the embedding row of the token is the input of qkv and the residual of o_proj
                 const float* xrow = ph.tok ? ph.x + (size_t)(ph.tok[P.tok_by_pos ? pos : 0]) * (size_t)ph.res_ld : ph.x;
                 const int nitems = tp.run * 32;
-                float* xs = reinterpret_cast<float*>(digb + (size_t)tp.run * 2048);
                 float ss = 0.0f, mx = 0.0f;
                 {
                     // Sum of squares of the whole input: per-tile sums published by the producing epilogue, added in tile
@@ -763,7 +762,7 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                             if (u >= nunits) continue;
                             const float v0 = kk[j] >= 0 ? ll_val(w[j][0]) * gg[j].x : 0.0f, v1 = kk[j] >= 0 ? ll_val(w[j][1]) * gg[j].y : 0.0f;
                             mx = fmaxf(mx, fmaxf(fabsf(v0), fabsf(v1)));
-                            *reinterpret_cast<float2*>(xs + u * 2) = make_float2(v0, v1);
+                            *reinterpret_cast<float2*>(digb + (size_t)(u >> 7) * 2048 + (u & 127) * 8) = make_float2(v0, v1);
                         }
                     }
                 }
@@ -784,7 +783,9 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                 const float mul = (inv / Sg) * 2147483648.0f;             // |x_n| / Sg * 2^31 < 2^32
                 #pragma unroll 1
                 for (int it = tid; it < nitems; it += NCT) {
-                    const float4 va = *reinterpret_cast<const float4*>(xs + it * 8), vb = *reinterpret_cast<const float4*>(xs + it * 8 + 4);
+                    const float4* xs = reinterpret_cast<const float4*>(digb + (size_t)(it >> 5) * 2048 + (it & 31) * 32);
+                    const float4 va = xs[0], vb = xs[1];
+                    __syncwarp();                                          // a warp turns a whole cell over: read, then written
                     const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
                     uint32_t M[8]; uint32_t sg = 0u;
 #pragma unroll

@@ -561,8 +561,7 @@ int build_phases(hx_model* m, bool from_prompt, bool with_head, HxPhase** out, i
             p.pieces = maxp;
             if ((size_t)p.ntiles * maxp > m->tc_units_max) m->tc_units_max = (size_t)p.ntiles * maxp;
             if (p.ntiles > m->tc_tiles_max) m->tc_tiles_max = p.ntiles;
-            const int per_cell = m->use_df ? 3072 : 2048;       // digit cells (+ the staged input values of the dataflow engine)
-            if (maxrun * per_cell > m->bdig_bytes) m->bdig_bytes = maxrun * per_cell;
+            if (maxrun * 2048 > m->bdig_bytes) m->bdig_bytes = maxrun * 2048;
         }
         p.N = N; p.x = x; p.K = f.K; p.norm = HX_NORM_NONE; p.epi = epi; p.y = y;
         p.ts[0] = f.ts[0]; p.ts[1] = f.ts[1]; p.ts[2] = f.ts[2]; p.bound0 = f.bound0; p.bound1 = f.bound1;
@@ -601,12 +600,6 @@ int build_phases(hx_model* m, bool from_prompt, bool with_head, HxPhase** out, i
             const int i_att = (int)v.size(); v.push_back(at);
             HxPhase o = linear(ly.o, nullptr, nullptr, HX_EPI_RESID, ly.o.N);
             o.in_ll = m->ctxll; o.in_dep = i_att;
-            {   // the CTA's K slice of the input is staged in shared memory behind its digit cells
-                int maxp = 1, maxrun = 1;
-                std::vector<HxCtaPlan> tab((size_t)m->grid_persist);
-                hx_df_plan(o.ntiles, o.ksteps / 4, m->grid_persist, tab.data(), &maxp, &maxrun);
-                if (maxrun * 3072 > m->bdig_bytes) m->bdig_bytes = maxrun * 3072;
-            }
             if (dep_x < 0) { o.x = m->emb; o.tok = from_prompt ? m->d_prompt : m->d_tok; o.res_ld = c.d_model; }
             else { o.res_ll = m->xll[1]; o.res_dep = dep_x; }
             o.out_ll = m->xll[0]; o.out_stat = m->statll[0]; o.part_ll = m->part_ll[1];
