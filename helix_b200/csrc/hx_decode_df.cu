@@ -217,16 +217,19 @@ __device__ __noinline__ AttPlan att_plan_df(const HxPersist& P, int cta, int pos
 // Attention phase of one CTA: (kv head, split of the cached positions); the split of the work depends on the
 // position only and is worked out once per launch (SmemDf::ap).  q (normed, rotated) and this position's k and v
 // arrive as pairs from the qkv epilogue; older rows stream through the ring from the cache in tiles of up to four slots.
-//  * scores: a warp takes four rows at a time against all heads of the group, eight lanes per row; the heads' sums are
-//    reduced across the eight lanes together (each exchange halves the values a lane carries);
+//  * scores: a warp takes eight rows at a time against all heads of the group, eight lanes per row and two rows per lane
+//    (reading the queries from shared memory is most of the traffic); the heads' sums are reduced across the eight lanes
+//    together (each exchange halves the values a lane carries);
 //  * soft-max statistics (online, m seeded -1e8 like the reference, fused_decode_attn_kernel.hx:74-102): one warp
 //    per head;
 //  * P*V: a thread owns four output dimensions of ALL heads of the group over a contiguous run of the tile's rows, four
 //    rows per step (a V row and a vector of four probabilities are read once); the runs are folded through shared memory.
-// The split's partial output and (max, sum) leave as pairs; one CTA per head merges the splits.
-// What bounds it: the arithmetic of the two products for groups of eight heads at long contexts (228 rows x 8 heads: about
-// 4 us), latency below.  (A thread per (row, head, eighth), with the row looked up in every step, took 44 ns per row for
-// eight heads: 25 us of a 30 us phase at 4096 positions.)
+// The split's partial output and (max, sum) leave as pairs; one CTA per head merges the splits (attention_merge_df, called
+// from the phase loop: nested in this function its registers pushed values of the caller to local memory, and a reload a
+// phase later comes from L2).
+// What bounds it: shared memory and the arithmetic of the two products for groups of eight heads at long contexts, latency
+// below.  32 layers' shape at 4096 positions (228 rows x 8 heads a CTA): 29.8 us a phase with a thread per (row, head,
+// eighth), 20.4 with all heads per row, 18.9 with two rows per lane.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ring_adv(uint32_t& slot, uint32_t& par, uint32_t n, uint32_t nring) {
     slot += n;
@@ -328,7 +331,6 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
             const int hs = (ap.kv * GRP + i / DH) * ns + ap.split;
             ll_st(ph.pacc_ll + (size_t)hs * DH + i % DH, 0.0f, ep);
         }
-        attention_merge_df(P, ph, S, reinterpret_cast<float4*>(sp), ap.kv, ap.split, ns, GRP, ep);
         return;
     }
     float4 acc[GRP];
@@ -382,26 +384,31 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         {
             const int p = lane & 7;
             #pragma unroll 1
-            for (int r0 = warp * 4; r0 < ntot; r0 += NCW * 4) {
-                const int r = r0 + (lane >> 3);
-                const float* kr = ringf + S.rowk[min(r, ntot - 1)];
-                float4 k4[4];
+            for (int r0 = warp * 8; r0 < ntot; r0 += NCW * 8) {
+                const int ra = r0 + (lane >> 3), rb = ra + 4;
+                const float* ka = ringf + S.rowk[min(ra, ntot - 1)];
+                const float* kb = ringf + S.rowk[min(rb, ntot - 1)];
+                float4 k4[2][4];
 #pragma unroll
-                for (int c = 0; c < 4; c++) k4[c] = *reinterpret_cast<const float4*>((c < CPT ? kr : sq) + (p + 8 * c) * 4);     // narrow heads: zeros
-                float v[GP];
+                for (int c = 0; c < 4; c++) {                       // narrow heads: zeros
+                    k4[0][c] = *reinterpret_cast<const float4*>((c < CPT ? ka : sq) + (p + 8 * c) * 4);
+                    k4[1][c] = *reinterpret_cast<const float4*>((c < CPT ? kb : sq) + (p + 8 * c) * 4);
+                }
+                float v[2][GP];
 #pragma unroll
                 for (int i = 0; i < GP; i++) {
-                    v[i] = 0.0f;
+                    v[0][i] = v[1][i] = 0.0f;
                     if (i < GRP) {
-                        float d0 = 0.0f, d1 = 0.0f;
+                        float d0 = 0.0f, d1 = 0.0f, e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
                         for (int c = 0; c < 4; c++) {
                             const float4 q4 = *reinterpret_cast<const float4*>(sq + i * 128 + (p + 8 * c) * 4);
-                            d0 = fmaf(q4.x, k4[c].x, d0); d1 = fmaf(q4.y, k4[c].y, d1); d0 = fmaf(q4.z, k4[c].z, d0); d1 = fmaf(q4.w, k4[c].w, d1);
+                            d0 = fmaf(q4.x, k4[0][c].x, d0); d1 = fmaf(q4.y, k4[0][c].y, d1); d0 = fmaf(q4.z, k4[0][c].z, d0); d1 = fmaf(q4.w, k4[0][c].w, d1);
+                            e0 = fmaf(q4.x, k4[1][c].x, e0); e1 = fmaf(q4.y, k4[1][c].y, e1); e0 = fmaf(q4.z, k4[1][c].z, e0); e1 = fmaf(q4.w, k4[1][c].w, e1);
                         }
-                        v[i] = d0 + d1;
+                        v[0][i] = d0 + d1; v[1][i] = e0 + e1;
                     }
-                    if (i & 1) asm volatile("" ::: "memory");          // two heads' queries in registers at a time
+                    asm volatile("" ::: "memory");                      // one head at a time: registers
                 }
 #pragma unroll
                 for (int st = 0; st < 3; st++) {
@@ -410,14 +417,19 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
                         const int hh = GP >> (st + 1);
                         const bool up = (lane & o) != 0;
 #pragma unroll
-                        for (int k = 0; k < hh; k++) {
-                            const float send = up ? v[k] : v[k + hh], keep = up ? v[k + hh] : v[k];
-                            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                        }
-                    } else v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                        for (int u = 0; u < 2; u++)
+#pragma unroll
+                            for (int k = 0; k < hh; k++) {
+                                const float send = up ? v[u][k] : v[u][k + hh], keep = up ? v[u][k + hh] : v[u][k];
+                                v[u][k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                            }
+                    } else { v[0][0] += __shfl_xor_sync(0xffffffffu, v[0][0], o); v[1][0] += __shfl_xor_sync(0xffffffffu, v[1][0], o); }
                 }
                 const int i = p >> (3 - LG);
-                if ((p & ((1 << (3 - LG)) - 1)) == 0 && i < GRP && r < ntot) sp[i * ATT_ROWS + r] = v[0] * ph.scale;
+                if ((p & ((1 << (3 - LG)) - 1)) == 0 && i < GRP) {
+                    if (ra < ntot) sp[i * ATT_ROWS + ra] = v[0][0] * ph.scale;
+                    if (rb < ntot) sp[i * ATT_ROWS + rb] = v[1][0] * ph.scale;
+                }
             }
         }
         consumer_sync();
@@ -488,7 +500,6 @@ __device__ __noinline__ void attention_df(const HxPersist& P, const HxPhase& ph,
         if (c == 0) ll_st2(ph.pml_ll + 2 * hs, S.att_m[i], S.att_l[i], ep);
     }
     DF_MARK(4);
-    attention_merge_df(P, ph, S, reinterpret_cast<float4*>(sp), ap.kv, ap.split, ns, GRP, ep);
 }
 
 
@@ -1011,6 +1022,8 @@ __global__ void __launch_bounds__(PT, 1) k_decode_df(const __grid_constant__ HxP
                     case 7: attention_df<7>(P, ph, S, ring, digb, cslot, cpar, pi, pos); break;
                     default: attention_df<8>(P, ph, S, ring, digb, cslot, cpar, pi, pos); break;
                 }
+                // (scratch: the probabilities, free since the last barrier of the tiles)
+                if (S.ap.active) attention_merge_df(P, ph, S, reinterpret_cast<float4*>(digb + (8 * 128 + 128 + 128) * 4), S.ap.kv, S.ap.split, S.att_ns, ph.NH / ph.NKV, ep);
             }
             DF_STAMP(2); DF_MARK(5);
             // ---------- phase boundary: the digit columns and the attention scratch are free again ----------
