@@ -353,7 +353,7 @@ def batch64_leg(hb, L, check, dist, rank, ngpus, shape):
     return {"sequences": n_seq, "sequences_asked": BATCH_SEQS, "per_gpu": S_run, "prompt": BATCH_PROMPT, "new_tokens": BATCH_NEW,
             "prefill_s": prefill_s, "prefill_tok_per_s": ptok / prefill_s, "decode_s": dms * 1e-3, "decode_tok_per_s": dtok / (dms * 1e-3),
             "total_tok_per_s": (ptok + dtok) / (prefill_s + dms * 1e-3),
-            "path": "hx_prefill_seq per sequence (64-token chunks through the tcgen05 GEMM), then hx_decode_batch_loop "
+            "path": "hx_prefill_seq per sequence (chunks of up to 1008 tokens through the tcgen05 GEMM), then hx_decode_batch_loop "
                     "(64 sequences per pass over the weights); replicas, no exchange between GPUs"}
 
 
@@ -647,7 +647,7 @@ def run_ours(args):
                 "roofline": roofline, "cpu_baseline": cpu, "parity": parity, "e2e": e2e, "gpu_launches": int(launches), "clocks": clocks,
                 "reference_gpu": ref_gpu, "batch64": batch64, "tp": tpl, "speculative": spec, "tensor_probe": tprobe, "quantizer": quant, "gpt2": gpt2,
                 "prefill": {"tokens": PROMPT_LEN, "ms": prefill_s * 1e3, "tok_per_s": PROMPT_LEN / prefill_s,
-                            "path": "chunks of 64 tokens, one tcgen05 block-scaled GEMM per linear (ten base-9 digit columns per activation), host ids in"},
+                            "path": "chunks of up to 1008 tokens, one tcgen05 block-scaled GEMM per linear (ten base-9 digit columns per activation), host ids in"},
                 "ms_per_token": ms_max / args.steps / NEW_TOKENS, "last_tokens": [int(t) for t in toks[-4:]]}
         print(json.dumps(line), flush=True)
     if dist is not None:

@@ -67,7 +67,7 @@ int hx_kpad(int K);
  *   sc     [rows*(Kpad/16)] f32, e4m3_decode(micro)*ts                          (may be NULL)
  *   ts     [1] f32 per-tensor scale amax/(6*448), 1.0 for an all-zero tensor    (may be NULL)
  * stream is a cudaStream_t (NULL = default stream); the call is asynchronous.  The first call on a device
- * allocates 256 bytes for the tensor maxima (64 words handed out in turn): calls on different streams may
+ * allocates a small scratch for the partial maxima (64 sets handed out in turn): calls on different streams may
  * overlap as long as no more than 64 are in flight on one device. */
 int hx_quantize_nvfp4(const float* w, int rows, int K, int32_t* words, uint8_t* micro, float* sc,
                       float* ts, void* stream);
@@ -75,7 +75,7 @@ int hx_quantize_nvfp4(const float* w, int rows, int K, int32_t* words, uint8_t* 
 /* hx_quantize_nvfp4 for callers that must not allocate device memory (a host that owns all of it in an
  * arena of its own, a service that cannot take the device-wide stall of an allocation).  Same arguments,
  * same bytes out.  No counterpart in the reference: its quantizer runs on the CPU.
- * The per-row maxima live in an array inside the library (1 MiB, found with cudaGetSymbolAddress):
+ * The partial maxima live in a small array inside the library (found with cudaGetSymbolAddress):
  *   - rows <= hx_noalloc_max_rows() (262144), else HX_ERR_ARG;
  *   - the first call on a device looks the array up (and loads the device code if nothing has yet): make
  *     it during start-up, ahead of any stream capture;
