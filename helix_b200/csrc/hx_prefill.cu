@@ -1,7 +1,7 @@
 // hx_prefill.cu -- batched prefill around the tcgen05 GEMM.
 //
 // Replaces forward_layer_llama / forward_full (helixc/runtime/gpt2_infer.c:1231-1333): where the reference runs
-// f32 tiled_matmul_abt over a dequantized weight copy per layer, a chunk of HX_PF_TB prompt tokens here is one
+// f32 tiled_matmul_abt over a dequantized weight copy per layer, a chunk of prompt tokens here is one
 // block-scaled NVFP4 GEMM per linear with the weights read in their packed form.  The activations enter the FP4
 // tensor path as digits: after the optional RMSNorm each element is x = s * sum_d digit_d 9^(9-d) with ten balanced
 // base-9 digits (-4 .. 4: E2M1 values, sign included) of the integer |x| / S * 2^29 (S: the power of two at or below
@@ -9,6 +9,7 @@
 // epilogue folds the ten accumulators of a token.  The digits resolve 2^-29 of the vector's largest element, beyond
 // what an f32 dot product keeps.  (The decode kernel uses sixteen exact base-4 digits: there the column count is free.)
 // Norm, RoPE, KV append and attention are small f32 kernels over the chunk.
+#include "hx_tc.cuh"
 #include "hx_prefill.cuh"
 #include "hx_gemm_tc.cuh"
 #include "hx_kernels.cuh"
@@ -30,25 +31,36 @@ __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, H
     }
 }
 
-// grid (token, slice of 2048 columns), 256 threads: every CTA of a token computes the token's statistics (all its loads in
-// flight together: one round trip to L2 bounds the small launches), then a thread turns eight consecutive elements into one
-// 32-bit word per digit.
+// grid (token, slice of 4096 columns), 512 threads: a thread takes eight consecutive elements and turns them into one 32-bit
+// word per digit.  The statistics of a token with several slices are put together by a cluster (up to PFD_CL slices) through
+// distributed shared memory; beyond that every CTA reads the whole vector.
 // A value becomes the integer X = round(x / S * 2^29), |X| < 2^30 (S: the power of two at or below the vector's largest
 // element), spelled with ten balanced base-9 digits (-4 .. 4).  Adding sum_i 4 * 9^i makes it a plain base-9 number whose
-// digits are the balanced ones plus 4 -- no carries, no separate sign -- and a division by 9^5 makes two independent chains
-// of five.  Digit d (d = 0: weight 9^9) of token t lies in row 24 d + t % 24 of the token group t / 24 of a cell, as the E2M1
-// code of its value.  (Before: a chain of ten dependent 32-bit divisions per element on 128 of 512 threads; 64 tokens x 4096
-// columns 6.9 us, 64 x 12288 15.8 us.)
-#define PFD_T 256
+// digits are the balanced ones plus 4 -- no carries, no separate sign -- taken two at a time: a pair of digits is an index
+// into a table of 81 bytes (21 words in as many banks: no conflicts), each with the two E2M1 codes.  Digit d (d = 0: weight
+// 9^9) of token t lies in row 24 d + t % 24 of the token group t / 24 of a cell.
+// Bound by instruction issue.  (Digit by digit, with six CTAs each reading the whole vector at K = 12288: 12 us for 512 tokens
+// x 4096 columns, 33 us for 512 x 12288.)
+#define PFD_T 512
+#define PFD_CL 8                    // CTAs of a token at most for a cluster
+template <bool CL>
 __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g, const float* __restrict__ lb,
                                                      float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ float part[PFD_CL][2];    // (sum of squares, largest) of the token's slices
     hx_grid_dep_launch();
+    if (CL) hxtc::cl_sync();             // every CTA of the cluster runs before a store into it
     hx_grid_dep_wait();
     const float* x = src + (size_t)t * ld;
     __shared__ float red[2 * PFD_T / 32];
-    const int k0 = (blockIdx.y * PFD_T + tid) * 8;       // this thread's item, fetched with the rest
-    float v[8];
+    __shared__ uint8_t codes[84];        // a pair of digits (each + 4) -> two codes, the more significant one in the high nibble
+    if (tid < 81) {
+        // E2M1 codes of -4, -3, -2, -1, 0, 1, 2, 3, 4: E D C A 0 2 4 5 6
+        const uint32_t h = (uint32_t)tid / 9u, l = (uint32_t)tid - 9u * h;
+        codes[tid] = (uint8_t)(((__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * h) & 0xFu) << 4) | (__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * l) & 0xFu));
+    }
+    const int k0 = (blockIdx.y * PFD_T + tid) * 8;       // this thread's item
+    float v[8], ss = 0.0f, mx = 0.0f;
     {
         const bool in0 = k0 < K, in1 = k0 + 4 < K;       // K is a multiple of four
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -56,8 +68,9 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
         const float4 ga = (g && in0) ? __ldg(reinterpret_cast<const float4*>(g + k0)) : one, gb = (g && in1) ? __ldg(reinterpret_cast<const float4*>(g + k0 + 4)) : one;
         v[0] = a.x * ga.x; v[1] = a.y * ga.y; v[2] = a.z * ga.z; v[3] = a.w * ga.w;
         v[4] = b.x * gb.x; v[5] = b.y * gb.y; v[6] = b.z * gb.z; v[7] = b.w * gb.w;
+        ss = ((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w));
     }
-    float inv = 1.0f, mx = 0.0f;
+    float inv = 1.0f;
     if (lb) {
         // LayerNorm (GPT-2): mean, then variance about it, then the largest result
         float mean = 0.0f;
@@ -91,49 +104,65 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
         __syncthreads();
     } else {
     // sum of squares (of x) and largest |x * g| of the whole vector
-    float ss = 0.0f;
-    #pragma unroll 4
-    for (int k = tid * 4; k < K; k += PFD_T * 4) {
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k));
-        const float4 ga = g ? __ldg(reinterpret_cast<const float4*>(g + k)) : make_float4(1.f, 1.f, 1.f, 1.f);
-        ss = fmaf(a.x, a.x, ss); ss = fmaf(a.y, a.y, ss); ss = fmaf(a.z, a.z, ss); ss = fmaf(a.w, a.w, ss);
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(a.x * ga.x), fabsf(a.y * ga.y)), fmaxf(fabsf(a.z * ga.z), fabsf(a.w * ga.w))));
+    if (CL || gridDim.y == 1) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(v[e]));
+    } else {
+        ss = 0.0f;
+        #pragma unroll 4
+        for (int k = tid * 4; k < K; k += PFD_T * 4) {
+            const float4 a = __ldcg(reinterpret_cast<const float4*>(x + k));
+            const float4 ga = g ? __ldg(reinterpret_cast<const float4*>(g + k)) : make_float4(1.f, 1.f, 1.f, 1.f);
+            ss = fmaf(a.x, a.x, ss); ss = fmaf(a.y, a.y, ss); ss = fmaf(a.z, a.z, ss); ss = fmaf(a.w, a.w, ss);
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(a.x * ga.x), fabsf(a.y * ga.y)), fmaxf(fabsf(a.z * ga.z), fabsf(a.w * ga.w))));
+        }
     }
     ss = hx_warp_sum(ss); mx = hx_warp_max(mx);
     if (lane == 0) { red[warp] = ss; red[PFD_T / 32 + warp] = mx; }
     __syncthreads();
     float tss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < PFD_T / 32; i++) tss += red[i];
+    for (int i = 0; i < PFD_T / 32; i++) { tss += red[i]; if (CL) mx = fmaxf(mx, red[PFD_T / 32 + i]); }
+    if (CL) {
+        if (tid < (int)gridDim.y) {
+            const uint32_t to = hxtc::cl_map(hxtc::s_u32(&part[blockIdx.y][0]), (uint32_t)tid);
+            hxtc::cl_st(to, tss); hxtc::cl_st(to + 4, mx);
+        }
+        hxtc::cl_sync();
+        tss = 0.0f;
+        for (int i = 0; i < (int)gridDim.y; i++) { tss += part[i][0]; mx = fmaxf(mx, part[i][1]); }
+    }
     if (g) inv = rsqrtf(tss / (float)K + eps);
     }
-    float tmx = 0.0f;
+    float tmx = mx;
+    if (!CL) {
 #pragma unroll
-    for (int i = 0; i < PFD_T / 32; i++) tmx = fmaxf(tmx, red[PFD_T / 32 + i]);
+        for (int i = 0; i < PFD_T / 32; i++) tmx = fmaxf(tmx, red[PFD_T / 32 + i]);
+    }
     float Sg = 1.0f;
     const float vmax = tmx * inv * 1.0000005f;
     if (vmax > 0.0f && vmax < INFINITY) Sg = __uint_as_float(__float_as_uint(vmax) & 0x7F800000u);
     if (tid == 0 && blockIdx.y == 0) scale[t] = Sg * (1.0f / HX_TC_DIGIT_UNIT);
     const float mul = (inv / Sg) * HX_TC_DIGIT_UNIT;
     if (k0 >= ((K + 255) & ~255)) return;
-    uint32_t word[HX_TC_DIGITS];
-#pragma unroll
-    for (int n = 0; n < HX_TC_DIGITS; n++) word[n] = 0u;
+    // two digits at a time: five pairs (base 81) per element, each a byte of two codes from the table
+    uint32_t pair[HX_TC_DIGITS / 2][8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
         const uint32_t u = 1743392200u + (uint32_t)__float2int_rn(v[e] * mul);      // (9^10 - 1) / 2 + X
-        const uint32_t hi = u / 59049u;
-        uint32_t part[2] = {hi, u - hi * 59049u};                                    // both below 2^16
+        uint32_t q = u;
 #pragma unroll
-        for (int h = 0; h < 2; h++)
+        for (int i = HX_TC_DIGITS / 2 - 1; i > 0; i--) { const uint32_t qn = q / 81u; pair[i][e] = codes[q - qn * 81u]; q = qn; }
+        pair[0][e] = codes[q];
+    }
+    uint32_t word[HX_TC_DIGITS];
 #pragma unroll
-            for (int n = 4; n >= 0; n--) {
-                const uint32_t qn = (part[h] * 58255u) >> 19;                        // / 9, exact below 2^16
-                const uint32_t r = part[h] - 9u * qn;                                // digit + 4
-                part[h] = qn;
-                // E2M1 codes of -4, -3, -2, -1, 0, 1, 2, 3, 4: E D C A 0 2 4 5 6
-                word[h * 5 + n] |= (__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * r) & 0xFu) << (4 * e);
-            }
+    for (int i = 0; i < HX_TC_DIGITS / 2; i++) {
+        const uint32_t (&p)[8] = pair[i];
+        const uint32_t ev = __byte_perm(__byte_perm(p[0], p[2], 0x0040), __byte_perm(p[4], p[6], 0x0040), 0x5410);
+        const uint32_t od = __byte_perm(__byte_perm(p[1], p[3], 0x0040), __byte_perm(p[5], p[7], 0x0040), 0x5410);
+        word[2 * i] = ((ev >> 4) & 0x0F0F0F0Fu) | (od & 0xF0F0F0F0u);               // the more significant digit of the pair
+        word[2 * i + 1] = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
     }
     const int it = k0 >> 3, j = (it >> 2) & 7, w = it & 3;
     const int tg = t / HX_TC_MAX_TOK, tl = t - tg * HX_TC_MAX_TOK;
@@ -145,39 +174,68 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
     }
 }
 
-// grid (NH + 2 NKV, n_tok), block DH threads (DH <= 256)
-__global__ void __launch_bounds__(256) k_pf_qkpost(float* __restrict__ qkv, int ld, HxPfWhere wh, int NH, int NKV, int DH,
+// q/k norm, rotate_half RoPE and KV append: a warp per (head section, token), EPL = DH / 32 consecutive elements per lane, so a
+// row is one vector load per lane, the sum of squares one warp reduction and the rotation partner one exchange with lane ^ 16;
+// grid (head sections / 8, n_tok).  Latency is what bounds it: loads of a row, gains and angles in flight together, no barrier.
+// (A CTA of DH threads per row with three barriers: 9.5 us for 77 tokens of the 8B shape, 22 for 512.)
+#define PF_QK_W 8
+template <int EPL>
+__global__ void __launch_bounds__(PF_QK_W * 32) k_pf_qkpost(float* __restrict__ qkv, int ld, HxPfWhere wh, int NH, int NKV,
                                                     const float* __restrict__ qn_g, const float* __restrict__ kn_g, float eps,
                                                     const float* __restrict__ cosT, const float* __restrict__ sinT,
                                                     float* __restrict__ kc, float* __restrict__ vc, int cap) {
+    constexpr int DH = 32 * EPL, half = DH / 2, VEC = EPL < 4 ? EPL : 4, NV = EPL / VEC;
+    struct __align__(4 * VEC) Vec { float f[VEC]; };
     hx_grid_dep_launch();
-    hx_grid_dep_wait();
-    const int hs = blockIdx.x, t = blockIdx.y, e = threadIdx.x, half = DH >> 1, pos = wh.pos_arr ? __ldcg(wh.pos_arr + t) : __ldcg(wh.posp) + t;
-    const size_t seq_off = wh.seq_arr ? (size_t)__ldcg(wh.seq_arr + t) * wh.seq_stride : (wh.seqp ? (size_t)__ldcg(wh.seqp) * wh.seq_stride : 0);
-    const int sec = hs < NH ? 0 : (hs < NH + NKV ? 1 : 2);
-    float* row = qkv + (size_t)t * ld + (size_t)hs * DH;
-    __shared__ float sm[256]; __shared__ float red[8];
-    float v = e < DH ? __ldcg(row + e) : 0.0f;
+    const int hs = blockIdx.x * PF_QK_W + (threadIdx.x >> 5), t = blockIdx.y, lane = threadIdx.x & 31;
+    if (hs >= NH + 2 * NKV) return;
+    const int sec = hs < NH ? 0 : (hs < NH + NKV ? 1 : 2), e0 = lane * EPL, er = e0 & (half - 1);
     const float* gg = sec == 0 ? qn_g : (sec == 1 ? kn_g : nullptr);
-    float ssq = hx_warp_sum(v * v);
-    if ((e & 31) == 0) red[e >> 5] = ssq;
-    __syncthreads();
-    ssq = 0.0f;
-    for (int i = 0; i < (DH + 31) / 32; i++) ssq += red[i];
-    if (gg) v = gg[e] * (v * rsqrtf(ssq / (float)DH + eps));
-    if (cosT && sec < 2) {
-        sm[e] = v;
-        __syncthreads();
-        const float other = sm[e < half ? e + half : e - half];
-        const float cs = cosT[(size_t)pos * half + (e < half ? e : e - half)], sn = sinT[(size_t)pos * half + (e < half ? e : e - half)];
-        v = e < half ? v * cs - other * sn : v * cs + other * sn;
-    }
-    if (e < DH) {
-        if (sec == 0) row[e] = v;
-        else {
-            const int kvh = hs - NH - (sec == 2 ? NKV : 0);
-            (sec == 1 ? kc : vc)[seq_off + ((size_t)kvh * cap + pos) * DH + e] = v;
+    auto load = [](const float* p, float (&v)[EPL], bool fresh) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            Vec x;
+            if (EPL == 1) x.f[0] = fresh ? __ldcg(p) : __ldg(p);
+            else if (EPL == 2) { const float2 y = fresh ? __ldcg(reinterpret_cast<const float2*>(p)) : __ldg(reinterpret_cast<const float2*>(p)); x.f[0] = y.x; x.f[VEC > 1 ? 1 : 0] = y.y; }
+            else {
+                const float4 y = fresh ? __ldcg(reinterpret_cast<const float4*>(p) + i) : __ldg(reinterpret_cast<const float4*>(p) + i);
+                x.f[0] = y.x; x.f[VEC > 1 ? 1 : 0] = y.y; x.f[VEC > 2 ? 2 : 0] = y.z; x.f[VEC > 3 ? 3 : 0] = y.w;
+            }
+#pragma unroll
+            for (int c = 0; c < VEC; c++) v[i * VEC + c] = x.f[c];
         }
+    };
+    float v[EPL], g[EPL], cs[EPL], sn[EPL];
+    if (gg) load(gg + e0, g, false);
+    hx_grid_dep_wait();
+    const int pos = wh.pos_arr ? __ldcg(wh.pos_arr + t) : __ldcg(wh.posp) + t;
+    const size_t seq_off = wh.seq_arr ? (size_t)__ldcg(wh.seq_arr + t) * wh.seq_stride : (wh.seqp ? (size_t)__ldcg(wh.seqp) * wh.seq_stride : 0);
+    float* row = qkv + (size_t)t * ld + (size_t)hs * DH;
+    load(row + e0, v, true);
+    const bool rot = cosT && sec < 2;
+    if (rot) { load(cosT + (size_t)pos * half + er, cs, false); load(sinT + (size_t)pos * half + er, sn, false); }
+    if (gg) {
+        float ssq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < EPL; i++) ssq = fmaf(v[i], v[i], ssq);
+        const float inv = rsqrtf(hx_warp_sum(ssq) / (float)DH + eps);
+#pragma unroll
+        for (int i = 0; i < EPL; i++) v[i] = g[i] * (v[i] * inv);
+    }
+    if (rot) {
+#pragma unroll
+        for (int i = 0; i < EPL; i++) {
+            const float other = __shfl_xor_sync(0xffffffffu, v[i], 16);
+            v[i] = lane < 16 ? v[i] * cs[i] - other * sn[i] : v[i] * cs[i] + other * sn[i];
+        }
+    }
+    float* dst = sec == 0 ? row + e0 : (sec == 1 ? kc : vc) + seq_off + ((size_t)(hs - NH - (sec == 2 ? NKV : 0)) * cap + pos) * DH + e0;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        Vec x;
+#pragma unroll
+        for (int c = 0; c < VEC; c++) x.f[c] = v[i * VEC + c];
+        reinterpret_cast<Vec*>(dst)[i] = x;
     }
 }
 
@@ -659,17 +717,34 @@ void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wp
 void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
     const int groups = (n_tok + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
     const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
+    const bool cl = grid.y > 1 && grid.y <= PFD_CL && !b;
     // Started early, this kernel's CTAs wait beside the GEMM's and the step got slower up to some hundred tokens (64 sequences
     // 3.72 -> 3.85 ms for twelve layers, five sequences 0.97 -> 1.03); at 512 tokens it gains 3 %.
-    if (n_tok >= 256) hx_launch_pdl(k_pf_digits, grid, dim3(PFD_T), 0, st, src, ld, K, g, b, eps, cells, groups, scale);
-    else k_pf_digits<<<grid, PFD_T, 0, st>>>(src, ld, K, g, b, eps, cells, groups, scale);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(PFD_T); cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    cfg.attrs = at;
+    if (n_tok >= 256) { at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
+    if (cl) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = grid.y; at[cfg.numAttrs++].val.clusterDim.z = 1;
+        cudaLaunchKernelEx(&cfg, k_pf_digits<true>, src, ld, K, g, b, eps, cells, groups, scale);
+    } else cudaLaunchKernelEx(&cfg, k_pf_digits<false>, src, ld, K, g, b, eps, cells, groups, scale);
     HX_COUNT_LAUNCH(1);
 }
 
 void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
                   float eps, const float* cosT, const float* sinT, float* kc, float* vc, int cap, cudaStream_t st) {
-    const int threads = ((DH + 31) / 32) * 32;
-    hx_launch_pdl(k_pf_qkpost, dim3(NH + 2 * NKV, n_tok), dim3(threads), 0, st, qkv, ld, wh, NH, NKV, DH, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap);
+    const dim3 grid((NH + 2 * NKV + PF_QK_W - 1) / PF_QK_W, n_tok);
+#define PF_QKPOST(E) hx_launch_pdl(k_pf_qkpost<E>, grid, dim3(PF_QK_W * 32), 0, st, qkv, ld, wh, NH, NKV, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap)
+    switch (DH) {                    // (the head sizes that the attention of a chunk takes; it reports the others)
+        case 32: PF_QKPOST(1); break;
+        case 64: PF_QKPOST(2); break;
+        case 128: PF_QKPOST(4); break;
+        case 256: PF_QKPOST(8); break;
+        default: return;
+    }
+#undef PF_QKPOST
     HX_COUNT_LAUNCH(1);
 }
 
