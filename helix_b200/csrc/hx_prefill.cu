@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, H
 // x 4096 columns, 33 us for 512 x 12288.)
 #define PFD_T 512
 #define PFD_CL 8                    // CTAs of a token at most for a cluster
-template <bool CL>
-__global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g, const float* __restrict__ lb,
+template <bool CL, bool LN>              // statistics by a cluster; LayerNorm instead of RMSNorm
+__global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict__ src, int ld, int K, const float* __restrict__ g, const float* __restrict__ lb,
                                                      float eps, uint8_t* __restrict__ cells, int groups, float* __restrict__ scale) {
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __shared__ float part[PFD_CL][2];    // (sum of squares, largest) of the token's slices
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
         ss = ((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w));
     }
     float inv = 1.0f;
-    if (lb) {
+    if (LN) {
         // LayerNorm (GPT-2): mean, then variance about it, then the largest result
         float mean = 0.0f;
         for (int ps = 0; ps < 2; ps++) {
@@ -145,24 +145,26 @@ __global__ void __launch_bounds__(PFD_T) k_pf_digits(const float* __restrict__ s
     if (tid == 0 && blockIdx.y == 0) scale[t] = Sg * (1.0f / HX_TC_DIGIT_UNIT);
     const float mul = (inv / Sg) * HX_TC_DIGIT_UNIT;
     if (k0 >= ((K + 255) & ~255)) return;
-    // two digits at a time: five pairs (base 81) per element, each a byte of two codes from the table
-    uint32_t pair[HX_TC_DIGITS / 2][8];
+    // two digits at a time: five pairs (base 81) per element, each a byte of two codes from the table; the bytes of the even
+    // and of the odd elements are collected in a word each
+    uint32_t ev[HX_TC_DIGITS / 2], od[HX_TC_DIGITS / 2];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
-        const uint32_t u = 1743392200u + (uint32_t)__float2int_rn(v[e] * mul);      // (9^10 - 1) / 2 + X
-        uint32_t q = u;
+        uint32_t q = 1743392200u + (uint32_t)__float2int_rn(v[e] * mul);            // (9^10 - 1) / 2 + X
 #pragma unroll
-        for (int i = HX_TC_DIGITS / 2 - 1; i > 0; i--) { const uint32_t qn = q / 81u; pair[i][e] = codes[q - qn * 81u]; q = qn; }
-        pair[0][e] = codes[q];
+        for (int i = HX_TC_DIGITS / 2 - 1; i >= 0; i--) {
+            const uint32_t qn = i ? q / 81u : 0u, c = codes[q - qn * 81u];
+            uint32_t& to = (e & 1) ? od[i] : ev[i];
+            to = e < 2 ? c : to + (c << (8 * (e >> 1)));
+            q = qn;
+        }
+        if (e & 1) asm volatile("" ::: "memory");        // two elements at a time: 40 registers, three CTAs per SM
     }
     uint32_t word[HX_TC_DIGITS];
 #pragma unroll
     for (int i = 0; i < HX_TC_DIGITS / 2; i++) {
-        const uint32_t (&p)[8] = pair[i];
-        const uint32_t ev = __byte_perm(__byte_perm(p[0], p[2], 0x0040), __byte_perm(p[4], p[6], 0x0040), 0x5410);
-        const uint32_t od = __byte_perm(__byte_perm(p[1], p[3], 0x0040), __byte_perm(p[5], p[7], 0x0040), 0x5410);
-        word[2 * i] = ((ev >> 4) & 0x0F0F0F0Fu) | (od & 0xF0F0F0F0u);               // the more significant digit of the pair
-        word[2 * i + 1] = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
+        word[2 * i] = ((ev[i] >> 4) & 0x0F0F0F0Fu) | (od[i] & 0xF0F0F0F0u);         // the more significant digit of the pair
+        word[2 * i + 1] = (ev[i] & 0x0F0F0F0Fu) | ((od[i] << 4) & 0xF0F0F0F0u);
     }
     const int it = k0 >> 3, j = (it >> 2) & 7, w = it & 3;
     const int tg = t / HX_TC_MAX_TOK, tl = t - tg * HX_TC_MAX_TOK;
@@ -728,8 +730,9 @@ void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, co
     if (cl) {
         at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
         at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = grid.y; at[cfg.numAttrs++].val.clusterDim.z = 1;
-        cudaLaunchKernelEx(&cfg, k_pf_digits<true>, src, ld, K, g, b, eps, cells, groups, scale);
-    } else cudaLaunchKernelEx(&cfg, k_pf_digits<false>, src, ld, K, g, b, eps, cells, groups, scale);
+        cudaLaunchKernelEx(&cfg, k_pf_digits<true, false>, src, ld, K, g, b, eps, cells, groups, scale);
+    } else if (b) cudaLaunchKernelEx(&cfg, k_pf_digits<false, true>, src, ld, K, g, b, eps, cells, groups, scale);
+    else cudaLaunchKernelEx(&cfg, k_pf_digits<false, false>, src, ld, K, g, b, eps, cells, groups, scale);
     HX_COUNT_LAUNCH(1);
 }
 
