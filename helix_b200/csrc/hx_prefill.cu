@@ -120,9 +120,11 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     ss = hx_warp_sum(ss); mx = hx_warp_max(mx);
     if (lane == 0) { red[warp] = ss; red[PFD_T / 32 + warp] = mx; }
     __syncthreads();
-    float tss = 0.0f;
+    static_assert(PFD_T / 32 == 16, "the warps' results are folded by sixteen lanes");
+    float tss = red[lane & 15];
+    mx = red[PFD_T / 32 + (lane & 15)];
 #pragma unroll
-    for (int i = 0; i < PFD_T / 32; i++) { tss += red[i]; if (CL) mx = fmaxf(mx, red[PFD_T / 32 + i]); }
+    for (int d = 8; d >= 1; d >>= 1) { tss += __shfl_xor_sync(0xffffffffu, tss, d); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d)); }
     if (CL) {
         if (tid < (int)gridDim.y) {
             const uint32_t to = hxtc::cl_map(hxtc::s_u32(&part[blockIdx.y][0]), (uint32_t)tid);
@@ -134,13 +136,13 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     }
     if (g) inv = rsqrtf(tss / (float)K + eps);
     }
-    float tmx = mx;
-    if (!CL) {
+    if (LN) {
+        mx = red[PFD_T / 32 + (lane & 15)];
 #pragma unroll
-        for (int i = 0; i < PFD_T / 32; i++) tmx = fmaxf(tmx, red[PFD_T / 32 + i]);
+        for (int d = 8; d >= 1; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
     }
     float Sg = 1.0f;
-    const float vmax = tmx * inv * 1.0000005f;
+    const float vmax = mx * inv * 1.0000005f;
     if (vmax > 0.0f && vmax < INFINITY) Sg = __uint_as_float(__float_as_uint(vmax) & 0x7F800000u);
     if (tid == 0 && blockIdx.y == 0) scale[t] = Sg * (1.0f / HX_TC_DIGIT_UNIT);
     const float mul = (inv / Sg) * HX_TC_DIGIT_UNIT;
@@ -153,7 +155,8 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
         uint32_t q = 1743392200u + (uint32_t)__float2int_rn(v[e] * mul);            // (9^10 - 1) / 2 + X
 #pragma unroll
         for (int i = HX_TC_DIGITS / 2 - 1; i >= 0; i--) {
-            const uint32_t qn = i ? q / 81u : 0u, c = codes[q - qn * 81u];
+            // q / 81; below 2^27 (after the first step) ceil(2^32 / 81) needs no shift: its error times q stays under 2^32
+            const uint32_t qn = i == 0 ? 0u : (i == HX_TC_DIGITS / 2 - 1 ? q / 81u : __umulhi(q, 53024288u)), c = codes[q - qn * 81u];
             uint32_t& to = (e & 1) ? od[i] : ev[i];
             to = e < 2 ? c : to + (c << (8 * (e >> 1)));
             q = qn;
@@ -168,12 +171,10 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     }
     const int it = k0 >> 3, j = (it >> 2) & 7, w = it & 3;
     const int tg = t / HX_TC_MAX_TOK, tl = t - tg * HX_TC_MAX_TOK;
-    uint8_t* dst = cells + ((size_t)(it >> 5) * groups + tg) * (HX_TC_GROUP_COLS * 128) + w * 4;
+    static_assert(HX_TC_MAX_TOK % 8 == 0, "the swizzle of a token's rows does not depend on the digit");
+    uint8_t* dst = cells + ((size_t)(it >> 5) * groups + tg) * (HX_TC_GROUP_COLS * 128) + tl * 128 + ((j ^ (tl & 7)) << 4) + w * 4;
 #pragma unroll
-    for (int n = 0; n < HX_TC_DIGITS; n++) {
-        const int row = n * HX_TC_MAX_TOK + tl;
-        *reinterpret_cast<uint32_t*>(dst + (size_t)row * 128 + ((j ^ (row & 7)) << 4)) = word[n];
-    }
+    for (int n = 0; n < HX_TC_DIGITS; n++) *reinterpret_cast<uint32_t*>(dst + n * HX_TC_MAX_TOK * 128) = word[n];
 }
 
 // q/k norm, rotate_half RoPE and KV append: a warp per (head section, token), EPL = DH / 32 consecutive elements per lane, so a
