@@ -228,8 +228,8 @@ __device__ __noinline__ AttPlan att_plan_df(const HxPersist& P, int cta, int pos
 // from the phase loop: nested in this function its registers pushed values of the caller to local memory, and a reload a
 // phase later comes from L2).
 // What bounds it: shared memory and the arithmetic of the two products for groups of eight heads at long contexts, latency
-// below.  32 layers' shape at 4096 positions (228 rows x 8 heads a CTA): 29.8 us a phase with a thread per (row, head,
-// eighth), 20.4 with all heads per row, 18.9 with two rows per lane.
+// below.  The 64-layer shape at 4096 positions (228 rows x 8 heads a CTA): 29.8 us a phase with a thread per (row, head,
+// eighth), 20.4 with all heads per row, 17.1 with two rows per lane.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ring_adv(uint32_t& slot, uint32_t& par, uint32_t n, uint32_t nring) {
     slot += n;
