@@ -592,7 +592,7 @@ def run_ours(args):
         g2.generate(gp, 16)
         _, gms_p, gms_d = g2.generate(gp, 128)
         gpt2 = {"shape": "gpt2-124m", "prompt": 32, "new_tokens": 128, "decode_tok_per_s": 127 / (gms_d * 1e-3), "prefill_ms": gms_p,
-                "engine": g2.engine(), "note": "per-op kernels in one CUDA graph per token (LayerNorm/bias/GELU fused into the NVFP4 GEMV)"}
+                "engine": g2.engine(), "note": "one CUDA graph per token: the layers in one launch on a cluster of sixteen CTAs, then the lm_head"}
         g2.close(); del gw
 
     # prompt-lookup speculative decode: the same tokens as plain greedy are required.  (a) the benchmark's own model:

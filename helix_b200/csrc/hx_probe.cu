@@ -1,9 +1,10 @@
 // hx_probe.cu -- what the tensor pipe can issue for the MMA this library uses: tcgen05.mma kind::mxf4nvf4
 // block_scale block16, M = 128, K = 64, N = ncols, both operands resident in shared memory, optionally with the four
 // tcgen05.cp scale-factor copies a weight cell needs.  One thread per SM issues `iters` cells of four MMAs through a
-// ring of eight commit barriers and the cycles are read from clock64.  The figure is the denominator of the
-// tensor-side roofline of the batched GEMM (no vendor figure exists for this MMA shape at small N), and shows why
-// the N = 16 decode formulation cannot run ahead of HBM.  Measurement only: no data leaves the kernel.
+// ring of eight commit barriers and the cycles are read from clock64.  Measurement only: no data leaves the kernel.
+// The loop is a single-thread branch (tid == 0), and at small N that branch, not the pipe, sets the pace: 130 cycles an MMA
+// at any N and 175 with the copies, where an elected lane of a converged warp reaches 57 at N = 16 (87 with the copies) and
+// 120 at N = 240.  The engines issue in the second way (hx_decode_df.cu, hx_gemm_dig.cu).
 #include "hx_common.cuh"
 
 namespace {
