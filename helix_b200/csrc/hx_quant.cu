@@ -284,9 +284,10 @@ static int quantize_launch(const float* w, int rows, int K, int32_t* words, uint
     const size_t want = (n / 4 + AMAX_THREADS * 4 - 1) / (AMAX_THREADS * 4);      // four float4 per thread and round
     const int g1 = (int)(want < 1 ? 1 : (want < AMAX_CTAS ? want : AMAX_CTAS));
     k_amax<<<g1, AMAX_THREADS, 0, st>>>(w, n, part);
-    // pass 2 is launched while pass 1 drains; it waits for its results before the first read
+    // pass 2 is launched while pass 1 drains; it waits for its results before the first read.  One wave: four CTAs fit an SM
+    // (two waves 85.9 us for 12288 x 4096, one 84.5).
     const size_t ctas = (items + Q_THREADS / 32 - 1) / (Q_THREADS / 32);
-    HX_CUDA(hx_launch_pdl(k_quantize, dim3((unsigned)(ctas < 148 * 8 ? ctas : 148 * 8)), dim3(Q_THREADS), 0, st, w, rows, K, units, (const float*)part, g1, o, ts));
+    HX_CUDA(hx_launch_pdl(k_quantize, dim3((unsigned)(ctas < 148 * 4 ? ctas : 148 * 4)), dim3(Q_THREADS), 0, st, w, rows, K, units, (const float*)part, g1, o, ts));
     HX_COUNT_LAUNCH(2);
     HX_CUDA(cudaGetLastError());
     return HX_OK;
