@@ -11,9 +11,10 @@
 // arithmetic (5 us of a layer at D = 768), so the layers run on one cluster:
 //  * every CTA owns a sixteenth of the rows of each linear; its weights stream through two shared-memory buffers by bulk
 //    copies, a phase ahead;
-//  * a half-warp takes a row: its lanes hold the (normed) input in registers, 16 * NB elements each (D = 256 * NB), decode
-//    the codes with cvt.f16x2.e2m1x2 and multiply in f32; the second projection (K = 4 D) is cut into four K quarters over
-//    the warps;
+//  * a warp takes sixteen rows and 256 columns at a time: codes decoded by cvt.f16x2.e2m1x2, times their scale (exact in
+//    f16), mma.sync m16n8k16 against the input as three f16 terms (33 bits of the largest element) in three of the eight
+//    columns.  The decode engines' tcgen05 form needs 128-row tiles: eighteen of them do not share out over sixteen CTAs.
+//    (A half-warp per row in f32 was bound by the f16 -> f32 conversions: 20 000 of a layer's 38 000 cycles.)
 //  * results leave as 8-byte (value, epoch) pairs stored into all sixteen CTAs (q, k, v: into the head's CTA), and the
 //    reader polls its own shared memory until the epoch of the layer shows up.  An aligned 8-byte store is single-copy
 //    atomic, so a matching epoch proves the value.  No buffer is written for the next layer before every CTA has read this
@@ -22,6 +23,7 @@
 // Waits are bounded; after one that ran out the CTA goes on with what is there, raises *err and the call reports it.
 #include "hx_tc.cuh"
 #include "hx_kernels.cuh"
+#include "hx_persist.cuh"
 #include "hx_gpt2_step.cuh"
 #include <cuda_fp16.h>
 
@@ -33,7 +35,6 @@ constexpr int G2_CTAS = 16, G2_WARPS = 16, G2_CT = G2_WARPS * 32, G2_THREADS = G
 constexpr int G2_CAP = 2048;                          // cached positions at most (scores in shared memory)
 
 __device__ __forceinline__ void g2_sync() { asm volatile("bar.sync 1, %0;" :: "n"(G2_CT) : "memory"); }
-__device__ __forceinline__ int g2_pad(int e) { return (e >> 4) * 20 + (e & 15); }      // blocks of sixteen 20 words apart: no bank conflicts
 __device__ __forceinline__ void g2_send(uint32_t addr, float v, unsigned ep) {
     const unsigned long long w = ((unsigned long long)ep << 32) | (unsigned long long)__float_as_uint(v);
     asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" :: "r"(addr), "l"(w) : "memory");
@@ -54,41 +55,54 @@ __device__ __forceinline__ float g2_gelu(float x) {   // gpu_gelu_stable_kernel.
     const float th = sgn * ((1.0f - e) / (1.0f + e));
     return 0.5f * x * (1.0f + th);
 }
-// sum of sixteen products with the codes of one block
-__device__ __forceinline__ float g2_dot16(uint2 c, const float* x) {
-    float a = 0.0f, b = 0.0f;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        uint32_t p0, p1, p2, p3;
-        asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\t"
-            "cvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\tcvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
-            : "=r"(p0), "=r"(p1), "=r"(p2), "=r"(p3) : "r"(h ? c.y : c.x));
-        const float* y = x + 8 * h;
-        float2 f;
-        f = __half22float2(*reinterpret_cast<__half2*>(&p0)); a = fmaf(y[0], f.x, a); b = fmaf(y[1], f.y, b);
-        f = __half22float2(*reinterpret_cast<__half2*>(&p1)); a = fmaf(y[2], f.x, a); b = fmaf(y[3], f.y, b);
-        f = __half22float2(*reinterpret_cast<__half2*>(&p2)); a = fmaf(y[4], f.x, a); b = fmaf(y[5], f.y, b);
-        f = __half22float2(*reinterpret_cast<__half2*>(&p3)); a = fmaf(y[6], f.x, a); b = fmaf(y[7], f.y, b);
-    }
-    return a + b;
+__device__ __forceinline__ void g2_cvt8(uint32_t w, uint32_t (&h)[4]) {       // eight codes -> four pairs of halves
+    asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\tcvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
+        : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(w));
 }
-__device__ __forceinline__ float g2_scale(uint32_t byte) {
-    uint32_t h;
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"((unsigned short)byte));
-    return __half2float(__ushort_as_half((unsigned short)h));
+__device__ __forceinline__ uint32_t g2_scale2(uint32_t s) { uint32_t h; asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"((unsigned short)s)); return h; }
+__device__ __forceinline__ uint32_t g2_mul2(uint32_t a, uint32_t b) { uint32_t d; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d; }
+__device__ __forceinline__ void g2_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
 }
-// row . x over NB blocks per lane: lane l of the half-warp owns blocks l, l + 16, ...; every lane of the half gets the sum
-template <int NB>
-__device__ __forceinline__ float g2_row(const uint8_t* codes, const uint8_t* scales, const float (&x)[16 * NB], int l) {
-    float s = 0.0f;
+// where the first term of element k of the input lies among the halves (the next two 16 and 32 behind): a B fragment of an
+// MMA is eight consecutive bytes per lane (hx_repack_t16 pairs the elements of two blocks the same way)
+__device__ __forceinline__ int g2_place(int k) {
+    const int e = k & 127, blk = e >> 4, j = e & 15, m = (blk & ~1) | (j >> 3);
+    return ((k >> 7) * 8 + m) * 48 + (((j >> 2) & 1) << 1 | (blk & 1)) + (j & 3) * 4;
+}
+// sixteen rows times `n` cells of 128 columns (T16: 1024 bytes of codes in A-fragment order, eight scales per row).  A weight
+// is code times scale, exact in f16; the input is three f16 terms in columns 0 .. 2.
+__device__ __forceinline__ void g2_cells(const uint8_t* cell, int n, const __half* x, float& lo, float& hi) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    float c[4] = {0.f, 0.f, 0.f, 0.f}, d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int i = 0; i < n; i++, cell += HX_T16_CELL, x += 8 * 48) {
+        const uint4 qa = *reinterpret_cast<const uint4*>(cell + lane * 16), qb = *reinterpret_cast<const uint4*>(cell + 512 + lane * 16);
+        const uint2 sa = *reinterpret_cast<const uint2*>(cell + 1024 + g * 8), sb = *reinterpret_cast<const uint2*>(cell + 1024 + (g + 8) * 8);
+        const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
-    for (int j = 0; j < NB; j++) {
-        const uint2 c = *reinterpret_cast<const uint2*>(codes + (l + 16 * j) * 8);
-        s = fmaf(g2_dot16(c, x + 16 * j), g2_scale(scales[l + 16 * j]), s);
+        for (int p = 0; p < 4; p++) {
+            uint32_t a[4], b[4];
+            g2_cvt8(wa[p], a); g2_cvt8(wb[p], b);
+            const uint32_t sA = g2_scale2((p < 2 ? sa.x : sa.y) >> (16 * (p & 1))), sB = g2_scale2((p < 2 ? sb.x : sb.y) >> (16 * (p & 1)));
+            uint2 x0 = make_uint2(0u, 0u), x1 = make_uint2(0u, 0u);
+            if (g < 3) {
+                x0 = *reinterpret_cast<const uint2*>(x + (2 * p * 3 + g) * 16 + t * 4);
+                x1 = *reinterpret_cast<const uint2*>(x + ((2 * p + 1) * 3 + g) * 16 + t * 4);
+            }
+            g2_mma(c, g2_mul2(a[0], sA), g2_mul2(b[0], sB), g2_mul2(a[1], sA), g2_mul2(b[1], sB), x0);
+            g2_mma(d, g2_mul2(a[2], sA), g2_mul2(b[2], sB), g2_mul2(a[3], sA), g2_mul2(b[3], sB), x1);
+        }
     }
+    // columns 0 and 1 of rows g, g + 8 are with the lanes t == 0, column 2 with t == 1
 #pragma unroll
-    for (int d = 1; d < 16; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    return s;
+    for (int q = 0; q < 4; q++) c[q] += d[q];
+    const float n0 = __shfl_down_sync(0xffffffffu, c[0], 1), n2 = __shfl_down_sync(0xffffffffu, c[2], 1);
+    constexpr float k1 = 1.0f / 2048.0f, k2 = k1 * k1;
+    lo = c[0] + c[1] * k1 + n0 * k2;
+    hi = c[2] + c[3] * k1 + n2 * k2;
 }
 
 template <int NB> struct G2Smem {
@@ -96,12 +110,13 @@ template <int NB> struct G2Smem {
     static constexpr int WB = 36 * D * D / 256;       // bytes of the largest phase: 4 D / 16 rows of D, or D / 16 rows of 4 D
     uint8_t w[2][WB];
     unsigned long long xa[D], xb[D], ctx[D], h[4 * D], qkv[192];
-    static constexpr int XS = 5 * D > G2_CAP + 1024 ? 5 * D : G2_CAP + 1024;
-    float xs[XS];                                     // input of the phase, padded; attention: scores, then [warp][64] partial outputs from G2_CAP on
-    float xres[D];                                    // residual stream
-    float part[4 * (D / 16)];                         // K quarters of the second projection
+    static constexpr int XS = 6 * D > G2_CAP + 1216 ? 6 * D : G2_CAP + 1216;
+    // input of a linear: three halves per element (then, for inputs of D elements, the K parts of its rows and the rows);
+    // attention: scores, from G2_CAP on [warp][64] partial outputs, then q, k and v of the position
+    float xs[XS];
+    float xres[D / 16];                               // this CTA's rows of the residual stream
+    float part[256];                                  // K parts of the second projection
     float red[4][G2_WARPS];
-    float q[64], k[64], v[64];
     uint64_t full[2], empty[2];
     volatile int abort_flag;
 };
@@ -133,43 +148,82 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 for (int ph = 0; ph < 4 && ok; ph++, n++) {
                     const HxGpt2LayerDev& ly = P.layers[L];
                     const uint32_t rows = ph == 0 ? 3 * ROWS : (ph == 2 ? 4 * ROWS : ROWS), kb = ph == 3 ? 4 * D : D;
-                    const uint32_t cb = rows * kb / 2, sb = rows * kb / 16;
+                    const uint32_t bytes = rows * kb / 16 * 9;
                     const int b = n & 1;
                     if (n >= 2 && !mb_wait(&S.empty[b], (uint32_t)((n >> 1) - 1) & 1u, ab)) { ok = false; break; }
-                    mb_expect(&S.full[b], cb + sb);
-                    bulk_load(S.w[b], ly.codes[ph] + (size_t)cta * cb, cb, &S.full[b]);
-                    bulk_load(S.w[b] + cb, ly.scales[ph] + (size_t)cta * sb, sb, &S.full[b]);
+                    mb_expect(&S.full[b], bytes);
+                    bulk_load(S.w[b], ly.t16[ph] + (size_t)cta * bytes, bytes, &S.full[b]);
                 }
             for (int i = n > 2 ? n - 2 : 0; i < n && !ok; i++) mb_drain(&S.full[i & 1], (uint32_t)(i >> 1) & 1u);
         }
     } else {
-        const int l = lane & 15, hw = warp * 2 + (lane >> 4);      // half-warp of the CTA
+        const int l = lane & 15, g = lane >> 2, t = lane & 3;
         // where this lane's stores go: CTA l of the cluster
         const uint32_t base = cl_map(s_u32(smem_raw), (uint32_t)l), me = s_u32(smem_raw);
-        const uint32_t d_xa = base + s_u32(S.xa) - me, d_xb = base + s_u32(S.xb) - me, d_h = base + s_u32(S.h) - me, d_qkv = base + s_u32(S.qkv) - me;
+        const uint32_t d_xa = base + s_u32(S.xa) - me, d_xb = base + s_u32(S.xb) - me, d_h = base + s_u32(S.h) - me;
         hx_grid_dep_wait();                                        // the token and the position come from the launch before
         const int pos = __ldcg(P.pos), tok = __ldcg(P.tok);
-        float xr[16 * NB];
+        __half* dig = reinterpret_cast<__half*>(S.xs);
+        float* part = S.xs + 3 * D / 2;                            // [NB][rows] of a linear with D inputs
+        float* yrow = part + NB * 4 * ROWS;
         int n = 0;                                                 // weight phases so far
-        auto take = [&](int slice) {                               // the phase's input into registers, its weights complete
-            const float* src = S.xs + slice * (D / 16) * 20;
-#pragma unroll
-            for (int j = 0; j < NB; j++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const float4 v = *reinterpret_cast<const float4*>(src + (l + 16 * j) * 20 + c * 4);
-                    xr[16 * j + 4 * c] = v.x; xr[16 * j + 4 * c + 1] = v.y; xr[16 * j + 4 * c + 2] = v.z; xr[16 * j + 4 * c + 3] = v.w;
-                }
-            (void)mb_wait(&S.full[n & 1], (uint32_t)(n >> 1) & 1u, ab);
-            __syncwarp();
-        };
+        auto take = [&]() { (void)mb_wait(&S.full[n & 1], (uint32_t)(n >> 1) & 1u, ab); __syncwarp(); };      // the phase's weights are complete
         auto give = [&]() { __syncwarp(); if (lane == 0) mb_arrive(&S.empty[n & 1]); n++; };
-        // LayerNorm of the values this thread fetched (elements tid and tid + 512), result to xs, the values to xres
+        // The phase's input (elements tid, tid + 512, ... of K) scaled to at most one by a power of two, as three f16 terms
+        // (33 bits); returns the power.  Every thread is past its use of xs when the first barrier lets go.
+        auto split = [&](const auto& v, int K, int slot) {
+            constexpr int N = sizeof(v) / sizeof(float);
+            float mx = 0.0f;
+#pragma unroll
+            for (int i = 0; i < N; i++) if (tid + i * G2_CT < K) mx = fmaxf(mx, fabsf(v[i]));
+            mx = hx_warp_max(mx);
+            if (lane == 0) S.red[slot][warp] = mx;
+            g2_sync();
+            mx = 0.0f;
+#pragma unroll
+            for (int i = 0; i < G2_WARPS; i++) mx = fmaxf(mx, S.red[slot][i]);
+            float sx = 1.0f;
+            if (mx > 0.0f && mx < INFINITY) sx = __uint_as_float(min((__float_as_uint(mx) >> 23) + 1u, 254u) << 23);
+            const float inv = 1.0f / sx;
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int k = tid + i * G2_CT;
+                if (k >= K) continue;
+                const float x = v[i] * inv;
+                const __half a = __float2half_rn(x);
+                const float r = (x - __half2float(a)) * 2048.0f;
+                const __half b = __float2half_rn(r);
+                __half* to = dig + g2_place(k);
+                to[0] = a; to[16] = b; to[32] = __float2half_rn((r - __half2float(b)) * 2048.0f);
+            }
+            g2_sync();
+            return sx;
+        };
+        // `rows` rows of D inputs: a warp takes (sixteen rows, 256 columns) at a time
+        auto linear = [&](int rows) {
+            take();
+            #pragma unroll 1
+            for (int u = warp; u < rows / 16 * NB; u += G2_WARPS) {
+                const int tile = u / NB, pt = u - tile * NB;
+                float lo, hi;
+                g2_cells(S.w[n & 1] + u * 2 * HX_T16_CELL, 2, dig + pt * 2 * 384, lo, hi);
+                if (t == 0) { part[pt * rows + tile * 16 + g] = lo; part[pt * rows + tile * 16 + g + 8] = hi; }
+            }
+            give();
+            g2_sync();
+        };
+        auto row_sum = [&](int rows, int rl) {
+            float s = part[rl];
+#pragma unroll
+            for (int i = 1; i < NB; i++) s += part[i * rows + rl];
+            return s;
+        };
+        // LayerNorm of the values this thread fetched (elements tid and tid + 512), this CTA's rows of them to xres; the result's terms to xs
         constexpr int PT = (D + G2_CT - 1) / G2_CT;
         auto layer_norm = [&](const float (&v)[PT], const float (&gg)[PT], const float (&bb)[PT]) {
             float s = 0.0f;
 #pragma unroll
-            for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) { s += v[i]; S.xres[tid + i * G2_CT] = v[i]; }
+            for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) { s += v[i]; const int e = tid + i * G2_CT - cta * ROWS; if (e >= 0 && e < ROWS) S.xres[e] = v[i]; }
             s = hx_warp_sum(s);
             if (lane == 0) S.red[0][warp] = s;
             g2_sync();
@@ -187,9 +241,10 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
 #pragma unroll
             for (int i = 0; i < G2_WARPS; i++) var += S.red[1][i];
             const float inv = rsqrtf(var / (float)D + P.eps);
+            float y[PT];
 #pragma unroll
-            for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) S.xs[g2_pad(tid + i * G2_CT)] = gg[i] * ((v[i] - mean) * inv) + bb[i];
-            g2_sync();
+            for (int i = 0; i < PT; i++) y[i] = gg[i] * ((v[i] - mean) * inv) + bb[i];
+            return split(y, D, 2);
         };
         #pragma unroll 1
         for (int L = 0; L < P.n_layers; L++) {
@@ -199,28 +254,22 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
             float* vc = P.vc + (size_t)L * (D / 64) * P.cap * 64;
             // ---- LayerNorm, qkv ----
             {
-                float v[PT], gg[PT], bb[PT], bias[(3 * ROWS + 31) / 32];
+                float v[PT], gg[PT], bb[PT];
 #pragma unroll
                 for (int i = 0; i < PT; i++) { const int e = tid + i * G2_CT; gg[i] = e < D ? __ldg(ly.ln1g + e) : 0.0f; bb[i] = e < D ? __ldg(ly.ln1b + e) : 0.0f; }
-#pragma unroll
-                for (int i = 0; i < (3 * ROWS + 31) / 32; i++) bias[i] = hw + 32 * i < 3 * ROWS ? __ldg(ly.bias[0] + cta * 3 * ROWS + hw + 32 * i) : 0.0f;
+                const float bias = tid < 3 * ROWS ? __ldg(ly.bias[0] + cta * 3 * ROWS + tid) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < PT; i++) {
                     const int e = tid + i * G2_CT;
                     v[i] = e >= D ? 0.0f : (L == 0 ? __ldg(P.emb + (size_t)tok * D + e) + __ldg(P.wpe + (size_t)pos * D + e) : g2_wait(&S.xb[e], (unsigned)L, ab));
                 }
-                layer_norm(v, gg, bb);
-                take(0);
-                const uint8_t* w = S.w[n & 1];
-                const float ts = ly.ts[0];
-#pragma unroll
-                for (int i = 0; i < (3 * ROWS + 31) / 32; i++) {
-                    const int rl = min(hw + 32 * i, 3 * ROWS - 1);
-                    const float y = g2_row<NB>(w + rl * (D / 2), w + 3 * ROWS * (D / 2) + rl * (D / 16), xr, l) * ts + bias[i];
-                    const int row = cta * 3 * ROWS + rl, sec = row / D, r = row - sec * D;
-                    if (hw + 32 * i < 3 * ROWS && l == (r >> 6)) g2_send(d_qkv + (uint32_t)(sec * 64 + (r & 63)) * 8, y, ep);
+                const float sc = layer_norm(v, gg, bb) * ly.ts[0];
+                linear(3 * ROWS);
+                if (tid < 3 * ROWS) {
+                    const int row = cta * 3 * ROWS + tid, sec = row / D, r = row - sec * D;
+                    g2_send(cl_map(s_u32(&S.qkv[sec * 64 + (r & 63)]), (uint32_t)(r >> 6)), row_sum(3 * ROWS, tid) * sc + bias, ep);
                 }
-                give();
+                g2_sync();                                         // (the head's own attention writes over the parts)
             }
             // ---- attention of head `cta` ----
             if (cta < D / 64) {
@@ -242,16 +291,17 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
 #pragma unroll
                     for (int i = 0; i < 8; i++) { const int key = k0 + kg + 32 * i; kr[i] = key < pos ? __ldcg(reinterpret_cast<const float4*>(vb + (size_t)key * 64 + c4 * 4)) : make_float4(0.f, 0.f, 0.f, 0.f); }
                 };
+                float* sq = S.xs + G2_CAP + 1024;                 // q, k, v of the position
                 load_k(0);
                 if (tid < 192) {
                     const float x = g2_wait(&S.qkv[tid], ep, ab);
-                    (tid < 64 ? S.q : (tid < 128 ? S.k : S.v))[tid & 63] = x;
+                    sq[tid] = x;
                     if (tid >= 64) (tid < 128 ? kc : vc)[((size_t)cta * P.cap + pos) * 64 + (tid & 63)] = x;
                 }
                 g2_sync();
                 float4 q4[4];
 #pragma unroll
-                for (int c = 0; c < 4; c++) q4[c] = *reinterpret_cast<const float4*>(S.q + (kp + 4 * c) * 4);
+                for (int c = 0; c < 4; c++) q4[c] = *reinterpret_cast<const float4*>(sq + (kp + 4 * c) * 4);
                 float* sc = S.xs;
                 float* pv = S.xs + G2_CAP;
                 float mx = -INFINITY;
@@ -263,7 +313,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                         float d = 0.0f;
 #pragma unroll
                         for (int c = 0; c < 4; c++) {
-                            const float4 k4 = key == pos ? *reinterpret_cast<const float4*>(S.k + (kp + 4 * c) * 4) : kr[4 * p + c];
+                            const float4 k4 = key == pos ? *reinterpret_cast<const float4*>(sq + 64 + (kp + 4 * c) * 4) : kr[4 * p + c];
                             d = fmaf(q4[c].x, k4.x, d); d = fmaf(q4[c].y, k4.y, d); d = fmaf(q4[c].z, k4.z, d); d = fmaf(q4[c].w, k4.w, d);
                         }
                         d += __shfl_xor_sync(0xffffffffu, d, 1); d += __shfl_xor_sync(0xffffffffu, d, 2);
@@ -291,7 +341,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                         const int key = k0 + kg + 32 * i;
                         if (key > pos) break;
                         const float p = sc[key];
-                        const float4 v4 = key == pos ? *reinterpret_cast<const float4*>(S.v + c4 * 4) : kr[i];
+                        const float4 v4 = key == pos ? *reinterpret_cast<const float4*>(sq + 128 + c4 * 4) : kr[i];
                         acc.x = fmaf(p, v4.x, acc.x); acc.y = fmaf(p, v4.y, acc.y); acc.z = fmaf(p, v4.z, acc.z); acc.w = fmaf(p, v4.w, acc.w);
                     }
                 }
@@ -312,71 +362,66 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
             }
             // ---- proj + residual ----
             {
-                float bias[(ROWS + 31) / 32];
+                constexpr int RT = (ROWS * 16 + G2_CT - 1) / G2_CT;
+                float bias[RT], cv[PT];
 #pragma unroll
-                for (int i = 0; i < (ROWS + 31) / 32; i++) bias[i] = hw + 32 * i < ROWS ? __ldg(ly.bias[1] + cta * ROWS + hw + 32 * i) : 0.0f;
-                float cv[PT];
+                for (int i = 0; i < RT; i++) bias[i] = tid + i * G2_CT < ROWS * 16 ? __ldg(ly.bias[1] + cta * ROWS + ((tid + i * G2_CT) >> 4)) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < PT; i++) cv[i] = tid + i * G2_CT < D ? g2_wait(&S.ctx[tid + i * G2_CT], ep, ab) : 0.0f;
-                g2_sync();                                         // (the head's own attention has used xs)
+                const float sc = split(cv, D, 0) * ly.ts[1];
+                linear(ROWS);
 #pragma unroll
-                for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) S.xs[g2_pad(tid + i * G2_CT)] = cv[i];
-                g2_sync();
-                take(0);
-                const uint8_t* w = S.w[n & 1];
-                const float ts = ly.ts[1];
-#pragma unroll
-                for (int i = 0; i < (ROWS + 31) / 32; i++) {
-                    const int rl = min(hw + 32 * i, ROWS - 1), row = cta * ROWS + rl;
-                    const float y = S.xres[row] + (g2_row<NB>(w + rl * (D / 2), w + ROWS * (D / 2) + rl * (D / 16), xr, l) * ts + bias[i]);
-                    if (hw + 32 * i < ROWS) g2_send(d_xa + (uint32_t)row * 8, y, ep);
+                for (int i = 0; i < RT; i++) {                     // (the sixteen lanes of a row send it to the sixteen CTAs)
+                    const int rl = (tid + i * G2_CT) >> 4;
+                    if (rl < ROWS) g2_send(d_xa + (uint32_t)(cta * ROWS + rl) * 8, S.xres[rl] + (row_sum(ROWS, rl) * sc + bias[i]), ep);
                 }
-                give();
             }
             // ---- LayerNorm, c_fc, gelu ----
             {
-                float v[PT], gg[PT], bb[PT], bias[(4 * ROWS + 31) / 32];
+                float v[PT], gg[PT], bb[PT];
 #pragma unroll
                 for (int i = 0; i < PT; i++) { const int e = tid + i * G2_CT; gg[i] = e < D ? __ldg(ly.ln2g + e) : 0.0f; bb[i] = e < D ? __ldg(ly.ln2b + e) : 0.0f; }
-#pragma unroll
-                for (int i = 0; i < (4 * ROWS + 31) / 32; i++) bias[i] = hw + 32 * i < 4 * ROWS ? __ldg(ly.bias[2] + cta * 4 * ROWS + hw + 32 * i) : 0.0f;
+                const float bias = tid < 4 * ROWS ? __ldg(ly.bias[2] + cta * 4 * ROWS + tid) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < PT; i++) v[i] = tid + i * G2_CT < D ? g2_wait(&S.xa[tid + i * G2_CT], ep, ab) : 0.0f;
-                layer_norm(v, gg, bb);
-                take(0);
-                const uint8_t* w = S.w[n & 1];
-                const float ts = ly.ts[2];
+                const float sc = layer_norm(v, gg, bb) * ly.ts[2];
+                linear(4 * ROWS);
+                if (tid < 4 * ROWS) yrow[tid] = g2_gelu(row_sum(4 * ROWS, tid) * sc + bias);
+                g2_sync();
 #pragma unroll
-                for (int i = 0; i < (4 * ROWS + 31) / 32; i++) {
-                    const int rl = min(hw + 32 * i, 4 * ROWS - 1);
-                    const float y = g2_gelu(g2_row<NB>(w + rl * (D / 2), w + 4 * ROWS * (D / 2) + rl * (D / 16), xr, l) * ts + bias[i]);
-                    if (hw + 32 * i < 4 * ROWS) g2_send(d_h + (uint32_t)(cta * 4 * ROWS + rl) * 8, y, ep);
-                }
-                give();
+                for (int i = tid; i < 4 * ROWS * 16; i += G2_CT) g2_send(d_h + (uint32_t)(cta * 4 * ROWS + (i >> 4)) * 8, yrow[i >> 4], ep);
             }
-            // ---- second projection + residual: K quarter warp & 3, rows (warp >> 2) * 2 + half, + 8, ... ----
+            // ---- second projection + residual: WT warps per sixteen rows, each every WT-th part of 256 columns ----
             {
-                float hv[4 * PT];
+                constexpr int WT = G2_WARPS / NB, RT = (ROWS * 16 + G2_CT - 1) / G2_CT;
+                float hv[4 * PT], bias[RT];
+#pragma unroll
+                for (int i = 0; i < RT; i++) bias[i] = tid + i * G2_CT < ROWS * 16 ? __ldg(ly.bias[3] + cta * ROWS + ((tid + i * G2_CT) >> 4)) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < 4 * PT; i++) hv[i] = tid + i * G2_CT < 4 * D ? g2_wait(&S.h[tid + i * G2_CT], ep, ab) : 0.0f;
-#pragma unroll
-                for (int i = 0; i < 4 * PT; i++) if (tid + i * G2_CT < 4 * D) S.xs[g2_pad(tid + i * G2_CT)] = hv[i];
-                g2_sync();
-                const int sl = warp & 3, r0 = (warp >> 2) * 2 + (lane >> 4);
-                take(sl);
-                const uint8_t* w = S.w[n & 1];
-                const float ts = ly.ts[3];
-#pragma unroll
-                for (int i = 0; i < ROWS / 8; i++) {
-                    const int rl = r0 + 8 * i;
-                    const float y = g2_row<NB>(w + rl * (2 * D) + sl * (D / 2), w + ROWS * (2 * D) + rl * (D / 4) + sl * (D / 16), xr, l);
-                    if (l == 0) S.part[sl * ROWS + rl] = y;
+                const float sc = split(hv, 4 * D, 0) * ly.ts[3];
+                take();
+                const int tile = warp % NB, j = warp / NB;
+                if (j < WT) {
+                    float lo = 0.0f, hi = 0.0f;
+                    #pragma unroll 1
+                    for (int pt = j; pt < 4 * NB; pt += WT) {
+                        float a, b;
+                        g2_cells(S.w[n & 1] + (tile * 8 * NB + pt * 2) * HX_T16_CELL, 2, dig + pt * 2 * 384, a, b);
+                        lo += a; hi += b;
+                    }
+                    if (t == 0) { S.part[j * ROWS + tile * 16 + g] = lo; S.part[j * ROWS + tile * 16 + g + 8] = hi; }
                 }
                 give();
                 g2_sync();
-                for (int i = tid; i < ROWS * 16; i += G2_CT) {     // (i & 15 is this lane's l: the row goes to CTA l)
-                    const int rl = i >> 4, row = cta * ROWS + rl;
-                    const float y = S.xres[row] + (((S.part[rl] + S.part[ROWS + rl]) + (S.part[2 * ROWS + rl] + S.part[3 * ROWS + rl])) * ts + __ldg(ly.bias[3] + row));
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    const int rl = (tid + i * G2_CT) >> 4, row = cta * ROWS + rl;
+                    if (rl >= ROWS) continue;
+                    float s = S.part[rl];
+#pragma unroll
+                    for (int q = 1; q < WT; q++) s += S.part[q * ROWS + rl];
+                    const float y = S.xres[rl] + (s * sc + bias[i]);
                     if (L + 1 < P.n_layers) g2_send(d_xb + (uint32_t)row * 8, y, ep);
                     else if (l == 0) P.x_out[row] = y;
                 }

@@ -3,7 +3,7 @@
 #include "hx_common.cuh"
 
 struct HxGpt2LayerDev {                     // one layer, in device memory; order: qkv, proj, c_fc, second proj
-    const uint8_t* codes[4]; const uint8_t* scales[4];      // dense decode layout (hx_repack_d16)
+    const uint8_t* t16[4];                  // A-fragment order (hx_repack_t16)
     const float* bias[4]; float ts[4];
     const float *ln1g, *ln1b, *ln2g, *ln2b;
 };

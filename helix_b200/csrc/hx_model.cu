@@ -80,6 +80,7 @@ struct hx_model {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool pdl = true;
     bool persist = true;                 // one cooperative kernel per token instead of the launch graph
+    bool want_t16 = false;                // T16 cells beside the dense layout (GPT-2 layers in one launch)
     bool want_t128 = true, use_tc = true; // linear phases on the tensor cores (tcgen05) inside the persistent kernel
     float* tc_partial = nullptr; unsigned* tc_cnt = nullptr; int bdig_bytes = 0, tc_ring = 0; size_t tc_units_max = 0; int tc_tiles_max = 0;
     HxPhase *ph_decode = nullptr, *ph_prefill = nullptr; int nph_decode = 0, nph_prefill = 0;
@@ -150,7 +151,8 @@ int alloc_fused(hx_model* m, Fused& f, int N, int K) {
     if (!m->persist) {
         rc = dalloc(m, &f.codes, (size_t)N * (f.Kd / 2)); if (rc) return rc;
         rc = dalloc(m, &f.scales, (size_t)N * (f.Kd / 16)); if (rc) return rc;
-    } else if (!m->use_tc) {
+    }
+    if (m->persist ? !m->use_tc : m->want_t16) {
         rc = dalloc(m, &f.t16, hx_t16_bytes(N, K)); if (rc) return rc;
         HX_CUDA(cudaMemsetAsync(f.t16, 0, hx_t16_bytes(N, K), m->st));
     }
@@ -855,13 +857,13 @@ int finish_init(hx_model* m) {
         if (rc) return rc;
     }
     if (m->persist) return HX_OK;               // the per-op launch graphs belong to the graph engine alone
-    if (m->cfg.arch == 0 && hx_gpt2_step_fits(m->cfg, m->kv_cap)) {
+    if (m->cfg.arch == 0 && m->layers[0].qkv.t16 && hx_gpt2_step_fits(m->cfg, m->kv_cap)) {
         std::vector<HxGpt2LayerDev> tab;
         for (auto& ly : m->layers) {
             HxGpt2LayerDev d = {};
             const Fused* f[4] = {&ly.qkv, &ly.o, &ly.gu, &ly.down};
             const float* b[4] = {ly.b_qkv, ly.b_o, ly.b_fc, ly.b_down};
-            for (int i = 0; i < 4; i++) { d.codes[i] = f[i]->codes; d.scales[i] = f[i]->scales; d.bias[i] = b[i]; d.ts[i] = f[i]->ts[0]; }
+            for (int i = 0; i < 4; i++) { d.t16[i] = f[i]->t16; d.bias[i] = b[i]; d.ts[i] = f[i]->ts[0]; }
             d.ln1g = ly.in_g; d.ln1b = ly.ln1_b; d.ln2g = ly.post_g; d.ln2b = ly.ln2_b;
             tab.push_back(d);
         }
@@ -1007,6 +1009,7 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
         if (cudaMalloc(&stage, maxel * 4) != cudaSuccess || cudaMalloc(&wtmp, maxrows * (kp / 7) * 4) != cudaSuccess ||
             cudaMalloc(&mtmp, maxrows * (kp / 16)) != cudaSuccess || cudaMalloc(&tstmp, 256) != cudaSuccess) { rc = hx_fail(HX_ERR_NOMEM, "GPT-2 staging"); break; }
         m->layers.resize(c.n_layers);
+        m->want_t16 = hx_gpt2_step_fits(c, kv_cap);
         for (int L = 0; L < c.n_layers && !rc; L++) {
             Layer& ly = m->layers[L]; const hx_gpt2_layer& hl = w->layers[L];
             if (!hl.ln1_g || !hl.ln1_b || !hl.w_qkv || !hl.b_qkv || !hl.w_proj || !hl.b_proj || !hl.ln2_g || !hl.ln2_b || !hl.w_fc || !hl.b_fc || !hl.w_proj2 || !hl.b_proj2) {
@@ -1023,6 +1026,7 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
         if (rc) break;
         if ((rc = gpt2_upload(m, &m->emb, w->wte, (size_t)NV * DM)) || (rc = gpt2_upload(m, &m->wpe, w->wpe, (size_t)c.max_ctx * DM)) ||
             (rc = gpt2_upload(m, &m->final_g, w->lnf_g, DM)) || (rc = gpt2_upload(m, &m->final_b, w->lnf_b, DM))) break;
+        m->want_t16 = false;
         if ((rc = gpt2_linear(m, m->head, w->wte, NV, DM, stage, wtmp, mtmp, tstmp))) break;       // tied lm_head
         HX_CUDA(cudaStreamSynchronize(m->st));
         rc = finish_init(m);
