@@ -157,10 +157,12 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
             for (int i = n > 2 ? n - 2 : 0; i < n && !ok; i++) mb_drain(&S.full[i & 1], (uint32_t)(i >> 1) & 1u);
         }
     } else {
-        const int l = lane & 15, g = lane >> 2, t = lane & 3;
-        // where this lane's stores go: CTA l of the cluster
-        const uint32_t base = cl_map(s_u32(smem_raw), (uint32_t)l), me = s_u32(smem_raw);
-        const uint32_t d_xa = base + s_u32(S.xa) - me, d_xb = base + s_u32(S.xb) - me, d_h = base + s_u32(S.h) - me;
+        const int g = lane >> 2, t = lane & 3;
+        // What every CTA needs is sent to CTA w by warp w, consecutive rows by consecutive lanes: whole lines through the
+        // cluster's network (the sixteen lanes of a row each to another CTA took 4500 cycles for the 192 rows of c_fc).
+        static_assert(G2_WARPS == G2_CTAS, "a warp per destination");
+        const uint32_t base = cl_map(s_u32(smem_raw), (uint32_t)warp), me = s_u32(smem_raw);
+        const uint32_t d_xa = base + s_u32(S.xa) - me, d_xb = base + s_u32(S.xb) - me, d_h = base + s_u32(S.h) - me, d_ctx = base + s_u32(S.ctx) - me;
         hx_grid_dep_wait();                                        // the token and the position come from the launch before
         const int pos = __ldcg(P.pos), tok = __ldcg(P.tok);
         __half* dig = reinterpret_cast<__half*>(S.xs);
@@ -223,10 +225,12 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
         auto layer_norm = [&](const float (&v)[PT], const float (&gg)[PT], const float (&bb)[PT]) {
             float s = 0.0f;
 #pragma unroll
-            for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) { s += v[i]; const int e = tid + i * G2_CT - cta * ROWS; if (e >= 0 && e < ROWS) S.xres[e] = v[i]; }
+            for (int i = 0; i < PT; i++) if (tid + i * G2_CT < D) s += v[i];
             s = hx_warp_sum(s);
             if (lane == 0) S.red[0][warp] = s;
-            g2_sync();
+            g2_sync();                                             // (every warp has sent its rows: xres may change)
+#pragma unroll
+            for (int i = 0; i < PT; i++) { const int e = tid + i * G2_CT - cta * ROWS; if (e >= 0 && e < ROWS) S.xres[e] = v[i]; }
             float mean = 0.0f;
 #pragma unroll
             for (int i = 0; i < G2_WARPS; i++) mean += S.red[0][i];
@@ -355,24 +359,24 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 const int dim = tid >> 3, p8 = tid & 7;
                 float o = pv[p8 * 64 + dim] + pv[(p8 + 8) * 64 + dim];
                 o += __shfl_xor_sync(0xffffffffu, o, 1); o += __shfl_xor_sync(0xffffffffu, o, 2); o += __shfl_xor_sync(0xffffffffu, o, 4);
-                o /= lsum;
-                const uint32_t off = s_u32(&S.ctx[cta * 64 + dim]);
-                g2_send(cl_map(off, (uint32_t)p8), o, ep);
-                g2_send(cl_map(off, (uint32_t)p8 + 8u), o, ep);
+                if (p8 == 0) sq[dim] = o / lsum;                   // (q has been used)
+                g2_sync();
+#pragma unroll
+                for (int i = 0; i < 64; i += 32) g2_send(d_ctx + (uint32_t)(cta * 64 + i + lane) * 8, sq[i + lane], ep);
             }
             // ---- proj + residual ----
             {
-                constexpr int RT = (ROWS * 16 + G2_CT - 1) / G2_CT;
-                float bias[RT], cv[PT];
+                constexpr int RL = (ROWS + 31) / 32;
+                float bias[RL], cv[PT];
 #pragma unroll
-                for (int i = 0; i < RT; i++) bias[i] = tid + i * G2_CT < ROWS * 16 ? __ldg(ly.bias[1] + cta * ROWS + ((tid + i * G2_CT) >> 4)) : 0.0f;
+                for (int i = 0; i < RL; i++) bias[i] = lane + 32 * i < ROWS ? __ldg(ly.bias[1] + cta * ROWS + lane + 32 * i) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < PT; i++) cv[i] = tid + i * G2_CT < D ? g2_wait(&S.ctx[tid + i * G2_CT], ep, ab) : 0.0f;
                 const float sc = split(cv, D, 0) * ly.ts[1];
                 linear(ROWS);
 #pragma unroll
-                for (int i = 0; i < RT; i++) {                     // (the sixteen lanes of a row send it to the sixteen CTAs)
-                    const int rl = (tid + i * G2_CT) >> 4;
+                for (int i = 0; i < RL; i++) {
+                    const int rl = lane + 32 * i;
                     if (rl < ROWS) g2_send(d_xa + (uint32_t)(cta * ROWS + rl) * 8, S.xres[rl] + (row_sum(ROWS, rl) * sc + bias[i]), ep);
                 }
             }
@@ -389,14 +393,14 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 if (tid < 4 * ROWS) yrow[tid] = g2_gelu(row_sum(4 * ROWS, tid) * sc + bias);
                 g2_sync();
 #pragma unroll
-                for (int i = tid; i < 4 * ROWS * 16; i += G2_CT) g2_send(d_h + (uint32_t)(cta * 4 * ROWS + (i >> 4)) * 8, yrow[i >> 4], ep);
+                for (int i = 0; i < 4 * ROWS; i += 32) g2_send(d_h + (uint32_t)(cta * 4 * ROWS + i + lane) * 8, yrow[i + lane], ep);
             }
             // ---- second projection + residual: WT warps per sixteen rows, each every WT-th part of 256 columns ----
             {
-                constexpr int WT = G2_WARPS / NB, RT = (ROWS * 16 + G2_CT - 1) / G2_CT;
-                float hv[4 * PT], bias[RT];
+                constexpr int WT = G2_WARPS / NB, RL = (ROWS + 31) / 32;
+                float hv[4 * PT], bias[RL];
 #pragma unroll
-                for (int i = 0; i < RT; i++) bias[i] = tid + i * G2_CT < ROWS * 16 ? __ldg(ly.bias[3] + cta * ROWS + ((tid + i * G2_CT) >> 4)) : 0.0f;
+                for (int i = 0; i < RL; i++) bias[i] = lane + 32 * i < ROWS ? __ldg(ly.bias[3] + cta * ROWS + lane + 32 * i) : 0.0f;
 #pragma unroll
                 for (int i = 0; i < 4 * PT; i++) hv[i] = tid + i * G2_CT < 4 * D ? g2_wait(&S.h[tid + i * G2_CT], ep, ab) : 0.0f;
                 const float sc = split(hv, 4 * D, 0) * ly.ts[3];
@@ -415,15 +419,15 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 give();
                 g2_sync();
 #pragma unroll
-                for (int i = 0; i < RT; i++) {
-                    const int rl = (tid + i * G2_CT) >> 4, row = cta * ROWS + rl;
+                for (int i = 0; i < RL; i++) {
+                    const int rl = lane + 32 * i, row = cta * ROWS + rl;
                     if (rl >= ROWS) continue;
                     float s = S.part[rl];
 #pragma unroll
                     for (int q = 1; q < WT; q++) s += S.part[q * ROWS + rl];
                     const float y = S.xres[rl] + (s * sc + bias[i]);
                     if (L + 1 < P.n_layers) g2_send(d_xb + (uint32_t)row * 8, y, ep);
-                    else if (l == 0) P.x_out[row] = y;
+                    else if (warp == 0) P.x_out[row] = y;
                 }
             }
         }
