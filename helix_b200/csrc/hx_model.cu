@@ -994,9 +994,10 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
     m->cfg = c; m->gcfg = c; m->cfg.qk_norm = 0; m->QD = c.d_model; m->KVD = c.d_model;
     m->kv_cap = kv_cap; m->batch = 1; m->flags = 0;
     // tokens one at a time through per-op kernels in one CUDA graph, prompts through the chunk GEMM (its weight cells beside
-    // the dense layout: 0.56 bytes per weight once more)
-    m->persist = false; m->use_tc = false; m->want_t128 = true;
-    { const char* pf = getenv("HX_PREFILL"); m->pf_batched = !(pf && strcmp(pf, "token") == 0); }
+    // the dense layout: 0.56 bytes per weight once more) where its attention takes the head size, else token by token
+    m->persist = false; m->use_tc = false;
+    { const char* pf = getenv("HX_PREFILL"); m->pf_batched = !(pf && strcmp(pf, "token") == 0) && hx_pf_head_dim(c.head_dim); }
+    m->want_t128 = m->pf_batched;
     int rc = HX_OK;
     float* stage = nullptr; int32_t* wtmp = nullptr; uint8_t* mtmp = nullptr; float* tstmp = nullptr;
     do {

@@ -737,6 +737,9 @@ void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, co
     HX_COUNT_LAUNCH(1);
 }
 
+// The threads of an attention CTA split into whole rows of the head size (P*V), and the q/k kernel has a variant per size.
+bool hx_pf_head_dim(int DH) { return DH == 32 || DH == 64 || DH == 128 || DH == 256; }
+
 void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
                   float eps, const float* cosT, const float* sinT, float* kc, float* vc, int cap, cudaStream_t st) {
     const dim3 grid((NH + 2 * NKV + PF_QK_W - 1) / PF_QK_W, n_tok);
@@ -784,7 +787,7 @@ int hx_pf_attn(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NK
                int cap, float scale, float* ctx, int ld_ctx, float* part, unsigned* tickets, int* err, cudaStream_t st) {
     const int GRP = NH / NKV;
     if (DH > 256 || DH % 32) return hx_fail(HX_ERR_ARG, "batched prefill attention: head_dim %d is not a multiple of 32 up to 256", DH);
-    if (PF_AT % DH) return hx_fail(HX_ERR_ARG, "batched prefill attention: head_dim %d does not divide %d", DH, PF_AT);
+    if (!hx_pf_head_dim(DH)) return hx_fail(HX_ERR_ARG, "batched prefill attention: head_dim %d does not divide %d", DH, PF_AT);
     if (!part || !tickets) return hx_fail(HX_ERR_ARG, "batched prefill attention: no scratch for the key runs");
     // a prefill chunk (one sequence, consecutive positions): four tokens share the tiles of a CTA
     auto smem_of = [&](int tg) { return (size_t)PF_ST * 2 * PF_TILE_BYTES + ((size_t)tg * GRP * DH + (size_t)tg * GRP * 128 + (size_t)(PF_AT / DH) * GRP * DH) * 4; };

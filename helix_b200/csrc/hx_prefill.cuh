@@ -36,6 +36,7 @@ void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, 
 // the tokens of a group in a prefill chunk.  `part` (hx_pf_attn_scratch floats) and `tickets` (n_tok * NKV words, zero
 // between launches) carry the runs' partial results; *err is raised when a bounded wait ran out.
 size_t hx_pf_attn_scratch(int n_tok, int NH, int NKV, int DH);
+bool hx_pf_head_dim(int DH);       // head sizes of the chunk kernels
 int hx_pf_attn(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* kc, const float* vc,
                int cap, float scale, float* ctx, int ld_ctx, float* part, unsigned* tickets, int* err, cudaStream_t st);
 

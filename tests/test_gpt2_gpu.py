@@ -71,3 +71,21 @@ def test_gpt2_teacher_forced_and_greedy(shape, seed):
     got, _ = gm.decode_loop(int(nx), 20, 12)
     assert list(got) == want
     gm.close()
+
+
+@pytest.mark.parametrize("d_model,n_heads", [(192, 2), (320, 2), (384, 2), (448, 2)])
+def test_prompt_with_a_head_size_the_chunk_attention_does_not_take(d_model, n_heads):
+    """head_dim 96, 160, 192, 224: prompt and continuation token by token, in prefill() and in generate()."""
+    shape = dict(n_layers=2, d_model=d_model, n_heads=n_heads, d_ff=2 * d_model, vocab=301, max_ctx=40)
+    wt = synth(shape, d_model)
+    om, gm = OracleGpt2(shape, wt, 40), hb.Model.gpt2(shape, wt, kv_cap=40)
+    ids = np.random.default_rng(d_model).integers(0, 301, 27).astype(np.int32)
+    for p, t in enumerate(ids):
+        lo = om.decode(int(t), p)
+    nx, lg = gm.prefill(ids, want_logits=True)
+    assert np.max(np.abs(lo - lg)) < 2e-4 and nx == int(np.argmax(lo))
+    want = [nx]
+    for i in range(5):
+        want.append(int(np.argmax(om.decode(want[-1], 27 + i))))
+    assert list(gm.generate(ids, 6)[0]) == want
+    gm.close()
