@@ -99,7 +99,8 @@ struct hx_model {
     float* tp_buf = nullptr; size_t tp_buf_floats = 0; float* tp_peer[8] = {nullptr}; bool tp_connected = false; unsigned tp_launches = 0;
     float* x2 = nullptr; int tp_nbar = 0;
     HxGpt2LayerDev* g2_layers = nullptr;           // GPT-2: layer table of the one-launch layers (null: per-op launches)
-    // batched prefill (chunks of up to pf_tb tokens through the tcgen05 GEMM); buffers are created on first use
+    // chunk path (up to pf_tb tokens through the tcgen05 GEMM); one allocation, pf_buf, made on first use: pf_tb > 0 says it stands
+    void* pf_buf = nullptr;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
     int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
     uint8_t* pf_pieces = nullptr; size_t pf_pieces_bytes = 0; int pf_ctx_hint = 0;      // bf16 terms of K and V of a layer for the tensor-core attention, grown to the longest context seen
@@ -118,6 +119,12 @@ struct hx_model {
 
 namespace {
 
+cudaError_t dev_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(p, bytes); }
+    return e;
+}
+
 // Device memory of a model.  Small buffers (gains, biases, scratch words: several hundred of them) are cut from slabs, since
 // an allocation of the driver's costs tens of microseconds whatever its size; `own`: an allocation of its own all the same.
 template <typename T>
@@ -132,8 +139,7 @@ int dalloc(hx_model* m, T** p, size_t n, bool own = false) {
     }
     void* q = nullptr;
     const size_t want = small ? SLAB : bytes;
-    cudaError_t e = cudaMalloc(&q, want);
-    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(&q, want); }
+    const cudaError_t e = dev_malloc(&q, want);
     if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want, cudaGetErrorString(e));
     m->allocs.push_back(q);
     if (small) { m->slab = (uint8_t*)q + bytes; m->slab_left = SLAB - bytes; }
@@ -925,6 +931,7 @@ HX_API int hx_model_free(hx_model* m) {
     for (int w = 0; w < 8; w++)                      // mappings of the peers' exchange buffers
         if (m->tp_peer[w] && w != m->tp_rank) cudaIpcCloseMemHandle(m->tp_peer[w]);
     for (void* p : m->allocs) cudaFree(p);
+    if (m->pf_buf) cudaFree(m->pf_buf);
     if (m->pf_pieces) cudaFree(m->pf_pieces);
     if (m->h_flags) cudaFreeHost(m->h_flags);
     for (cudaEvent_t e : m->prof_ev) cudaEventDestroy(e);
@@ -1305,35 +1312,60 @@ HX_API int hx_decode_step(hx_model* m, const int32_t* ids, int pos, int32_t* nex
 }
 
 // ---- batched prefill ---------------------------------------------------------------------------------
-static int pf_alloc(hx_model* m) {
-    if (m->pf_x) return HX_OK;
-    { const int prc = hx_gemm_dig_prepare(); if (prc) return prc; }
+// Buffers for chunks of `want` tokens: a batch step, a verify window and a shard's chunk take HX_PF_TB, a prompt what the cache
+// holds up to HX_PF_MAX.  Where memory is short a prompt makes do with smaller chunks; a failed attempt leaves what was there.
+static int pf_alloc(hx_model* m, int want) {
     const hx_config& c = m->cfg;
-    int tb = m->kv_cap < HX_PF_MAX ? m->kv_cap : HX_PF_MAX;
-    if (tb < HX_PF_TB || m->tp_world > 1) tb = HX_PF_TB;       // (a shard's exchange areas hold HX_PF_TB tokens)
-    tb = (tb + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK * HX_TC_MAX_TOK;
-    int maxK = c.d_model > m->QD ? c.d_model : m->QD; if (c.d_ff > maxK) maxK = c.d_ff;
-    const size_t cells = (size_t)((maxK + 255) / 256) * (tb / HX_TC_MAX_TOK) * (HX_TC_GROUP_COLS * 128);
-    m->pf_gu_ld = m->layers.empty() ? 64 : m->layers[0].gu.tiles128 * (c.arch == 0 ? 128 : 64);      // hidden size rounded up to whole tiles
+    auto groups_of = [](int t) { return (t + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK; };
+    if (want > HX_PF_MAX) want = HX_PF_MAX;
+    if (want < HX_PF_TB || m->tp_world > 1) want = HX_PF_TB;       // (a shard's exchange areas hold HX_PF_TB tokens)
+    int tb = groups_of(want) * HX_TC_MAX_TOK;
+    if (m->pf_tb >= tb) return HX_OK;
     int rc;
-    if ((rc = dalloc(m, &m->pf_x, (size_t)tb * c.d_model))) return rc;
-    if ((rc = dalloc(m, &m->pf_qkv, (size_t)tb * (m->QD + 2 * m->KVD)))) return rc;
-    if ((rc = dalloc(m, &m->pf_ctx, (size_t)tb * m->QD))) return rc;
-    if ((rc = dalloc(m, &m->pf_gu, (size_t)tb * m->pf_gu_ld))) return rc;
-    if ((rc = dalloc(m, &m->pf_scale, (size_t)tb))) return rc;
-    if ((rc = dalloc(m, &m->pf_cells, cells))) return rc;
-    if (m->tp_world > 1 && (rc = dalloc(m, &m->pf_part, (size_t)HX_PF_TB * c.d_model))) return rc;
-    if ((rc = dalloc(m, &m->pf_err, (size_t)4))) return rc;
-    if ((rc = dalloc(m, &m->d_pf_pos, (size_t)4))) return rc;
-    if ((rc = dalloc(m, &m->pf_att_part, hx_pf_attn_scratch(tb, c.n_heads, c.n_kv_heads, c.head_dim)))) return rc;
-    if ((rc = dalloc(m, &m->pf_att_tickets, (size_t)tb * c.n_kv_heads))) return rc;
+    if (!m->pf_tb && (rc = hx_gemm_dig_prepare())) return rc;
+    int maxK = c.d_model > m->QD ? c.d_model : m->QD; if (c.d_ff > maxK) maxK = c.d_ff;
+    const size_t cell_n = (size_t)((maxK + 255) / 256) * (HX_TC_GROUP_COLS * 128);      // per group of tokens
+    const int gu_rows = m->layers.empty() ? 128 : m->layers[0].gu.tiles128 * 128;
+    const int gu_ld = c.arch == 0 ? gu_rows : gu_rows / 2;         // hidden size rounded up to whole tiles
+    // sums so far of the linears whose K is done in blocks: residual ones (d_model rows) and gate/up
+    const size_t acc_n = (size_t)(gu_rows > c.d_model ? gu_rows : c.d_model);
+    struct { void** p; size_t bytes; } item[11];
+    void* q = nullptr;
+    size_t total = 0, off = 0;
+    int n = 0;
+    for (;; tb = groups_of(tb / 2) * HX_TC_MAX_TOK) {
+        const size_t t = (size_t)tb;
+        n = 0;
+        item[n++] = {(void**)&m->pf_x, t * c.d_model * 4};
+        item[n++] = {(void**)&m->pf_qkv, t * (m->QD + 2 * m->KVD) * 4};
+        item[n++] = {(void**)&m->pf_ctx, t * m->QD * 4};
+        item[n++] = {(void**)&m->pf_gu, t * gu_ld * 4};
+        item[n++] = {(void**)&m->pf_scale, t * 4};
+        item[n++] = {(void**)&m->pf_cells, groups_of(tb) * cell_n};
+        item[n++] = {(void**)&m->pf_acc, t * acc_n * 4};
+        item[n++] = {(void**)&m->pf_att_part, hx_pf_attn_scratch(tb, c.n_heads, c.n_kv_heads, c.head_dim) * 4};
+        item[n++] = {(void**)&m->pf_att_tickets, t * c.n_kv_heads * 4};
+        item[n++] = {(void**)&m->pf_err, 16};
+        if (m->tp_world > 1) item[n++] = {(void**)&m->pf_part, (size_t)HX_PF_TB * c.d_model * 4};
+        total = 256;                                               // (the chunk's position)
+        for (int i = 0; i < n; i++) total += (item[i].bytes + 255) & ~(size_t)255;
+        const cudaError_t e = dev_malloc(&q, total);
+        if (e == cudaSuccess) break;
+        (void)cudaGetLastError();
+        if (e != cudaErrorMemoryAllocation) return hx_fail(HX_ERR_CUDA, "cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
+        if (m->pf_tb && groups_of(tb / 2) * HX_TC_MAX_TOK <= m->pf_tb) return HX_OK;
+        if (tb / 2 < HX_PF_TB) return hx_fail(HX_ERR_NOMEM, "chunk path: cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
+    }
+    cudaError_t e = cudaStreamSynchronize(m->st);
+    if (e != cudaSuccess) { cudaFree(q); return hx_fail(HX_ERR_CUDA, "chunk path: %s", cudaGetErrorString(e)); }
+    if (m->g_bstep) { cudaGraphExecDestroy(m->g_bstep); m->g_bstep = nullptr; }      // (it holds the old addresses)
+    if (m->pf_buf) cudaFree(m->pf_buf);
+    m->pf_buf = q; m->pf_tb = 0;
+    m->d_pf_pos = (int*)q; off = 256;
+    for (int i = 0; i < n; i++) { *item[i].p = (uint8_t*)q + off; off += (item[i].bytes + 255) & ~(size_t)255; }
+    m->pf_gu_ld = gu_ld;
     HX_CUDA(cudaMemsetAsync(m->pf_att_tickets, 0, (size_t)tb * c.n_kv_heads * 4, m->st));
     HX_CUDA(cudaMemsetAsync(m->pf_err, 0, 16, m->st));
-    {   // sums so far of the linears whose K is done in blocks: residual ones (d_model rows) and gate/up
-        size_t w = (size_t)c.d_model;
-        for (auto& ly : m->layers) if ((size_t)ly.gu.tiles128 * 128 > w) w = (size_t)ly.gu.tiles128 * 128;
-        if ((rc = dalloc(m, &m->pf_acc, (size_t)tb * w))) return rc;
-    }
     m->pf_tb = tb;
     return HX_OK;
 }
@@ -1422,18 +1454,16 @@ static int pf_enqueue_chunk(hx_model* m, int t0, int n) {
 }
 
 // ---- batched decode: n_seq independent sequences, one token each, in chunks of HX_PF_TB ----------------
-static int bd_alloc(hx_model* m) {
-    int rc = pf_alloc(m); if (rc) return rc;
-    if (m->d_bids) return HX_OK;
-    m->b_cap = ((m->batch + HX_PF_TB - 1) / HX_PF_TB) * HX_PF_TB;
-    if ((rc = dalloc(m, &m->d_bids, (size_t)m->b_cap))) return rc;
-    if ((rc = dalloc(m, &m->d_bpos, (size_t)m->b_cap))) return rc;
-    if ((rc = dalloc(m, &m->d_bseq, (size_t)m->b_cap))) return rc;
-    if ((rc = dalloc(m, &m->d_bnext, (size_t)m->b_cap))) return rc;
+static int bd_alloc(hx_model* m) {      // b_cap > 0 says the buffers stand; a failed attempt goes on from what it got
+    int rc = pf_alloc(m, HX_PF_TB); if (rc) return rc;
+    if (m->b_cap) return HX_OK;
+    const int cap = ((m->batch + HX_PF_TB - 1) / HX_PF_TB) * HX_PF_TB;
+    for (int** p : {&m->d_bids, &m->d_bpos, &m->d_bseq, &m->d_bnext}) if (!*p && (rc = dalloc(m, p, (size_t)cap))) return rc;
     if (!m->pf_logits && (rc = dalloc(m, &m->pf_logits, (size_t)HX_PF_TB * m->cfg.vocab))) return rc;
-    std::vector<int> seq(m->b_cap);
-    for (int i = 0; i < m->b_cap; i++) seq[i] = i;
-    HX_CUDA(cudaMemcpy(m->d_bseq, seq.data(), (size_t)m->b_cap * 4, cudaMemcpyHostToDevice));
+    std::vector<int> seq(cap);
+    for (int i = 0; i < cap; i++) seq[i] = i;
+    HX_CUDA(cudaMemcpy(m->d_bseq, seq.data(), (size_t)cap * 4, cudaMemcpyHostToDevice));
+    m->b_cap = cap;
     return HX_OK;
 }
 
@@ -1468,7 +1498,7 @@ static int bd_enqueue_step(hx_model* m, int n_seq) {
 // *d_pos = T.
 static int run_prefill_batched(hx_model* m, int T, int seq) {
     const hx_config& c = m->cfg;
-    int rc = pf_alloc(m); if (rc) return rc;
+    int rc = pf_alloc(m, m->kv_cap); if (rc) return rc;
     const int ps[2] = {0, seq};                      // first position of the chunk, KV slot of the sequence
     HX_CUDA(cudaMemcpyAsync(m->d_pf_pos, ps, 8, cudaMemcpyHostToDevice, m->st));
     const int nch = (T + m->pf_tb - 1) / m->pf_tb, gr = (T + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
@@ -1491,7 +1521,7 @@ static int run_prefill(hx_model* m, const int32_t* ids, int T, int seq = 0) {
     if (m->tp_world > 1 && m->use_tc && m->pf_batched && m->head.t128 && m->use_df) {
         // a shard: positions [0, T-1) in chunks (the exchanges are epoch-numbered kernel arguments, so no graph replay),
         // the last position through the decode kernel, which holds the arg-max over the ranks' vocabulary slices
-        int rc = pf_alloc(m); if (rc) return rc;
+        int rc = pf_alloc(m, HX_PF_TB); if (rc) return rc;
         const hx_config& c = m->cfg;
         const bool slot = seq != 0 || m->batch > 1;       // a slot of a batch: everything through the chunk path
         const int Tc = slot ? T : T - 1;
@@ -1638,7 +1668,7 @@ HX_API int hx_pld_draft(const int32_t* ids, int T, int k_min, int k_max, int m, 
 static int spec_alloc(hx_model* m) {
     if (!m->use_tc || !m->pf_batched || !m->head.t128 || m->tp_world > 1 || m->cfg.arch == 0)
         return hx_fail(HX_ERR_STATE, "speculative decode needs the tensor-core engine with batched prefill on one GPU");
-    int rc = pf_alloc(m); if (rc) return rc;
+    int rc = pf_alloc(m, m->kv_cap); if (rc) return rc;
     if (!m->pf_logits && (rc = dalloc(m, &m->pf_logits, (size_t)HX_PF_TB * m->cfg.vocab))) return rc;
     if (!m->sp_next && (rc = dalloc(m, &m->sp_next, (size_t)HX_PF_TB))) return rc;
     if (!m->sp_margin && (rc = dalloc(m, &m->sp_margin, (size_t)HX_PF_TB))) return rc;

@@ -5,7 +5,7 @@
 
 #define HX_PF_TB 64                // tokens per chunk of the batched decode (its logits take vocab floats each), of a verify window and inside a tensor-parallel group
 #define HX_PF_MAX 1008             // tokens per chunk of a prompt: 42 groups of 24.  A launch's ramp and drain (about 6 us) are a
-                                   // twentieth of its work there; the activations of a chunk stay within about 200 MB
+                                   // twentieth of its work there; the chunk's buffers are 270 MB at the 8B shape, 536 at the 32B
 
 // Where the tokens of a chunk sit.  Prefill: consecutive positions of one sequence starting at *posp (device memory, so
 // that captured launches can be replayed).  Batched decode: token t is at position pos_arr[t] of
