@@ -80,11 +80,11 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 
 // ---- thread-block clusters ----
 __device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cl_map(uint32_t saddr, uint32_t rank) { uint32_t a; asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank)); return a; }
+__device__ __forceinline__ uint32_t cl_map(uint32_t saddr, uint32_t rank) { uint32_t a; asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank)); return a; }
 __device__ __forceinline__ void cl_st(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory"); }
 __device__ __forceinline__ void cl_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory"); }
-// An arrival that orders nothing: for handing back a buffer whose values have been used.  (A release at cluster scope waits
-// for the thread's global stores as well, about a microsecond.)
+// An arrival that orders nothing by itself: for handing back a buffer after reads that the caller knows to be over.  (A release at
+// cluster scope waits for the thread's global stores as well, about a microsecond.)
 __device__ __forceinline__ void cl_arrive_relaxed(uint32_t bar) { asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory"); }
 __device__ __forceinline__ void cl_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -34,3 +34,18 @@ def test_prompt_logits_and_cache_rows(model, T):
         for a, b in zip(gm.kv_read(layer, head, 0, T), one.kv_read(layer, head, 0, T)):
             assert np.max(np.abs(a - b)) < 1e-4 * max(1.0, float(np.max(np.abs(b))))
     om.close(); gm.close(); one.close()
+
+
+def test_repeated_prompts_are_bit_equal(model):
+    """Many units per CTA through the two receive buffers of the cluster: what a buffer held for one unit is read before the next
+    unit's sums arrive, so a prompt gives the same bits every time."""
+    gm = hb.Model.load(model, kv_cap=320)
+    ids = np.random.default_rng(7).integers(0, CFG["NV"], 301).astype(np.int32)
+    _, want = gm.prefill(ids, want_logits=True)
+    rows = gm.kv_read(0, 5, 0, 301)
+    for _ in range(40):
+        _, lg = gm.prefill(ids, want_logits=True)
+        assert np.array_equal(lg.view(np.uint32), want.view(np.uint32))
+    for a, b in zip(gm.kv_read(0, 5, 0, 301), rows):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    gm.close()
