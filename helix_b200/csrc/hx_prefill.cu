@@ -53,8 +53,10 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     hx_grid_dep_wait();
     const float* x = src + (size_t)t * ld;
     __shared__ float red[2 * PFD_T / 32];
-    __shared__ uint8_t codes[84];        // a pair of digits (each + 4) -> two codes, the more significant one in the high nibble
-    if (tid < 81) {
+    // a pair of digits (each + 4) -> two codes, the more significant one in the high nibble; indexes 81 to
+    // 99 come from infinite values (the conversion to an integer saturates), whose scale says what they are
+    __shared__ uint8_t codes[100];
+    if (tid < 100) {
         // E2M1 codes of -4, -3, -2, -1, 0, 1, 2, 3, 4: E D C A 0 2 4 5 6
         const uint32_t h = (uint32_t)tid / 9u, l = (uint32_t)tid - 9u * h;
         codes[tid] = (uint8_t)(((__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * h) & 0xFu) << 4) | (__funnelshift_rc(0x5420ACDEu, 0x6u, 4u * l) & 0xFu));
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
         v[4] = b.x * gb.x; v[5] = b.y * gb.y; v[6] = b.z * gb.z; v[7] = b.w * gb.w;
         ss = ((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((b.x * b.x + b.y * b.y) + (b.z * b.z + b.w * b.w));
     }
-    float inv = 1.0f;
+    float inv = 1.0f, probe;             // probe: not a number when an element of the vector is not
     if (LN) {
         // LayerNorm (GPT-2): mean, then variance about it, then the largest result
         float mean = 0.0f;
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
         }
 #pragma unroll
         for (int e = 0; e < 8; e++) v[e] = k0 + e < K ? __ldg(g + k0 + e) * ((__ldcg(x + k0 + e) - mean) * inv) + __ldg(lb + k0 + e) : 0.0f;
-        inv = 1.0f;
+        probe = inv; inv = 1.0f;
         mx = hx_warp_max(mx);
         __syncthreads();
         if (lane == 0) red[PFD_T / 32 + warp] = mx;
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
         tss = 0.0f;
         for (int i = 0; i < (int)gridDim.y; i++) { tss += part[i][0]; mx = fmaxf(mx, part[i][1]); }
     }
+    probe = tss;
     if (g) inv = rsqrtf(tss / (float)K + eps);
     }
     if (LN) {
@@ -144,7 +147,8 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     float Sg = 1.0f;
     const float vmax = mx * inv * 1.0000005f;
     if (vmax > 0.0f && vmax < INFINITY) Sg = __uint_as_float(__float_as_uint(vmax) & 0x7F800000u);
-    if (tid == 0 && blockIdx.y == 0) scale[t] = Sg * (1.0f / HX_TC_DIGIT_UNIT);
+    // digits cannot spell infinities or NaN: the scale does, so that the token's outputs show them
+    if (tid == 0 && blockIdx.y == 0) scale[t] = (vmax < INFINITY && probe == probe) ? Sg * (1.0f / HX_TC_DIGIT_UNIT) : __int_as_float(0x7FC00000);
     const float mul = (inv / Sg) * HX_TC_DIGIT_UNIT;
     if (k0 >= ((K + 255) & ~255)) return;
     // two digits at a time: five pairs (base 81) per element, each a byte of two codes from the table; the bytes of the even
