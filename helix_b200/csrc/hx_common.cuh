@@ -17,9 +17,11 @@ int  hx_fail(int code, const char* fmt, ...);
 #define HX_CUDA(call)                                                                         \
     do {                                                                                      \
         cudaError_t _e = (call);                                                              \
-        if (_e != cudaSuccess)                                                                \
+        if (_e != cudaSuccess) {                                                              \
+            (void)cudaGetLastError();   /* reported here, not by the next call's launch check */ \
             return hx_fail(HX_ERR_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(_e), \
                            __FILE__, __LINE__);                                               \
+        }                                                                                     \
     } while (0)
 
 #define HX_CHECK_ARG(cond)                                                                    \

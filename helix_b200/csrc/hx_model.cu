@@ -121,7 +121,8 @@ namespace {
 
 cudaError_t dev_malloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) { (void)cudaGetLastError(); e = cudaMalloc(p, bytes); }
+    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) (void)cudaGetLastError();        // the caller reports it
     return e;
 }
 
@@ -1351,7 +1352,6 @@ static int pf_alloc(hx_model* m, int want) {
         for (int i = 0; i < n; i++) total += (item[i].bytes + 255) & ~(size_t)255;
         const cudaError_t e = dev_malloc(&q, total);
         if (e == cudaSuccess) break;
-        (void)cudaGetLastError();
         if (e != cudaErrorMemoryAllocation) return hx_fail(HX_ERR_CUDA, "cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
         if (m->pf_tb && groups_of(tb / 2) * HX_TC_MAX_TOK <= m->pf_tb) return HX_OK;
         if (tb / 2 < HX_PF_TB) return hx_fail(HX_ERR_NOMEM, "chunk path: cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
@@ -1373,7 +1373,7 @@ static int pf_alloc(hx_model* m, int want) {
 // one linear of a chunk: digits of `src` -> GEMM against f -> out (token-major)
 static int pf_linear(hx_model* m, const Fused& f, const float* src, int ld_src, int n, int swiglu, const float* g,
                      float* out, int ld_out, int rows, int resid, int pair64, const float* nb = nullptr, const float* bias = nullptr, int gelu = 0) {
-    hx_pf_digits(src, ld_src, n, f.K, g, nb, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st);
+    const int rc = hx_pf_digits(src, ld_src, n, f.K, g, nb, m->cfg.norm_eps, m->pf_cells, m->pf_scale, m->st); if (rc) return rc;
     HxGemmDig q = {};
     q.a = f.t128; q.b = m->pf_cells; q.rows = rows; q.ntiles = f.tiles128; q.kcells = f.ksteps / 4; q.ntok = n;
     q.err = m->pf_err; q.col_scale = m->pf_scale; q.out = out; q.ld_out = ld_out; q.resid = resid; q.acc = m->pf_acc;
@@ -1416,13 +1416,13 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, i
             else m->pf_pieces_bytes = need;
         }
     }
-    hx_pf_embed(ids, wh, m->emb, c.arch == 0 ? m->wpe : nullptr, m->pf_x, n, DM, m->st);
+    if ((rc = hx_pf_embed(ids, wh, m->emb, c.arch == 0 ? m->wpe : nullptr, m->pf_x, n, DM, m->st))) return rc;
     for (int L = 0; L < c.n_layers; L++) {
         Layer& ly = m->layers[L];
         float* kc = m->kc + (size_t)L * c.n_kv_heads * cap * DH; float* vc = m->vc + (size_t)L * c.n_kv_heads * cap * DH;
         const bool g2 = c.arch == 0;         // GPT-2: LayerNorm, biases, gelu_new, no rotation, no q/k norm
         if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0, ly.ln1_b, ly.b_qkv))) return rc;
-        hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, g2 ? nullptr : m->cosT, g2 ? nullptr : m->sinT, kc, vc, cap, m->st);
+        if ((rc = hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, g2 ? nullptr : m->cosT, g2 ? nullptr : m->sinT, kc, vc, cap, m->st))) return rc;
         if (tc) {
             if ((rc = hx_pf_attn_tc(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_pieces, ctx_end, m->pf_err, m->st))) return rc;
         } else if ((rc = hx_pf_attn(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_att_part, m->pf_att_tickets, m->pf_err, m->st))) return rc;
@@ -1449,8 +1449,7 @@ static int pf_enqueue_chunk(hx_model* m, int t0, int n) {
     const hx_config& c = m->cfg;
     HxPfWhere wh = {m->d_pf_pos, nullptr, nullptr, (size_t)c.n_layers * c.n_kv_heads * m->kv_cap * c.head_dim, m->d_pf_pos + 1};
     int rc = pf_enqueue_layers(m, n, m->d_prompt, wh, t0 + n); if (rc) return rc;
-    hx_pf_advance(m->d_pf_pos, n, m->st);
-    return HX_OK;
+    return hx_pf_advance(m->d_pf_pos, n, m->st);
 }
 
 // ---- batched decode: n_seq independent sequences, one token each, in chunks of HX_PF_TB ----------------

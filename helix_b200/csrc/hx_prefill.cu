@@ -716,12 +716,14 @@ __global__ void __launch_bounds__(1024) k_pf_argmax(const float* __restrict__ lo
 
 }  // namespace
 
-void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st) {
+int hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st) {
     k_pf_embed<<<n_tok, 256, 0, st>>>(ids, wh, emb, wpe, X, DM);
+    HX_CUDA(cudaGetLastError());
     HX_COUNT_LAUNCH(1);
+    return HX_OK;
 }
 
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
+int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st) {
     const int groups = (n_tok + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
     const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
     const bool cl = grid.y > 1 && grid.y <= PFD_CL && !b;
@@ -735,28 +737,30 @@ void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, co
     if (cl) {
         at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
         at[cfg.numAttrs].val.clusterDim.x = 1; at[cfg.numAttrs].val.clusterDim.y = grid.y; at[cfg.numAttrs++].val.clusterDim.z = 1;
-        cudaLaunchKernelEx(&cfg, k_pf_digits<true, false>, src, ld, K, g, b, eps, cells, groups, scale);
-    } else if (b) cudaLaunchKernelEx(&cfg, k_pf_digits<false, true>, src, ld, K, g, b, eps, cells, groups, scale);
-    else cudaLaunchKernelEx(&cfg, k_pf_digits<false, false>, src, ld, K, g, b, eps, cells, groups, scale);
+        HX_CUDA(cudaLaunchKernelEx(&cfg, k_pf_digits<true, false>, src, ld, K, g, b, eps, cells, groups, scale));
+    } else if (b) HX_CUDA(cudaLaunchKernelEx(&cfg, k_pf_digits<false, true>, src, ld, K, g, b, eps, cells, groups, scale));
+    else HX_CUDA(cudaLaunchKernelEx(&cfg, k_pf_digits<false, false>, src, ld, K, g, b, eps, cells, groups, scale));
     HX_COUNT_LAUNCH(1);
+    return HX_OK;
 }
 
 // The threads of an attention CTA split into whole rows of the head size (P*V), and the q/k kernel has a variant per size.
 bool hx_pf_head_dim(int DH) { return DH == 32 || DH == 64 || DH == 128 || DH == 256; }
 
-void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
+int hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
                   float eps, const float* cosT, const float* sinT, float* kc, float* vc, int cap, cudaStream_t st) {
     const dim3 grid((NH + 2 * NKV + PF_QK_W - 1) / PF_QK_W, n_tok);
-#define PF_QKPOST(E) hx_launch_pdl(k_pf_qkpost<E>, grid, dim3(PF_QK_W * 32), 0, st, qkv, ld, wh, NH, NKV, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap)
-    switch (DH) {                    // (the head sizes that the attention of a chunk takes; it reports the others)
+#define PF_QKPOST(E) HX_CUDA(hx_launch_pdl(k_pf_qkpost<E>, grid, dim3(PF_QK_W * 32), 0, st, qkv, ld, wh, NH, NKV, qn_g, kn_g, eps, cosT, sinT, kc, vc, cap))
+    switch (DH) {
         case 32: PF_QKPOST(1); break;
         case 64: PF_QKPOST(2); break;
         case 128: PF_QKPOST(4); break;
         case 256: PF_QKPOST(8); break;
-        default: return;
+        default: return hx_fail(HX_ERR_ARG, "chunk path: head_dim %d", DH);
     }
 #undef PF_QKPOST
     HX_COUNT_LAUNCH(1);
+    return HX_OK;
 }
 
 // Runs of key tiles per (token group, kv head): as many as one wave of CTAs holds (a CTA fills an SM's shared memory; with
@@ -832,9 +836,10 @@ void hx_pf_tp_argmax_rows(const float* logits, int n, int ld, int rows, int voca
     HX_COUNT_LAUNCH(1);
 }
 
-void hx_pf_advance(int* posp, int n, cudaStream_t st) {
-    hx_launch_pdl(k_pf_advance, dim3(1), dim3(32), 0, st, posp, n);
+int hx_pf_advance(int* posp, int n, cudaStream_t st) {
+    HX_CUDA(hx_launch_pdl(k_pf_advance, dim3(1), dim3(32), 0, st, posp, n));
     HX_COUNT_LAUNCH(1);
+    return HX_OK;
 }
 
 void hx_pf_argmax(const float* logits, int n, int* tok, int* hist, int* pos_out, int pos, cudaStream_t st) {

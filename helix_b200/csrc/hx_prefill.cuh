@@ -16,7 +16,7 @@ struct HxPfWhere { const int* posp; const int* pos_arr; const int* seq_arr; size
 // Positions are read from device memory (*posp = position of the chunk's first token) so that the launches of a
 // chunk can be captured once and replayed.
 // X[t][:] = emb[ids[*posp + t]][:] (+ wpe[*posp + t][:])
-void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st);
+int hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st);
 
 // Digit columns of a chunk of activation vectors, in the B-cell layout of the digit-mode GEMM.
 //   src [n_tok][ld] f32, K a multiple of four;
@@ -24,11 +24,11 @@ void hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wp
 //   cells: K rounded up to 256 columns; per 256-column cell and group of 24 tokens 240 rows of 128 bytes, row 24 d + t % 24 =
 //   digit d of token t (ten balanced base-9 digits, most significant first, as E2M1 codes);
 //   scale[t]: x_n = scale[t] * sum_d digit_d 9^(9-d)  (a power of two).
-void hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st);
+int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, cudaStream_t st);
 
 // Per token and head of a chunk: RMSNorm (gains qn_g / kn_g, may be null) + rotate_half RoPE at position *posp + t on
 // q (in place) and k; k and v are written to the cache rows of their positions.
-void hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
+int hx_pf_qkpost(float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, int DH, const float* qn_g, const float* kn_g,
                   float eps, const float* cosT, const float* sinT, float* kc, float* vc, int cap, cudaStream_t st);
 
 // Causal attention of a chunk over the cache: query t (position *posp + t) attends to positions 0 .. *posp + t.
@@ -48,7 +48,7 @@ int hx_pf_attn_tc(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int
                   float* ctx, int ld_ctx, uint8_t* pieces, int ctx_len, int* err, cudaStream_t st);
 
 // *posp += n
-void hx_pf_advance(int* posp, int n, cudaStream_t st);
+int hx_pf_advance(int* posp, int n, cudaStream_t st);
 
 // First maximum of logits[0..n): index to *tok and hist[pos + 1]; *pos_out = pos + 1.
 void hx_pf_argmax(const float* logits, int n, int* tok, int* hist, int* pos_out, int pos, cudaStream_t st);

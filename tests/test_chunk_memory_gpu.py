@@ -62,3 +62,11 @@ def test_batch_step_then_longer_prompts_then_the_captured_step(gqa4_file):
     for s, p in enumerate(prompts):
         assert list(one.generate(p, 5)[0]) == [first[s]] + list(got[:, s])
     gm.close(); one.close()
+
+
+def test_a_failed_allocation_is_not_reported_again_by_the_next_call(tiny_file):
+    with pytest.raises(hb.HxError) as e:
+        hb.Model.load(tiny_file, kv_cap=1 << 30)              # a KV cache larger than the device
+    assert e.value.code == HX_ERR_NOMEM
+    w = np.random.default_rng(0).standard_normal((48, 1000)).astype(np.float32)
+    assert np.array_equal(hb.quantize_host(w)[0], ol.quantize(w)[0])
