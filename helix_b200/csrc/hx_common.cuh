@@ -140,6 +140,8 @@ __device__ __forceinline__ float hx_warp_max(float v) {
     for (int d = 16; d >= 1; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
     return v;
 }
+#define HX_TC_WAIT_NS 2000000000u        // limit of a device-side wait that is bounded by time
+
 // Programmatic dependent launch: wait for the kernels this one depends on / let dependents start.
 __device__ __forceinline__ void hx_grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void hx_grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -39,13 +39,13 @@ __device__ __forceinline__ void g2_send(uint32_t addr, float v, unsigned ep) {
     const unsigned long long w = ((unsigned long long)ep << 32) | (unsigned long long)__float_as_uint(v);
     asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" :: "r"(addr), "l"(w) : "memory");
 }
-__device__ __forceinline__ float g2_wait(const unsigned long long* p, unsigned ep, volatile int* ab) {
+__device__ __forceinline__ float g2_wait(const unsigned long long* p, unsigned ep, volatile int* ab, unsigned limit_ns) {
     unsigned long long w = 0;
     const uint32_t a = s_u32(p);
     (void)mb_bounded([&] {
         asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(w) : "r"(a) : "memory");
         return (unsigned)(w >> 32) == ep || *ab != 0;
-    }, ab);
+    }, ab, limit_ns);
     return __uint_as_float((unsigned)w);
 }
 __device__ __forceinline__ float g2_gelu(float x) {   // gpu_gelu_stable_kernel.hx:15-28
@@ -117,7 +117,8 @@ template <int NB> struct G2Smem {
     float xres[D / 16];                               // this CTA's rows of the residual stream
     float part[256];                                  // K parts of the second projection
     float red[4][G2_WARPS];
-    uint64_t full[2], empty[2];
+    uint64_t full[2], empty[2], never;
+    int loads;                                        // copies issued, for a launch that gives up
     volatile int abort_flag;
 };
 
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
     hx_grid_dep_launch();
     if (tid == 0) {
         for (int i = 0; i < 2; i++) { mb_init(&S.full[i], 1); mb_init(&S.empty[i], G2_WARPS); }
+        mb_init(&S.never, 1);
         S.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
     if (warp == G2_WARPS) {
         // ------------------------------ weights: a phase ahead ------------------------------
         if (lane == 0) {
-            bool ok = true;
+            bool ok = !P.stall || mb_wait(&S.never, 0, ab, P.wait_ns);
             int n = 0;
             for (int L = 0; L < P.n_layers && ok; L++)
                 for (int ph = 0; ph < 4 && ok; ph++, n++) {
@@ -150,11 +152,11 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                     const uint32_t rows = ph == 0 ? 3 * ROWS : (ph == 2 ? 4 * ROWS : ROWS), kb = ph == 3 ? 4 * D : D;
                     const uint32_t bytes = rows * kb / 16 * 9;
                     const int b = n & 1;
-                    if (n >= 2 && !mb_wait(&S.empty[b], (uint32_t)((n >> 1) - 1) & 1u, ab)) { ok = false; break; }
+                    if (n >= 2 && !mb_wait(&S.empty[b], (uint32_t)((n >> 1) - 1) & 1u, ab, P.wait_ns)) { ok = false; break; }
                     mb_expect(&S.full[b], bytes);
                     bulk_load(S.w[b], ly.t16[ph] + (size_t)cta * bytes, bytes, &S.full[b]);
                 }
-            for (int i = n > 2 ? n - 2 : 0; i < n && !ok; i++) mb_drain(&S.full[i & 1], (uint32_t)(i >> 1) & 1u);
+            S.loads = n;
         }
     } else {
         const int g = lane >> 2, t = lane & 3;
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
         float* part = S.xs + 3 * D / 2;                            // [NB][rows] of a linear with D inputs
         float* yrow = part + NB * 4 * ROWS;
         int n = 0;                                                 // weight phases so far
-        auto take = [&]() { (void)mb_wait(&S.full[n & 1], (uint32_t)(n >> 1) & 1u, ab); __syncwarp(); };      // the phase's weights are complete
+        auto take = [&]() { (void)mb_wait(&S.full[n & 1], (uint32_t)(n >> 1) & 1u, ab, P.wait_ns); __syncwarp(); };      // the phase's weights are complete
         auto give = [&]() { __syncwarp(); if (lane == 0) mb_arrive(&S.empty[n & 1]); n++; };
         // The phase's input (elements tid, tid + 512, ... of K) scaled to at most one by a power of two, as three f16 terms
         // (33 bits); returns the power.  Every thread is past its use of xs when the first barrier lets go.
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
 #pragma unroll
                 for (int i = 0; i < PT; i++) {
                     const int e = tid + i * G2_CT;
-                    v[i] = e >= D ? 0.0f : (L == 0 ? __ldg(P.emb + (size_t)tok * D + e) + __ldg(P.wpe + (size_t)pos * D + e) : g2_wait(&S.xb[e], (unsigned)L, ab));
+                    v[i] = e >= D ? 0.0f : (L == 0 ? __ldg(P.emb + (size_t)tok * D + e) + __ldg(P.wpe + (size_t)pos * D + e) : g2_wait(&S.xb[e], (unsigned)L, ab, P.wait_ns));
                 }
                 const float sc = layer_norm(v, gg, bb) * ly.ts[0];
                 linear(3 * ROWS);
@@ -298,7 +300,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 float* sq = S.xs + G2_CAP + 1024;                 // q, k, v of the position
                 load_k(0);
                 if (tid < 192) {
-                    const float x = g2_wait(&S.qkv[tid], ep, ab);
+                    const float x = g2_wait(&S.qkv[tid], ep, ab, P.wait_ns);
                     sq[tid] = x;
                     if (tid >= 64) (tid < 128 ? kc : vc)[((size_t)cta * P.cap + pos) * 64 + (tid & 63)] = x;
                 }
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
 #pragma unroll
                 for (int i = 0; i < RL; i++) bias[i] = lane + 32 * i < ROWS ? __ldg(ly.bias[1] + cta * ROWS + lane + 32 * i) : 0.0f;
 #pragma unroll
-                for (int i = 0; i < PT; i++) cv[i] = tid + i * G2_CT < D ? g2_wait(&S.ctx[tid + i * G2_CT], ep, ab) : 0.0f;
+                for (int i = 0; i < PT; i++) cv[i] = tid + i * G2_CT < D ? g2_wait(&S.ctx[tid + i * G2_CT], ep, ab, P.wait_ns) : 0.0f;
                 const float sc = split(cv, D, 0) * ly.ts[1];
                 linear(ROWS);
 #pragma unroll
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
                 for (int i = 0; i < PT; i++) { const int e = tid + i * G2_CT; gg[i] = e < D ? __ldg(ly.ln2g + e) : 0.0f; bb[i] = e < D ? __ldg(ly.ln2b + e) : 0.0f; }
                 const float bias = tid < 4 * ROWS ? __ldg(ly.bias[2] + cta * 4 * ROWS + tid) : 0.0f;
 #pragma unroll
-                for (int i = 0; i < PT; i++) v[i] = tid + i * G2_CT < D ? g2_wait(&S.xa[tid + i * G2_CT], ep, ab) : 0.0f;
+                for (int i = 0; i < PT; i++) v[i] = tid + i * G2_CT < D ? g2_wait(&S.xa[tid + i * G2_CT], ep, ab, P.wait_ns) : 0.0f;
                 const float sc = layer_norm(v, gg, bb) * ly.ts[2];
                 linear(4 * ROWS);
                 if (tid < 4 * ROWS) yrow[tid] = g2_gelu(row_sum(4 * ROWS, tid) * sc + bias);
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
 #pragma unroll
                 for (int i = 0; i < RL; i++) bias[i] = lane + 32 * i < ROWS ? __ldg(ly.bias[3] + cta * ROWS + lane + 32 * i) : 0.0f;
 #pragma unroll
-                for (int i = 0; i < 4 * PT; i++) hv[i] = tid + i * G2_CT < 4 * D ? g2_wait(&S.h[tid + i * G2_CT], ep, ab) : 0.0f;
+                for (int i = 0; i < 4 * PT; i++) hv[i] = tid + i * G2_CT < 4 * D ? g2_wait(&S.h[tid + i * G2_CT], ep, ab, P.wait_ns) : 0.0f;
                 const float sc = split(hv, 4 * D, 0) * ly.ts[3];
                 take();
                 const int tile = warp % NB, j = warp / NB;
@@ -433,7 +435,11 @@ __global__ void __launch_bounds__(G2_THREADS, 1) k_gpt2_layers(const __grid_cons
         }
     }
     __syncthreads();
-    if (S.abort_flag && tid == 0) *P.err = 1;
+    if (S.abort_flag && tid == 0) {
+        // given up: the CTA must not end with a copy of its own in flight
+        for (int i = S.loads > 2 ? S.loads - 2 : 0; i < S.loads; i++) mb_drain(&S.full[i & 1], (uint32_t)(i >> 1) & 1u);
+        *P.err = 1;
+    }
     cl_sync();      // nobody leaves while a CTA of the cluster may still write into its shared memory
 }
 

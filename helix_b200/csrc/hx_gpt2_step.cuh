@@ -14,6 +14,7 @@ struct HxGpt2Step {
     float* x_out;                                           // [d_model] residual stream behind the last layer
     float eps, scale;
     int* err;                                               // set when a bounded wait ran out
+    unsigned wait_ns; int stall;                            // limit of a wait; 1: begin with a wait for something that nothing does (tests)
 };
 bool hx_gpt2_step_fits(const hx_config& c, int kv_cap);
 int hx_gpt2_step_launch(const HxGpt2Step& p, int d_model, cudaStream_t st, bool pdl);

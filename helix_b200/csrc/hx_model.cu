@@ -113,7 +113,7 @@ struct hx_model {
     bool use_df = false;
     unsigned long long *xll[2] = {nullptr, nullptr}, *statll[2] = {nullptr, nullptr}, *qll = nullptr, *kvll = nullptr, *hll = nullptr;
     unsigned long long *pacc_ll = nullptr, *pml_ll = nullptr, *ctxll = nullptr, *part_ll[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    unsigned ep_count = 0, wait_limit = 1u << 24; int inject_stall = 0; unsigned* done_cnt = nullptr;
+    unsigned ep_count = 0, wait_limit = 1u << 24, wait_ns = HX_TC_WAIT_NS; int inject_stall = 0; unsigned* done_cnt = nullptr;
     std::vector<long long> plan_keys; std::vector<HxCtaPlan*> plan_tabs;
 };
 
@@ -475,6 +475,7 @@ int enqueue_step(hx_model* m, bool from_prompt, bool with_head, bool prof = fals
         HxGpt2Step s = {};
         s.layers = m->g2_layers; s.n_layers = c.n_layers; s.emb = m->emb; s.wpe = m->wpe; s.tok = m->d_tok; s.pos = m->d_pos;
         s.kc = m->kc; s.vc = m->vc; s.cap = cap; s.x_out = m->x; s.eps = c.norm_eps; s.scale = 1.0f / sqrtf((float)DH); s.err = m->d_err;
+        s.wait_ns = m->wait_ns; s.stall = m->inject_stall;
         if ((rc = hx_gpt2_step_launch(s, DM, m->st, pdl))) return rc;
         return enqueue_head_gpt2(m, pdl, false);
     }
@@ -1180,13 +1181,18 @@ HX_API const char* hx_model_engine(const hx_model* m) {
     if (m->use_df) return "persistent-tcgen05-dataflow";
     return m->use_tc ? "persistent-tcgen05" : "persistent-mma";
 }
-// Test hook of the bounded waits: polls before a device-side wait gives up (0 = the default) and, with
-// inject_stall != 0, a wait at the start of every launch on a word that nothing writes.
+// Test hook of the bounded waits: polls before a device-side wait gives up (0 = the default; 100 ns a poll in the GPT-2 layer
+// kernel, which bounds its waits by time) and, with inject_stall != 0, a wait at the start of every launch for something that
+// nothing does.
 HX_API int hx_model_debug_waits(hx_model* m, unsigned wait_limit, int inject_stall) {
     HX_CHECK_ARG(m);
     m->wait_limit = wait_limit ? wait_limit : (1u << 24);
+    m->wait_ns = wait_limit && wait_limit < HX_TC_WAIT_NS / 100 ? wait_limit * 100u : HX_TC_WAIT_NS;
     m->inject_stall = inject_stall;
-    return HX_OK;
+    if (!m->g2_layers) return HX_OK;
+    HX_CUDA(cudaStreamSynchronize(m->st));                    // the captured token holds the old values
+    if (m->g_decode) { cudaGraphExecDestroy(m->g_decode); m->g_decode = nullptr; }
+    return capture(m, false, true, &m->g_decode);
 }
 HX_API int hx_model_set_profile(hx_model* m, int on) { HX_CHECK_ARG(m); m->profile = on != 0; return HX_OK; }
 

@@ -3,7 +3,7 @@
 #pragma once
 #include "hx_common.cuh"
 
-#define TC_WAIT_NS 2000000000ull        // a wait gives up after two seconds (a poll may itself be suspended, so polls do not measure time)
+// A wait gives up after two seconds, or what the caller says (a poll may itself be suspended, so polls do not measure time).
 
 namespace hxtc {
 
@@ -18,24 +18,24 @@ __device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity) {
 }
 __device__ __forceinline__ unsigned long long now_ns() { unsigned long long v; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v)); return v; }
 template <class Try>
-__device__ __forceinline__ bool mb_bounded(Try&& poll, volatile int* abort_flag) {
+__device__ __forceinline__ bool mb_bounded(Try&& poll, volatile int* abort_flag, unsigned limit_ns = HX_TC_WAIT_NS) {
     unsigned long long t0 = 0;
     for (uint32_t i = 1; ; i++) {
         if (poll()) return true;
         if ((i & 255) == 0) {
             if (*abort_flag) return false;
             if (!t0) t0 = now_ns();
-            else if (now_ns() - t0 > TC_WAIT_NS) { *abort_flag = 1; return false; }
+            else if (now_ns() - t0 > limit_ns) { *abort_flag = 1; return false; }
         }
     }
 }
-__device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-    return mb_bounded([&] { return mb_try(b, parity); }, abort_flag);
+__device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag, unsigned limit_ns = HX_TC_WAIT_NS) {
+    return mb_bounded([&] { return mb_try(b, parity); }, abort_flag, limit_ns);
 }
 // For copies of one's own that are in flight when the work is given up: waits whatever the abort flag says.
 __device__ __forceinline__ void mb_drain(uint64_t* b, uint32_t parity) {
     const unsigned long long t0 = now_ns();
-    while (!mb_try(b, parity) && now_ns() - t0 < TC_WAIT_NS) { }
+    while (!mb_try(b, parity) && now_ns() - t0 < HX_TC_WAIT_NS) { }
 }
 // A wait of the whole warp: every lane gets the same answer, so the warp leaves a loop together.
 __device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {

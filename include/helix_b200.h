@@ -298,10 +298,12 @@ int hx_model_last_stats(const hx_model* m, hx_step_stats* st);
  * HX_LINEAR=mma) or "graph" (one CUDA graph of per-op kernels, HX_DECODE=graph and GPT-2; the only engine for which
  * hx_model_set_profile yields per-category times). */
 const char* hx_model_engine(const hx_model* m);
-/* Test hook of the bounded device-side waits.  Every wait of the decode kernels polls at most wait_limit times
- * (0 restores the default, about ten seconds) and then makes the call return HX_ERR_TIMEOUT with the model still
- * usable.  inject_stall != 0 makes every launch begin with a wait on a word that nothing writes, so that the
- * time-out path can be exercised without faulting or hanging the GPU.  No reference counterpart. */
+/* Test hook of the bounded device-side waits.  Every wait of the default decode engine polls at most wait_limit times (0
+ * restores the default, about ten seconds) and then makes the call return HX_ERR_TIMEOUT with the model still usable; the
+ * GPT-2 layer kernel waits 100 ns for each of wait_limit (0: two seconds).  inject_stall != 0 makes every launch of these
+ * two kernels begin with a wait for something that nothing does, so that the time-out path can be exercised without
+ * faulting or hanging the GPU.  The chunk kernels (two seconds) and the other engines take neither.  No reference
+ * counterpart. */
 int hx_model_debug_waits(hx_model* m, unsigned wait_limit, int inject_stall);
 int hx_model_set_profile(hx_model* m, int on);
 
