@@ -80,7 +80,7 @@ struct hx_model {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool pdl = true;
     bool persist = true;                 // one cooperative kernel per token instead of the launch graph
-    bool want_t16 = false;                // T16 cells beside the dense layout (GPT-2 layers in one launch)
+    bool want_d16 = true, want_t16 = false;      // without `persist`: the dense layout of the per-op kernels, the T16 cells of the GPT-2 layer kernel
     bool want_t128 = true, use_tc = true; // linear phases on the tensor cores (tcgen05) inside the persistent kernel
     float* tc_partial = nullptr; unsigned* tc_cnt = nullptr; int bdig_bytes = 0, tc_ring = 0; size_t tc_units_max = 0; int tc_tiles_max = 0;
     HxPhase *ph_decode = nullptr, *ph_prefill = nullptr; int nph_decode = 0, nph_prefill = 0;
@@ -153,9 +153,9 @@ int alloc_fused(hx_model* m, Fused& f, int N, int K) {
     int rc = HX_OK;
     m->decode_bytes += f.bytes();
     f.KG = hx_t16_kgroups(K); f.ntiles = hx_t16_tiles(N);
-    // one resident layout: the one the selected engine reads (D16 for the per-op graph engine, T16 for the mma.sync
-    // persistent engine, T128 for the tensor-core engines)
-    if (!m->persist) {
+    // the layouts that the selected engine reads: D16 for the per-op graph engine, T16 for the mma.sync persistent engine and
+    // the GPT-2 layer kernel, T128 for the tensor-core engines and the chunk path
+    if (!m->persist && m->want_d16) {
         rc = dalloc(m, &f.codes, (size_t)N * (f.Kd / 2)); if (rc) return rc;
         rc = dalloc(m, &f.scales, (size_t)N * (f.Kd / 16)); if (rc) return rc;
     }
@@ -885,7 +885,7 @@ int finish_init(hx_model* m) {
         m->pdl = false;
         rc = capture(m, false, true, &m->g_decode);
     }
-    if (rc) return rc;
+    if (rc || (m->cfg.arch == 0 && m->pf_batched)) return rc;      // (prompts go through the chunk path)
     return capture(m, true, false, &m->g_prefill);
 }
 
@@ -1020,6 +1020,7 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
             cudaMalloc(&mtmp, maxrows * (kp / 16)) != cudaSuccess || cudaMalloc(&tstmp, 256) != cudaSuccess) { rc = hx_fail(HX_ERR_NOMEM, "GPT-2 staging"); break; }
         m->layers.resize(c.n_layers);
         m->want_t16 = hx_gpt2_step_fits(c, kv_cap);
+        m->want_d16 = !(m->want_t16 && m->pf_batched);       // nothing runs a layer op by op then (but see hx_model_set_profile)
         for (int L = 0; L < c.n_layers && !rc; L++) {
             Layer& ly = m->layers[L]; const hx_gpt2_layer& hl = w->layers[L];
             if (!hl.ln1_g || !hl.ln1_b || !hl.w_qkv || !hl.b_qkv || !hl.w_proj || !hl.b_proj || !hl.ln2_g || !hl.ln2_b || !hl.w_fc || !hl.b_fc || !hl.w_proj2 || !hl.b_proj2) {
@@ -1036,7 +1037,7 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
         if (rc) break;
         if ((rc = gpt2_upload(m, &m->emb, w->wte, (size_t)NV * DM)) || (rc = gpt2_upload(m, &m->wpe, w->wpe, (size_t)c.max_ctx * DM)) ||
             (rc = gpt2_upload(m, &m->final_g, w->lnf_g, DM)) || (rc = gpt2_upload(m, &m->final_b, w->lnf_b, DM))) break;
-        m->want_t16 = false;
+        m->want_t16 = false; m->want_d16 = true;
         if ((rc = gpt2_linear(m, m->head, w->wte, NV, DM, stage, wtmp, mtmp, tstmp))) break;       // tied lm_head
         HX_CUDA(cudaStreamSynchronize(m->st));
         rc = finish_init(m);
@@ -1194,7 +1195,22 @@ HX_API int hx_model_debug_waits(hx_model* m, unsigned wait_limit, int inject_sta
     if (m->g_decode) { cudaGraphExecDestroy(m->g_decode); m->g_decode = nullptr; }
     return capture(m, false, true, &m->g_decode);
 }
-HX_API int hx_model_set_profile(hx_model* m, int on) { HX_CHECK_ARG(m); m->profile = on != 0; return HX_OK; }
+HX_API int hx_model_set_profile(hx_model* m, int on) {
+    HX_CHECK_ARG(m);
+    // profiled steps run op by op: a GPT-2 model that keeps only the cells of its layer kernel gets the dense layout now
+    if (on && m->g2_layers && !m->layers[0].qkv.codes) {
+        for (auto& ly : m->layers)
+            for (Fused* f : {&ly.qkv, &ly.o, &ly.gu, &ly.down}) {
+                int rc;
+                if (!f->codes && (rc = dalloc(m, &f->codes, (size_t)f->N * (f->Kd / 2)))) return rc;
+                if (!f->scales && (rc = dalloc(m, &f->scales, (size_t)f->N * (f->Kd / 16)))) return rc;
+                if ((rc = hx_repack_d16_t16(f->t16, f->N, f->K, f->KG, f->codes, f->scales, m->st))) return rc;
+            }
+        HX_CUDA(cudaStreamSynchronize(m->st));
+    }
+    m->profile = on != 0;
+    return HX_OK;
+}
 
 // ---- HXGW v3 image ---------------------------------------------------------------------------------
 namespace {

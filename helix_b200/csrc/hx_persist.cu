@@ -74,6 +74,33 @@ void hx_repack_t16(const int32_t* words, const uint8_t* micro, int rows, int K, 
     HX_COUNT_LAUNCH(1);
 }
 
+// T16 -> D16: a thread per eight columns of a row.  (Only for profiling a model whose layers run from T16 cells.)
+__global__ void __launch_bounds__(256) k_repack_d16_t16(const uint8_t* __restrict__ t16, int rows, int K, int KG, uint32_t* __restrict__ codes, uint8_t* __restrict__ scales) {
+    const int c8 = K / 8;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)rows * c8; i += (size_t)gridDim.x * blockDim.x) {
+        const int r = (int)(i / c8), g = (int)(i % c8), kg = g >> 4, blk = (g >> 1) & 7;
+        const uint8_t* cell = t16 + ((size_t)(r / 16) * KG + kg) * HX_T16_CELL;
+        uint32_t o = 0;
+#pragma unroll
+        for (int e = 0; e < 8; e++) {                     // element 8 (g & 1) + e of block blk
+            const int m = (blk & ~1) | (g & 1), nib = (e >> 2) * 2 + (blk & 1);
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(cell + (r % 16) * 64 + (e & 3) * 16 + (m >> 1) * 4);
+            o |= ((w >> ((m & 1) * 16 + nib * 4)) & 15u) << (4 * e);
+        }
+        codes[i] = o;
+        if (!(g & 1)) scales[(size_t)r * (K / 16) + kg * 8 + blk] = cell[1024 + (r % 16) * 8 + blk];
+    }
+}
+
+int hx_repack_d16_t16(const uint8_t* t16, int rows, int K, int KG, uint8_t* codes, uint8_t* scales, cudaStream_t st) {
+    HX_CHECK_ARG(t16 && codes && scales && K % 128 == 0);
+    const size_t n = (size_t)rows * (K / 8);
+    k_repack_d16_t16<<<(unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16), 256, 0, st>>>(t16, rows, K, KG, reinterpret_cast<uint32_t*>(codes), scales);
+    HX_COUNT_LAUNCH(1);
+    HX_CUDA(cudaGetLastError());
+    return HX_OK;
+}
+
 __device__ __forceinline__ void cvt_e2m1x8(uint32_t w, uint32_t& h0, uint32_t& h1, uint32_t& h2, uint32_t& h3) {
     asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
         "mov.b32 {b0, b1, b2, b3}, %4;\n\t"

@@ -24,6 +24,8 @@ static inline size_t hx_t16_bytes(int N, int K) { return (size_t)hx_t16_tiles(N)
 
 // committed layout -> T16.  Source row r goes to destination row (r / grp) * grp * row_mul + row_off * grp + r % grp
 // (grp = 16, row_mul = 2 interleaves gate and up tile by tile; grp = 1 is a plain offset).
+// T16 -> D16 (rows of K / 2 code bytes and K / 16 scale bytes), K a multiple of 128.
+int hx_repack_d16_t16(const uint8_t* t16, int rows, int K, int KG, uint8_t* codes, uint8_t* scales, cudaStream_t st);
 void hx_repack_t16(const int32_t* words, const uint8_t* micro, int rows, int K, int Kpad, uint8_t* dst,
                    int dstKG, int grp, int row_mul, int row_off, cudaStream_t st);
 

@@ -26,3 +26,22 @@ def test_prompt_then_tokens_match_checker(d_model, n_layers, T, cap):
         assert np.max(np.abs(lg - want)) < 2e-4, p
         assert tok == int(np.argmax(want))
     gm.close()
+
+
+@pytest.mark.parametrize("d_model", [256, 768])
+def test_profiled_steps_run_op_by_op_with_the_same_tokens(d_model):
+    """The layers' dense layout is made from the layer kernel's cells when profiling asks for it."""
+    shape = dict(n_layers=2, d_model=d_model, n_heads=d_model // 64, d_ff=4 * d_model, vocab=517, max_ctx=40)
+    wt = synth(shape, d_model)
+    om, gm = OracleGpt2(shape, wt, 40), hb.Model.gpt2(shape, wt, kv_cap=40)
+    tok, want = 11, []
+    for p in range(8):
+        tok = int(np.argmax(om.decode(tok, p))); want.append(tok)
+    assert list(gm.decode_loop(11, 0, 8)[0]) == want
+    gm.set_profile(True)
+    assert list(gm.decode_loop(11, 0, 8)[0]) == want
+    st = gm.last_stats()
+    assert st["ms_gemv"] > 0 and st["ms_attn"] > 0
+    gm.set_profile(False)
+    assert list(gm.decode_loop(11, 0, 8)[0]) == want
+    gm.close()
