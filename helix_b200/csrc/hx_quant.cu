@@ -201,9 +201,12 @@ __global__ void __launch_bounds__(Q_THREADS, 4) k_quantize(const float* __restri
 }
 
 // Both passes of a small tensor in one launch: a cluster of eight CTAs, the maxima exchanged through distributed shared
-// memory.  Launches are what a small call costs (a fill and two kernels before: 12.5 us for 48 x 1000); up to Q_SMALL
-// elements eight SMs are not slower than two launches over all of them.
+// memory.  Launches are what a small call costs (a fill and two kernels before: 12.5 us for 48 x 1000).  Up to Q_SMALL elements
+// eight SMs are not slower than two launches over all of them, unless the rows are narrow: the cluster's time goes with the pairs
+// of units, 256 at a time, whatever their columns hold.  8.5 us up to 768 pairs, 8.9 to 11 at 1024, 12.3 at 1536, 24.6 at 4096
+// (4096 x 16), against 10.6 for two launches at each of these: up to Q_SMALL_PAIRS pairs.
 #define Q_SMALL 131072
+#define Q_SMALL_PAIRS 1024
 #define QS_THREADS 1024
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(QS_THREADS) k_quantize_small(const float* __restrict__ w, int rows, int K, int units, QOut o, float* __restrict__ ts_out) {
     __shared__ float sm[32];
@@ -275,7 +278,7 @@ static int quantize_launch(const float* w, int rows, int K, int32_t* words, uint
     const size_t items = (size_t)rows * ((units + 1) / 2);
     if (items > 0x7FFFFFFFu) return hx_fail(HX_ERR_ARG, "quantizer: %d x %d elements are more than a call takes", rows, K);
     const QOut o = {words, micro, sc};
-    if (n <= Q_SMALL) {
+    if (n <= Q_SMALL && items <= Q_SMALL_PAIRS) {
         k_quantize_small<<<8, QS_THREADS, 0, st>>>(w, rows, K, units, o, ts);
         HX_COUNT_LAUNCH(1);
         HX_CUDA(cudaGetLastError());

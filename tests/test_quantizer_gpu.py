@@ -148,3 +148,11 @@ def test_device_pointer_calls_and_layouts():
     y2 = dy.to_array(np.float32)
     assert np.max(np.abs(y2 - y_asc) / np.maximum(np.abs(y_asc), 1e-6)) < 1e-3
     assert np.max(np.abs(y2 - y_asc)) < 1e-5
+
+
+@pytest.mark.parametrize("rows,K", [(1023, 16), (1024, 16), (1025, 16), (4096, 16), (585, 224), (586, 224), (512, 225), (513, 225), (131, 1000), (132, 1000)])
+def test_around_the_line_between_one_launch_and_two(rows, K):
+    """Up to 1024 pairs of 112-column units and 131072 elements go through the one-launch kernel, more through two launches."""
+    w = (0.02 * np.random.default_rng(rows + K).standard_normal((rows, K))).astype(np.float32)
+    w[rows - 1, K - 1] = 1.5                              # the tensor's largest value is the last one
+    assert same(ol.quantize(w), hb.quantize_host(w))
