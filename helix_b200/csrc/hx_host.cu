@@ -4,6 +4,7 @@
 // Reference: sha256* helixc/runtime/gpt2_infer.c:137-213; run_v3_receipt_from_logits :2827-2871;
 // run_v3_receipt_check :2876-2912; calib_tau :2765-2769; argmax_row :1735-1739.
 #include "hx_common.cuh"
+#include "hx_stage.cuh"
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string>
@@ -24,7 +25,7 @@ HX_API const char* hx_version(void) { return "helix_b200 0.1 (sm_100a)"; }
 // ---- device helpers ------------------------------------------------------------------------------
 HX_API int hx_device_count(int* n) { HX_CHECK_ARG(n); HX_CUDA(cudaGetDeviceCount(n)); return HX_OK; }
 HX_API int hx_set_device(int dev) { HX_CUDA(cudaSetDevice(dev)); return HX_OK; }
-HX_API int hx_malloc(void** dptr, size_t bytes) { HX_CHECK_ARG(dptr); HX_CUDA(cudaMalloc(dptr, bytes ? bytes : 1)); return HX_OK; }
+HX_API int hx_malloc(void** dptr, size_t bytes) { HX_CHECK_ARG(dptr); HX_CUDA(hx_dev_malloc(dptr, bytes ? bytes : 1)); return HX_OK; }
 HX_API int hx_free(void* dptr) { HX_CUDA(cudaFree(dptr)); return HX_OK; }
 HX_API int hx_memcpy_h2d(void* dst, const void* src, size_t bytes) { HX_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice)); return HX_OK; }
 HX_API int hx_memcpy_d2h(void* dst, const void* src, size_t bytes) { HX_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost)); return HX_OK; }

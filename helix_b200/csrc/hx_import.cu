@@ -11,6 +11,7 @@
 // (copy of chunk i+1 from the page cache overlaps the transfer of chunk i), are widened there if BF16,
 // quantized there, and the results come back through the same staging buffers straight into fwrite.
 #include "hx_common.cuh"
+#include "hx_stage.cuh"
 #include <errno.h>
 #include <fcntl.h>
 #include <string>
@@ -223,7 +224,7 @@ struct DevBuf {
     int need(size_t n) {
         if (n <= cap) return HX_OK;
         if (p) { cudaFree(p); p = nullptr; cap = 0; }
-        if (cudaMalloc(&p, n) != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "device allocation of %zu bytes failed", n);
+        if (hx_dev_malloc(&p, n) != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "device allocation of %zu bytes failed", n);
         cap = n; return HX_OK;
     }
 };

@@ -119,13 +119,6 @@ struct hx_model {
 
 namespace {
 
-cudaError_t dev_malloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && hx_stage_trim()) e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) (void)cudaGetLastError();        // the caller reports it
-    return e;
-}
-
 // Device memory of a model.  Small buffers (gains, biases, scratch words: several hundred of them) are cut from slabs, since
 // an allocation of the driver's costs tens of microseconds whatever its size; `own`: an allocation of its own all the same.
 template <typename T>
@@ -140,7 +133,7 @@ int dalloc(hx_model* m, T** p, size_t n, bool own = false) {
     }
     void* q = nullptr;
     const size_t want = small ? SLAB : bytes;
-    const cudaError_t e = dev_malloc(&q, want);
+    const cudaError_t e = hx_dev_malloc(&q, want);
     if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want, cudaGetErrorString(e));
     m->allocs.push_back(q);
     if (small) { m->slab = (uint8_t*)q + bytes; m->slab_left = SLAB - bytes; }
@@ -263,7 +256,7 @@ int build(hx_model* m, Source& s) {
     int rc;
     std::vector<void*> staging;
     auto salloc = [&](void** p, size_t bytes) -> int {
-        cudaError_t e = cudaMalloc(p, bytes);
+        cudaError_t e = hx_dev_malloc(p, bytes);
         if (e != cudaSuccess) return hx_fail(HX_ERR_NOMEM, "staging cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
         staging.push_back(*p); return HX_OK;
     };
@@ -1016,8 +1009,8 @@ HX_API int hx_model_gpt2(hx_model** out, const hx_config* cfg, const hx_gpt2_wei
         size_t maxel = (size_t)NV * DM; if ((size_t)3 * DM * DM > maxel) maxel = (size_t)3 * DM * DM; if ((size_t)DFF * DM > maxel) maxel = (size_t)DFF * DM;
         const int kp = hx_kpad(DM > DFF ? DM : DFF);
         size_t maxrows = (size_t)NV; if ((size_t)3 * DM > maxrows) maxrows = 3 * DM; if ((size_t)DFF > maxrows) maxrows = DFF;
-        if (cudaMalloc(&stage, maxel * 4) != cudaSuccess || cudaMalloc(&wtmp, maxrows * (kp / 7) * 4) != cudaSuccess ||
-            cudaMalloc(&mtmp, maxrows * (kp / 16)) != cudaSuccess || cudaMalloc(&tstmp, 256) != cudaSuccess) { rc = hx_fail(HX_ERR_NOMEM, "GPT-2 staging"); break; }
+        if (hx_dev_malloc((void**)&stage, maxel * 4) != cudaSuccess || hx_dev_malloc((void**)&wtmp, maxrows * (kp / 7) * 4) != cudaSuccess ||
+            hx_dev_malloc((void**)&mtmp, maxrows * (kp / 16)) != cudaSuccess || hx_dev_malloc((void**)&tstmp, 256) != cudaSuccess) { rc = hx_fail(HX_ERR_NOMEM, "GPT-2 staging"); break; }
         m->layers.resize(c.n_layers);
         m->want_t16 = hx_gpt2_step_fits(c, kv_cap);
         m->want_d16 = !(m->want_t16 && m->pf_batched);       // nothing runs a layer op by op then (but see hx_model_set_profile)
@@ -1372,7 +1365,7 @@ static int pf_alloc(hx_model* m, int want) {
         if (m->tp_world > 1) item[n++] = {(void**)&m->pf_part, (size_t)HX_PF_TB * c.d_model * 4};
         total = 256;                                               // (the chunk's position)
         for (int i = 0; i < n; i++) total += (item[i].bytes + 255) & ~(size_t)255;
-        const cudaError_t e = dev_malloc(&q, total);
+        const cudaError_t e = hx_dev_malloc(&q, total);
         if (e == cudaSuccess) break;
         if (e != cudaErrorMemoryAllocation) return hx_fail(HX_ERR_CUDA, "cudaMalloc(%zu bytes): %s", total, cudaGetErrorString(e));
         if (m->pf_tb && groups_of(tb / 2) * HX_TC_MAX_TOK <= m->pf_tb) return HX_OK;
@@ -1433,8 +1426,8 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, i
             HX_CUDA(cudaStreamSynchronize(m->st));
             if (m->pf_pieces) cudaFree(m->pf_pieces);
             m->pf_pieces_bytes = 0;
-            const cudaError_t e = cudaMalloc(&m->pf_pieces, need);
-            if (e != cudaSuccess) { m->pf_pieces = nullptr; (void)cudaGetLastError(); tc = false; }      // no room: the vector kernel needs none
+            const cudaError_t e = hx_dev_malloc((void**)&m->pf_pieces, need);
+            if (e != cudaSuccess) { m->pf_pieces = nullptr; tc = false; }      // no room: the vector kernel needs none
             else m->pf_pieces_bytes = need;
         }
     }

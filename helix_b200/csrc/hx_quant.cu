@@ -265,7 +265,7 @@ static float* amax_scratch() {
     float* q = p[dev].load();
     if (!q) {
         float* fresh = nullptr;
-        if (cudaMalloc(&fresh, (size_t)64 * AMAX_CTAS * 4) != cudaSuccess) return nullptr;
+        if (hx_dev_malloc((void**)&fresh, (size_t)64 * AMAX_CTAS * 4) != cudaSuccess) return nullptr;
         if (p[dev].compare_exchange_strong(q, fresh)) q = fresh;
         else cudaFree(fresh);                             // another thread was first
     }

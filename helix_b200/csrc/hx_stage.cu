@@ -4,9 +4,10 @@
 // call that allocates and frees its device buffers pays for mapping them each time.  Here up to eight threads copy slices of
 // one megabyte between the caller's memory and page-locked slots, two per thread, while the link moves the slot before;
 // slots, streams and a device workspace stay with the device for the next call.  They are bounded (16 MB page-locked, 256 MB
-// of device memory; a larger workspace is freed when the call ends), handed to one call at a time, and freed when memory is
-// short elsewhere (hx_stage_trim) or the process ends.  The threads live for one call: a call that needs one slice starts none.
+// of device memory; a larger workspace is freed when the call ends), handed to one call at a time, and the workspace is
+// given back when device memory is short elsewhere in the library (hx_dev_malloc).  The threads live for one call: a call that needs one slice starts none.
 #include "hx_stage.cuh"
+#include <condition_variable>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -17,8 +18,9 @@ constexpr size_t ST_SLICE = 1u << 20;
 constexpr size_t ST_KEEP = (size_t)256 << 20;
 }
 
-struct Area {
-    std::mutex mu;
+struct HxStageArea {
+    std::mutex mu; std::condition_variable cv;
+    bool busy = false;                                    // a call has the area (mu is held for moments only)
     int dev = -1;
     bool ready = false;
     uint8_t* pinned = nullptr;                            // [worker][2] slots
@@ -41,7 +43,7 @@ struct Area {
     }
 };
 
-static Area* areas() { static Area* a = new Area[64]; return a; }      // never destroyed: the driver outlives no destructor order
+static HxStageArea* areas() { static HxStageArea* a = new HxStageArea[64]; return a; }      // never destroyed: the driver outlives no destructor order
 
 HxStage::HxStage() : a_(nullptr), rc_(HX_OK) {
     int dev = 0;
@@ -49,14 +51,19 @@ HxStage::HxStage() : a_(nullptr), rc_(HX_OK) {
     if (e != cudaSuccess) { rc_ = hx_fail(HX_ERR_CUDA, "cudaGetDevice: %s", cudaGetErrorString(e)); return; }
     if (dev < 0 || dev >= 64) { rc_ = hx_fail(HX_ERR_ARG, "device index %d not supported", dev); return; }
     a_ = areas() + dev;
-    a_->mu.lock();
+    {
+        std::unique_lock<std::mutex> lk(a_->mu);
+        a_->cv.wait(lk, [&] { return !a_->busy; });
+        a_->busy = true;
+    }
     rc_ = a_->prepare();
 }
 
 HxStage::~HxStage() {
     if (!a_) return;
     if (big_ && a_->work) { cudaStreamSynchronize(a_->st); cudaFree(a_->work); a_->work = nullptr; a_->work_bytes = 0; }
-    a_->mu.unlock();
+    { std::lock_guard<std::mutex> lk(a_->mu); a_->busy = false; }
+    a_->cv.notify_one();
 }
 
 cudaStream_t HxStage::stream() const { return a_->st; }
@@ -65,8 +72,8 @@ int HxStage::workspace(void** dptr, size_t bytes) {
     if (bytes > a_->work_bytes) {
         HX_CUDA(cudaStreamSynchronize(a_->st));
         if (a_->work) { cudaFree(a_->work); a_->work = nullptr; a_->work_bytes = 0; }
-        const cudaError_t e = cudaMalloc(&a_->work, bytes);
-        if (e != cudaSuccess) { a_->work = nullptr; (void)cudaGetLastError(); return hx_fail(HX_ERR_CUDA, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e)); }
+        const cudaError_t e = hx_dev_malloc(&a_->work, bytes);
+        if (e != cudaSuccess) { a_->work = nullptr; return hx_fail(HX_ERR_CUDA, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e)); }
         a_->work_bytes = bytes;
     }
     big_ = a_->work_bytes > ST_KEEP;
@@ -75,7 +82,7 @@ int HxStage::workspace(void** dptr, size_t bytes) {
 }
 
 int HxStage::run(const HxCopy* c, int n, bool up) {
-    Area& A = *a_;
+    HxStageArea& A = *a_;
     struct Slice { uint8_t *dev, *host; size_t bytes; };
     std::vector<Slice> sl;
     for (int i = 0; i < n; i++)
@@ -130,13 +137,15 @@ int HxStage::run(const HxCopy* c, int n, bool up) {
 int HxStage::upload(const HxCopy* c, int n) { return run(c, n, true); }
 int HxStage::download(const HxCopy* c, int n) { return run(c, n, false); }
 
-bool hx_stage_trim() {
-    bool freed = false;
-    Area* a = areas();
-    for (int d = 0; d < 64; d++) {
-        if (!a[d].mu.try_lock()) continue;
-        if (a[d].work) { cudaFree(a[d].work); a[d].work = nullptr; a[d].work_bytes = 0; freed = true; }
-        a[d].mu.unlock();
+cudaError_t hx_dev_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    int dev = 0;
+    if (e != cudaSuccess) (void)cudaGetLastError();       // no error stays behind: the caller reports it
+    if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        HxStageArea& A = areas()[dev];
+        std::lock_guard<std::mutex> lk(A.mu);             // (a call that has the area keeps its workspace)
+        if (!A.busy && A.work) { cudaFree(A.work); A.work = nullptr; A.work_bytes = 0; e = cudaMalloc(p, bytes); }
+        if (e != cudaSuccess) (void)cudaGetLastError();
     }
-    return freed;
+    return e;
 }

@@ -17,11 +17,12 @@ public:
     int upload(const HxCopy* c, int n);          // later work on stream() sees the data; the host buffers have been read
     int download(const HxCopy* c, int n);        // what stream() has produced so far; the host buffers have been written
 private:
-    struct Area* a_;
+    struct HxStageArea* a_;
     int rc_;
     bool big_ = false;
     int run(const HxCopy* c, int n, bool up);
 };
 
-// Frees the idle staging areas' device memory (an allocation elsewhere failed); returns true when something was freed.
-bool hx_stage_trim();
+// cudaMalloc on the current device; where memory is short the idle staging area gives its workspace back first.  Leaves no error
+// behind for the next launch check.
+cudaError_t hx_dev_malloc(void** p, size_t bytes);
