@@ -3,9 +3,10 @@
 // A cudaMemcpy from pageable memory stages through the driver on one thread (about 12 GB/s where the link does 50), and a
 // call that allocates and frees its device buffers pays for mapping them each time.  Here up to eight threads copy slices of
 // one megabyte between the caller's memory and page-locked slots, two per thread, while the link moves the slot before;
-// slots, streams and a device workspace stay with the device for the next call.  They are bounded (16 MB page-locked, 256 MB
-// of device memory; a larger workspace is freed when the call ends), handed to one call at a time, and the workspace is
-// given back when device memory is short elsewhere in the library (hx_dev_malloc).  The threads live for one call: a call that needs one slice starts none.
+// slots, streams and a device workspace stay with the device for the next call.  They are bounded (16 MB page-locked, made per
+// thread when a call first needs it; 256 MB of device memory; a larger workspace is freed when the call ends), handed to one
+// call at a time, and the workspace is given back when device memory is short elsewhere in the library (hx_dev_malloc).  The
+// threads live for one call: a call that needs one slice starts none.
 #include "hx_stage.cuh"
 #include <condition_variable>
 #include <mutex>
@@ -22,23 +23,21 @@ struct HxStageArea {
     std::mutex mu; std::condition_variable cv;
     bool busy = false;                                    // a call has the area (mu is held for moments only)
     int dev = -1;
-    bool ready = false;
-    uint8_t* pinned = nullptr;                            // [worker][2] slots
+    uint8_t* pinned[ST_WORKERS] = {};                     // two slots each
     cudaStream_t st = nullptr, wst[ST_WORKERS] = {};
     cudaEvent_t ev[ST_WORKERS][2] = {}, done[ST_WORKERS] = {}, mark = nullptr;
     void* work = nullptr; size_t work_bytes = 0;
     int prepare() {
-        if (ready) return HX_OK;
         HX_CUDA(cudaGetDevice(&dev));
-        if (!pinned) HX_CUDA(cudaHostAlloc((void**)&pinned, ST_WORKERS * 2 * ST_SLICE, cudaHostAllocDefault));
         if (!st) HX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         if (!mark) HX_CUDA(cudaEventCreateWithFlags(&mark, cudaEventDisableTiming));
-        for (int w = 0; w < ST_WORKERS; w++) {
-            if (!wst[w]) HX_CUDA(cudaStreamCreateWithFlags(&wst[w], cudaStreamNonBlocking));
-            if (!done[w]) HX_CUDA(cudaEventCreateWithFlags(&done[w], cudaEventDisableTiming));
-            for (int i = 0; i < 2; i++) if (!ev[w][i]) HX_CUDA(cudaEventCreateWithFlags(&ev[w][i], cudaEventDisableTiming));
-        }
-        ready = true;
+        return HX_OK;
+    }
+    int prepare_worker(int w) {
+        if (!pinned[w]) HX_CUDA(cudaHostAlloc((void**)&pinned[w], 2 * ST_SLICE, cudaHostAllocDefault));
+        if (!wst[w]) HX_CUDA(cudaStreamCreateWithFlags(&wst[w], cudaStreamNonBlocking));
+        if (!done[w]) HX_CUDA(cudaEventCreateWithFlags(&done[w], cudaEventDisableTiming));
+        for (int i = 0; i < 2; i++) if (!ev[w][i]) HX_CUDA(cudaEventCreateWithFlags(&ev[w][i], cudaEventDisableTiming));
         return HX_OK;
     }
 };
@@ -61,6 +60,10 @@ HxStage::HxStage() : a_(nullptr), rc_(HX_OK) {
 
 HxStage::~HxStage() {
     if (!a_) return;
+    if (open_) {      // a call that failed: its copies must not meet the next call's in the slots or in the workspace
+        for (cudaStream_t s : a_->wst) if (s) cudaStreamSynchronize(s);
+        if (a_->st) cudaStreamSynchronize(a_->st);
+    }
     if (big_ && a_->work) { cudaStreamSynchronize(a_->st); cudaFree(a_->work); a_->work = nullptr; a_->work_bytes = 0; }
     { std::lock_guard<std::mutex> lk(a_->mu); a_->busy = false; }
     a_->cv.notify_one();
@@ -84,16 +87,22 @@ int HxStage::workspace(void** dptr, size_t bytes) {
 int HxStage::run(const HxCopy* c, int n, bool up) {
     HxStageArea& A = *a_;
     struct Slice { uint8_t *dev, *host; size_t bytes; };
-    std::vector<Slice> sl;
-    for (int i = 0; i < n; i++)
-        for (size_t o = 0; o < c[i].bytes; o += ST_SLICE)
-            sl.push_back({(uint8_t*)c[i].dev + o, (uint8_t*)c[i].host + o, c[i].bytes - o < ST_SLICE ? c[i].bytes - o : ST_SLICE});
-    if (sl.empty()) return HX_OK;
+    auto slices_of = [](const HxCopy& x) { return (x.bytes + ST_SLICE - 1) / ST_SLICE; };
+    size_t nsl = 0;
+    for (int i = 0; i < n; i++) nsl += slices_of(c[i]);
+    if (!nsl) return HX_OK;
+    auto slice = [&](size_t k) {
+        int i = 0;
+        while (k >= slices_of(c[i])) k -= slices_of(c[i++]);
+        const size_t o = k * ST_SLICE, left = c[i].bytes - o;
+        return Slice{(uint8_t*)c[i].dev + o, (uint8_t*)c[i].host + o, left < ST_SLICE ? left : ST_SLICE};
+    };
+    open_ = true;
     std::atomic<size_t> next{0};
     std::atomic<int> err{0};
     auto work = [&](int w) {
         cudaError_t e = cudaSetDevice(A.dev);
-        uint8_t* slot[2] = {A.pinned + (size_t)(2 * w) * ST_SLICE, A.pinned + (size_t)(2 * w + 1) * ST_SLICE};
+        uint8_t* slot[2] = {A.pinned[w], A.pinned[w] + ST_SLICE};
         Slice held[2]; bool full[2] = {false, false};
         auto finish = [&](int s) {                        // the slot's copy over the link is done; a download goes on to the caller's memory
             if (!full[s]) return;
@@ -103,10 +112,10 @@ int HxStage::run(const HxCopy* c, int n, bool up) {
         };
         for (int s = 0; e == cudaSuccess && !err.load(std::memory_order_relaxed); s ^= 1) {
             const size_t i = next.fetch_add(1);
-            if (i >= sl.size()) break;
+            if (i >= nsl) break;
             finish(s);
             if (e != cudaSuccess) break;
-            held[s] = sl[i];
+            held[s] = slice(i);
             if (up) {
                 memcpy(slot[s], held[s].host, held[s].bytes);
                 e = cudaMemcpyAsync(held[s].dev, slot[s], held[s].bytes, cudaMemcpyHostToDevice, A.wst[w]);
@@ -119,8 +128,13 @@ int HxStage::run(const HxCopy* c, int n, bool up) {
     };
     size_t nw = std::thread::hardware_concurrency() / 2;
     if (nw > ST_WORKERS) nw = ST_WORKERS;
-    if (nw > (sl.size() + 1) / 2) nw = (sl.size() + 1) / 2;      // two slices are worth a thread
+    if (nw > (nsl + 1) / 2) nw = (nsl + 1) / 2;      // two slices are worth a thread
     if (nw < 1) nw = 1;
+    for (size_t w = 0; w < nw; w++) {
+        const int rc = A.prepare_worker((int)w);
+        if (rc && w == 0) return rc;
+        if (rc) nw = w;                              // page-locked memory is short: the others take its slices
+    }
     // downloads follow what stream() has been given so far, uploads what it still reads from the workspace
     HX_CUDA(cudaEventRecord(A.mark, A.st));
     for (size_t w = 0; w < nw; w++) HX_CUDA(cudaStreamWaitEvent(A.wst[w], A.mark, 0));
@@ -131,6 +145,7 @@ int HxStage::run(const HxCopy* c, int n, bool up) {
     for (auto& t : th) t.join();
     if (err.load()) return hx_fail(HX_ERR_CUDA, "host copy: %s", cudaGetErrorString((cudaError_t)err.load()));
     if (up) for (size_t w = 0; w < started; w++) HX_CUDA(cudaStreamWaitEvent(A.st, A.done[w], 0));
+    else open_ = false;                                   // (downloads have been waited for, and they follow all that came before)
     return HX_OK;
 }
 

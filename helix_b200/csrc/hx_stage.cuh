@@ -19,7 +19,7 @@ public:
 private:
     struct HxStageArea* a_;
     int rc_;
-    bool big_ = false;
+    bool big_ = false, open_ = false;            // open_: copies may be in flight
     int run(const HxCopy* c, int n, bool up);
 };
 

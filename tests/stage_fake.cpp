@@ -55,13 +55,14 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) { std::lock_guard<std::recursi
 #define CHECK(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
 
 int main() {
+    // a small call page-locks what one thread needs
     std::vector<uint8_t> a(1000, 1), b(1000, 0);
     {
         HxStage s; void* d = nullptr;
         CHECK(!s.status() && !s.workspace(&d, 1000));
         HxCopy c = {d, a.data(), 1000}, e = {d, b.data(), 1000};
         CHECK(!s.upload(&c, 1) && !s.download(&e, 1));
-        CHECK(b == a);
+        CHECK(b == a && pinned_bytes <= (size_t)2 << 20);
     }
     // several copies, slices of a megabyte that do not divide them
     const size_t n0 = (5u << 20) + 17, n1 = 3;
@@ -75,6 +76,14 @@ int main() {
         CHECK(!s.upload(in, 2) && !s.download(out, 2));
         CHECK(u == x && v == y && in_flight() == 0);
     }
+    // a call that ends between its upload and its download leaves nothing in flight
+    {
+        HxStage s; void* d = nullptr;
+        CHECK(!s.workspace(&d, n0));
+        HxCopy in = {d, x.data(), n0};
+        CHECK(!s.upload(&in, 1));
+    }
+    CHECK(in_flight() == 0);
     // the idle workspace is given back to an allocation that needs it, the workspace of a call is not
     room = live + 100;
     void* p = nullptr;
