@@ -103,6 +103,7 @@ struct hx_model {
     void* pf_buf = nullptr;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
     int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
+    int pf_chunk = HX_PF_MAX, pf_attn = 0;      // tokens of a prompt chunk at most (HX_PF_CHUNK); HX_PF_ATTN: 1 tc, -1 vec, 0 by the rule
     uint8_t* pf_pieces = nullptr; size_t pf_pieces_bytes = 0; int pf_ctx_hint = 0;      // bf16 terms of K and V of a layer for the tensor-core attention, grown to the longest context seen
     float* pf_part = nullptr; size_t tp_pf_off = 0, tp_pf_area = 0; unsigned tp_pf_ep = 0;      // tensor-parallel chunk exchange
     int *d_bids = nullptr, *d_bpos = nullptr, *d_bseq = nullptr, *d_bnext = nullptr; float* pf_logits = nullptr; int b_cap = 0;   // batched decode
@@ -851,6 +852,8 @@ int persist_check(hx_model* m) {
 
 int finish_init(hx_model* m) {
     int rc = alloc_state(m); if (rc) return rc;
+    if (const char* e = getenv("HX_PF_CHUNK")) { const int v = atoi(e) / HX_TC_MAX_TOK * HX_TC_MAX_TOK; if (v >= HX_TC_MAX_TOK && v < HX_PF_MAX) m->pf_chunk = v; }
+    if (const char* e = getenv("HX_PF_ATTN")) m->pf_attn = strcmp(e, "tc") == 0 ? 1 : (strcmp(e, "vec") == 0 ? -1 : 0);
     const char* np = getenv("HX_NO_PDL");
     m->pdl = !(np && *np == '1');
     if (m->persist) {
@@ -1418,7 +1421,7 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, i
     const int ldq = QD + 2 * KVD;
     const float att_scale = 1.0f / sqrtf((float)DH);
     int rc;
-    bool tc = ctx_end > 0 && hx_pf_attn_tc_wanted(n, ctx_end, c.n_heads, c.n_kv_heads, DH);
+    bool tc = ctx_end > 0 && m->pf_attn >= 0 && hx_pf_attn_tc_takes(c.n_heads, c.n_kv_heads, DH) && (m->pf_attn > 0 || hx_pf_attn_tc_wanted(n, ctx_end, c.n_heads, c.n_kv_heads));
     if (tc) {
         size_t need = hx_pf_attn_tc_bytes(ctx_end, c.n_kv_heads);
         if (need > m->pf_pieces_bytes) {
@@ -1515,7 +1518,7 @@ static int run_prefill_batched(hx_model* m, int T, int seq) {
     int rc = pf_alloc(m, m->kv_cap); if (rc) return rc;
     const int ps[2] = {0, seq};                      // first position of the chunk, KV slot of the sequence
     HX_CUDA(cudaMemcpyAsync(m->d_pf_pos, ps, 8, cudaMemcpyHostToDevice, m->st));
-    const int nch = (T + m->pf_tb - 1) / m->pf_tb, gr = (T + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
+    const int tb = m->pf_chunk < m->pf_tb ? m->pf_chunk : m->pf_tb, nch = (T + tb - 1) / tb, gr = (T + HX_TC_MAX_TOK - 1) / HX_TC_MAX_TOK;
     const int chunk = (gr + nch - 1) / nch * HX_TC_MAX_TOK;
     int nlast = 0;
     for (int t0 = 0; t0 < T; t0 += chunk) {

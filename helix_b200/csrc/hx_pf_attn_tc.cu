@@ -303,12 +303,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_pf_attn_tc(const float* __res
 // Bytes of the term pieces for a context of `ctx` positions.
 size_t hx_pf_attn_tc_bytes(int ctx, int NKV) { return (size_t)NKV * ((ctx + AT_KT - 1) / AT_KT) * 12 * AT_PIECE; }
 
-// Whether a chunk of n_tok tokens that ends at position ctx should go this way: head_dim 128 and a group that shares a row
-// tile.  A row tile costs about 4.5 us per key tile however few of its rows exist and the key runs are not split over CTAs,
+// head_dim 128 and a group that shares a row tile
+bool hx_pf_attn_tc_takes(int NH, int NKV, int DH) { return DH == AT_DH && NH % NKV == 0 && NH / NKV <= 8; }
+
+// Whether a chunk of n_tok tokens that ends at position ctx should go this way (if it can).  A row tile costs about 4.5 us per key tile however few of its rows exist and the key runs are not split over CTAs,
 // while the vector kernel (hx_pf_attn) costs about 1.5 ns per (token, key) of eight kv heads plus 8 us and splits them: it
 // keeps the small windows at a long context.
-bool hx_pf_attn_tc_wanted(int n_tok, int ctx, int NH, int NKV, int DH) {
-    if (DH != AT_DH || NH % NKV || NH / NKV > 8) return false;
+bool hx_pf_attn_tc_wanted(int n_tok, int ctx, int NH, int NKV) {
     const int tpt = 128 / (NH / NKV), rt = (n_tok + tpt - 1) / tpt, kt = (ctx + AT_KT - 1) / AT_KT;
     const double waves = (rt * NKV + 147) / 148;
     const double tc = 8.0 + waves * (3.0 + 4.5 * (kt - 0.5 * (double)n_tok / AT_KT)), vec = 8.0 + 1.5e-3 * n_tok * (ctx - 0.5 * n_tok) * NH / 32.0;

@@ -43,7 +43,8 @@ int hx_pf_attn(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NK
 // The same on the tensor cores (hx_pf_attn_tc.cu), head_dim 128, one sequence: `pieces` holds hx_pf_attn_tc_bytes(ctx_len, NKV)
 // bytes, ctx_len = position of the chunk's last token + 1.
 size_t hx_pf_attn_tc_bytes(int ctx, int NKV);
-bool hx_pf_attn_tc_wanted(int n_tok, int ctx, int NH, int NKV, int DH);
+bool hx_pf_attn_tc_takes(int NH, int NKV, int DH);
+bool hx_pf_attn_tc_wanted(int n_tok, int ctx, int NH, int NKV);
 int hx_pf_attn_tc(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int NKV, const float* kc, const float* vc, int cap, float scale,
                   float* ctx, int ld_ctx, uint8_t* pieces, int ctx_len, int* err, cudaStream_t st);
 

@@ -1,6 +1,6 @@
-"""The chunk GEMM's kinds (pairs of CTAs, clusters over K, K in several blocks, an odd number of row tiles) and the prompt
-attention at token counts around their groups of 24 and row tiles, through a prompt's logits and cached rows
-against the CPU restatement."""
+"""The chunk GEMM's kinds (pairs of CTAs, clusters over K, K in several blocks, an odd number of row tiles) at token
+counts around its groups of 24, through a prompt's logits and cached rows against the CPU restatement.  (The prompt attention
+has tests/test_prompt_attention_gpu.py.)"""
 import numpy as np
 import pytest
 

@@ -1,5 +1,5 @@
 """GPT-2 prompts through the chunk GEMM and tokens through the one-launch layer kernel (d_model 256, 512 and 768), against the
-fp32 CPU restatement: contexts around the kernel's passes of 128 keys, the first position, and the last of the cache."""
+fp32 CPU restatement: contexts around the kernel's passes of 256 keys and beyond two of them, the first position, and the last of the cache."""
 import numpy as np
 import pytest
 
@@ -9,7 +9,7 @@ from test_gpt2_gpu import OracleGpt2, synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("d_model,n_layers,T,cap", [(256, 3, 1, 40), (256, 2, 126, 136), (512, 2, 25, 40), (768, 2, 255, 262)])
+@pytest.mark.parametrize("d_model,n_layers,T,cap", [(256, 3, 1, 40), (256, 2, 126, 136), (512, 2, 25, 40), (768, 2, 255, 262), (256, 2, 510, 520), (512, 2, 34, 40)])
 def test_prompt_then_tokens_match_checker(d_model, n_layers, T, cap):
     shape = dict(n_layers=n_layers, d_model=d_model, n_heads=d_model // 64, d_ff=4 * d_model, vocab=517, max_ctx=cap)
     wt = synth(shape, d_model + T)

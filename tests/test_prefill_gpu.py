@@ -1,5 +1,5 @@
-"""Batched prefill (chunks of 64 tokens = four groups of 16 through the tcgen05 GEMM in digit mode) against the fp32 CPU restatement
-and against the token-by-token path of the same library."""
+"""Batched prefill (one chunk here: up to 1008 tokens in groups of 24 through the tcgen05 GEMM) against the fp32 CPU
+restatement and against the token-by-token path of the same library."""
 import os
 
 import numpy as np
