@@ -191,7 +191,7 @@ __device__ __forceinline__ void df_wait2(const u64* p, unsigned ep, float& a, fl
     df_fail(S, P);
     a = ll_val(x); b = ll_val(y);
 }
-// ---- attention work split: the number of splits follows the context length (about 64 positions each) ----
+// ---- attention work split: the number of splits follows the context length (about 16 positions each) ----
 __device__ __noinline__ AttPlan att_plan_df(const HxPersist& P, int cta, int pos, int nring, int* ns_out, int* tile_rows, int* ntiles) {
 #ifndef DF_SPLIT_ROWS_LOG2
 #define DF_SPLIT_ROWS_LOG2 4          // about 16 cached positions per attention split while CTAs are left (measured best: 8..16)

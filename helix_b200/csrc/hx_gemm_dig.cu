@@ -6,7 +6,10 @@
 //
 // A unit of work is a 128-row tile of W times a group of 24 tokens: 240 digit columns, tcgen05.mma kind::mxf4nvf4 with
 // M = 128, N = 240, K = 64, 120 cycles each (the pipe's rate; the scale-factor copies of a weight cell hide behind it).
-// What bounds a large chunk is that pipe; what bounds a small one (a group or two) is the weights from HBM.
+// What bounds a large chunk: the MMA's operands (98 bytes per cycle) and the weights that arrive (38) ask more than the 128 that
+// shared memory moves, so the pipe is busy for about 155 cycles per MMA, and for a third of a launch (512 tokens, 8B shape) it
+// waits for ramps, read-outs and the passage between blocks of K.  What bounds a small one (a group or two) is the weights
+// from HBM and the fixed part of a launch.
 //
 // K is cut over the CTAs of a cluster, not over time: CTA q of C keeps the digit cells of its part of K (at most four
 // 256-column cells, 120 KB) in shared memory and streams only weight cells (18 KB per four MMAs = 38 bytes per cycle and

@@ -728,7 +728,8 @@ int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, con
     const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
     const bool cl = grid.y > 1 && grid.y <= PFD_CL && !b;
     // Started early, this kernel's CTAs wait beside the GEMM's and the step got slower up to some hundred tokens (64 sequences
-    // 3.72 -> 3.85 ms for twelve layers, five sequences 0.97 -> 1.03); at 512 tokens it gains 3 %.
+    // 3.72 -> 3.85 ms for twelve layers, five sequences 0.97 -> 1.03); at 512 tokens it gains 3 %.  Measured at 5, 64 and 512 tokens:
+    // the line between is a guess.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(PFD_T); cfg.stream = st;
     cudaLaunchAttribute at[2];

@@ -13,8 +13,8 @@
 // With pos_arr == null and seqp != null the whole chunk belongs to sequence *seqp (prefill into one KV slot of a batch).
 struct HxPfWhere { const int* posp; const int* pos_arr; const int* seq_arr; size_t seq_stride; const int* seqp; };
 
-// Positions are read from device memory (*posp = position of the chunk's first token) so that the launches of a
-// chunk can be captured once and replayed.
+// Positions are read from device memory (*posp = position of the chunk's first token), so that a captured batch step can be
+// replayed; chunks of a prompt are launched one by one.
 // X[t][:] = emb[ids[*posp + t]][:] (+ wpe[*posp + t][:])
 int hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe, float* X, int n_tok, int DM, cudaStream_t st);
 

@@ -7,9 +7,10 @@
 // (amax/2688, ts*6, bamax/(ts*6), decode(micro)*ts, v/eff) are issued as separately rounded IEEE
 // operations (__fdiv_rn / __fmul_rn are never contracted), the rest is compares and integers.
 //
-// Data flow (HBM-bound): pass 1 reads the tensor once for the per-tensor amax; pass 2 reads it again -- last rows first, so
+// Data flow: pass 1 reads the tensor once for the per-tensor amax (bound by HBM); pass 2 reads it again -- last rows first, so
 // that what pass 1 left in L2 is met before it is evicted -- and writes 4.57 bits of codes + 0.5 bits of scale per element.
-// Small tensors do both passes in one launch by one cluster.
+// Pass 2 is bound by latency: a warp's loads and its arithmetic take turns (12288 x 4096: 57.6 us at 50 % of DRAM and 59 % of SM
+// throughput).  Small tensors do both passes in one launch by one cluster.
 #include "hx_common.cuh"
 #include "hx_stage.cuh"
 
