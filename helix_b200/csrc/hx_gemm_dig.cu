@@ -332,24 +332,36 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         // A block per CTA by one bulk copy between shared memories, which counts its bytes at the receiver's barrier: nobody waits
         // for stores to arrive.  (st.async of single words counts a transaction per lane
         // and was unusable.)
+        // Nothing at the source says when such a copy has read its block (bulk groups hold only copies that complete by group), so the
+        // staging is given back when every other CTA has taken its sums of the unit: rx_free of unit u follows the reads of what the
+        // copies wrote, these follow rx_full there, which counts the copies' bytes.  No circle: a CTA takes unit u as soon as its own
+        // read-out and the copies of unit u are done, and both wait only for units before.
         if (C > 1) {
             const uint32_t to = lane < C ? cl_map(s_u32(rx) + (uint32_t)((q < lane ? q : q - 1) * blk), (uint32_t)lane) : 0u;
             const uint32_t bar = lane < C ? cl_map(s_u32(&S.rx_full), (uint32_t)lane) : 0u;
-            int ou = 0;
+            int ou = 0, announced = 0;
+            bool ok = true;
             dg_walk(g, u0, u1, [&](int, int, int, bool, bool) {
-                if (!warp_wait(&S.st_full, (uint32_t)ou & 1u, ab_flag)) return false;
-                if (ou >= 1 && !warp_wait(&S.rx_full, (uint32_t)(ou - 1) & 1u, ab_flag)) return false;      // the unit before has arrived here: announce this one
+                ok = warp_wait(&S.st_full, (uint32_t)ou & 1u, ab_flag) &&
+                     (ou == 0 || warp_wait(&S.rx_full, (uint32_t)(ou - 1) & 1u, ab_flag));                  // the unit before has arrived here: announce this one
+                if (!ok) return false;
                 if (lane == 0) mb_expect(&S.rx_full, (uint32_t)((C - 1) * blk));
-                if (ou >= 1 && !warp_wait(&S.rx_free, (uint32_t)(ou - 1) & 1u, ab_flag)) return false;      // and has been taken there
-                if (lane < C && lane != q) cl_bulk(to, s_u32(stage + lane * blk), (uint32_t)blk, bar);
-                bulk_commit();
-                bulk_wait_read();
-                __syncwarp();
+                announced = ou + 1;
+                if (lane < C && lane != q) cl_bulk(to, s_u32(stage + lane * blk), (uint32_t)blk, bar);      // (the unit before has been taken there)
+                if (!(ok = warp_wait(&S.rx_free, (uint32_t)ou & 1u, ab_flag))) return false;
                 if (lane == 0) mb_arrive(&S.st_free);
                 ou++;
                 return true;
             });
-            bulk_wait_all();      // the CTA must not end with a copy of its own in flight
+            // Given up: no CTA may end with copies to or from it in flight.  A CTA waits for those to it, the cluster leaves together.
+            // What can still come is the unit announced last and, as the others cannot finish one without this CTA's part, one more.
+            if (!ok && lane == 0) {
+                const bool came = !announced || mb_drain(&S.rx_full, (uint32_t)(announced - 1) & 1u);
+                if (came && announced < (u1 - u0) * g.nblk) {
+                    mb_expect(&S.rx_full, (uint32_t)((C - 1) * blk));
+                    mb_drain(&S.rx_full, (uint32_t)announced & 1u);
+                }
+            }
         }
     } else {
         // ------------------------------ finish: add the K parts, scale, store ------------------------------

@@ -32,10 +32,12 @@ __device__ __forceinline__ bool mb_bounded(Try&& poll, volatile int* abort_flag,
 __device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag, unsigned limit_ns = HX_TC_WAIT_NS) {
     return mb_bounded([&] { return mb_try(b, parity); }, abort_flag, limit_ns);
 }
-// For copies of one's own that are in flight when the work is given up: waits whatever the abort flag says.
-__device__ __forceinline__ void mb_drain(uint64_t* b, uint32_t parity) {
+// For copies that are in flight when the work is given up: waits whatever the abort flag says.
+__device__ __forceinline__ bool mb_drain(uint64_t* b, uint32_t parity) {
     const unsigned long long t0 = now_ns();
-    while (!mb_try(b, parity) && now_ns() - t0 < HX_TC_WAIT_NS) { }
+    bool over;
+    while (!(over = mb_try(b, parity)) && now_ns() - t0 < HX_TC_WAIT_NS) { }
+    return over;
 }
 // A wait of the whole warp: every lane gets the same answer, so the warp leaves a loop together.
 __device__ __forceinline__ bool warp_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
@@ -90,13 +92,10 @@ __device__ __forceinline__ void cl_arrive(uint32_t bar) { asm volatile("mbarrier
 // An arrival that orders nothing by itself: for handing back a buffer after reads that the caller knows to be over.  (A release at
 // cluster scope waits for the thread's global stores as well, about a microsecond.)
 __device__ __forceinline__ void cl_arrive_relaxed(uint32_t bar) { asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory"); }
-// A block of this CTA's shared memory into another CTA's; the bytes count at a barrier there.
+// A block of this CTA's shared memory into another CTA's; the bytes count at a barrier there, which is all that tells its end.
 __device__ __forceinline__ void cl_bulk(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" :: "r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }      // the sources may change
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void cl_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
