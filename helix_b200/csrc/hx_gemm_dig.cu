@@ -47,13 +47,10 @@ constexpr int DG_EP = (DG_TOK / 2 + 1) / 2;      // token pairs of a read-out wa
 constexpr float DG_13P7 = 62748516.0f;       // 13^7 - 1: fmaf(v, DG_13P7, v) is v * 13^7, rounded once
 static_assert(HX_TC_DIGITS == 8, "a token is eight columns");
 
-// Columns of a resident cell's scale factors: 128 accumulator columns in four.
-__host__ __device__ constexpr int dg_sf_cols(int group) { return 8 * group > 128 ? 8 : 4; }
 // Token pairs that a CTA of the cluster finishes, and their sums in one unit: [pair][128 rows][2 tokens].
 __host__ __device__ constexpr int dg_pairs(int group, int C) { return (group / 2 + C - 1) / C; }
 __host__ __device__ constexpr int dg_blk(int group, int C) { return dg_pairs(group, C) * 1024; }
-// Digit cells that fit beside a ring of four, the staged sums (a block per CTA), a received block per other CTA and, in TMEM,
-// beside two accumulators and the scales of two weight cells.
+// Digit cells that fit beside a ring of four, the staged sums (a block per CTA) and a received block per other CTA.
 __host__ __device__ constexpr int dg_sum_bytes(int group, int C) { return (2 * C - 1) * dg_blk(group, C); }
 // Token pairs per finishing thread for `shares` threads per row; a thread reads as many as a full group has, so the last block is
 // followed by as many pairs as it may read too far.
@@ -65,11 +62,10 @@ constexpr int dg_over(int group, int C) {
 constexpr int DG_HDR = 2048, DG_SMEM = 227 * 1024;
 constexpr int dg_room(int group, int C) { return DG_SMEM - 1024 - DG_HDR - dg_sum_bytes(group, C) - dg_over(group, C); }
 constexpr int dg_res_cells(int group, int C) {
-    int n = (dg_room(group, C) - 4 * HX_T128_CELL) / HX_TC_DCELL(group);
-    const int t = (512 - 16 * group - 32) / dg_sf_cols(group);
-    if (n > t) n = t;
+    const int n = (dg_room(group, C) - 4 * HX_T128_CELL) / HX_TC_DCELL(group);
     return n < DG_RES ? n : DG_RES;
 }
+static_assert(16 * DG_TOK + 2 * 16 + 2 * 8 <= 512, "two accumulators, row scales and column scales of either issuing warp in TMEM");
 static_assert(dg_res_cells(DG_TOK, 1) >= 4 && dg_res_cells(DG_TOK, 2) >= 4 && dg_res_cells(DG_TOK, 4) >= 4, "four cells of a full group");
 // What the digit cells leave goes to the ring: loads in flight are what the MMAs wait for.
 constexpr int dg_stages(int group, int C, int res) { const int n = (dg_room(group, C) - res * HX_TC_DCELL(group)) / HX_T128_CELL; return n < DG_STAGES ? n : DG_STAGES; }
@@ -79,7 +75,7 @@ struct DgSmem {
     // ring of weight cells: a pair of barriers per slot for each MMA warp.  (One for both would pass two uses on between two looks of a
     // warp, and a parity tells a use from the next one only.)
     uint64_t full[2][DG_STAGES], empty[2][DG_STAGES], bfull[DG_RES], bempty[DG_RES];
-    uint64_t accum[2], acc_free[2], st_full, st_free, rx_full, rx_free, sfb_ready;
+    uint64_t accum[2], acc_free[2], st_full, st_free, rx_full, rx_free;
     uint32_t tmem_base;
     volatile uint32_t zero;                  // see the hand-back of the finishing warps
     volatile int abort_flag;
@@ -152,7 +148,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         for (int i = 0; i < DG_RES; i++) { mb_init(&S.bfull[i], 1); mb_init(&S.bempty[i], 2); }
         for (int i = 0; i < 2; i++) { mb_init(&S.accum[i], 1); mb_init(&S.acc_free[i], DG_EPI); }
         mb_init(&S.rx_full, 1); mb_init(&S.rx_free, C > 1 ? DG_FIN * (C - 1) : 1);
-        mb_init(&S.sfb_ready, 1); mb_init(&S.st_full, DG_EPI); mb_init(&S.st_free, DG_FIN + (C > 1 ? 1 : 0));
+        mb_init(&S.st_full, DG_EPI); mb_init(&S.st_free, DG_FIN + (C > 1 ? 1 : 0));
         S.abort_flag = 0; S.zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -164,7 +160,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
     cl_sync();
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    const uint32_t ncols = 8u * (uint32_t)G, col_sfa = 2u * ncols, col_sfb = col_sfa + 32u, sfb_w = (uint32_t)dg_sf_cols(G);
+    const uint32_t ncols = 8u * (uint32_t)G, col_sfa = 2u * ncols, col_sfb = col_sfa + 32u;
     volatile int* ab_flag = &S.abort_flag;
 
     if (warp == 0) {
@@ -229,27 +225,29 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
     } else if (warp == 1 || warp == DG_W_MMA2) {
         // ------------------------------ MMA issuers ------------------------------
         // Two warps, one per accumulator: what lies between two units in a warp (waits, the walk, the issue of the first instructions:
-        // about 1100 cycles) is more than the one or two MMAs that the pipe holds, so the other warp's unit fills it.  A pass's column
-        // scales are copied by the warp of its first unit; the other one waits for them.
+        // about 1100 cycles) is more than the one or two MMAs that the pipe holds, so the other warp's unit fills it.  Each warp copies
+        // the column scales of a cell before its MMAs, as it does the row scales, so neither depends on what the other has copied.  (Copied once
+        // per pass over the tiles by the warp of its first unit, with a barrier that the other one waited at: 1 to 2 % slower, and that warp could take
+        // the barrier of the pass before for this one's.)
         // instruction descriptor: E2M1 x E2M1, UE4M3 scales, K-major both, M = 128, N = 8 G, K = 64
         const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)G << 17) | (8u << 24);
         const int mw = warp == 1 ? 0 : 1;
         const uint64_t dA0 = smem_desc(s_u32(ring), 16, 1024, SW128), dS0 = smem_desc(s_u32(ring) + 16384, 16, 128);
         const uint64_t dB0 = smem_desc(s_u32(bres), 16, 1024, SW128);
         const uint64_t dC0 = smem_desc(s_u32(bres) + (uint32_t)G * 1024u, 16, 128);      // column scales of a digit cell
-        const uint32_t acc = tmem + (uint32_t)mw * ncols, sfa = tmem + col_sfa + (uint32_t)mw * 16u;
-        uint32_t slot = 0, fpar = 0, bpar = 0, pass = 0;             // (fpar, bpar: a parity per slot and digit cell)
+        const uint32_t acc = tmem + (uint32_t)mw * ncols, sfa = tmem + col_sfa + (uint32_t)mw * 16u, sfb = tmem + col_sfb + (uint32_t)mw * 8u;
+        const bool wide = ncols > 128u;
+        uint32_t slot = 0, fpar = 0, bpar = 0;             // (fpar, bpar: a parity per slot and digit cell)
         int ou = 0;
         bool ok = true;
         for (int u = u0; u < u1 && ok; ) {
             const int t0 = u % g.ntiles, nt = min(g.ntiles - t0, u1 - u);
-            for (int kb = 0; kb < g.nblk && ok; kb++, pass++) {
+            for (int kb = 0; kb < g.nblk && ok; kb++) {
                 const int p = kb * C + q, nc = (p + 1) * g.kcells / NP - p * g.kcells / NP;
                 const int first = (ou ^ mw) & 1;                     // this warp's first unit of the pass
                 for (int ci = 0; ci < nc && ok && first > 0; ci++) ok = warp_wait(&S.bfull[ci], (bpar >> ci) & 1u, ab_flag);
-                if (first >= nt) {                                   // none: the cells are not used here
-                    if (ok && lane == 0) for (int ci = 0; ci < nc; ci++) mb_arrive(&S.bempty[ci]);
-                } else if (ok && first > 0) ok = warp_wait(&S.sfb_ready, pass & 1u, ab_flag);
+                if (first >= nt && ok && lane == 0)                  // none: the cells are not used here
+                    for (int ci = 0; ci < nc; ci++) mb_arrive(&S.bempty[ci]);
                 for (int t = 0; t < nt && ok; t++, ou++) {
                     if ((ou & 1) != mw) { slot = (slot + (uint32_t)nc) % stages; continue; }
                     const bool done = t + 2 >= nt;
@@ -262,13 +260,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                         // the descriptors of a cell's four steps differ by constants (the address field counts 16-byte units)
                         const uint64_t dA = dA0 + (uint64_t)(slot * (HX_T128_CELL >> 4)), dS = dS0 + (uint64_t)(slot * (HX_T128_CELL >> 4));
                         const uint64_t dB = dB0 + (uint64_t)((uint32_t)ci * (dcell >> 4)), dC = dC0 + (uint64_t)((uint32_t)ci * (dcell >> 4));
-                        const uint32_t sfb = tmem + col_sfb + (uint32_t)ci * sfb_w;
                         if (tc_elect()) {
-                            if (t == 0) {
-                                tc_cp_sf(sfb, dC);
-                                if (sfb_w > 4) tc_cp_sf(sfb + 4, dC + 32u);
-                                if (ci + 1 == nc) tc_commit(&S.sfb_ready);
-                            }
+                            tc_cp_sf(sfb, dC);
+                            if (wide) tc_cp_sf(sfb + 4, dC + 32u);
 #pragma unroll
                             for (int k = 0; k < 4; k++) tc_cp_sf(sfa + k * 4, dS + (uint64_t)(k * 32));
 #pragma unroll

@@ -1,5 +1,6 @@
-"""Hand-overs between the roles of the chunk GEMM where little time lies between them: one or two cells of K per CTA, token groups of two
-and of 26.  A prompt gives the same bits every time, and the K and V rows of the second layer, which depend on every token's sums in the first, are those
+"""Hand-overs between the roles of the chunk GEMM where little time lies between them: one to three cells of K per CTA, token groups of two
+and of 26, and plans in which a cluster goes from the last tile of a token group to several tiles of the next with fewer cells of K.
+A prompt gives the same bits every time, and the K and V rows of the second layer, which depend on every token's sums in the first, are those
 of the token-by-token path (f32 sums of the same values in another order through one layer)."""
 import numpy as np
 import pytest
@@ -10,6 +11,8 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = {
     "K768": dict(n_layers=2, d_model=768, n_heads=6, n_kv_heads=6, head_dim=128, d_ff=3072, vocab=300),
+    "K12288": dict(n_layers=2, d_model=4096, n_heads=32, n_kv_heads=8, head_dim=128, d_ff=12288, vocab=300),
+    "K25600": dict(n_layers=2, d_model=5120, n_heads=64, n_kv_heads=8, head_dim=128, d_ff=25600, vocab=300),
 }
 
 
@@ -17,7 +20,8 @@ def _rows(m, T):
     return [a for h in range(m.cfg.n_kv_heads) for a in m.kv_read(1, h, 0, T)]
 
 
-@pytest.mark.parametrize("shape,T,repeats", [("K768", 2, 60), ("K768", 26, 60), ("K768", 53, 60), ("K768", 300, 40)])
+@pytest.mark.parametrize("shape,T,repeats", [("K768", 2, 60), ("K768", 26, 60), ("K768", 53, 60), ("K768", 300, 40),
+                                             ("K12288", 212, 12), ("K12288", 262, 12), ("K25600", 128, 12), ("K25600", 270, 8)])
 def test_repeated_prompts_are_bit_equal_and_near_the_token_path(shape, T, repeats):
     ids = np.random.default_rng(T).integers(0, 300, T).astype(np.int32)
     m, one = (hb.Model.synth(SHAPES[shape], seed=T, kv_cap=T + 4) for _ in range(2))
