@@ -75,7 +75,7 @@ struct DgSmem {
     // ring of weight cells: a pair of barriers per slot for each MMA warp.  (One for both would pass two uses on between two looks of a
     // warp, and a parity tells a use from the next one only.)
     uint64_t full[2][DG_STAGES], empty[2][DG_STAGES], bfull[DG_RES], bempty[DG_RES];
-    uint64_t accum[2], acc_free[2], st_full, st_free, rx_full, rx_free;
+    uint64_t accum[2], acc_free[2], st_full, st_free, rx_full, rx_free, given_up[2];
     uint32_t tmem_base;
     volatile uint32_t zero;                  // see the hand-back of the finishing warps
     volatile int abort_flag;
@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         for (int i = 0; i < 2; i++) { mb_init(&S.accum[i], 1); mb_init(&S.acc_free[i], DG_EPI); }
         mb_init(&S.rx_full, 1); mb_init(&S.rx_free, C > 1 ? DG_FIN * (C - 1) : 1);
         mb_init(&S.st_full, DG_EPI); mb_init(&S.st_free, DG_FIN + (C > 1 ? 1 : 0));
+        mb_init(&S.given_up[0], 1); mb_init(&S.given_up[1], 1);
         S.abort_flag = 0; S.zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -279,6 +280,11 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                 bpar ^= (1u << nc) - 1u;
             }
             u += nt;
+        }
+        if (!ok) {       // given up: the tensor memory and the cells must outlive the MMAs that were issued
+            if (tc_elect()) tc_commit(&S.given_up[mw]);
+            __syncwarp();
+            mb_drain(&S.given_up[mw], 0);
         }
     } else if (warp < DG_W_FIN) {
         // ------------------------------ read-out: TMEM -> fold -> the token's CTA ------------------------------
