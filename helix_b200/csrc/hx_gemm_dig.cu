@@ -2,7 +2,7 @@
 // times f32 activations that enter the FP4 tensor cores as digit columns (hx_prefill.cu: k_pf_digits).  Replaces the f32
 // tiled_matmul_abt projections of forward_layer_llama, helixc/runtime/gpt2_infer.c:1231-1287.
 //
-//   out[t][row] (+)= scale_t * ts(row) * 13^7 * sum_d 13^-d ( sum_k W[row,k] * SF[row,k/16] * CS[t,k/256] * digit_d[t,k] )
+//   out[t][row] (+)= scale_t * ts(row) * 13^7 * sum_d 13^-d ( sum_k W[row,k] * SF[row,k/16] * CS[t,block of k] * digit_d[t,k] )
 //
 // A unit of work is a 128-row tile of W times a group of G <= 26 tokens: 8 G digit columns, tcgen05.mma kind::mxf4nvf4 with
 // M = 128, N = 8 G, K = 64, N / 2 cycles each at large N (the pipe's rate, which neither the scale copies nor loads, TMEM reads and
@@ -11,7 +11,7 @@
 // brought from L2 (385 cycles of the SM's port each), used -- and the ring holds five; then ramp, drain and the passage
 // between blocks of K.  What bounds a small one (a group or two): the weights from HBM and the fixed part of a launch.
 //
-// K is cut over the CTAs of a cluster, not over time: CTA q of C keeps the digit cells of its part of K (27 KB each at 26 tokens,
+// K is cut over the CTAs of a cluster, not over time: CTA q of C keeps the digit cells of its part of K (28 KB each at 26 tokens,
 // as many as fit: four, or sixteen for six tokens) in shared memory and streams only weight cells (18 KB per four MMAs).  Two
 // accumulators lie in TMEM, each with an issuing warp of its own, so a unit's MMAs run while the unit before is read out: a thread folds
 // a row's eight digit accumulators of two tokens at a time (f32x2), the small ones first (v = D7; v = D6 + v / 13; ...: every step's
@@ -22,8 +22,11 @@
 //
 // Digits, GEMM and epilogue of the four linears of a layer of the 8B shape, launch by launch, before / now (ten base-9 digits, 24 tokens a group, one issuing
 // warp, sums sent by plain stores and a cluster-scope release that held the read-out up for 1500 cycles a unit): 5 tokens 80 / 74 us,
-// 64 119 / 109, 77 137 / 113, 512 447 / 370, 1008 795 / 690.  Error against 64 bits (2-norm, relative; N(0, 1), heavy-tailed and
-// vectors with one element 64 or 1000 times the others): 6.5e-8 .. 9e-8 / 4e-8 .. 7e-8.
+// 64 119 / 109, 77 137 / 113, 512 447 / 370, 1008 795 / 690.  Error against 64 bits (relative, 2-norm over
+// the rows; K = 768 .. 12288; ten base-9 digits / now): 6e-8 .. 9e-8 / 5e-8 .. 8e-8 for N(0, 1), heavy-tailed vectors and those with an element 64 to a
+// million times the others.  Rows whose weight on the large element is zero, which see the resolution of the elements beside it: 64 times
+// 1.0e-7 .. 1.3e-7 / 7e-8 .. 9e-8, 1000 times 1.1e-6 .. 1.3e-6 / 2.6e-7 .. 9.6e-7, one in every 256 elements 64 times 1.3e-7 .. 1.5e-7 / 1.4e-7 ..
+// 1.6e-7 (K = 256, one element 1000 times: 1.0e-6 / 1.5e-6).
 //
 // K beyond the resident cells is done in blocks, one pass over the tiles each; the sums so far wait in global memory between
 // the passes (the same thread writes and reads them).  Every wait is bounded; the roles meet only at mbarriers.
@@ -65,7 +68,7 @@ constexpr int dg_res_cells(int group, int C) {
     const int n = (dg_room(group, C) - 4 * HX_T128_CELL) / HX_TC_DCELL(group);
     return n < DG_RES ? n : DG_RES;
 }
-static_assert(16 * DG_TOK + 2 * 16 + 2 * 8 <= 512, "two accumulators, row scales and column scales of either issuing warp in TMEM");
+static_assert(16 * DG_TOK + 2 * 16 + 2 * 16 <= 512, "two accumulators, row scales and column scales of either issuing warp in TMEM");
 static_assert(dg_res_cells(DG_TOK, 1) >= 4 && dg_res_cells(DG_TOK, 2) >= 4 && dg_res_cells(DG_TOK, 4) >= 4, "four cells of a full group");
 // What the digit cells leave goes to the ring: loads in flight are what the MMAs wait for.
 constexpr int dg_stages(int group, int C, int res) { const int n = (dg_room(group, C) - res * HX_TC_DCELL(group)) / HX_T128_CELL; return n < DG_STAGES ? n : DG_STAGES; }
@@ -235,9 +238,10 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
         const int mw = warp == 1 ? 0 : 1;
         const uint64_t dA0 = smem_desc(s_u32(ring), 16, 1024, SW128), dS0 = smem_desc(s_u32(ring) + 16384, 16, 128);
         const uint64_t dB0 = smem_desc(s_u32(bres), 16, 1024, SW128);
-        const uint64_t dC0 = smem_desc(s_u32(bres) + (uint32_t)G * 1024u, 16, 128);      // column scales of a digit cell
-        const uint32_t acc = tmem + (uint32_t)mw * ncols, sfa = tmem + col_sfa + (uint32_t)mw * 16u, sfb = tmem + col_sfb + (uint32_t)mw * 8u;
+        const uint64_t dC0 = smem_desc(s_u32(bres) + (uint32_t)G * 1024u, 16, 128);      // column scales of a digit cell: MMA steps 0 and 1, 2 and 3
+        const uint32_t acc = tmem + (uint32_t)mw * ncols, sfa = tmem + col_sfa + (uint32_t)mw * 16u, sfb = tmem + col_sfb + (uint32_t)mw * 16u;
         const bool wide = ncols > 128u;
+        const uint32_t dsf = (uint32_t)HX_TC_DSF(G) >> 4;
         uint32_t slot = 0, fpar = 0, bpar = 0;             // (fpar, bpar: a parity per slot and digit cell)
         int ou = 0;
         bool ok = true;
@@ -263,12 +267,13 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                         const uint64_t dB = dB0 + (uint64_t)((uint32_t)ci * (dcell >> 4)), dC = dC0 + (uint64_t)((uint32_t)ci * (dcell >> 4));
                         if (tc_elect()) {
                             tc_cp_sf(sfb, dC);
-                            if (wide) tc_cp_sf(sfb + 4, dC + 32u);
+                            tc_cp_sf(sfb + 8, dC + dsf);
+                            if (wide) { tc_cp_sf(sfb + 4, dC + 32u); tc_cp_sf(sfb + 12, dC + dsf + 32u); }
 #pragma unroll
                             for (int k = 0; k < 4; k++) tc_cp_sf(sfa + k * 4, dS + (uint64_t)(k * 32));
 #pragma unroll
                             for (int k = 0; k < 4; k++)
-                                tc_mma(acc, dA + (uint64_t)(k * 2), dB + (uint64_t)(k * 2), idesc, sfa + k * 4, sfb, (k > 0 || ci > 0) ? 1u : 0u);
+                                tc_mma(acc, dA + (uint64_t)(k * 2), dB + (uint64_t)(k * 2), idesc, sfa + k * 4, sfb + (k >> 1) * 8, (k > 0 || ci > 0) ? 1u : 0u);
                             tc_commit(&S.empty[mw][slot]);
                             if (done) tc_commit(&S.bempty[ci]);
                             if (ci + 1 == nc) tc_commit(&S.accum[mw]);

@@ -9,8 +9,11 @@
 #define HX_TC_RES_CELLS 16         // digit cells of a (part of K, token group) that a CTA keeps at most (as many as fit beside the ring of weight cells)
 #define HX_TC_DIGITS 8             // base-13 digits of a 29-bit signed integer per activation, digit values 0, 1, 2, 3, 4, 6, 8 and their negatives
 #define HX_TC_MAX_TOK 26           // tokens per group at most: digit d of token t is column 16 (t / 2) + 2 d + t % 2, up to 208 columns per MMA
-#define HX_TC_DCELL(G) (((G) + 1) * 1024)  // bytes of a digit cell: 1024 per token (8 swizzled rows of 128), then 1024 of column scales
-#define HX_TC_DIGIT_UNIT 134217728.0f      // 2^27: the integer is |x| / (scale of the cell) * 2^27 <= 2^28
+// Bytes of a digit cell: 1024 per token (8 swizzled rows of 128), then the column scales of the first and of the second 128 columns of K: 512 bytes
+// per 128 digit columns each.
+#define HX_TC_DSF(G) ((G) > 16 ? 1024 : 512)
+#define HX_TC_DCELL(G) ((G) * 1024 + ((G) > 16 ? 2048 : 1024))
+#define HX_TC_DIGIT_UNIT 134217728.0f      // 2^27: the integer is |x| / (scale of the block) * 2^27 <= 2^28
 
 struct HxGemmTC {                  // raw GEMM
     const uint8_t* a;              // T128 cells, [tile][kstep]
@@ -26,7 +29,7 @@ size_t hx_gemm_tc_smem(int ncols, int stage_ksteps);
 //   y = act(col_scale[t] * ts(row) * 13^7 * sum_d 13^-d D_d[row][t] + bias[row])
 struct HxGemmDig {
     const uint8_t* a;              // T128 weight cells [tile][cell of 256 columns]
-    const uint8_t* b;              // digit cells [cell of 256 columns][token group] of HX_TC_DCELL(group) bytes
+    const uint8_t* b;              // digit cells [cell of 256 columns][token group] of HX_TC_DCELL(tokens of a group) bytes
     int rows, ntiles, kcells, ntok;
     const float* col_scale;        // [ntok] scale of each token's digits (a power of two)
     float* out; int ld_out;        // token-major output

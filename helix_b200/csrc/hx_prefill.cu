@@ -3,9 +3,9 @@
 // Replaces forward_layer_llama / forward_full (helixc/runtime/gpt2_infer.c:1231-1333): where the reference runs
 // f32 tiled_matmul_abt over a dequantized weight copy per layer, a chunk of prompt tokens here is one
 // block-scaled NVFP4 GEMM per linear with the weights read in their packed form.  The activations enter the FP4
-// tensor path as digits: after the optional RMSNorm each element is x = s_c * sum_d digit_d 13^(7-d) with eight base-13 digits
-// of the integer x / S_c * 2^27 (S_c: the power of two at or below the largest element of the vector's 256-column cell c), every
-// digit an E2M1 column; S_c over the vector's S is the column's block scale, the GEMM epilogue folds the eight accumulators
+// tensor path as digits: after the optional RMSNorm each element is x = s_b * sum_d digit_d 13^(7-d) with eight base-13 digits
+// of the integer x / S_b * 2^27 (S_b: the power of two at or below the largest element of the value's 32-column block b), every
+// digit an E2M1 column; S_b over the vector's S is the column's block scale, the GEMM epilogue folds the eight accumulators
 // of a token.  (The decode kernel uses sixteen exact base-4 digits: there the column count is free.)
 // Norm, RoPE, KV append and attention are small f32 kernels over the chunk.
 #include "hx_tc.cuh"
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) k_pf_embed(const int* __restrict__ ids, H
 // distributed shared memory; beyond that every CTA reads the whole vector.
 // A warp holds a 256-column cell of the token; the digits are those of hx_digits.cuh.
 // (Ten balanced base-9 digits against the vector's S: 25 % more columns for the tensor pipe, and the digits of a vector with one
-// large element resolved 2^-29 of it everywhere; now 2^-27 of it in its own cell and 2^-27 of the cell's largest in the others.)
+// large element resolved 2^-29 of it everywhere; now 2^-27 of it in its own block and 2^-27 of the block's largest in the others.)
 #define PFD_T 512
 #define PFD_CL 8                    // CTAs of a token at most for a cluster
 template <bool CL, bool LN>              // statistics by a cluster; LayerNorm instead of RMSNorm
@@ -137,11 +137,7 @@ __global__ void __launch_bounds__(PFD_T, 3) k_pf_digits(const float* __restrict_
     // digits cannot spell infinities or NaN: the scale does, so that the token's outputs show them
     if (tid == 0 && blockIdx.y == 0) scale[t] = (vmax < INFINITY && probe == probe) ? Sg * (2.0f / HX_TC_DIGIT_UNIT) : __int_as_float(0x7FC00000);
     if (k0 >= ((K + 255) & ~255)) return;
-    // the warp's 256 columns are a cell
-    float cm = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) cm = fmaxf(cm, fabsf(v[e]));
-    const int r = dig_cell_exp(Sg, hx_warp_max(cm) * inv * 1.0000005f);
+    const int r = dig_block_exp(Sg, dig_block_max(v) * inv * 1.0000005f);        // the warp's 256 columns are a cell
     uint32_t word[HX_TC_DIGITS];
     dig_words(v, (inv / Sg) * (float)(1 << r) * HX_TC_DIGIT_UNIT, codes, word);
     const int tg = t / group;
@@ -186,12 +182,10 @@ __global__ void __launch_bounds__(PFL_T, 5) k_pf_digits_long(const float* __rest
     const int tg = t / group, tl = t - tg * group;
     #pragma unroll 1
     for (int c = warp; c < kcells; c += PFL_T / 32) {
-        float v[8], cm = 0.0f;
+        float v[8];
         const float4 a = *reinterpret_cast<const float4*>(xs + c * 256 + lane * 8), b = *reinterpret_cast<const float4*>(xs + c * 256 + lane * 8 + 4);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-#pragma unroll
-        for (int e = 0; e < 8; e++) cm = fmaxf(cm, fabsf(v[e]));
-        const int r = dig_cell_exp(Sg, hx_warp_max(cm) * inv * 1.0000005f);
+        const int r = dig_block_exp(Sg, dig_block_max(v) * inv * 1.0000005f);
         uint32_t word[HX_TC_DIGITS];
         dig_words(v, (inv / Sg) * (float)(1 << r) * HX_TC_DIGIT_UNIT, codes, word);
         dig_store(cells + ((size_t)c * groups + tg) * HX_TC_DCELL(group), group, tl, lane, word, r);
