@@ -29,15 +29,30 @@ int  hx_fail(int code, const char* fmt, ...);
         if (!(cond)) return hx_fail(HX_ERR_ARG, "bad argument: %s (%s:%d)", #cond, __FILE__, __LINE__); \
     } while (0)
 
-// A function attribute belongs to the device that is current when it is set, so "done once" is tracked per
-// device: returns true the first time it is called for `seen` on the current device (devices 0..63).
+// A function attribute belongs to the device that is current when it is set, so "done once" is tracked per device (the first 64; on
+// others it is set every time).  A caller that comes while another thread is setting waits for it; what failed is tried again.
 #include <atomic>
-static inline bool hx_first_on_device(std::atomic<unsigned long long>& seen) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) return true;
-    const unsigned long long bit = 1ull << dev;
-    return (seen.fetch_or(bit) & bit) == 0;
+#include <mutex>
+struct HxOncePerDevice {
+    std::atomic<unsigned long long> done{0};
+    std::mutex mu;
+    template <class Set> int operator()(Set&& set) {
+        int dev = 0;
+        HX_CUDA(cudaGetDevice(&dev));
+        const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+        if (done.load(std::memory_order_acquire) & bit) return HX_OK;
+        std::lock_guard<std::mutex> lock(mu);
+        if (done.load(std::memory_order_relaxed) & bit) return HX_OK;
+        const int rc = set();
+        if (!rc) done.fetch_or(bit, std::memory_order_release);
+        return rc;
+    }
+};
+#ifdef __CUDACC__
+template <class Kernel> static int hx_max_smem(HxOncePerDevice& once, Kernel kernel, int bytes) {
+    return once([&]() -> int { HX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)); return HX_OK; });
 }
+#endif
 
 // Count of kernels this library launched (reported by the benchmark as gpu_launches).
 extern unsigned long long g_hx_launches;

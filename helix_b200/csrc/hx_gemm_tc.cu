@@ -159,8 +159,8 @@ int hx_gemm_tc_launch(const HxGemmTC& g, cudaStream_t st) {
     HX_CHECK_ARG(g.ncols >= 8 && g.ncols <= 256 && g.ncols % 8 == 0);
     const size_t smem = hx_gemm_tc_smem(g.ncols, g.stage_ksteps);
     if (smem > 227 * 1024) return hx_fail(HX_ERR_ARG, "tensor-core GEMM stage too large (%zu bytes of shared memory)", smem);
-    static std::atomic<unsigned long long> attr_seen{0};
-    if (hx_first_on_device(attr_seen)) HX_CUDA(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    static HxOncePerDevice once;
+    const int rc = hx_max_smem(once, k_gemm_tc, 227 * 1024); if (rc) return rc;
     k_gemm_tc<<<g.ntiles < 148 ? g.ntiles : 148, TC_THREADS, smem, st>>>(g);
     HX_COUNT_LAUNCH(1);
     HX_CUDA(cudaGetLastError());

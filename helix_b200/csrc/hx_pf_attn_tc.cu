@@ -323,8 +323,8 @@ int hx_pf_attn_tc(const float* qkv, int ld, int n_tok, HxPfWhere wh, int NH, int
     HX_CHECK_ARG(!wh.pos_arr && pieces && NH % NKV == 0 && NH / NKV <= 128);
     const int GRP = NH / NKV, tpt = 128 / GRP, kt = (ctx_len + AT_KT - 1) / AT_KT;
     const size_t smem = 1024 + AT_HDR + (size_t)(6 + AT_RING) * AT_PIECE;
-    static std::atomic<unsigned long long> attr_seen{0};
-    if (hx_first_on_device(attr_seen)) HX_CUDA(cudaFuncSetAttribute(k_pf_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    static HxOncePerDevice once;
+    const int rc = hx_max_smem(once, k_pf_attn_tc, 227 * 1024); if (rc) return rc;
     HX_CUDA(hx_launch_pdl(k_pf_kv_split, dim3(kt, NKV, 4), dim3(256), 0, st, kc, vc, wh, n_tok, cap, pieces));
     HX_CUDA(hx_launch_pdl(k_pf_attn_tc, dim3(NKV, (n_tok + tpt - 1) / tpt), dim3(AT_THREADS), smem, st, qkv, ld, wh, n_tok, GRP, pieces, kt, scale, ctx, ld_ctx, err));
     HX_COUNT_LAUNCH(2);

@@ -13,7 +13,6 @@
 #include "hx_digits.cuh"
 #include "hx_kernels.cuh"
 #include <math.h>
-#include <atomic>
 
 namespace {
 
@@ -771,8 +770,8 @@ int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, con
     // us, x 12288 26.8 -> 19.4, 1008 x 12288 52 -> 36; below that it is the slower one (24 x 12288 6 -> 10, 256 tokens a layer 201 -> 209).
     const size_t values = (size_t)((K + 255) / 256) * 1024;
     if (!b && n_tok >= 148 && (long long)n_tok * grid.y > 3 * 148 && values <= 192 * 1024) {
-        static std::atomic<unsigned long long> seen{0};
-        if (hx_first_on_device(seen)) HX_CUDA(cudaFuncSetAttribute(k_pf_digits_long, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024));
+        static HxOncePerDevice once;
+        const int rc = hx_max_smem(once, k_pf_digits_long, 192 * 1024); if (rc) return rc;
         cfg.gridDim = dim3(n_tok); cfg.blockDim = dim3(PFL_T); cfg.dynamicSmemBytes = values;
         HX_CUDA(cudaLaunchKernelEx(&cfg, k_pf_digits_long, src, ld, K, g, eps, cells, group, groups, scale));
     } else if (cl) {
@@ -829,8 +828,8 @@ size_t hx_pf_attn_scratch(int n_tok, int NH, int NKV, int DH) {
 template <int GRP, int TG>
 static int pf_attn_launch(dim3 grid, size_t smem, cudaStream_t st, const float* qkv, int ld, HxPfWhere wh, int n_tok, int NH, int DH, const float* kc,
                           const float* vc, int cap, float scale, float* ctx, int ld_ctx, float* part, unsigned* tickets, int* err) {
-    static std::atomic<unsigned long long> attr_seen{0};
-    if (hx_first_on_device(attr_seen)) HX_CUDA(cudaFuncSetAttribute(k_pf_attn<GRP, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));      // the kernel has some static shared memory too
+    static HxOncePerDevice once;
+    const int rc = hx_max_smem(once, k_pf_attn<GRP, TG>, 226 * 1024); if (rc) return rc;      // the kernel has some static shared memory too
     HX_CUDA(hx_launch_pdl(k_pf_attn<GRP, TG>, grid, dim3(PF_AT), smem, st, qkv, ld, wh, n_tok, NH, DH, kc, vc, cap, scale, ctx, ld_ctx, part, tickets, err));
     return HX_OK;
 }
