@@ -103,7 +103,6 @@ struct hx_model {
     void* pf_buf = nullptr;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_ctx = nullptr, *pf_gu = nullptr, *pf_scale = nullptr; uint8_t* pf_cells = nullptr; int* pf_err = nullptr; float* pf_acc = nullptr; float* pf_att_part = nullptr; unsigned* pf_att_tickets = nullptr;
     int pf_gu_ld = 0, pf_tb = 0; bool pf_batched = true;
-    bool pf_batch_step = false;                 // the chunk being launched is a step of batched decode
     int pf_chunk = HX_PF_MAX, pf_attn = 0;      // tokens of a prompt chunk at most (HX_PF_CHUNK); HX_PF_ATTN: 1 tc, -1 vec, 0 by the rule
     uint8_t* pf_pieces = nullptr; size_t pf_pieces_bytes = 0; int pf_ctx_hint = 0;      // bf16 terms of K and V of a layer for the tensor-core attention, grown to the longest context seen
     float* pf_part = nullptr; size_t tp_pf_off = 0, tp_pf_area = 0; unsigned tp_pf_ep = 0;      // tensor-parallel chunk exchange
@@ -1389,10 +1388,10 @@ static int pf_alloc(hx_model* m, int want) {
     return HX_OK;
 }
 
-// one linear of a chunk: digits of `src` -> GEMM against f -> out (token-major)
-static int pf_linear(hx_model* m, const Fused& f, const float* src, int ld_src, int n, int swiglu, const float* g,
+// one linear of a chunk: digits of `src` (early: see hx_pf_digits) -> GEMM against f -> out (token-major)
+static int pf_linear(hx_model* m, const Fused& f, const float* src, int ld_src, int n, bool early, int swiglu, const float* g,
                      float* out, int ld_out, int rows, int resid, int pair64, const float* nb = nullptr, const float* bias = nullptr, int gelu = 0) {
-    const int rc = hx_pf_digits(src, ld_src, n, f.K, g, nb, m->cfg.norm_eps, m->pf_cells, m->pf_scale, !m->pf_batch_step || n <= 12, m->st); if (rc) return rc;
+    const int rc = hx_pf_digits(src, ld_src, n, f.K, g, nb, m->cfg.norm_eps, m->pf_cells, m->pf_scale, early, m->st); if (rc) return rc;
     HxGemmDig q = {};
     q.a = f.t128; q.b = m->pf_cells; q.rows = rows; q.ntiles = f.tiles128; q.kcells = f.ksteps / 4; q.ntok = n;
     q.err = m->pf_err; q.col_scale = m->pf_scale; q.out = out; q.ld_out = ld_out; q.resid = resid; q.acc = m->pf_acc;
@@ -1418,7 +1417,7 @@ static int pf_tp_reduce(hx_model* m, int n) {
 // of one sequence ends at position ctx_end (0: batched decode, every token has a sequence of its own).
 static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, int ctx_end) {
     const hx_config& c = m->cfg;
-    m->pf_batch_step = ctx_end == 0;
+    const bool early = ctx_end > 0 || n <= HX_PF_EARLY_SEQ;
     const int DH = c.head_dim, DM = c.d_model, QD = m->QD, KVD = m->KVD, cap = m->kv_cap;
     const int ldq = QD + 2 * KVD;
     const float att_scale = 1.0f / sqrtf((float)DH);
@@ -1441,25 +1440,25 @@ static int pf_enqueue_layers(hx_model* m, int n, const int* ids, HxPfWhere wh, i
         Layer& ly = m->layers[L];
         float* kc = m->kc + (size_t)L * c.n_kv_heads * cap * DH; float* vc = m->vc + (size_t)L * c.n_kv_heads * cap * DH;
         const bool g2 = c.arch == 0;         // GPT-2: LayerNorm, biases, gelu_new, no rotation, no q/k norm
-        if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0, ly.ln1_b, ly.b_qkv))) return rc;
+        if ((rc = pf_linear(m, ly.qkv, m->pf_x, DM, n, early, 0, ly.in_g, m->pf_qkv, ldq, ly.qkv.N, 0, 0, ly.ln1_b, ly.b_qkv))) return rc;
         if ((rc = hx_pf_qkpost(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, ly.qn_g, ly.kn_g, c.norm_eps, g2 ? nullptr : m->cosT, g2 ? nullptr : m->sinT, kc, vc, cap, m->st))) return rc;
         if (tc) {
             if ((rc = hx_pf_attn_tc(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_pieces, ctx_end, m->pf_err, m->st))) return rc;
         } else if ((rc = hx_pf_attn(m->pf_qkv, ldq, n, wh, c.n_heads, c.n_kv_heads, DH, kc, vc, cap, att_scale, m->pf_ctx, QD, m->pf_att_part, m->pf_att_tickets, m->pf_err, m->st))) return rc;
         if (m->tp_world > 1) {
-            if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_part, DM, ly.o.N, 0, 0))) return rc;
+            if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, early, 0, nullptr, m->pf_part, DM, ly.o.N, 0, 0))) return rc;
             if ((rc = pf_tp_reduce(m, n))) return rc;
-        } else if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, 0, nullptr, m->pf_x, DM, ly.o.N, 1, 0, nullptr, ly.b_o))) return rc;
+        } else if ((rc = pf_linear(m, ly.o, m->pf_ctx, QD, n, early, 0, nullptr, m->pf_x, DM, ly.o.N, 1, 0, nullptr, ly.b_o))) return rc;
         if (g2) {
-            if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, 0, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 0, ly.ln2_b, ly.b_fc, 1))) return rc;
-            if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, 0, nullptr, m->pf_x, DM, ly.down.N, 1, 0, nullptr, ly.b_down))) return rc;
+            if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, early, 0, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 0, ly.ln2_b, ly.b_fc, 1))) return rc;
+            if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, early, 0, nullptr, m->pf_x, DM, ly.down.N, 1, 0, nullptr, ly.b_down))) return rc;
             continue;
         }
-        if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, 1, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 1))) return rc;       // SwiGLU in the epilogue
+        if ((rc = pf_linear(m, ly.gu, m->pf_x, DM, n, early, 1, ly.post_g, m->pf_gu, m->pf_gu_ld, c.d_ff, 0, 1))) return rc;       // SwiGLU in the epilogue
         if (m->tp_world > 1) {
-            if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, 0, nullptr, m->pf_part, DM, ly.down.N, 0, 0))) return rc;
+            if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, early, 0, nullptr, m->pf_part, DM, ly.down.N, 0, 0))) return rc;
             if ((rc = pf_tp_reduce(m, n))) return rc;
-        } else if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, 0, nullptr, m->pf_x, DM, ly.down.N, 1, 0))) return rc;
+        } else if ((rc = pf_linear(m, ly.down, m->pf_gu, m->pf_gu_ld, n, early, 0, nullptr, m->pf_x, DM, ly.down.N, 1, 0))) return rc;
     }
     return HX_OK;
 }
@@ -1496,7 +1495,7 @@ static int bd_enqueue_step(hx_model* m, int n_seq) {
         const int n = n_seq - c0 < HX_PF_TB ? n_seq - c0 : HX_PF_TB;
         HxPfWhere wh = {nullptr, m->d_bpos + c0, m->d_bseq + c0, seq_stride, nullptr};
         if ((rc = pf_enqueue_layers(m, n, m->d_bids + c0, wh, 0))) return rc;
-        if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
+        if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, n <= HX_PF_EARLY_SEQ, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
         if (m->tp_world > 1) {
             // every rank holds a slice of the vocabulary: local first maximum, then the best over the ranks
             if (!m->tp_connected) return hx_fail(HX_ERR_STATE, "tensor parallel: call hx_model_tp_connect before the first step");
@@ -1527,7 +1526,7 @@ static int run_prefill_batched(hx_model* m, int T, int seq) {
         nlast = T - t0 < chunk ? T - t0 : chunk;
         if ((rc = pf_enqueue_chunk(m, t0, nlast))) return rc;
     }
-    if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0, m->final_b))) return rc;
+    if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, true, 0, m->final_g, m->logits, 0, m->head.N, 0, 0, m->final_b))) return rc;
     hx_pf_argmax(m->logits, c.vocab, m->d_tok, m->d_hist, m->d_pos, T - 1, m->st);
     HX_CUDA(cudaGetLastError());
     return HX_OK;
@@ -1553,7 +1552,7 @@ static int run_prefill(hx_model* m, const int32_t* ids, int T, int seq = 0) {
         }
         if (slot) {
             // the head on the last position, then the first maximum over the ranks' vocabulary slices
-            if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, 0, m->final_g, m->logits, 0, m->head.N, 0, 0))) return rc;
+            if ((rc = pf_linear(m, m->head, m->pf_x + (size_t)(nlast - 1) * c.d_model, c.d_model, 1, true, 0, m->final_g, m->logits, 0, m->head.N, 0, 0))) return rc;
             const unsigned ep = ++m->tp_pf_ep;
             unsigned long long* areas[8] = {nullptr};
             for (int w = 0; w < m->tp_world; w++)
@@ -1707,7 +1706,7 @@ static int spec_verify(hx_model* m, const int32_t* win, int n, int pos, int32_t*
     HX_CUDA(cudaMemcpyAsync(m->d_pf_pos, ps, 8, cudaMemcpyHostToDevice, m->st));
     HxPfWhere wh = {m->d_pf_pos, nullptr, nullptr, (size_t)c.n_layers * c.n_kv_heads * m->kv_cap * c.head_dim, m->d_pf_pos + 1};
     int rc = pf_enqueue_layers(m, n, m->d_prompt, wh, pos + n); if (rc) return rc;
-    if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
+    if ((rc = pf_linear(m, m->head, m->pf_x, c.d_model, n, true, 0, m->final_g, m->pf_logits, c.vocab, m->head.N, 0, 0))) return rc;
     hx_pf_top2_rows(m->pf_logits, c.vocab, c.vocab, n, m->sp_next, m->sp_margin, m->st);
     HX_CUDA(cudaMemcpyAsync(a, m->sp_next, (size_t)n * 4, cudaMemcpyDeviceToHost, m->st));
     HX_CUDA(cudaMemcpyAsync(margin, m->sp_margin, (size_t)n * 4, cudaMemcpyDeviceToHost, m->st));

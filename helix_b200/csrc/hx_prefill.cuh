@@ -4,6 +4,7 @@
 #include "hx_common.cuh"
 
 #define HX_PF_TB 64                // tokens per chunk of the batched decode (its logits take vocab floats each), of a verify window and inside a tensor-parallel group
+#define HX_PF_EARLY_SEQ 12         // see hx_pf_digits
 #define HX_PF_MAX 1040             // tokens per chunk of a prompt: 40 groups of 26, so that 1024 tokens are one chunk and 2048 two.  A launch's ramp
                                    // and drain (about 6 us) are a twentieth of its work there; the chunk's buffers are 269 MB at the 8B shape
 
@@ -23,7 +24,7 @@ int hx_pf_embed(const int* ids, HxPfWhere wh, const float* emb, const float* wpe
 //   g != null: RMSNorm with gain g and eps first, or with b != null LayerNorm with gain g and bias b;
 //   cells: K rounded up to 256 columns; per 256-column cell and group of hx_gemm_dig_group(n_tok) tokens HX_TC_DCELL bytes: row
 //   16 (t / 2) + 2 d + t % 2 = digit d of the group's token t (eight base-13 digits, most significant first, as E2M1 codes), then the column scales;
-//   early: the launch may overlap the end of the kernel before;
+//   early: the launch may overlap the end of the kernel before (prompts, and batch steps of up to HX_PF_EARLY_SEQ sequences);
 //   scale[t]: x_n = scale[t] * column scale of the block * sum_d digit_d 13^(7-d)  (powers of two).
 int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, const float* b, float eps, uint8_t* cells, float* scale, bool early, cudaStream_t st);
 
