@@ -852,7 +852,10 @@ int persist_check(hx_model* m) {
 
 int finish_init(hx_model* m) {
     int rc = alloc_state(m); if (rc) return rc;
-    if (const char* e = getenv("HX_PF_CHUNK")) { const int v = atoi(e) / HX_TC_MAX_TOK * HX_TC_MAX_TOK; if (v >= HX_TC_MAX_TOK && v < HX_PF_MAX) m->pf_chunk = v; }
+    if (const char* e = getenv("HX_PF_CHUNK")) {      // rounded down to whole token groups, one at least
+        const int v = atoi(e), t = v > HX_TC_MAX_TOK ? v / HX_TC_MAX_TOK * HX_TC_MAX_TOK : HX_TC_MAX_TOK;
+        if (v > 0 && t < HX_PF_MAX) m->pf_chunk = t;
+    }
     if (const char* e = getenv("HX_PF_ATTN")) m->pf_attn = strcmp(e, "tc") == 0 ? 1 : (strcmp(e, "vec") == 0 ? -1 : 0);
     const char* np = getenv("HX_NO_PDL");
     m->pdl = !(np && *np == '1');

@@ -48,3 +48,25 @@ def test_prefill_throughput_reports(tiny_file):
     out, ms_p, ms_d = gm.generate(ids, 16)
     assert ms_p > 0 and ms_d > 0 and len(out) == 16
     gm.close()
+
+
+@pytest.mark.parametrize("asked,same_as", [("1", "26"), ("24", "26"), ("25", "26"), ("51", "26"), ("72", "52"), ("0", None), ("x", None)])
+def test_chunk_size_switch(tiny_file, monkeypatch, asked, same_as):
+    """HX_PF_CHUNK is rounded down to whole token groups of 26, to one group at least, and ignored where it is no positive number: seen in the launches."""
+    ids = np.random.default_rng(4).integers(0, 300, 100).astype(np.int32)
+
+    def launches(value):
+        monkeypatch.delenv("HX_PF_CHUNK", raising=False)
+        if value is not None:
+            monkeypatch.setenv("HX_PF_CHUNK", value)
+        m = hb.Model.load(tiny_file, kv_cap=128)
+        m.prefill(ids)
+        n = hb.launch_count()
+        m.prefill(ids)
+        n = hb.launch_count() - n
+        m.close()
+        return n
+
+    assert launches(asked) == launches(same_as)
+    if same_as:
+        assert launches(asked) > launches(None)
