@@ -766,10 +766,13 @@ int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, con
     cudaLaunchAttribute at[2];
     cfg.attrs = at;
     if (early) { at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
-    // As soon as the CTAs of k_pf_digits do not fit the SMs at once (three per SM) the long form takes over, if it has a CTA for every SM: 512 tokens x 4096 columns 10.4 -> 8.3
-    // us, x 12288 26.8 -> 19.4, 1008 x 12288 52 -> 36; below that it is the slower one (24 x 12288 6 -> 10, 256 tokens a layer 201 -> 209).
+    // The long form takes over where the CTAs of k_pf_digits fill the SMs more than twice (three per SM) and every SM has a token.  Alone, back to back, slices /
+    // long: 4096 columns, 300 tokens 8.3 / 8.3 us, 1008 14.4 / 12.4; 12288, 150 10.4 / 10.3, 256 14.8 / 10.4, 300 17.8 / 13.1, 512 25.3 / 16.5; 25600, 150 18.8 / 18.5,
+    // 512 59.5 / 45.1.  In a prompt it gives about 4 us a launch away: its CTAs hold the values in shared memory and cannot come up beside the GEMM
+    // that is leaving, those of k_pf_digits can.  Twelve layers of the 8B shape, never / from more than one wave / from two: 150 tokens 2287 / 2345 / 2287, 200 2653 / 2711 /
+    // 2652, 256 3058 / 3095 / 3052, 300 3532 / 3529 / 3521, 700 7269 / 7095 / 7113, 1024 10525 / 10322 / 10135.
     const size_t values = (size_t)((K + 255) / 256) * 1024;
-    if (!b && n_tok >= 148 && (long long)n_tok * grid.y > 3 * 148 && values <= 192 * 1024) {
+    if (!b && n_tok >= 148 && (long long)n_tok * grid.y > 2 * 3 * 148 && values <= 192 * 1024) {
         static HxOncePerDevice once;
         const int rc = hx_max_smem(once, k_pf_digits_long, 192 * 1024); if (rc) return rc;
         cfg.gridDim = dim3(n_tok); cfg.blockDim = dim3(PFL_T); cfg.dynamicSmemBytes = values;

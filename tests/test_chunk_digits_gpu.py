@@ -36,8 +36,8 @@ def plain(tmp_path_factory):
     om.close(); gm.close(); one.close()
 
 
-# groups of at most 26 tokens, all of one even size: one token, a pair and its half, full groups, one token more, odd remainders; 225 and
-# 449: the digit kernel of long chunks for the hidden vector (two slices of 4096 columns a token) and for all vectors
+# groups of at most 26 tokens, all of one even size: one token, a pair and its half, full groups, one token more, odd remainders; 449: the
+# digit kernel of long chunks for the hidden vector (two slices of 4096 columns a token)
 @pytest.mark.parametrize("T", [1, 2, 3, 25, 26, 27, 52, 53, 79, 105, 225, 449])
 def test_group_edges(plain, T):
     _check(*plain, np.random.default_rng(T).integers(0, CFG["NV"], T).astype(np.int32))
@@ -70,8 +70,9 @@ def _block_units(x):
     return (np.broadcast_to(s, a.shape) * 2.0 ** -27).reshape(K)[:len(x)]
 
 
-# T: groups up to 16 tokens (their column scales lie closer) and wider ones, several groups, the kernel of long chunks
-@pytest.mark.parametrize("DM,T", [(768, 6), (1024, 16), (1024, 18), (1024, 53), (4096, 7), (4096, 26), (4096, 450), (8192, 226)])
+# T: groups up to 16 tokens (their column scales lie closer) and wider ones, several groups, both sides of the line to the
+# kernel of long chunks
+@pytest.mark.parametrize("DM,T", [(768, 6), (1024, 16), (1024, 18), (1024, 53), (4096, 7), (4096, 26), (4096, 450), (8192, 444), (8192, 446)])
 def test_a_linear_against_64_bits(tmp_path, DM, T):
     """2-norm over the rows of a token.  Rows with weight on the vector's large element: below one unit of an f32, 2^-23, for every vector (an element times
     the norm's factor, the fold of the digits and the sums round; 5e-8 to 1e-7 seen).  Rows without: what the digits of the other elements resolve comes on
