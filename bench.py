@@ -559,8 +559,8 @@ def run_ours(args):
         for b in (dw, dW, dmic, dts):
             b.free()
 
-    # what the tensor pipe can issue for the MMA of this library (no vendor figure exists for it at small N): the
-    # denominator of the batched GEMM's tensor-side roofline
+    # the MMA of this library as one thread per SM issues it (no vendor figure exists for it at small N), and the pipe's own rate
+    # at the clock of that probe: the denominator of the batched GEMM's tensor-side roofline
     tprobe = None
     if rank == 0 and extras:
         c16, _ = hb.probe_mxf4_rate(16, True)
@@ -570,10 +570,11 @@ def run_ours(args):
         useful = PROMPT_LEN / prefill_s * 2.0 * lin_weights / 1e12
         tprobe = {"mma": "tcgen05.mma kind::mxf4nvf4 block16, M128 x N x K64, operands in shared memory, one issuing thread per SM",
                   "clk_per_mma_n16_with_scale_copies": c16, "clk_per_mma_n256": c256, "clk_per_mma_n256_with_scale_copies": c256s,
-                  "attainable_tflops_n256": tf256, "attainable_tflops_n256_with_scale_copies": tf256s,
+                  "probe_tflops_n256": tf256, "probe_tflops_n256_with_scale_copies": tf256s, "pipe_tflops": tf256 * c256 / 128.0,
                   "prefill_useful_tflops": useful, "prefill_issued_tflops": useful * 8.0,
-                  "prefill_issued_frac_of_attainable": useful * 8.0 / (tf256s * 208.0 / 256.0),
-                  "note": "the prefill issues eight digit columns per activation (base 13), up to 208 columns per MMA, so its issued work is 8 x the useful work"}
+                  "prefill_issued_frac_of_pipe": useful * 8.0 / (tf256 * c256 / 128.0),
+                  "note": "the probe's single-thread issue loop sets its pace; the pipe takes N / 2 cycles per MMA, which is pipe_tflops at the probe's clock.  "
+                          "The prefill issues eight digit columns per activation (base 13), up to 208 columns per MMA, so its issued work is 8 x the useful work"}
 
     # GPT-2-124M shape, all linears NVFP4, 32-token prompt + 128 greedy tokens, batch 1
     gpt2 = None

@@ -6,7 +6,7 @@
 //
 // A unit of work is a 128-row tile of W times a group of G <= 26 tokens: 8 G digit columns, tcgen05.mma kind::mxf4nvf4 with
 // M = 128, N = 8 G, K = 64, N / 2 cycles each at large N (the pipe's rate, which neither the scale copies nor loads, TMEM reads and
-// polling warps beside it lower).  What bounds a large chunk (512 tokens, 8B shape): the pipe is busy for 70 % of a launch.  A unit of sixteen
+// polling warps beside it lower).  What bounds a large chunk (512 tokens, 8B shape): the pipe is busy for 46 (o) to 66 % (gate+up) of a launch.  A unit of sixteen
 // MMAs takes 1664 cycles of it and 2270 in all, because a 18 KB weight cell is some 1900 cycles on its way round -- freed, asked for,
 // brought from L2 (385 cycles of the SM's port each), used -- and the ring holds five; then ramp, drain and the passage
 // between blocks of K.  What bounds a small one (a group or two): the weights from HBM and the fixed part of a launch.
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
             if (lane < C && lane != q) cl_arrive_relaxed(bar);
         };
         // This CTA's own part of a unit's sums is taken first, so that the read-out can go on; the other parts are added to it in K
-        // order.  Instructions are what a unit can run out of (its MMAs take 1800 cycles): tokens go in pairs, addresses are constants
+        // order.  Instructions are what a unit can run out of (its MMAs take 1664 cycles): tokens go in pairs, addresses are constants
         // or steps of a pointer, a thread reads NP pairs whether it has as many or not, and the common case loads and stores without
         // predicates.  (Token by token, with a comparison per token and part: 4000 cycles a unit.)
         const f32x2 c13p7 = x2(DG_13P7, DG_13P7);

@@ -759,8 +759,9 @@ int hx_pf_digits(const float* src, int ld, int n_tok, int K, const float* g, con
     const dim3 grid(n_tok, (K + PFD_T * 8 - 1) / (PFD_T * 8));
     const bool cl = grid.y > 1 && grid.y <= PFD_CL && !b;
     // `early`: launched while the kernel before drains.  A prompt gains (12 layers of the 8B shape: 77 tokens 1690 -> 1640 us, 128
-    // 2083 -> 1990, 512 5.35 -> 5.0 .. 5.5 ms) and a few sequences (5: 862 -> 852); from 16 sequences on the waiting CTAs are in the way
-    // (16: 913 -> 935, 48: 1490 -> 1536, 64: 1857 -> 1911).
+    // 2083 -> 1990, 512 5.35 -> 5.0 .. 5.5 ms).  A batch step gains where its kernels are launched one by one (hx_decode_batch: 5 sequences 924 -> 855,
+    // 12 903 -> 855, 16 926 -> 885) and loses where it is replayed from a graph (hx_decode_batch_loop: 5 724 -> 747, 12 727 -> 746, 16 757 -> 776,
+    // 48 1490 -> 1536, 64 1857 -> 1911): the line at HX_PF_EARLY_SEQ is a compromise between the two.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(PFD_T); cfg.stream = st;
     cudaLaunchAttribute at[2];

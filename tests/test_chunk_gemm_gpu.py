@@ -1,5 +1,5 @@
 """The chunk GEMM's kinds (pairs of CTAs, clusters over K, K in several blocks, an odd number of row tiles) at token
-counts around its groups of 24, through a prompt's logits and cached rows against the CPU restatement.  (The prompt attention
+counts around its groups of up to 26, through a prompt's logits and cached rows against the CPU restatement.  (The prompt attention
 has tests/test_prompt_attention_gpu.py.)"""
 import numpy as np
 import pytest
@@ -20,7 +20,7 @@ def model(tmp_path_factory):
     return path
 
 
-@pytest.mark.parametrize("T", [1, 24, 25, 130])
+@pytest.mark.parametrize("T", [1, 24, 25, 26, 27, 52, 53, 130])
 def test_prompt_logits_and_cache_rows(model, T):
     om, gm = ol.OracleModel(model, kv_cap=T + 8), hb.Model.load(model, kv_cap=T + 8)
     ids = np.random.default_rng(T).integers(0, CFG["NV"], T).astype(np.int32)
@@ -37,8 +37,8 @@ def test_prompt_logits_and_cache_rows(model, T):
 
 
 def test_repeated_prompts_are_bit_equal(model):
-    """Many units per CTA through the two receive buffers of the cluster: what a buffer held for one unit is read before the next
-    unit's sums arrive, so a prompt gives the same bits every time."""
+    """Many units per CTA through the staging and the receive buffer of the cluster's CTAs: what a buffer held for one unit is read before the
+    next unit's sums arrive, so a prompt gives the same bits every time."""
     gm = hb.Model.load(model, kv_cap=320)
     ids = np.random.default_rng(7).integers(0, CFG["NV"], 301).astype(np.int32)
     _, want = gm.prefill(ids, want_logits=True)

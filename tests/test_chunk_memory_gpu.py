@@ -9,7 +9,7 @@ import oracle_lib as ol
 
 pytestmark = pytest.mark.gpu
 HX_ERR_NOMEM = 6
-# wide hidden layer: 41 MB of chunk buffers at 72 tokens, 82 at 144, 143 at 252, 574 at 1008
+# wide hidden layer: 43 MB of chunk buffers at 78 tokens, 71 at 130, 142 at 260, 567 at 1040
 CFG = dict(NL=1, DM=512, NH=4, NKV=4, DH=128, DFF=32768, NV=300)
 
 

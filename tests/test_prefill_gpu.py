@@ -1,4 +1,4 @@
-"""Batched prefill (one chunk here: up to 1008 tokens in groups of 24 through the tcgen05 GEMM) against the fp32 CPU
+"""Batched prefill (one chunk here: up to 1040 tokens in groups of up to 26 through the tcgen05 GEMM) against the fp32 CPU
 restatement and against the token-by-token path of the same library."""
 import os
 

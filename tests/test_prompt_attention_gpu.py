@@ -1,5 +1,5 @@
 """Prompt attention, both kernels (HX_PF_ATTN forces one): the tensor-core kernel with every way a group of heads fills its 128-row tiles,
-token counts around row and key tiles, and chunks that begin inside a key tile (HX_PF_CHUNK); prompts of several chunks.  The K and V
+token counts around row and key tiles, and chunks that begin inside a key tile (HX_PF_CHUNK, in whole groups of 26: 52 and 104); prompts of several chunks.  The K and V
 rows of the second layer depend on every token's attention in the first; the logits are checked against the CPU restatement."""
 import numpy as np
 import pytest
@@ -59,7 +59,7 @@ def test_vector_kernel_in_chunks(tmp_path, monkeypatch):
 
 
 def test_prompt_longer_than_a_chunk(tmp_path, monkeypatch):
-    """1100 tokens: two chunks of 552 and 548 by the rule that also picks the kernel."""
+    """1100 tokens: two chunks of 572 and 528 by the rule that also picks the kernel."""
     path = _model(tmp_path, 4, 1, DM=128)
     om = ol.OracleModel(path, kv_cap=1104)
     ids = np.random.default_rng(6).integers(0, 300, 1100).astype(np.int32)
