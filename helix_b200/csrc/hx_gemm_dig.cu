@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
             if (!warp_wait(&S.accum[buf], (uint32_t)(ou >> 1) & 1u, ab_flag)) return false;
             tc_fence_after();
             const uint32_t col = tcol + (uint32_t)buf * ncols;
+            f32x2 v[DG_EP];
 #pragma unroll
             for (int h = 0; h < DG_EP; h += 3) {
                 if (h > 0 && h >= np) break;
@@ -316,16 +317,18 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_gemm_dig(const __grid_constan
                     tc_fence_before();
                     if (lane == 0) mb_arrive(&S.acc_free[buf]);
                 }
-                if (h == 0 && ou >= 1 && !warp_wait(&S.st_free, (uint32_t)(ou - 1) & 1u, ab_flag)) return false;
 #pragma unroll
                 for (int t = 0; t < 3; t++) {
                     if (h + t >= DG_EP) break;
-                    f32x2 v = x2(r[t][14], r[t][15]);
+                    v[h + t] = x2(r[t][14], r[t][15]);
 #pragma unroll
-                    for (int d = 6; d >= 0; d--) v = x2_fma(v, c13, x2(r[t][2 * d], r[t][2 * d + 1]));
-                    if (h + t < np) *reinterpret_cast<f32x2*>(to + (p0 + h + t) * 1024) = v;
+                    for (int d = 6; d >= 0; d--) v[h + t] = x2_fma(v[h + t], c13, x2(r[t][2 * d], r[t][2 * d + 1]));
                 }
             }
+            // The staging is free a trip to the other CTAs and back after the unit before was sent: the accumulator is not held up by that.
+            if (ou >= 1 && !warp_wait(&S.st_free, (uint32_t)(ou - 1) & 1u, ab_flag)) return false;
+#pragma unroll
+            for (int t = 0; t < DG_EP; t++) if (t < np) *reinterpret_cast<f32x2*>(to + (p0 + t) * 1024) = v[t];
             if (C > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mb_arrive(&S.st_full);
